@@ -423,6 +423,20 @@ static rs::StepScalars step_scalars(const rs_ctx *c, const rs_step_args *a, cons
   return P;
 }
 
+// the final reduction of nb partials (a dependent launch)
+static int reduce_partials(rs_ctx *c, int nb, double mass_offset, double *mass_out, int32_t *itip_out,
+                           cudaStream_t st, const char *what) {
+  rs::FinalRed fr = {};
+  fr.partials = c->partials;
+  fr.nparts = nb;
+  fr.mass_offset = mass_offset;
+  fr.mass_out = mass_out;
+  fr.itip_out = itip_out;
+  if (rs::launch_reduce_partials_dep(fr, st))
+    return fail(RS_E_CUDA, "%s: launch: %s", what, cudaGetErrorString(cudaGetLastError()));
+  return cuda_check(what);
+}
+
 int rs_step(rs_ctx *c, const rs_fields *cur, const rs_fields *next, const rs_step_args *a, rs_stream_t stream) {
   if (!c || !a) return fail(RS_E_INVALID, "rs_step: null argument");
   int rc = check_fields(c, cur, "rs_step cur");
@@ -478,8 +492,7 @@ int rs_step(rs_ctx *c, const rs_fields *cur, const rs_fields *next, const rs_ste
   // (the tile kernels reduce their partials themselves)
   if (red && !tmp) {
     const double off = cur->precision == RS_F32 ? (double)(c->p.nx_all - 2) * (c->p.ny_all - 2) * c->p.cinf : 0.0;
-    rs::launch_reduce_partials(c->partials, nb, off, a->mass_out, a->itip_out, st);
-    if ((rc = cuda_check("rs_step reduce"))) return rc;
+    if ((rc = reduce_partials(c, nb, off, a->mass_out, a->itip_out, st, "rs_step reduce"))) return rc;
   }
   return RS_OK;
 }
@@ -563,11 +576,11 @@ int rs_itip(rs_ctx *c, const rs_fields *f, int32_t *d_itip, rs_stream_t stream) 
   int rc = check_fields(c, f, "rs_itip");
   if (rc) return rc;
   int nb = 0;
-  if (rs::launch_grid_partials(f->precision, c->K, f->c, f->psi, c->p.cinf, c->partials, c->max_partials, &nb,
-                               (cudaStream_t)stream))
-    return fail(RS_E_INVALID, "rs_itip: workspace too small");
-  rs::launch_reduce_partials(c->partials, nb, 0.0, nullptr, d_itip, (cudaStream_t)stream);
-  return cuda_check("rs_itip");
+  const int lr = rs::launch_itip_partials(f->precision, c->K, f->psi, c->partials, c->max_partials, &nb,
+                                          (cudaStream_t)stream);
+  if (lr == -1) return fail(RS_E_INVALID, "rs_itip: workspace too small");
+  if (lr) return fail(RS_E_CUDA, "rs_itip: launch: %s", cudaGetErrorString(cudaGetLastError()));
+  return reduce_partials(c, nb, 0.0, nullptr, d_itip, (cudaStream_t)stream, "rs_itip");
 }
 
 int rs_mass(rs_ctx *c, const rs_fields *f, double *d_mass, rs_stream_t stream) {
@@ -575,11 +588,11 @@ int rs_mass(rs_ctx *c, const rs_fields *f, double *d_mass, rs_stream_t stream) {
   int rc = check_fields(c, f, "rs_mass");
   if (rc) return rc;
   int nb = 0;
-  if (rs::launch_grid_partials(f->precision, c->K, f->c, f->psi, c->p.cinf, c->partials, c->max_partials, &nb,
-                               (cudaStream_t)stream))
-    return fail(RS_E_INVALID, "rs_mass: workspace too small");
-  rs::launch_reduce_partials(c->partials, nb, 0.0, d_mass, nullptr, (cudaStream_t)stream);
-  return cuda_check("rs_mass");
+  const int lr = rs::launch_mass_partials(f->precision, c->K, f->c, c->p.cinf, c->partials, c->max_partials, &nb,
+                                          (cudaStream_t)stream);
+  if (lr == -1) return fail(RS_E_INVALID, "rs_mass: workspace too small");
+  if (lr) return fail(RS_E_CUDA, "rs_mass: launch: %s", cudaGetErrorString(cudaGetLastError()));
+  return reduce_partials(c, nb, 0.0, d_mass, nullptr, (cudaStream_t)stream, "rs_mass");
 }
 
 int rs_precise_tip(rs_ctx *c, const rs_fields *f, rs_tip *d_tip, rs_stream_t stream) {
@@ -587,7 +600,9 @@ int rs_precise_tip(rs_ctx *c, const rs_fields *f, rs_tip *d_tip, rs_stream_t str
   if (c->p.band) return fail(RS_E_UNSUPPORTED, "rs_precise_tip: needs the whole domain, not a band");
   int rc = check_fields(c, f, "rs_precise_tip", false);
   if (rc) return rc;
-  rs::launch_precise_tip(f->precision, c->K, f->psi, c->row_last, c->row_f, c->row_g, d_tip, (cudaStream_t)stream);
+  if (rs::launch_precise_tip(f->precision, c->K, f->psi, c->row_last, c->row_f, c->row_g, d_tip,
+                             (cudaStream_t)stream))
+    return fail(RS_E_CUDA, "rs_precise_tip: launch: %s", cudaGetErrorString(cudaGetLastError()));
   return cuda_check("rs_precise_tip");
 }
 

@@ -1,14 +1,14 @@
 // rs_frame.cu — moving frame, grid reductions and the device tip tracker.
 //
 //  * pull_back (fun.cu:1469-1492): standalone column shift of every cell.
-//  * grid partials: per-block FP64 sum of interior c and max tip column;
-//    replaces the full-grid D2H copy + host scan of set_pull_back
+//  * grid partials: per-block FP64 sum of interior c, and per-block max tip
+//    column; they replace the full-grid D2H copy + host scan of set_pull_back
 //    (fun.cu:693-699, get_itip_all_grain fun.cu:1745-1754).
 //  * precise tip (get_precise_tip, fun.cu:2895-2954): one warp per row finds
-//    the last psi > 0 column with a warp max-reduction; one thread replays the
-//    reference's sequential row scan (get_tip_int, fun.cu:2880-2893) over the
-//    per-row results and performs the quartic and parabola least-squares fits
-//    (fun.cu:2648-2865) in FP64.  This file is compiled with -fmad=false so that
+//    the last psi > 0 column; one block replays the reference's sequential row
+//    scan (get_tip_int, fun.cu:2880-2893) over the per-row results and
+//    performs the quartic and parabola least-squares fits (fun.cu:2648-2865)
+//    in FP64.  This file is compiled with -fmad=false so that
 //    the fits round like the reference's host code.
 #include <cstdio>
 #include <cstring>
@@ -51,109 +51,156 @@ void launch_pull_back(int precision, const StepCoef &K, const void *c, const voi
 }
 
 // ---------------------------------------------------------------- reductions
-template <typename R>
-__global__ void __launch_bounds__(256) grid_partials_kernel(const StepCoef K, const R *__restrict__ c,
-                                                            const R *__restrict__ psi, double c_offset,
-                                                            BlockPartial *out) {
-  // one block per 8 rows; every cell (ghosts included) for the tip column,
-  // interior cells for the mass
-  const int j0 = blockIdx.x * 8;
-  double m = 0.0;
-  int it = 0;
-  for (int jj = threadIdx.y; jj < 8; jj += blockDim.y) {
-    const int j = j0 + jj;
-    if (j >= K.ny) break;
-    const bool interior_row = j >= 1 && j <= K.ny - 2;
-    for (int i = threadIdx.x; i < K.nx; i += blockDim.x) {
-      const int64_t o = (int64_t)j * K.pitch + i;
-      if (psi[o] > R(0)) it = max(it, i);
-      if (interior_row && i >= 1 && i <= K.nx - 2) m += (double)c[o] + c_offset;
-    }
-  }
-  block_partial<256>(m, it, out);
-}
+// rs_itip, rs_mass and rs_precise_tip are two launches each: a pass over the
+// one field the figure needs, and a small kernel that is a programmatic
+// dependent of it.  The passes are programmatic dependents too: every kernel
+// here waits (griddepcontrol.wait) before it touches memory, so its launch
+// overlaps the kernel before it.  At 2048 x 2048 in FP64 (front at column 300)
+// itip takes 15, the precise tip 21 and the mass 9 us, 296 together before: the
+// tip's row scan was one thread's, and itip and mass read both fields.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-int launch_grid_partials(int precision, const StepCoef &K, const void *c, const void *psi,
-                         double c_offset, BlockPartial *partials, int max_partials,
-                         int *nblocks_out, cudaStream_t st) {
-  const int nb = (K.ny + 7) / 8;
-  if (nb > max_partials) return -1;
-  dim3 b(64, 4);
-  if (precision == RS_F64)
-    grid_partials_kernel<double><<<nb, b, 0, st>>>(K, (const double *)c, (const double *)psi, 0.0, partials);
-  else
-    grid_partials_kernel<float><<<nb, b, 0, st>>>(K, (const float *)c, (const float *)psi, c_offset, partials);
-  *nblocks_out = nb;
-  return 0;
-}
-
-__global__ void __launch_bounds__(256) reduce_partials_kernel(const BlockPartial *__restrict__ p, int n,
-                                                              double mass_offset, double *mass_out,
-                                                              int32_t *itip_out) {
-  __shared__ double s_m[256];
-  __shared__ int s_i[256];
-  double m = 0.0;
-  int it = 0;
-  for (int k = threadIdx.x; k < n; k += 256) {
-    m += p[k].mass;
-    it = max(it, p[k].itip);
-  }
-  s_m[threadIdx.x] = m;
-  s_i[threadIdx.x] = it;
-  __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      s_m[threadIdx.x] += s_m[threadIdx.x + s];
-      s_i[threadIdx.x] = max(s_i[threadIdx.x], s_i[threadIdx.x + s]);
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    if (mass_out) *mass_out = s_m[0] + mass_offset;
-    if (itip_out) *itip_out = max(1, s_i[0]);  // get_itip_all_grain starts at 1
-  }
-}
-
-void launch_reduce_partials(const BlockPartial *partials, int n, double mass_offset,
-                            double *mass_out, int32_t *itip_out, cudaStream_t st) {
-  reduce_partials_kernel<<<1, 256, 0, st>>>(partials, n, mass_offset, mass_out, itip_out);
-}
-
-__global__ void __launch_bounds__(128) reduce_partials_dep_kernel(const FinalRed FR) {
-  __shared__ double s_m[256];
-  __shared__ int s_i[256];
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // the step grid has completed, its writes visible
-  final_reduce(FR, s_m, s_i, (int)threadIdx.x, [] { __syncthreads(); });
-}
-
-int launch_reduce_partials_dep(const FinalRed &FR, cudaStream_t st) {
+template <typename T>
+struct Same {  // (the kernel's own parameter types: no deduction from the arguments)
+  using type = T;
+};
+template <typename... Args>
+cudaError_t launch_dep(void (*kernel)(Args...), unsigned blocks, unsigned threads, cudaStream_t st,
+                       typename Same<Args>::type... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(1);
-  cfg.blockDim = dim3(128);
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, reduce_partials_dep_kernel, FR) == cudaSuccess ? 0 : -3;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// The largest column in [0, hi] with psi > 0 of a row, or -1: the whole warp
+// walks from the right end, kScan cells per lane and turn (their loads in
+// flight together), and stops at the first turn that finds one, so it reads
+// the melt ahead of the front only.
+constexpr int kScan = 16;
+// all of v in registers at once: without it the compiler loads and compares a
+// few cells at a time (itip of 2048 x 2048 in FP64: 27 us)
+#define RS_HOLD8(C, v, k)                                                                                  \
+  "+" C(v[k]), "+" C(v[k + 1]), "+" C(v[k + 2]), "+" C(v[k + 3]), "+" C(v[k + 4]), "+" C(v[k + 5]), \
+      "+" C(v[k + 6]), "+" C(v[k + 7])
+__device__ __forceinline__ void hold(double (&v)[kScan]) { asm volatile("" : RS_HOLD8("d", v, 0), RS_HOLD8("d", v, 8)); }
+__device__ __forceinline__ void hold(float (&v)[kScan]) { asm volatile("" : RS_HOLD8("f", v, 0), RS_HOLD8("f", v, 8)); }
+#undef RS_HOLD8
+template <typename R>
+__device__ __forceinline__ int last_solid(const R *__restrict__ row, int hi, int lane) {
+  int last = -1;
+  for (; hi >= 0 && last < 0; hi -= 32 * kScan) {
+    R v[kScan];
+#pragma unroll
+    for (int u = 0; u < kScan; ++u) {
+      const int i = hi - 32 * u - lane;
+      v[u] = i >= 0 ? row[i] : R(0);
+    }
+    hold(v);
+#pragma unroll
+    for (int u = kScan - 1; u >= 0; --u)
+      if (v[u] > R(0)) last = hi - 32 * u - lane;
+    last = __reduce_max_sync(0xffffffffu, last);
+  }
+  return last;
+}
+
+// coarse tip of four rows per block, a warp each (every cell, ghosts included)
+constexpr int kRedRows = 4;
+template <typename R>
+__global__ void __launch_bounds__(32 * kRedRows) itip_partials_kernel(const StepCoef K, const R *__restrict__ psi,
+                                                                      BlockPartial *out) {
+  pdl_wait();
+  pdl_trigger();
+  const int j = blockIdx.x * kRedRows + (threadIdx.x >> 5);
+  int it = 0;
+  if (j < K.ny) it = last_solid(psi + (int64_t)j * K.pitch, K.nx - 1, threadIdx.x & 31);
+  block_partial<32 * kRedRows>(0.0, it, out);
+}
+
+// FP64 sum of c (+ c_offset) over the interior cells of four rows per block,
+// two warps per row, eight loads in flight per lane
+template <typename R>
+__global__ void __launch_bounds__(64 * kRedRows) mass_partials_kernel(const StepCoef K, const R *__restrict__ c,
+                                                                      const double c_offset, BlockPartial *out) {
+  pdl_wait();
+  pdl_trigger();
+  const int j = blockIdx.x * kRedRows + (threadIdx.x >> 6);
+  double m = 0.0;
+  if (j >= 1 && j <= K.ny - 2) {
+    const R *__restrict__ row = c + (int64_t)j * K.pitch;
+    constexpr int kU = 8;
+    int i = 1 + (threadIdx.x & 63);
+    for (; i + 64 * (kU - 1) <= K.nx - 2; i += 64 * kU) {
+      R v[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) v[u] = row[i + 64 * u];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) m += (double)v[u] + c_offset;
+    }
+    for (; i <= K.nx - 2; i += 64) m += (double)row[i] + c_offset;
+  }
+  block_partial<64 * kRedRows>(m, 0, out);
+}
+
+int launch_itip_partials(int precision, const StepCoef &K, const void *psi, BlockPartial *partials, int max_partials,
+                         int *nblocks_out, cudaStream_t st) {
+  const int nb = (K.ny + kRedRows - 1) / kRedRows;
+  if (nb > max_partials) return -1;
+  *nblocks_out = nb;
+  return (precision == RS_F64
+              ? launch_dep(itip_partials_kernel<double>, nb, 32 * kRedRows, st, K, (const double *)psi, partials)
+              : launch_dep(itip_partials_kernel<float>, nb, 32 * kRedRows, st, K, (const float *)psi, partials)) ==
+                 cudaSuccess
+             ? 0
+             : -3;
+}
+
+int launch_mass_partials(int precision, const StepCoef &K, const void *c, double c_offset, BlockPartial *partials,
+                         int max_partials, int *nblocks_out, cudaStream_t st) {
+  const int nb = (K.ny + kRedRows - 1) / kRedRows;
+  if (nb > max_partials) return -1;
+  *nblocks_out = nb;
+  return (precision == RS_F64
+              ? launch_dep(mass_partials_kernel<double>, nb, 64 * kRedRows, st, K, (const double *)c, 0.0, partials)
+              : launch_dep(mass_partials_kernel<float>, nb, 64 * kRedRows, st, K, (const float *)c, c_offset,
+                           partials)) == cudaSuccess
+             ? 0
+             : -3;
+}
+
+__global__ void __launch_bounds__(128) reduce_partials_dep_kernel(const FinalRed FR) {
+  __shared__ double s_m[256];
+  __shared__ int s_i[256];
+  pdl_wait();  // the kernel that wrote the partials has completed, its writes visible
+  final_reduce(FR, s_m, s_i, (int)threadIdx.x, [] { __syncthreads(); });
+}
+
+int launch_reduce_partials_dep(const FinalRed &FR, cudaStream_t st) {
+  return launch_dep(reduce_partials_dep_kernel, 1, 128, st, FR) == cudaSuccess ? 0 : -3;
 }
 
 // ---------------------------------------------------------------- precise tip
 // per row j: last column i in [0, nx-2] with psi > 0 (or -1), and the two
 // values get_tip_int can produce for the row: f_j at i0 = last, g_j at i0 = 0.
 template <typename R>
-__global__ void tip_rows_kernel(const StepCoef K, const R *__restrict__ psi, int *row_last,
-                                double *row_f, double *row_g) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__global__ void __launch_bounds__(128) tip_rows_kernel(const StepCoef K, const R *__restrict__ psi, int *row_last,
+                                                       double *row_f, double *row_g) {
+  pdl_wait();
+  pdl_trigger();
+  const int j = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (warp >= K.ny) return;
-  const int j = warp;
+  if (j >= K.ny) return;
   const R *row = psi + (int64_t)j * K.pitch;
-  int last = -1;
-  for (int i = lane; i <= K.nx - 2; i += 32)
-    if (row[i] > R(0)) last = i;
-  last = __reduce_max_sync(0xffffffffu, last);
+  const double g0 = (double)row[0], g1 = (double)row[1];
+  const int last = last_solid(row, K.nx - 2, lane);
   if (lane == 0) {
     row_last[j] = last;
     if (last >= 0) {
@@ -162,53 +209,74 @@ __global__ void tip_rows_kernel(const StepCoef K, const R *__restrict__ psi, int
     } else {
       row_f[j] = 0.0;
     }
-    const double a = (double)row[0], b = (double)row[1];
-    row_g[j] = (b - a) * (0.0 - a) + 0;
+    row_g[j] = (g1 - g0) * (0.0 - g0) + 0;
   }
 }
 
-// solve_5x5 (fun.cu:2648-2691): Gaussian elimination with partial pivoting
-__device__ void solve_5x5_d(double A[5][5], double b[5], double c[5]) {
-  int p[5];
-  for (int i = 0; i < 5; i++) p[i] = i;
+// solve_5x5 (fun.cu:2648-2691): Gaussian elimination with partial pivoting.
+// The reference permutes row indices; here the rows themselves change places
+// (the same operations on the same numbers in the same order), so that every
+// index is a compile-time one and the system stays in registers.
+__device__ __forceinline__ void solve_5x5_d(double A[5][5], double b[5], double c[5]) {
+#pragma unroll
   for (int k = 0; k < 4; k++) {
-    double max_val = fabs(A[p[k]][k]);
+    double max_val = fabs(A[k][k]);
     int max_idx = k;
+#pragma unroll
     for (int i = k + 1; i < 5; i++)
-      if (fabs(A[p[i]][k]) > max_val) {
-        max_val = fabs(A[p[i]][k]);
+      if (fabs(A[i][k]) > max_val) {
+        max_val = fabs(A[i][k]);
         max_idx = i;
       }
-    const int t = p[k];
-    p[k] = p[max_idx];
-    p[max_idx] = t;
+#pragma unroll
+    for (int i = k + 1; i < 5; i++)
+      if (max_idx == i) {
+#pragma unroll
+        for (int j = 0; j < 5; j++) {
+          const double t = A[k][j];
+          A[k][j] = A[i][j];
+          A[i][j] = t;
+        }
+        const double t = b[k];
+        b[k] = b[i];
+        b[i] = t;
+      }
+#pragma unroll
     for (int i = k + 1; i < 5; i++) {
-      const double factor = A[p[i]][k] / A[p[k]][k];
-      for (int j = k; j < 5; j++) A[p[i]][j] -= factor * A[p[k]][j];
-      b[p[i]] -= factor * b[p[k]];
+      const double factor = A[i][k] / A[k][k];
+#pragma unroll
+      for (int j = k; j < 5; j++) A[i][j] -= factor * A[k][j];
+      b[i] -= factor * b[k];
     }
   }
+#pragma unroll
   for (int i = 4; i >= 0; i--) {
     double sum = 0.0;
-    for (int j = i + 1; j < 5; j++) sum += A[p[i]][j] * c[j];
-    c[i] = (b[p[i]] - sum) / A[p[i]][i];
+#pragma unroll
+    for (int j = i + 1; j < 5; j++) sum += A[i][j] * c[j];
+    c[i] = (b[i] - sum) / A[i][i];
   }
 }
 
 // get_precise_x (fun.cu:2694-2738): quartic x(psi) through 5 points, x at psi = 0
-__device__ double precise_x_d(const double *x, const double *y) {
+__device__ __forceinline__ double precise_x_d(const double (&x)[5], const double (&y)[5]) {
   double A[5][5], b[5], c[5];
+#pragma unroll
   for (int j = 0; j < 5; ++j) {
     b[j] = 0.0;
     c[j] = 0.0;
     for (int k = 0; k < 5; ++k) A[j][k] = 0.0;
   }
+#pragma unroll
   for (int i = 0; i < 5; i++) {
     double yp[9];
     yp[0] = 1.0;
+#pragma unroll
     for (int k = 1; k <= 8; k++) yp[k] = yp[k - 1] * y[i];
+#pragma unroll
     for (int j = 0; j < 5; j++) {
       b[j] += x[i] * yp[j];
+#pragma unroll
       for (int k = 0; k < 5; k++) A[j][k] += yp[j + k];
     }
   }
@@ -273,29 +341,74 @@ __device__ int fit_parabola_d(const double *x, const double *y, double *x0, doub
   return 0;
 }
 
+// get_tip_int (fun.cu:2880-2893) is sequential over the rows: the scan start
+// of row j is the running tip int(itip), so row j offers f_j if its last solid
+// column is not behind that, else g_j, and becomes the tip if it is larger.
+// Here the block reads kFitRows rows at a time and takes the larger of f_j and
+// g_j over each group of 32; one warp then visits the groups that can raise
+// the tip, in order, and in a group the rows that do (ballots), with the
+// comparisons of the sequential scan.  The five quartic fits run on five lanes.
+constexpr int kFitThreads = 512;
+constexpr int kFitRows = 2048;
+constexpr int kFitGroups = kFitRows / 32;
 template <typename R>
-__global__ void tip_fit_kernel(const StepCoef K, const R *__restrict__ psi, const int *__restrict__ row_last,
-                               const double *__restrict__ row_f, const double *__restrict__ row_g,
-                               rs_tip *out) {
-  if (threadIdx.x != 0) return;
-  // get_tip_int (fun.cu:2880-2893): sequential over rows, the scan start of
-  // row j is the running tip int(itip)
+__global__ void __launch_bounds__(kFitThreads) tip_fit_kernel(const StepCoef K, const R *__restrict__ psi,
+                                                              const int *__restrict__ row_last,
+                                                              const double *__restrict__ row_f,
+                                                              const double *__restrict__ row_g, rs_tip *out) {
+  __shared__ int s_last[kFitRows];
+  __shared__ double s_f[kFitRows], s_g[kFitRows], s_max[kFitGroups];
+  static_assert(kFitGroups == 64, "two group maxima per lane");
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ny = K.ny;
   double itip = 0.0;
   int ti = 0, tj = 0;
-  for (int j = 0; j < K.ny; ++j) {
-    const int s = (int)itip;
-    const int last = row_last[j];
-    const double v = (last >= 0 && last >= s) ? row_f[j] : row_g[j];
-    if (v > itip) {
-      itip = v;
-      ti = (int)itip;
-      tj = j;
+  for (int base = 0; base < ny; base += kFitRows) {
+    if (base) __syncthreads();  // the warp has left the previous rows
+#pragma unroll
+    for (int q = 0; q < kFitRows / kFitThreads; ++q) {
+      const int r = threadIdx.x + q * kFitThreads, j = base + r;
+      const int last = j < ny ? __ldcg(row_last + j) : -1;
+      const double f = j < ny ? __ldcg(row_f + j) : 0.0, g = j < ny ? __ldcg(row_g + j) : 0.0;
+      s_last[r] = last;
+      s_f[r] = f;
+      s_g[r] = g;
+      double m = fmax(f, g);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if (lane == 0) s_max[r >> 5] = m;
+    }
+    __syncthreads();
+    if (warp != 0) continue;
+    const double m0 = s_max[lane], m1 = s_max[32 + lane];
+    for (int g = 0; g < kFitGroups; ++g) {  // the next group that can raise the tip
+      const unsigned long long can = ((unsigned long long)__ballot_sync(0xffffffffu, m1 > itip) << 32) |
+                                     __ballot_sync(0xffffffffu, m0 > itip);
+      const unsigned long long left = can >> g;
+      if (!left) break;
+      g += __ffsll((long long)left) - 1;
+      const int r = 32 * g + lane, last = s_last[r];
+      const double f = s_f[r], gv = s_g[r];
+      unsigned rest = 0xffffffffu;  // rows after the last one that raised it
+      for (;;) {
+        const int s = (int)itip;
+        const double v = (last >= 0 && last >= s) ? f : gv;
+        const unsigned hit = __ballot_sync(0xffffffffu, v > itip) & rest;
+        if (!hit) break;
+        const int l = __ffs(hit) - 1;
+        itip = __shfl_sync(0xffffffffu, v, l);
+        ti = (int)itip;
+        tj = base + 32 * g + l;
+        rest = l == 31 ? 0u : (0xffffffffu << (l + 1));
+        if (!rest) break;
+      }
     }
   }
-  double xd[5], yd[5];
-  const int ny = K.ny;
-  for (int k = 0; k < 5; ++k) {
-    int j = tj - 2 + k;
+  if (warp != 0) return;
+  double xk = 0.0, yk = 0.0;
+  if (lane < 5) {
+    int j = tj - 2 + lane;
     // deal_with_boundary (fun.cu:2624-2641) with (jmin, jmax)
     const int nmin = min(K.jmin, K.jmax), nmax = max(K.jmin, K.jmax);
     if (K.jmin > K.jmax) {  // periodic
@@ -307,17 +420,25 @@ __global__ void tip_fit_kernel(const StepCoef K, const R *__restrict__ psi, cons
     }
     j = min(max(j, 0), ny - 1);
     const int s = max(ti - 5, 0);
-    const int last = row_last[j];
+    const int last = __ldcg(row_last + j);
     const int i0 = (last >= 0 && last >= s) ? last : 0;
     double id[5], pd[5];
+#pragma unroll
     for (int m = 0; m < 5; ++m) {
       const int i = i0 - 2 + m;
       id[m] = i;
       pd[m] = (double)psi[(int64_t)j * K.pitch + min(max(i, 0), K.nx - 1)];
     }
-    xd[k] = precise_x_d(id, pd);
-    yd[k] = j;
+    xk = precise_x_d(id, pd);
+    yk = j;
   }
+  double xd[5], yd[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    xd[k] = __shfl_sync(0xffffffffu, xk, k);
+    yd[k] = __shfl_sync(0xffffffffu, yk, k);
+  }
+  if (lane != 0) return;
   double x0 = 0.0, y0 = 0.0, Rr = 0.0;
   const int status = fit_parabola_d(xd, yd, &x0, &y0, &Rr);
   rs_tip t;
@@ -334,17 +455,19 @@ __global__ void tip_fit_kernel(const StepCoef K, const R *__restrict__ psi, cons
   *out = t;
 }
 
-void launch_precise_tip(int precision, const StepCoef &K, const void *psi, int *row_last,
-                        double *row_f, double *row_g, rs_tip *out, cudaStream_t st) {
-  const int threads = 256, rows_per_block = threads / 32;
-  const int nb = (K.ny + rows_per_block - 1) / rows_per_block;
-  if (precision == RS_F64) {
-    tip_rows_kernel<double><<<nb, threads, 0, st>>>(K, (const double *)psi, row_last, row_f, row_g);
-    tip_fit_kernel<double><<<1, 32, 0, st>>>(K, (const double *)psi, row_last, row_f, row_g, out);
-  } else {
-    tip_rows_kernel<float><<<nb, threads, 0, st>>>(K, (const float *)psi, row_last, row_f, row_g);
-    tip_fit_kernel<float><<<1, 32, 0, st>>>(K, (const float *)psi, row_last, row_f, row_g, out);
-  }
+template <typename R>
+static int launch_precise_tip_t(const StepCoef &K, const R *psi, int *row_last, double *row_f, double *row_g,
+                                rs_tip *out, cudaStream_t st) {
+  if (launch_dep(tip_rows_kernel<R>, (K.ny + 3) / 4, 128, st, K, psi, row_last, row_f, row_g) != cudaSuccess ||
+      launch_dep(tip_fit_kernel<R>, 1, kFitThreads, st, K, psi, row_last, row_f, row_g, out) != cudaSuccess)
+    return -3;
+  return 0;
+}
+
+int launch_precise_tip(int precision, const StepCoef &K, const void *psi, int *row_last, double *row_f, double *row_g,
+                       rs_tip *out, cudaStream_t st) {
+  return precision == RS_F64 ? launch_precise_tip_t(K, (const double *)psi, row_last, row_f, row_g, out, st)
+                             : launch_precise_tip_t(K, (const float *)psi, row_last, row_f, row_g, out, st);
 }
 
 }  // namespace rs
@@ -439,9 +562,9 @@ extern "C" int rs_precise_tip_noalloc(const rs_params *p, const rs_fields *f, rs
   K.dx = p->dx;
   K.W0 = p->W0;
   K.S = p->S;
-  rs::launch_precise_tip(f->precision, K, f->psi, sc->last, sc->f, sc->g, d_tip, (cudaStream_t)stream);
+  const int lr = rs::launch_precise_tip(f->precision, K, f->psi, sc->last, sc->f, sc->g, d_tip, (cudaStream_t)stream);
   const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
+  if (lr || e != cudaSuccess) {
     char msg[256];
     snprintf(msg, sizeof(msg), "rs_precise_tip_noalloc: %s", cudaGetErrorString(e));
     return rs::set_error(RS_E_CUDA, msg);

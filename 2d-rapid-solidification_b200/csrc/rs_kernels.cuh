@@ -59,7 +59,7 @@ struct FinalRed {
   int32_t *itip_out;
 };
 // The fused final reduction, run by the 128 threads of the CTA that finished
-// last: the partials are summed in reduce_partials_kernel's order (slot v =
+// last: the partials are summed in a fixed order (slot v =
 // 0..255 adds partials v, v + 256, ... in turn, then a tree over the slots).
 // Each thread takes slots tid and tid + 128 and issues eight 16-byte loads
 // per slot before adding any of them, so the pass costs a few L2 round trips
@@ -167,22 +167,21 @@ int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScal
 // The final reduction of FR (counter unused) as a programmatic dependent of
 // the kernel just launched on st, which wrote the partials: it is scheduled
 // while that kernel runs and waits for its completion on the device
-// (griddepcontrol.wait), so no host-side launch gap follows the step.  The
-// step kernel must execute griddepcontrol.launch_dependents.  Same order of
-// summation as launch_reduce_partials.
+// (griddepcontrol.wait), so no host-side launch gap follows the step.  (A
+// kernel that does not execute griddepcontrol.launch_dependents lets it start
+// when it ends.)
 int launch_reduce_partials_dep(const FinalRed &FR, cudaStream_t st);
-void launch_reduce_partials(const BlockPartial *partials, int n, double mass_offset,
-                            double *mass_out, int32_t *itip_out, cudaStream_t st);
 
 // frame / reductions / tip (rs_frame.cu); precision 0 = double, 1 = float
 void launch_pull_back(int precision, const StepCoef &K, const void *c, const void *psi,
                       const void *phi, void *c_n, void *psi_n, void *phi_n, int i_offset,
                       cudaStream_t st);
-int launch_grid_partials(int precision, const StepCoef &K, const void *c, const void *psi,
-                         double c_offset, BlockPartial *partials, int max_partials,
+int launch_itip_partials(int precision, const StepCoef &K, const void *psi, BlockPartial *partials, int max_partials,
                          int *nblocks_out, cudaStream_t st);
-void launch_precise_tip(int precision, const StepCoef &K, const void *psi, int *row_last,
-                        double *row_f, double *row_g, rs_tip *out, cudaStream_t st);
+int launch_mass_partials(int precision, const StepCoef &K, const void *c, double c_offset, BlockPartial *partials,
+                         int max_partials, int *nblocks_out, cudaStream_t st);
+int launch_precise_tip(int precision, const StepCoef &K, const void *psi, int *row_last, double *row_f, double *row_g,
+                       rs_tip *out, cudaStream_t st);
 
 // initial conditions and coarse temperature (rs_init.cu)
 void launch_initial_reference(int precision, const StepCoef &K, int i_tip_target, void *c,
