@@ -727,7 +727,8 @@ int rs_mlp_grad(const rs_mlp_box *box, const float *d_w, int64_t n, const float 
 int rs_mlp_adam(float *d_w, const float *d_grad, float *d_m, float *d_v, int64_t t, float lr, float scale,
                 rs_stream_t stream) {
   if (!d_w || !d_grad || !d_m || !d_v || t < 1) return fail(RS_E_INVALID, "rs_mlp_adam: bad argument");
-  rs::launch_mlp_adam(d_w, d_grad, d_m, d_v, t, lr, scale, (cudaStream_t)stream);
+  if (rs::launch_mlp_adam(d_w, d_grad, d_m, d_v, t, lr, scale, (cudaStream_t)stream))
+    return fail(RS_E_CUDA, "rs_mlp_adam: launch: %s", cudaGetErrorString(cudaGetLastError()));
   return cuda_check("rs_mlp_adam");
 }
 

@@ -21,8 +21,7 @@ namespace cg = cooperative_groups;
 namespace rs {
 namespace {
 
-constexpr int kGradThreads = 128;
-constexpr int kGradCtas = 8;  // CTAs of the one gradient cluster (portable size)
+constexpr int kGradThreads = 256;
 
 // g: the interpolation weight, gg(phi) for the 2D model, 2 gS - 1 for the 3D one
 __device__ __forceinline__ double mu2_exact(double T, double c, double g, double cinf, double RR) {
@@ -62,138 +61,225 @@ __global__ void sample_kernel(const double cinf, const double RR, const MlpBox b
   y[2 * k + 1] = (float)dG_exact(T, c, RR);
 }
 
-// The gradient of one call is computed by ONE cluster of kGradCtas CTAs, so
-// that its sums have a fixed order and two trainings with the same seed give
-// the same weights: CTA r takes the sample chunks r, r + kGradCtas, ... of
-// kGradThreads samples; per chunk, one thread per sample runs forward, loss
-// and backward into shared memory, and each thread then adds the chunk's
-// contribution to the weight gradients it owns (parameters t, t + 128, ...)
-// in sample order.  At the end CTA 0 adds the CTAs' partial gradients and
-// losses, read from their shared memory (distributed shared memory), in rank
-// order, to grad and loss.
-constexpr int kParamsPerThread = (kMlpNParams + kGradThreads - 1) / kGradThreads;
+// The gradient of one call is computed by ONE cluster of CTAs (16, the opt-in
+// size; 8 where the device cannot place 16), so that its sums have a fixed
+// order and two trainings with the same seed give the same weights, with no
+// scratch beyond shared memory.  CTA r takes the chunks r, r + C, ... of `per`
+// samples (up to kGradThreads; fewer where n is small, so that every CTA has
+// some).
+//   samples: one thread per sample, forward, loss and backward; weights by
+//     16-byte broadcasts from shared memory, the sigmoid of a unit evaluated
+//     once for SiLU and its derivative; activations and deltas leave as
+//     16-byte stores into rows of kRow floats (8 lanes x 16 bytes at a stride
+//     of 36 words touch every bank once);
+//   weights: W2's 32 x 32 gradient as 4 x 4 register tiles (two 16-byte loads
+//     for 16 FMA per sample), the chunk's samples in four slices; the other
+//     226 parameters one per thread.
+// At the end the slices and then the CTAs' partial gradients (distributed
+// shared memory, every CTA a share of the parameters) are added in order.
+// At batch 4096 one thread per parameter and 32-way conflicting rows on 8 CTAs
+// took 205 us; this takes 25.  Shared-memory bandwidth bounds it (the 16-byte
+// weight broadcasts return 512 B each: 13 us), then the chain of its phases.
+constexpr int kRow = 36;
+constexpr int kSlices = 4;
+struct GradSmem {
+  float w[kMlpNParams + 2];
+  float part[kMlpNParams + 2];  // this CTA's gradient
+  alignas(16) float h1[kGradThreads][kRow];
+  alignas(16) float h2[kGradThreads][kRow];
+  alignas(16) float d1[kGradThreads][kRow];
+  alignas(16) float d2[kGradThreads][kRow];
+  float x[kGradThreads][4];  // inputs and 1
+  float d3[kGradThreads][2];
+  double wloss[kGradThreads / 32];
+  double loss;
+};
+static_assert(sizeof(GradSmem) <= 227 * 1024, "one CTA per SM");
+static_assert(kSlices * kMlpH * kMlpH <= kGradThreads * kRow, "the slices' W2 gradients fit the activations' room");
+static_assert(kOffW2 % 4 == 0 && kOffW3 % 4 == 0, "16-byte weight rows");
 
-__global__ void __cluster_dims__(kGradCtas, 1, 1) __launch_bounds__(kGradThreads)
-    grad_kernel(const MlpBox box, const float *__restrict__ w, const int64_t n, const float *__restrict__ x,
-                const float *__restrict__ y, float *__restrict__ grad, double *__restrict__ loss) {
-  extern __shared__ float sh[];
-  float *sx = sh;                                   // [kGradThreads][3]
-  float *h1 = sx + kGradThreads * 3;                // [kGradThreads][H]
-  float *h2 = h1 + kGradThreads * kMlpH;            // [kGradThreads][H]
-  float *d1 = h2 + kGradThreads * kMlpH;            // [kGradThreads][H]
-  float *d2 = d1 + kGradThreads * kMlpH;            // [kGradThreads][H]
-  float *d3 = d2 + kGradThreads * kMlpH;            // [kGradThreads][2]
-  float *part = d3 + kGradThreads * 2;              // [kMlpNParams] this CTA's gradient
-  __shared__ double sloss[kGradThreads / 32];
-  __shared__ double cta_loss;
+__device__ __forceinline__ float4 ld4s(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ void st4s(float *p, const float (&v)[4]) {
+  *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+
+__global__ void __launch_bounds__(kGradThreads, 1)
+    grad_kernel(const MlpBox box, const float *__restrict__ w, const int64_t n, const int per,
+                const float *__restrict__ x, const float *__restrict__ y, float *__restrict__ grad,
+                double *__restrict__ loss) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  GradSmem &sm = *reinterpret_cast<GradSmem *>(smem_raw);
   cg::cluster_group cluster = cg::this_cluster();
-  const unsigned rank = cluster.block_rank();
-  const MlpView W(w);
-  const int t = threadIdx.x;
-  float acc[kParamsPerThread];
-#pragma unroll
-  for (int i = 0; i < kParamsPerThread; ++i) acc[i] = 0.f;
-  double lsum = 0.0;  // thread 0: this CTA's loss
-  for (int64_t base = (int64_t)rank * kGradThreads; base < n; base += (int64_t)kGradCtas * kGradThreads) {
+  const unsigned rank = cluster.block_rank(), C = cluster.num_blocks();
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  for (int p = t; p < kMlpNParams; p += kGradThreads) sm.w[p] = w[p];
+  __syncthreads();
+  const MlpView W(sm.w);
+  const float *W2 = sm.w + kOffW2, *W3 = sm.w + kOffW3;
+  // this thread's W2 tile (rows 4 ti.., columns 4 tj..) and slice of a chunk
+  const int ti = ((warp & 1) * 32 + lane) >> 3, tj = lane & 7, slice = warp >> 1;
+  float acc[4][4] = {};
+  float one = 0.f;  // its other parameter
+  double l = 0.0;
+  for (int64_t base = (int64_t)rank * per; base < n; base += (int64_t)C * per) {
     const int64_t k = base + t;
-    const bool live = k < n;
-    float xi[3] = {0.f, 0.f, 0.f};
-    if (live)
-      for (int q = 0; q < 3; ++q) xi[q] = x[3 * k + q];
-    float z1[kMlpH], a1[kMlpH], z2[kMlpH], a2[kMlpH], o[2];
-    mlp_forward_full(W, xi, z1, a1, z2, a2, o);
-    float e[2] = {0.f, 0.f};
-    double l = 0.0;
-    if (live) {
-      for (int q = 0; q < 2; ++q) {
-        e[q] = o[q] - (float)((y[2 * k + q] - box.y_mean[q]) / box.y_scale[q]);
-        l += (double)e[q] * e[q];
+    if (t < per) {
+      const bool live = k < n;
+      float xi[3] = {0.f, 0.f, 0.f};
+      if (live)
+        for (int q = 0; q < 3; ++q) xi[q] = x[3 * k + q];
+      float a1[kMlpH], s1[kMlpH];  // activations and SiLU derivatives of layer 1
+#pragma unroll
+      for (int h = 0; h < kMlpH; ++h) {
+        const float z = W.b1(h) + W.w1(h, 0) * xi[0] + W.w1(h, 1) * xi[1] + W.w1(h, 2) * xi[2];
+        const float s = sigm(z);
+        a1[h] = z * s;
+        s1[h] = s * (1.f + z * (1.f - s));
       }
-    }
-    // backward: dL/do = 2 e (dead samples carry 0 deltas)
-    float g3[2] = {2.f * e[0], 2.f * e[1]};
-    float g2[kMlpH], g1[kMlpH];
 #pragma unroll
-    for (int i = 0; i < kMlpH; ++i) {
-      const float s = g3[0] * W.w3(0, i) + g3[1] * W.w3(1, i);
-      g2[i] = s * silu_grad(z2[i]);
-    }
+      for (int h = 0; h < kMlpH; h += 4) {
+        const float v[4] = {a1[h], a1[h + 1], a1[h + 2], a1[h + 3]};
+        st4s(&sm.h1[t][h], v);
+      }
+      float o[2] = {W.b3(0), W.b3(1)};
+#pragma unroll 1
+      for (int i = 0; i < kMlpH; i += 4) {
+        float a2[4], s2[4];
 #pragma unroll
-    for (int j = 0; j < kMlpH; ++j) {
-      float s = 0.f;
+        for (int u = 0; u < 4; ++u) {
+          float z = W.b2(i + u);
 #pragma unroll
-      for (int i = 0; i < kMlpH; ++i) s += g2[i] * W.w2(i, j);
-      g1[j] = s * silu_grad(z1[j]);
+          for (int j = 0; j < kMlpH; j += 4) {
+            const float4 r = ld4s(W2 + (i + u) * kMlpH + j);
+            z += r.x * a1[j];
+            z += r.y * a1[j + 1];
+            z += r.z * a1[j + 2];
+            z += r.w * a1[j + 3];
+          }
+          const float s = sigm(z);
+          a2[u] = z * s;
+          s2[u] = s * (1.f + z * (1.f - s));
+        }
+        st4s(&sm.h2[t][i], a2);
+        st4s(&sm.d2[t][i], s2);  // the derivative, until the delta replaces it
+        const float4 r0 = ld4s(W3 + i), r1 = ld4s(W3 + kMlpH + i);
+        const float w0[4] = {r0.x, r0.y, r0.z, r0.w}, w1[4] = {r1.x, r1.y, r1.z, r1.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {  // in the order of mlp_forward: the same outputs
+          o[0] += w0[u] * a2[u];
+          o[1] += w1[u] * a2[u];
+        }
+      }
+      float e[2] = {0.f, 0.f};
+      if (live) {
+        for (int q = 0; q < 2; ++q) {
+          e[q] = o[q] - (float)((y[2 * k + q] - box.y_mean[q]) / box.y_scale[q]);
+          l += (double)e[q] * e[q];
+        }
+      }
+      // backward: dL/do = 2 e (dead samples carry 0 deltas)
+      const float g3[2] = {2.f * e[0], 2.f * e[1]};
+      float g1[kMlpH];
+#pragma unroll
+      for (int j = 0; j < kMlpH; ++j) g1[j] = 0.f;
+#pragma unroll 1
+      for (int i = 0; i < kMlpH; i += 4) {
+        const float4 r0 = ld4s(W3 + i), r1 = ld4s(W3 + kMlpH + i), s2 = ld4s(&sm.d2[t][i]);
+        const float g2[4] = {(g3[0] * r0.x + g3[1] * r1.x) * s2.x, (g3[0] * r0.y + g3[1] * r1.y) * s2.y,
+                             (g3[0] * r0.z + g3[1] * r1.z) * s2.z, (g3[0] * r0.w + g3[1] * r1.w) * s2.w};
+        st4s(&sm.d2[t][i], g2);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int j = 0; j < kMlpH; j += 4) {
+            const float4 r = ld4s(W2 + (i + u) * kMlpH + j);
+            g1[j] += g2[u] * r.x;
+            g1[j + 1] += g2[u] * r.y;
+            g1[j + 2] += g2[u] * r.z;
+            g1[j + 3] += g2[u] * r.w;
+          }
+      }
+#pragma unroll
+      for (int h = 0; h < kMlpH; h += 4) {
+        const float v[4] = {g1[h] * s1[h], g1[h + 1] * s1[h + 1], g1[h + 2] * s1[h + 2], g1[h + 3] * s1[h + 3]};
+        st4s(&sm.d1[t][h], v);
+      }
+      const float xv[4] = {xi[0], xi[1], xi[2], 1.f};
+      st4s(sm.x[t], xv);
+      sm.d3[t][0] = g3[0];
+      sm.d3[t][1] = g3[1];
     }
-    for (int q = 0; q < 3; ++q) sx[t * 3 + q] = xi[q];
-    for (int i = 0; i < kMlpH; ++i) {
-      h1[t * kMlpH + i] = a1[i];
-      h2[t * kMlpH + i] = a2[i];
-      d1[t * kMlpH + i] = g1[i];
-      d2[t * kMlpH + i] = g2[i];
-    }
-    d3[t * 2 + 0] = g3[0];
-    d3[t * 2 + 1] = g3[1];
-    for (int off = 16; off > 0; off >>= 1) l += __shfl_down_sync(0xffffffffu, l, off);
-    if ((t & 31) == 0) sloss[t >> 5] = l;
     __syncthreads();
-    if (t == 0)
-      for (int q = 0; q < kGradThreads / 32; ++q) lsum += sloss[q];
-    // this chunk's weight gradients, summed over its samples in order
+    // this chunk's weight gradients
+    const int m0 = slice * (per / kSlices), m1 = m0 + per / kSlices;
+#pragma unroll 4
+    for (int m = m0; m < m1; ++m) {
+      const float4 d = ld4s(&sm.d2[m][4 * ti]), h = ld4s(&sm.h1[m][4 * tj]);
+      const float dv[4] = {d.x, d.y, d.z, d.w}, hv[4] = {h.x, h.y, h.z, h.w};
 #pragma unroll
-    for (int i = 0; i < kParamsPerThread; ++i) {
-      const int p = t + i * kGradThreads;
-      if (p >= kMlpNParams) break;
-      float s = 0.f;
-      if (p < kOffB1) {  // W1[h][q]
-        const int h = p / 3, q = p % 3;
-        for (int m = 0; m < kGradThreads; ++m) s += d1[m * kMlpH + h] * sx[m * 3 + q];
-      } else if (p < kOffW2) {
-        const int h = p - kOffB1;
-        for (int m = 0; m < kGradThreads; ++m) s += d1[m * kMlpH + h];
-      } else if (p < kOffB2) {  // W2[i][j]
-        const int i2 = (p - kOffW2) / kMlpH, j = (p - kOffW2) % kMlpH;
-        for (int m = 0; m < kGradThreads; ++m) s += d2[m * kMlpH + i2] * h1[m * kMlpH + j];
-      } else if (p < kOffW3) {
-        const int i2 = p - kOffB2;
-        for (int m = 0; m < kGradThreads; ++m) s += d2[m * kMlpH + i2];
-      } else if (p < kOffB3) {  // W3[q][i]
-        const int q = (p - kOffW3) / kMlpH, i2 = (p - kOffW3) % kMlpH;
-        for (int m = 0; m < kGradThreads; ++m) s += d3[m * 2 + q] * h2[m * kMlpH + i2];
-      } else {
-        const int q = p - kOffB3;
-        for (int m = 0; m < kGradThreads; ++m) s += d3[m * 2 + q];
-      }
-      acc[i] += s;
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) acc[u][v] += dv[u] * hv[v];
+    }
+    if (warp < 4) {  // W1 (column `warp`), b1
+#pragma unroll 8
+      for (int m = 0; m < per; ++m) one += sm.d1[m][lane] * sm.x[m][warp];
+    } else if (warp == 4) {  // b2
+#pragma unroll 8
+      for (int m = 0; m < per; ++m) one += sm.d2[m][lane];
+    } else if (warp < 7) {  // W3
+#pragma unroll 8
+      for (int m = 0; m < per; ++m) one += sm.d3[m][warp - 5] * sm.h2[m][lane];
+    } else if (lane < 2) {  // b3
+#pragma unroll 8
+      for (int m = 0; m < per; ++m) one += sm.d3[m][lane];
     }
     __syncthreads();  // the chunk's arrays are read before the next chunk writes them
   }
+  float *sw = &sm.h1[0][0];  // the slices' W2 gradients
 #pragma unroll
-  for (int i = 0; i < kParamsPerThread; ++i) {
-    const int p = t + i * kGradThreads;
-    if (p < kMlpNParams) part[p] = acc[i];
+  for (int u = 0; u < 4; ++u) st4s(sw + slice * (kMlpH * kMlpH) + (4 * ti + u) * kMlpH + 4 * tj, acc[u]);
+  if (warp < 3) sm.part[kOffW1 + 3 * lane + warp] = one;
+  else if (warp == 3) sm.part[kOffB1 + lane] = one;
+  else if (warp == 4) sm.part[kOffB2 + lane] = one;
+  else if (warp < 7) sm.part[kOffW3 + (warp - 5) * kMlpH + lane] = one;
+  else if (lane < 2) sm.part[kOffB3 + lane] = one;
+  for (int off = 16; off > 0; off >>= 1) l += __shfl_down_sync(0xffffffffu, l, off);
+  if (lane == 0) sm.wloss[warp] = l;
+  __syncthreads();
+  for (int p = t; p < kMlpH * kMlpH; p += kGradThreads) {
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < kSlices; ++q) s += sw[q * (kMlpH * kMlpH) + p];
+    sm.part[kOffW2 + p] = s;
   }
-  if (t == 0) cta_loss = lsum;
+  if (t == 0) {
+    double s = 0.0;
+    for (int q = 0; q < kGradThreads / 32; ++q) s += sm.wloss[q];
+    sm.loss = s;
+  }
   cluster.sync();  // every CTA's partial is in its shared memory
-  if (rank == 0) {
-    for (int p = t; p < kMlpNParams; p += kGradThreads) {
-      float s = 0.f;
-      for (unsigned r = 0; r < kGradCtas; ++r) s += cluster.map_shared_rank(part, r)[p];
-      grad[p] += s;
-    }
-    if (t == 0) {
-      double l = 0.0;
-      for (unsigned r = 0; r < kGradCtas; ++r) l += *cluster.map_shared_rank(&cta_loss, r);
-      *loss += l;
-    }
+  const int share = (kMlpNParams + (int)C - 1) / (int)C;
+  for (int p = (int)rank * share + t; p < min(kMlpNParams, ((int)rank + 1) * share); p += kGradThreads) {
+    float s = 0.f;
+    for (unsigned r = 0; r < C; ++r) s += cluster.map_shared_rank(sm.part, r)[p];
+    grad[p] += s;
   }
-  cluster.sync();  // CTA 0 has read the others' shared memory before they exit
+  if (rank == 0 && t == 0) {
+    double s = 0.0;
+    for (unsigned r = 0; r < C; ++r) s += *cluster.map_shared_rank(&sm.loss, r);
+    *loss += s;
+  }
+  cluster.sync();  // the others have read this CTA's shared memory before it exits
 }
 
 // Adam (Kingma & Ba 2015) on the gradient scaled by `scale` (1 / batch size)
 __global__ void adam_kernel(float *__restrict__ w, const float *__restrict__ grad, float *__restrict__ m,
                             float *__restrict__ v, const int64_t t, const float lr, const float scale) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (p >= kMlpNParams) return;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   const float g = grad[p] * scale;
@@ -227,20 +313,70 @@ int launch_mlp_sample(double cinf, double RR, const MlpBox &box, int64_t n, uint
   return 0;
 }
 
+// CTAs of the gradient's cluster on the current device: 16 where it can place
+// such a cluster, else 8 (the portable size); 0 on a CUDA error
+static int grad_cluster() {
+  static std::atomic<int> of[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  int c = dev < 64 ? of[dev].load(std::memory_order_acquire) : 0;
+  if (c) return c;
+  if (cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradSmem)) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+    return 0;
+  c = 8;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(16);
+  cfg.blockDim = dim3(kGradThreads);
+  cfg.dynamicSmemBytes = sizeof(GradSmem);
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim = {16, 1, 1};
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int placed = 0;
+  if (cudaOccupancyMaxActiveClusters(&placed, grad_kernel, &cfg) == cudaSuccess && placed > 0) c = 16;
+  cudaGetLastError();
+  if (dev < 64) of[dev].store(c, std::memory_order_release);
+  return c;
+}
+
 int launch_mlp_grad(const MlpBox &box, const float *w, int64_t n, const float *x, const float *y, float *grad,
                     double *loss, cudaStream_t st) {
   if (n <= 0) return 0;
-  const size_t smem = sizeof(float) * (kGradThreads * (3 + 4 * kMlpH + 2) + kMlpNParams);
-  static std::atomic<unsigned long long> attr{0};
-  if (!smem_limit_once((const void *)grad_kernel, (int)smem, attr)) return -3;
-  grad_kernel<<<kGradCtas, kGradThreads, smem, st>>>(box, w, n, x, y, grad, loss);  // one cluster
-  return 0;
+  const int C = grad_cluster();
+  if (!C) return -3;
+  // samples per chunk: every CTA one chunk where n allows, in whole warps
+  const int64_t even = ((n + C - 1) / C + 31) / 32 * 32;
+  const int per = even < kGradThreads ? (int)even : kGradThreads;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(C);  // one cluster
+  cfg.blockDim = dim3(kGradThreads);
+  cfg.dynamicSmemBytes = sizeof(GradSmem);
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim = {(unsigned)C, 1, 1};
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, grad_kernel, box, w, n, per, x, y, grad, loss) == cudaSuccess ? 0 : -3;
 }
 
 int launch_mlp_adam(float *w, const float *grad, float *m, float *v, int64_t t, float lr, float scale,
                     cudaStream_t st) {
-  adam_kernel<<<(kMlpNParams + 255) / 256, 256, 0, st>>>(w, grad, m, v, t, lr, scale);
-  return 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((kMlpNParams + 255) / 256);
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, adam_kernel, w, grad, m, v, t, lr, scale) == cudaSuccess ? 0 : -3;
 }
 
 int launch_mlp_forward(const MlpBox &box, const float *w, int64_t n, const float *x, float *out, cudaStream_t st) {
