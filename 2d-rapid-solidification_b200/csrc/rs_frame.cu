@@ -58,28 +58,6 @@ void launch_pull_back(int precision, const StepCoef &K, const void *c, const voi
 // overlaps the kernel before it.  At 2048 x 2048 in FP64 (front at column 300)
 // itip takes 15, the precise tip 21 and the mass 9 us, 296 together before: the
 // tip's row scan was one thread's, and itip and mass read both fields.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-template <typename T>
-struct Same {  // (the kernel's own parameter types: no deduction from the arguments)
-  using type = T;
-};
-template <typename... Args>
-cudaError_t launch_dep(void (*kernel)(Args...), unsigned blocks, unsigned threads, cudaStream_t st,
-                       typename Same<Args>::type... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(threads);
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 // The largest column in [0, hi] with psi > 0 of a row, or -1: the whole warp
 // walks from the right end, kScan cells per lane and turn (their loads in
 // flight together), and stops at the first turn that finds one, so it reads
@@ -156,8 +134,8 @@ int launch_itip_partials(int precision, const StepCoef &K, const void *psi, Bloc
   if (nb > max_partials) return -1;
   *nblocks_out = nb;
   return (precision == RS_F64
-              ? launch_dep(itip_partials_kernel<double>, nb, 32 * kRedRows, st, K, (const double *)psi, partials)
-              : launch_dep(itip_partials_kernel<float>, nb, 32 * kRedRows, st, K, (const float *)psi, partials)) ==
+              ? launch_dep(itip_partials_kernel<double>, dim3(nb), dim3(32 * kRedRows), st, K, (const double *)psi, partials)
+              : launch_dep(itip_partials_kernel<float>, dim3(nb), dim3(32 * kRedRows), st, K, (const float *)psi, partials)) ==
                  cudaSuccess
              ? 0
              : -3;
@@ -169,8 +147,8 @@ int launch_mass_partials(int precision, const StepCoef &K, const void *c, double
   if (nb > max_partials) return -1;
   *nblocks_out = nb;
   return (precision == RS_F64
-              ? launch_dep(mass_partials_kernel<double>, nb, 64 * kRedRows, st, K, (const double *)c, 0.0, partials)
-              : launch_dep(mass_partials_kernel<float>, nb, 64 * kRedRows, st, K, (const float *)c, c_offset,
+              ? launch_dep(mass_partials_kernel<double>, dim3(nb), dim3(64 * kRedRows), st, K, (const double *)c, 0.0, partials)
+              : launch_dep(mass_partials_kernel<float>, dim3(nb), dim3(64 * kRedRows), st, K, (const float *)c, c_offset,
                            partials)) == cudaSuccess
              ? 0
              : -3;
@@ -184,7 +162,7 @@ __global__ void __launch_bounds__(128) reduce_partials_dep_kernel(const FinalRed
 }
 
 int launch_reduce_partials_dep(const FinalRed &FR, cudaStream_t st) {
-  return launch_dep(reduce_partials_dep_kernel, 1, 128, st, FR) == cudaSuccess ? 0 : -3;
+  return launch_dep(reduce_partials_dep_kernel, dim3(1), dim3(128), st, FR) == cudaSuccess ? 0 : -3;
 }
 
 // ---------------------------------------------------------------- precise tip
@@ -458,8 +436,8 @@ __global__ void __launch_bounds__(kFitThreads) tip_fit_kernel(const StepCoef K, 
 template <typename R>
 static int launch_precise_tip_t(const StepCoef &K, const R *psi, int *row_last, double *row_f, double *row_g,
                                 rs_tip *out, cudaStream_t st) {
-  if (launch_dep(tip_rows_kernel<R>, (K.ny + 3) / 4, 128, st, K, psi, row_last, row_f, row_g) != cudaSuccess ||
-      launch_dep(tip_fit_kernel<R>, 1, kFitThreads, st, K, psi, row_last, row_f, row_g, out) != cudaSuccess)
+  if (launch_dep(tip_rows_kernel<R>, dim3((K.ny + 3) / 4), dim3(128), st, K, psi, row_last, row_f, row_g) != cudaSuccess ||
+      launch_dep(tip_fit_kernel<R>, dim3(1), dim3(kFitThreads), st, K, psi, row_last, row_f, row_g, out) != cudaSuccess)
     return -3;
   return 0;
 }

@@ -7,6 +7,31 @@
 
 namespace rs {
 
+// Programmatic dependent launch: the kernel is scheduled while the one before
+// it in the stream drains, and must execute pdl_wait() before it touches
+// memory (its launch latency hides; the order of the stream stays).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// the next kernel of the stream may be scheduled (if it is such a launch)
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename T>
+struct Same {  // (the kernel's own parameter types: no deduction from the arguments)
+  using type = T;
+};
+template <typename... Args>
+cudaError_t launch_dep(void (*kernel)(Args...), dim3 grid, dim3 block, cudaStream_t st,
+                       typename Same<Args>::type... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Per-block partial results of a grid pass: sum of interior c (FP64) and the
 // largest column with psi > 0 (the coarse tip, get_itip_all_grain fun.cu:1745).
 struct BlockPartial {

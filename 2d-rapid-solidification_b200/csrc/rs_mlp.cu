@@ -64,27 +64,28 @@ __global__ void sample_kernel(const double cinf, const double RR, const MlpBox b
 // The gradient of one call is computed by ONE cluster of CTAs (16, the opt-in
 // size; 8 where the device cannot place 16), so that its sums have a fixed
 // order and two trainings with the same seed give the same weights, with no
-// scratch beyond shared memory.  CTA r takes the chunks r, r + C, ... of `per`
-// samples (up to kGradThreads; fewer where n is small, so that every CTA has
-// some).
+// scratch beyond shared memory.  The order, which does not depend on the
+// cluster's size: each chunk of kChunk samples is summed sample by sample;
+// kChains chains add the sums of the chunks r, r + kChains, ...; the chains are
+// added in order.  A round takes two chunks per CTA:
 //   samples: one thread per sample, forward, loss and backward; weights by
 //     16-byte broadcasts from shared memory, the sigmoid of a unit evaluated
 //     once for SiLU and its derivative; activations and deltas leave as
 //     16-byte stores into rows of kRow floats (8 lanes x 16 bytes at a stride
 //     of 36 words touch every bank once);
-//   weights: W2's 32 x 32 gradient as 4 x 4 register tiles (two 16-byte loads
-//     for 16 FMA per sample), the chunk's samples in four slices; the other
-//     226 parameters one per thread.
-// At the end the slices and then the CTAs' partial gradients (distributed
-// shared memory, every CTA a share of the parameters) are added in order.
+//   weights: four warps per chunk, W2's 32 x 32 gradient as 4 x 2 register
+//     tiles, then the other 226 parameters one per thread and pass;
+//   sums: the owner of a parameter (each CTA a share of them) adds the round's
+//     chunk sums to its chains, read over distributed shared memory.
 // At batch 4096 one thread per parameter and 32-way conflicting rows on 8 CTAs
-// took 205 us; this takes 25.  Shared-memory bandwidth bounds it (the 16-byte
+// took 205 us; this takes 27.  Shared-memory bandwidth bounds it (the 16-byte
 // weight broadcasts return 512 B each: 13 us), then the chain of its phases.
+constexpr int kChunk = 128;
+constexpr int kChains = 8;
 constexpr int kRow = 36;
-constexpr int kSlices = 4;
 struct GradSmem {
   float w[kMlpNParams + 2];
-  float part[kMlpNParams + 2];  // this CTA's gradient
+  float part[2][kMlpNParams + 2];  // gradients of this CTA's two chunks
   alignas(16) float h1[kGradThreads][kRow];
   alignas(16) float h2[kGradThreads][kRow];
   alignas(16) float d1[kGradThreads][kRow];
@@ -95,7 +96,7 @@ struct GradSmem {
   double loss;
 };
 static_assert(sizeof(GradSmem) <= 227 * 1024, "one CTA per SM");
-static_assert(kSlices * kMlpH * kMlpH <= kGradThreads * kRow, "the slices' W2 gradients fit the activations' room");
+static_assert(kGradThreads == 2 * kChunk, "two chunks per CTA, a thread per sample");
 static_assert(kOffW2 % 4 == 0 && kOffW3 % 4 == 0, "16-byte weight rows");
 
 __device__ __forceinline__ float4 ld4s(const float *p) { return *reinterpret_cast<const float4 *>(p); }
@@ -104,7 +105,7 @@ __device__ __forceinline__ void st4s(float *p, const float (&v)[4]) {
 }
 
 __global__ void __launch_bounds__(kGradThreads, 1)
-    grad_kernel(const MlpBox box, const float *__restrict__ w, const int64_t n, const int per,
+    grad_kernel(const MlpBox box, const float *__restrict__ w, const int64_t n,
                 const float *__restrict__ x, const float *__restrict__ y, float *__restrict__ grad,
                 double *__restrict__ loss) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -118,14 +119,21 @@ __global__ void __launch_bounds__(kGradThreads, 1)
   __syncthreads();
   const MlpView W(sm.w);
   const float *W2 = sm.w + kOffW2, *W3 = sm.w + kOffW3;
-  // this thread's W2 tile (rows 4 ti.., columns 4 tj..) and slice of a chunk
-  const int ti = ((warp & 1) * 32 + lane) >> 3, tj = lane & 7, slice = warp >> 1;
-  float acc[4][4] = {};
-  float one = 0.f;  // its other parameter
+  // this thread's chunk of a round, and its W2 tile (rows 4 ti.., columns 2 tj..) of it
+  const int half = warp >> 2, id = t & (kChunk - 1), ti = id >> 4, tj = id & 15;
+  float chain[kChains];  // the chains of the parameter this thread owns
+#pragma unroll
+  for (int r = 0; r < kChains; ++r) chain[r] = 0.f;
+  const int share = (kMlpNParams + (int)C - 1) / (int)C, own = (int)rank * share + t;
+  const bool owner = t < share && own < kMlpNParams;
   double l = 0.0;
-  for (int64_t base = (int64_t)rank * per; base < n; base += (int64_t)C * per) {
-    const int64_t k = base + t;
-    if (t < per) {
+  const int64_t round = (int64_t)2 * C * kChunk;
+  for (int64_t first = 0; first < n; first += round) {
+    // chunk `rank` + C half of the round
+    const int64_t base = first + (int64_t)(rank + C * half) * kChunk;
+    const bool some = base < n;
+    const int64_t k = base + id;
+    if (some) {
       const bool live = k < n;
       float xi[3] = {0.f, 0.f, 0.f};
       if (live)
@@ -212,67 +220,80 @@ __global__ void __launch_bounds__(kGradThreads, 1)
       sm.d3[t][1] = g3[1];
     }
     __syncthreads();
-    // this chunk's weight gradients
-    const int m0 = slice * (per / kSlices), m1 = m0 + per / kSlices;
+    if (some) {  // this chunk's weight gradients
+      const int m0 = half * kChunk, m1 = m0 + kChunk, wq = warp & 3;
+      float *part = sm.part[half];
+      float acc[4][2] = {};
 #pragma unroll 4
-    for (int m = m0; m < m1; ++m) {
-      const float4 d = ld4s(&sm.d2[m][4 * ti]), h = ld4s(&sm.h1[m][4 * tj]);
-      const float dv[4] = {d.x, d.y, d.z, d.w}, hv[4] = {h.x, h.y, h.z, h.w};
+      for (int m = m0; m < m1; ++m) {
+        const float4 d = ld4s(&sm.d2[m][4 * ti]);
+        const float2 h = *reinterpret_cast<const float2 *>(&sm.h1[m][2 * tj]);
+        const float dv[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < 4; ++u) {
+          acc[u][0] += dv[u] * h.x;
+          acc[u][1] += dv[u] * h.y;
+        }
+      }
 #pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] += dv[u] * hv[v];
+      for (int u = 0; u < 4; ++u) {
+        part[kOffW2 + (4 * ti + u) * kMlpH + 2 * tj] = acc[u][0];
+        part[kOffW2 + (4 * ti + u) * kMlpH + 2 * tj + 1] = acc[u][1];
+      }
+      float one = 0.f, two = 0.f;
+      if (wq < 3) {  // W1, column wq
+#pragma unroll 8
+        for (int m = m0; m < m1; ++m) one += sm.d1[m][lane] * sm.x[m][wq];
+        part[kOffW1 + 3 * lane + wq] = one;
+      } else {  // b1
+#pragma unroll 8
+        for (int m = m0; m < m1; ++m) one += sm.d1[m][lane];
+        part[kOffB1 + lane] = one;
+      }
+      if (wq < 2) {  // W3
+#pragma unroll 8
+        for (int m = m0; m < m1; ++m) two += sm.d3[m][wq] * sm.h2[m][lane];
+        part[kOffW3 + wq * kMlpH + lane] = two;
+      } else if (wq == 2) {  // b2
+#pragma unroll 8
+        for (int m = m0; m < m1; ++m) two += sm.d2[m][lane];
+        part[kOffB2 + lane] = two;
+      } else if (lane < 2) {  // b3
+#pragma unroll 8
+        for (int m = m0; m < m1; ++m) two += sm.d3[m][lane];
+        part[kOffB3 + lane] = two;
+      }
     }
-    if (warp < 4) {  // W1 (column `warp`), b1
-#pragma unroll 8
-      for (int m = 0; m < per; ++m) one += sm.d1[m][lane] * sm.x[m][warp];
-    } else if (warp == 4) {  // b2
-#pragma unroll 8
-      for (int m = 0; m < per; ++m) one += sm.d2[m][lane];
-    } else if (warp < 7) {  // W3
-#pragma unroll 8
-      for (int m = 0; m < per; ++m) one += sm.d3[m][warp - 5] * sm.h2[m][lane];
-    } else if (lane < 2) {  // b3
-#pragma unroll 8
-      for (int m = 0; m < per; ++m) one += sm.d3[m][lane];
+    cluster.sync();  // every CTA's chunk sums are in its shared memory
+    if (owner) {
+#pragma unroll
+      for (int r = 0; r < kChains; ++r)
+        for (unsigned c = r; c < 2 * C && first + (int64_t)c * kChunk < n; c += kChains)
+          chain[r] += cluster.map_shared_rank(sm.part[c / C], c % C)[own];
     }
-    __syncthreads();  // the chunk's arrays are read before the next chunk writes them
+    cluster.sync();  // they are read before the next round, or the CTA's end
   }
-  float *sw = &sm.h1[0][0];  // the slices' W2 gradients
+  if (owner) {
+    float s = 0.f;
 #pragma unroll
-  for (int u = 0; u < 4; ++u) st4s(sw + slice * (kMlpH * kMlpH) + (4 * ti + u) * kMlpH + 4 * tj, acc[u]);
-  if (warp < 3) sm.part[kOffW1 + 3 * lane + warp] = one;
-  else if (warp == 3) sm.part[kOffB1 + lane] = one;
-  else if (warp == 4) sm.part[kOffB2 + lane] = one;
-  else if (warp < 7) sm.part[kOffW3 + (warp - 5) * kMlpH + lane] = one;
-  else if (lane < 2) sm.part[kOffB3 + lane] = one;
+    for (int r = 0; r < kChains; ++r) s += chain[r];
+    grad[own] += s;
+  }
   for (int off = 16; off > 0; off >>= 1) l += __shfl_down_sync(0xffffffffu, l, off);
   if (lane == 0) sm.wloss[warp] = l;
   __syncthreads();
-  for (int p = t; p < kMlpH * kMlpH; p += kGradThreads) {
-    float s = 0.f;
-#pragma unroll
-    for (int q = 0; q < kSlices; ++q) s += sw[q * (kMlpH * kMlpH) + p];
-    sm.part[kOffW2 + p] = s;
-  }
   if (t == 0) {
     double s = 0.0;
     for (int q = 0; q < kGradThreads / 32; ++q) s += sm.wloss[q];
     sm.loss = s;
   }
-  cluster.sync();  // every CTA's partial is in its shared memory
-  const int share = (kMlpNParams + (int)C - 1) / (int)C;
-  for (int p = (int)rank * share + t; p < min(kMlpNParams, ((int)rank + 1) * share); p += kGradThreads) {
-    float s = 0.f;
-    for (unsigned r = 0; r < C; ++r) s += cluster.map_shared_rank(sm.part, r)[p];
-    grad[p] += s;
-  }
+  cluster.sync();
   if (rank == 0 && t == 0) {
     double s = 0.0;
     for (unsigned r = 0; r < C; ++r) s += *cluster.map_shared_rank(&sm.loss, r);
     *loss += s;
   }
-  cluster.sync();  // the others have read this CTA's shared memory before it exits
+  cluster.sync();  // the others' shared memory is read before they exit
 }
 
 // Adam (Kingma & Ba 2015) on the gradient scaled by `scale` (1 / batch size)
@@ -347,9 +368,6 @@ int launch_mlp_grad(const MlpBox &box, const float *w, int64_t n, const float *x
   if (n <= 0) return 0;
   const int C = grad_cluster();
   if (!C) return -3;
-  // samples per chunk: every CTA one chunk where n allows, in whole warps
-  const int64_t even = ((n + C - 1) / C + 31) / 32 * 32;
-  const int per = even < kGradThreads ? (int)even : kGradThreads;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C);  // one cluster
   cfg.blockDim = dim3(kGradThreads);
@@ -362,21 +380,15 @@ int launch_mlp_grad(const MlpBox &box, const float *w, int64_t n, const float *x
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, grad_kernel, box, w, n, per, x, y, grad, loss) == cudaSuccess ? 0 : -3;
+  return cudaLaunchKernelEx(&cfg, grad_kernel, box, w, n, x, y, grad, loss) == cudaSuccess ? 0 : -3;
 }
 
 int launch_mlp_adam(float *w, const float *grad, float *m, float *v, int64_t t, float lr, float scale,
                     cudaStream_t st) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((kMlpNParams + 255) / 256);
-  cfg.blockDim = dim3(256);
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, adam_kernel, w, grad, m, v, t, lr, scale) == cudaSuccess ? 0 : -3;
+  return launch_dep(adam_kernel, dim3((kMlpNParams + 255) / 256), dim3(256), st, w, grad, m, v, t, lr, scale) ==
+                 cudaSuccess
+             ? 0
+             : -3;
 }
 
 int launch_mlp_forward(const MlpBox &box, const float *w, int64_t n, const float *x, float *out, cudaStream_t st) {
