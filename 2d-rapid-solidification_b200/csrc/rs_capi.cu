@@ -320,12 +320,11 @@ static void make_coef(const rs_params *p, const rs_derived *d, rs::StepCoef *K, 
   T->dx = dx;
   T->dxT = dx * p->ratio_dxT_dx;
   T->dtT = d->dtT;
-  T->Lcp = p->latent_heat / p->cp;
   T->W0 = p->W0;
   T->GG = p->GG;
   T->S = p->S;
-  T->DT = p->DT;
-  T->Gmuk = p->Gamma * p->muk0;
+  T->diff = p->DT / (p->Gamma * p->muk0) / (T->dxT * T->dxT);
+  T->source = p->latent_heat / p->cp / ((double)d->ratio_dt_dtT * p->ratio_dxT_dx * p->ratio_dxT_dx);
 }
 
 int rs_create(const rs_params *p, rs_ctx **out) {
@@ -645,16 +644,14 @@ int rs_temperature_step(rs_ctx *c, double *d_T, double *d_T_next, const double *
   const double adv = vp_ramp(c->p, step * c->d.tau0 * c->d.dt) * c->d.tau0 / (c->p.S * c->p.W0);
   double *a = d_T, *b = d_T_next;
   for (int s = 0; s < c->d.ratio_dt_dtT; ++s) {
-    rs::launch_temperature_substep(c->T, a, b, d_dphidt, adv, st);
+    if (rs::launch_temperature_substep(c->T, a, b, d_dphidt, adv, st))
+      return fail(RS_E_CUDA, "rs_temperature_step: launch: %s", cudaGetErrorString(cudaGetLastError()));
     double *t = a;
     a = b;
     b = t;
   }
-  if (a != d_T) {
-    const size_t bytes = sizeof(double) * (size_t)c->d.NxT_all * c->d.NyT_all;
-    if (cudaMemcpyAsync(d_T, a, bytes, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-      return cuda_check("rs_temperature_step copy");
-  }
+  if (a != d_T && rs::launch_temperature_copy(c->T, a, d_T, st))
+    return fail(RS_E_CUDA, "rs_temperature_step: launch: %s", cudaGetErrorString(cudaGetLastError()));
   return cuda_check("rs_temperature_step");
 }
 
@@ -673,8 +670,9 @@ int rs_integrate_phi(rs_ctx *c, const rs_fields *cur, const rs_fields *next, dou
   if (rc) return rc;
   // a pull-back fused into the last rs_step on this cur shifted its read side only
   const int off = (c->pb_cur && cur->psi == c->pb_cur) ? c->pb_offset : 0;
-  rs::launch_integrate_phi(cur->precision, c->T, cur->psi, next->psi, d_dphidt, i_left_end, off,
-                           (cudaStream_t)stream);
+  if (rs::launch_integrate_phi(cur->precision, c->T, cur->psi, next->psi, d_dphidt, i_left_end, off,
+                               (cudaStream_t)stream))
+    return fail(RS_E_CUDA, "rs_integrate_phi: launch: %s", cudaGetErrorString(cudaGetLastError()));
   return cuda_check("rs_integrate_phi");
 }
 

@@ -220,16 +220,19 @@ struct TfcCoef {
   int32_t NxT, NyT, NxT_all, NyT_all;
   int32_t jTmin, jTmax;
   int32_t ratio_dt_dtT, Sint;
-  double Tcold, Thot, dx, dxT, dtT, Lcp, W0, GG, S, DT, Gmuk;
+  double Tcold, Thot, dx, dxT, dtT, W0, GG, S;
+  double diff;    // DT / (Gamma muk0 dxT^2)
+  double source;  // Lcp / (ratio_dt_dtT ratio^2)
 };
 void launch_temperature_init(const TfcCoef &T, double *d_T, cudaStream_t st);
 // adv = Vp_ramp(step tau0 dt) tau0 / (S W0), per step (fun.cu:1563)
-void launch_temperature_substep(const TfcCoef &T, const double *Tin, double *Tout,
-                                const double *dphidt, double adv, cudaStream_t st);
+int launch_temperature_substep(const TfcCoef &T, const double *Tin, double *Tout, const double *dphidt, double adv,
+                               cudaStream_t st);
+int launch_temperature_copy(const TfcCoef &T, const double *src, double *dst, cudaStream_t st);
 void launch_interpolate_temperature(const TfcCoef &T, const StepCoef &K, const double *d_T,
                                     double *d_T_fine, int i_left_end, cudaStream_t st);
-void launch_integrate_phi(int precision, const TfcCoef &T, const void *psi, const void *psi_n,
-                          double *dphidt, int i_left_end, int i_offset, cudaStream_t st);
+int launch_integrate_phi(int precision, const TfcCoef &T, const void *psi, const void *psi_n, double *dphidt,
+                         int i_left_end, int i_offset, cudaStream_t st);
 
 // records a message for rs_last_error() and returns code (rs_capi.cu)
 int set_error(int code, const char *msg);
