@@ -343,7 +343,10 @@ int rs_create(const rs_params *p, rs_ctx **out) {
     return fail(RS_E_CUDA, "rs_create: no CUDA device");
   }
   const int ni = p->nx_all - 2, nj = p->ny_all - 2;
-  c->max_partials = ((ni + 31) / 32) * ((nj + 7) / 8) + (p->ny_all + 7) / 8 + 64;
+  // the largest of the step kernels' grids (register kernel: 32-column strips,
+  // FP64 tiles: 64 columns by 4 rows and more)
+  c->max_partials = std::max(((ni + 31) / 32) * ((nj + 7) / 8), ((p->nx_all + 63) / 64) * ((nj + 3) / 4)) +
+                    (p->ny_all + 7) / 8 + 64;
   cudaError_t e = cudaMalloc(&c->partials, sizeof(rs::BlockPartial) * c->max_partials);
   if (e == cudaSuccess) e = cudaMalloc(&c->row_last, sizeof(int) * p->ny_all);
   if (e == cudaSuccess) e = cudaMalloc(&c->row_f, sizeof(double) * p->ny_all);
@@ -458,7 +461,10 @@ int rs_step(rs_ctx *c, const rs_fields *cur, const rs_fields *next, const rs_ste
   const uintptr_t vec = 16;
   const bool out_aligned =
       ((uintptr_t)next->psi % vec) == 0 && ((uintptr_t)next->c % vec) == 0 && ((uintptr_t)next->phi % vec) == 0;
-  const int box_rows = c->p.tfc && cur->precision == RS_F32 ? rs::kTfcTileRows32 + 2 : rs::kTmaBoxH;
+  const int rows = cur->precision == RS_F64 ? rs::tile_rows_f64(c->p.nx_all, c->p.ny_all, c->p.tfc != 0)
+                   : c->p.tfc               ? rs::kTfcTileRows32
+                                            : rs::kTileRows;
+  const int box_rows = rows + 2;
   if (c->use_tma && out_aligned && field_map(c, cur->psi, cur->precision, box_rows, &tm.psi) &&
       field_map(c, cur->c, cur->precision, box_rows, &tm.c)) {
     tm.col_tab = c->col_tab;
@@ -467,6 +473,7 @@ int rs_step(rs_ctx *c, const rs_fields *cur, const rs_fields *next, const rs_ste
     tm.col_tab64_len = c->col_tab64_len;
     tm.surr = c->surr.w && cur->precision == RS_F32 ? &c->surr : nullptr;
     tm.pipeline = c->pipeline;
+    tm.rows = rows;
     tm.red = {};
     if (red) {  // both tile kernels reduce their partials themselves
       tm.red.counter = c->red_counter;

@@ -47,6 +47,19 @@ inline int resident_ctas(const void *kfn, int threads, size_t smem, std::atomic<
 }
 }  // namespace rs
 
+namespace rs {
+// SMs of the current device (148 if it cannot be asked), once per device
+inline int sm_count() {
+  static std::atomic<int> cache[64];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 148;
+  if (dev < 64 && (n = cache[dev].load(std::memory_order_relaxed)) != 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 148;
+  if (dev < 64) cache[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+}  // namespace rs
+
 #define RS_HD __host__ __device__ __forceinline__
 
 namespace rs {

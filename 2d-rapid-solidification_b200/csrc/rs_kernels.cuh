@@ -154,6 +154,7 @@ struct TmaMaps {
   const SurrArgs *surr;  // learned CALPHAD surrogate, or nullptr (exact)
   FinalRed red;          // counter, offset and outputs (partials, nparts set by the launcher)
   int pipeline;          // the persistent warp-role kernel instead of one tile per CTA
+  int rows;              // output rows of a tile (the maps' boxes are two rows higher)
 };
 constexpr int kTileOutW = 128;                  // output columns of an FP32 tile
 constexpr int kTmaBoxW32 = kTileOutW + 8;        // input columns (4 each side keep x 16-byte aligned)
@@ -161,6 +162,7 @@ constexpr int kTileOutW64 = 64;                  // output columns of an FP64 ti
 constexpr int kTmaBoxW64 = kTileOutW64 + 8;      // its input columns
 constexpr int kTileRows = 16;    // output rows of a tile
 constexpr int kTmaBoxH = kTileRows + 2;  // input rows of a tile
+int tile_rows_f64(int nx, int ny, bool tfc);  // output rows of an FP64 tile: 4, 8 or 16
 constexpr int kTfcTileRows32 = 8;        // output rows of an FP32 coarse-grid-temperature tile
 constexpr int kColTabFields = 5;
 // length of the per-column table (entry k is column k - 4) for nx_all columns

@@ -298,9 +298,13 @@ __device__ __forceinline__ double log_near(const LogRef &L, double T) {
 // term is the cell form itself (groups_at) at T0.  Cells farther than 4 K from
 // T0, or all cells when T0 is not in [1945, 2746) K (so that the cells within
 // 4 K of it stay in [1941, 2750) K), take groups_at.
+// The driving-force groups have the same form: A_Ti = G_Ti_Liq - G_Ti_BCC by its
+// own Taylor polynomial (its remainder below 7e-16 J/mol), A_Nb = G_Nb_Liq -
+// G_Nb_BCC in closed form, as the SGTE pieces of Nb differ by a + bT + hT^7 only.
 struct KcPoly {
   LogRef lr;     // T0, log T0, 1 / T0 (also log_near's reference)
   double c[7];   // KC^(k)(T0) / k!
+  double a[7];   // A_Ti^(k)(T0) / k!
   int ok;        // T0 in [1945, 2746)
 };
 __device__ __forceinline__ KcPoly kc_poly(const StepCoef &K, double T0) {
@@ -319,7 +323,29 @@ __device__ __forceinline__ KcPoly kc_poly(const StepCoef &K, double T0) {
   P.c[4] = (2.0 * c * i3 + 24.0 * f * i5 + 840.0 * h * T3) / 24.0;
   P.c[5] = (-6.0 * c * i4 - 120.0 * f * i6 + 2520.0 * h * T2) / 120.0;
   P.c[6] = (24.0 * c * i5 + 720.0 * f * i7 + 5040.0 * h * T) / 720.0;
+  // G_Ti_Liq - G_Ti_BCC above 1941 K (fun.cu:1628-1647)
+  constexpr double ab = 298.7367 + 182.426471, ac = -46.29 - 19.0900905, ad = 22.00832e-3, ae = -1.228863e-6,
+                   af = -1400501.0;
+  P.a[0] = P.ok ? g_ti_liq(T, lT) - g_ti_bcc(T, lT) : 0.0;
+  P.a[1] = ab + ac * (lT + 1.0) + 2.0 * ad * T + 3.0 * ae * T2 - af * i2;
+  P.a[2] = (ac * i1 + 2.0 * ad + 6.0 * ae * T + 2.0 * af * i3) / 2.0;
+  P.a[3] = (-ac * i2 + 6.0 * ae - 6.0 * af * i4) / 6.0;
+  P.a[4] = (2.0 * ac * i3 + 24.0 * af * i5) / 24.0;
+  P.a[5] = (-6.0 * ac * i4 - 120.0 * af * i6) / 120.0;
+  P.a[6] = (24.0 * ac * i5 + 720.0 * af * i7) / 720.0;
   return P;
+}
+// the driving-force groups at T from P, or false where it does not apply
+__device__ __forceinline__ bool drive_eval(const KcPoly &P, double T, double &Anb, double &Ati) {
+  const double u = T - P.lr.T0;
+  if (!(P.ok && fabs(u) <= 4.0)) return false;
+  double r = P.a[6];
+#pragma unroll
+  for (int k = 5; k >= 0; --k) r = fma(r, u, P.a[k]);
+  Ati = r;
+  const double T2 = T * T, T4 = T2 * T2;
+  Anb = fma(131.229057 - 142.045475, T, 21262.202 + 8519.353) - 306.098e-25 * (T4 * T2 * T);
+  return true;
 }
 // K + C0 at T from P, or false where the polynomial does not apply
 __device__ __forceinline__ bool kc_eval(const KcPoly &P, double T, double &kc) {
@@ -341,17 +367,29 @@ static __device__ __noinline__ CellGroups groups_cell(const StepCoef &K, const L
 static __device__ __noinline__ CellGroups groups_exact(const StepCoef &K, double T) {
   return groups_at(K, T, log(T), true);
 }
+// the driving-force groups of a cell (phase 3)
+__device__ __forceinline__ void drive_tfc(const StepCoef &K, const KcPoly &P, double T, double &Anb, double &Ati) {
+  if (drive_eval(P, T, Anb, Ati)) return;
+  const CellGroups g = groups_cell(K, P.lr, T, true);
+  Anb = g.Anb;
+  Ati = g.Ati;
+}
 // the groups a cell needs: RT and K + C0 always, C0 where full (the general
 // row form; the melt forms multiply C0 by g + 1 = 0)
 __device__ __forceinline__ void cell_tfc(const StepCoef &K, const KcPoly &P, double T, bool full, double &RT,
                                          double &C0, double &KC) {
   RT = K.RR * T;
   C0 = 0.0;
-  const bool poly = kc_eval(P, T, KC);
-  if (!poly || full) {
+  if (kc_eval(P, T, KC)) {
+    if (full) {  // C0 from the driving-force groups: (G_Ti - G_Nb)_BCC - (G_Ti - G_Nb)_Liq = A_Nb - A_Ti
+      double Anb, Ati;
+      drive_eval(P, T, Anb, Ati);
+      C0 = -0.5 * (Anb - Ati) - 0.5 * (kL0Bcc - kL0Liq) * (1.0 - 2.0 * K.cinf);
+    }
+  } else {
     const CellGroups g = groups_cell(K, P.lr, T, full);
     C0 = g.C0;
-    if (!poly) KC = g.KC;
+    KC = g.KC;
   }
 }
 // interpolate_temperature's coordinates (fun.cu:1588-1594), split into the

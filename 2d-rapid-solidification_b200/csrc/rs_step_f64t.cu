@@ -8,29 +8,42 @@
 // launches:
 //   * column_table_kernel_f64: the per-column CALPHAD groups of this step's
 //     frozen temperature (col_terms, get_delta fun.cu:1610-1619) in FP64;
-//   * tile_kernel_f64, launched as a programmatic dependent of the table
-//     kernel: its CTAs start, issue their TMA loads, and wait for the table
-//     only where they first read it.
+//   * tile_kernel_f64.
+// Both are programmatic dependent launches: they are scheduled while the
+// kernel before them drains and wait for it on the device, so a run's steps
+// follow one another without launch gaps (2048^2, all solid: 28.7 -> 26.4 us).
 //
-// A CTA of 128 threads owns a tile of 16 output rows x 64 output columns
-// (x0 .. x0+63, x0 a multiple of 64).  Its input, 18 rows x 72 columns
-// (x0-4 .. x0+67, so the TMA x coordinate stays 16-byte aligned), arrives in
-// shared memory by one TMA box per field.  Two adjacent columns per lane
-// (16-byte double2 shared-memory accesses).
-//   phase 1  per-cell S = q(psi) c (1-c) and mu'' of the 18 input rows into
+// A CTA of 128 threads owns a tile of TR output rows x 64 output columns
+// (x0 .. x0+63, x0 a multiple of 64; TR = 4, 8 or 16 by tile_rows_f64).  Its
+// input, TR + 2 rows x 72 columns (x0-4 .. x0+67, so the TMA x coordinate stays
+// 16-byte aligned), arrives in shared memory by one TMA box per field.  Two
+// adjacent columns per lane (16-byte double2 shared-memory accesses).  The CTA
+// votes on the tile's form:
+//   * far melt everywhere (the bulk of a run ahead of its front): the c update
+//     straight from registers to global memory (melt_tile), one barrier after
+//     the load;
+//   * deep solid everywhere: psi and c stay (solid_tile);
+//   * anything else, the phases:
+//   phase 1  per-cell S = q(psi) c (1-c) and mu'' of the input rows into
 //            shared memory, with per-row flags "every psi == -1" / "== +1"
 //            and per-lane phi masks; the halo columns x0-1 and x0+64 are
 //            computed by 36 threads of warps 2 and 3 (one input row fewer);
-//   phase 2  each warp computes 4 output rows: face fluxes from the shared S
+//   phase 2  each warp computes its output rows: face fluxes from the shared S
 //            and mu'' (neighbours straight from shared memory), the c update
 //            (kept in registers); cells whose 3x3 phi neighbourhood is not
 //            uniformly +-1 are listed;
-//   phase 3  the listed interface cells are updated one per thread;
+//   phase 3  the listed interface cells are updated one per thread, those that
+//            draw noise (a third of the tail cells of a planar front, at more
+//            than twice the cost) apart from the others;
 //   phase 4  new psi and c are written into the shared tile, ghost columns
 //            copied there, and each output row leaves by one bulk async copy
 //            per field (ghost rows by one more, except in row-band mode);
-//   partials the solute mass (FP64) and coarse tip of the tile; the last CTA
-//            to finish reduces them all.
+//   partials the solute mass (FP64) and coarse tip of the tile; a dependent
+//            launch reduces them all.
+// What bounds it: a 2048^2 grid ahead of a planar front (34.8 us a step, 43.0
+// without the melt form and the chained launches, floor 20.5) its instruction
+// issue and the load -> compute -> store chain of a CTA; small grids (256^2:
+// 12.4 us, 15.0 with 16-row tiles) and fronts the chain of the phases.
 // Arithmetic (identical mathematics to the reference, regrouped as in the
 // FP32 tile kernel):
 //   * mu = K(T) + C0(T) + mu'', C0 = -D - (L0_BCC - L0_Liq)(1 - 2 cinf)/2, so
@@ -50,15 +63,16 @@
 //     1.5 / 0.25 weights, the 4 folded into the flux constant); face fluxes
 //     are rounded products, so a cell's result does not depend on the tiling.
 // Launch order: the tile columns from the one holding the front
-// (front_first_block).  After phase 1 each CTA prefetches into L2 the input
-// tile of the block launched one resident wave later.
+// (front_first_block).  Once its own tile has arrived each CTA prefetches into
+// L2 the input tile of the block launched one resident wave later.
 // The coarse-grid temperature (TFC, interpolate_temperature
 // fun.cu:1580-1608): no table kernel; every cell evaluates its CALPHAD groups
 // from its own bilinear temperature (K + C0 by its Taylor polynomial about
-// the tile's centre temperature, kc_poly; C0 in general rows and cells out of
-// the polynomial's range by the Gibbs functions) and stores
-// mu = mu'' + (K + C0), so the faces take plain differences of mu.  The tile kernel then runs in plain stream
-// order: it issues its TMA loads before griddepcontrol.wait.
+// the tile's centre temperature, kc_poly, and C0 and the driving-force groups
+// likewise; cells out of the polynomials' range by the Gibbs functions) and
+// stores mu = mu'' + (K + C0), so the faces take plain differences of mu.
+// 768 x 832 with a cellular front: 22.5 us a step (41 with the Gibbs functions
+// per cell).
 //
 // Two kernels run these phases (same functions, same results bit for bit):
 //   * tile_kernel_f64: one tile per CTA of 128 threads, the phases in series
@@ -78,72 +92,16 @@ namespace {
 
 constexpr int kW = kTileOutW64;   // output columns of a tile
 constexpr int kWin = kTmaBoxW64;  // input columns of a tile (kW + 8)
-constexpr int kTR = kTileRows;    // output rows of a tile
-constexpr int kTRin = kTmaBoxH;   // input rows of a tile
 constexpr int kThreads = 128;     // threads of a phase group
 constexpr int kWarps = kThreads / 32;
-constexpr int kRowsPerWarp = kTR / kWarps;
 constexpr int kHaloL = 3, kHaloR = kW + 4;  // box columns of x0-1 and x0+kW
 constexpr uint32_t kWaitLimit = 1u << 20;
 constexpr unsigned FULL = 0xffffffffu;
 constexpr unsigned long long kMinus1 = 0xBFF0000000000000ull, kPlus1 = 0x3FF0000000000000ull;
-constexpr uint32_t kTileBytes = 2u * kTRin * kWin * sizeof(double);
 static_assert(kW == 32 * 2, "two columns per lane");
-static_assert(kTR % kWarps == 0 && kRowsPerWarp == 4, "four output rows per warp");
-static_assert(kTRin <= 32, "row flags are 32-bit masks");
-static_assert(64 + 2 * kTRin <= kThreads && 4 * kTR <= kThreads, "one thread per halo cell and per row copy");
-
 // column table arrays (kColTabFields of them, len doubles each); entry k
 // describes column k - 4
 enum { kTabRT = 0, kTabC0 = 1, kTabDK = 2, kTabAnb = 3, kTabAti = 4 };
-
-// the input tile: TMA destinations (128-byte aligned); after phase 3 rows
-// 1..16 receive the new psi / c for the bulk stores
-struct alignas(128) InSlot {  // both arrays are TMA destinations: 128-byte aligned
-  alignas(128) double psi[kTRin][kWin];
-  alignas(128) double c[kTRin][kWin];
-};
-// phase 1 -> phases 2-4: per-cell terms and row flags
-struct alignas(16) StSlot {
-  double S[kTRin][kWin];  // after phase 2: new psi of the listed cells
-  double mu[kTRin][kWin];
-  uint8_t pmask[kTRin][32];  // per lane: bits 0-1 psi <= -1, bits 4-5 psi >= 1 of its two cells
-                             // (rows flagged in liq / sol store none)
-  uint8_t hmask[kTRin][2];   // halo cells: bit 0 psi <= -1, bit 1 psi >= 1
-  uint32_t liq, sol;         // bit r: every cell of input row r has psi == -1 / +1
-  double ty[kTRin];          // TFC: the row part of each input row's temperature
-  int tj[kTRin];             // (tfc_row), once per tile
-  KcPoly kp;                 // TFC: K + C0 near the tile's temperature
-  double hx[2];              // TFC: column part of the halo columns' temperatures
-  int hiT[2];
-};
-// phases 2-4: the interface list and the partial sums
-struct P2Smem {
-  uint16_t list[kTR * kW];  // interface cells: row << 8 | output column
-  int nlist;
-  int last;  // this CTA finished last (fused final reduction)
-  double part_mass[kWarps];
-  int part_itip[kWarps];
-};
-struct alignas(128) TileSmem64 {
-  InSlot in;
-  StSlot st;
-  P2Smem p2;
-  uint64_t full;
-};
-constexpr int kRing = 3, kStage = 2;
-struct alignas(128) PipeSmem64 {
-  InSlot in[kRing];
-  StSlot st[kStage];
-  P2Smem p2;
-  uint64_t in_full[kRing], in_empty[kRing], st_full[kStage], st_empty[kStage];
-  int abort;  // a wait gave up: every role stops
-};
-static_assert(sizeof(InSlot) % 128 == 0 && offsetof(InSlot, psi) % 128 == 0 && offsetof(InSlot, c) % 128 == 0,
-              "ring slots and their TMA destinations stay 128-byte aligned");
-static_assert(offsetof(PipeSmem64, in) % 128 == 0 && offsetof(TileSmem64, in) % 128 == 0,
-              "the input slots start on 128-byte boundaries");
-static_assert((kWin * sizeof(double)) % 16 == 0, "rows stay 16-byte aligned for double2 and bulk copies");
 
 __device__ __forceinline__ double2 ld2(const double *p) { return *reinterpret_cast<const double2 *>(p); }
 __device__ __forceinline__ void st2(double *p, double a, double b) {
@@ -185,6 +143,33 @@ __device__ __forceinline__ void cell_terms(const Coef<double> &F, double pv, dou
   mu = -(g + 1.0) * C0 - dv * fma(2.0 * L0half, g, L0sum) + RT * lam;
 }
 
+// A far-melt cell (psi = -1 exactly, |delta| <= melt_tiny): g = -1, q = 1, lam
+// by its Taylor polynomial in delta (Coef::melt_a, six terms, ma),
+// mu'' = RT lam - 2 L0_Liq delta = delta (RT p + KL), lam = delta p; with TFC
+// plus the cell's K + C0.  Rounded products: phase 1 and the melt tiles give
+// the same bits.
+template <bool TFC>
+__device__ __forceinline__ void far_cell(const double (&ma)[6], double c, double dv, double RT, double KC, double &S,
+                                         double &mu) {
+  constexpr double KL = -2.0 * kL0Liq;
+  double p = ma[5];
+#pragma unroll
+  for (int k = 4; k >= 0; --k) p = fma(p, dv, ma[k]);
+  S = __dmul_rn(c, 1.0 - c);
+  const double w = fma(RT, p, KL);
+  mu = TFC ? fma(dv, w, KC) : __dmul_rn(dv, w);
+}
+// a bulk-melt cell (psi = -1 exactly, delta in the series range)
+template <bool TFC>
+__device__ __forceinline__ void bulk_cell(double cinf, double c, double dv, double RT, double KC, double &S,
+                                          double &mu) {
+  const double om = 1.0 - c;
+  const double sv = dv / fma(2.0 * cinf, om, dv);
+  S = __dmul_rn(c, om);
+  mu = fma(RT, lam_series(sv), __dmul_rn(dv, -2.0 * kL0Liq));
+  if (TFC) mu += KC;
+}
+
 // shared -> global bulk copy (16-byte aligned addresses, size a multiple of 16)
 __device__ __forceinline__ void bulk_store(void *gdst, const void *ssrc, uint32_t bytes) {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gdst), "r"(smem_u32(ssrc)),
@@ -209,6 +194,8 @@ __global__ void __launch_bounds__(kTabBlock) column_table_kernel_f64(const StepC
   const double C0 = -ct.D - 0.5 * (kL0Bcc - kL0Liq) * (1.0 - 2.0 * K.cinf);
   kc[threadIdx.x] = ct.Kc + C0;
   __syncthreads();
+  // the previous step's tiles have read the table
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (threadIdx.x == kTabBlock - 1 || k >= len) return;
   tab[kTabRT * len + k] = ct.RT;
   tab[kTabC0 * len + k] = C0;
@@ -225,6 +212,73 @@ struct Tab {
         Anb(tab + kTabAnb * len + 4), Ati(tab + kTabAti * len + 4) {}
 };
 
+// Everything that depends on the tile's height: TR output rows (4, 8 or 16), a
+// warp taking every fourth of them.  A tile's latency is the chain load ->
+// phases -> stores of its four warps, and a tile at the front takes long (its
+// phase 3 alone 6 to 8 rounds at 16 rows), so a grid whose 16-row tiles would
+// leave SMs idle takes lower ones (tile_rows).
+template <int TR>
+struct TileOps {
+static constexpr int kTR = TR, kTRin = TR + 2;  // output and input rows
+static constexpr int kRowsPerWarp = TR / kWarps;
+static constexpr uint32_t kTileBytes = 2u * kTRin * kWin * sizeof(double);
+static_assert(TR % kWarps == 0 && kRowsPerWarp * kWarps == TR, "output rows split evenly over the warps");
+static_assert(kTRin <= 32, "row flags are 32-bit masks");
+static_assert(64 + 2 * kTRin <= kThreads && 4 * kTR <= kThreads, "one thread per halo cell and per row copy");
+
+// the input tile: TMA destinations (128-byte aligned); after phase 3 rows
+// 1..16 receive the new psi / c for the bulk stores
+struct alignas(128) InSlot {  // both arrays are TMA destinations: 128-byte aligned
+  alignas(128) double psi[kTRin][kWin];
+  alignas(128) double c[kTRin][kWin];
+};
+// phase 1 -> phases 2-4: per-cell terms
+struct alignas(128) StArr {
+  double S[kTRin][kWin];  // after phase 2: new psi of the listed cells
+  double mu[kTRin][kWin];
+};
+// and row flags
+struct alignas(16) StFlags {
+  uint8_t pmask[kTRin][32];  // per lane: bits 0-1 psi <= -1, bits 4-5 psi >= 1 of its two cells
+                             // (rows flagged in liq / sol store none)
+  uint8_t hmask[kTRin][2];   // halo cells: bit 0 psi <= -1, bit 1 psi >= 1
+  uint32_t liq, sol;         // bit r: every cell of input row r has psi == -1 / +1
+};
+// TFC: what a tile's temperatures need, once per tile
+struct TfcTile {
+  double ty[kTRin];  // the row part of each input row's temperature (tfc_row)
+  int tj[kTRin];
+  KcPoly kp;         // K + C0 near the tile's temperature
+  double hx[2];      // column part of the halo columns' temperatures
+  int hiT[2];
+  double tx[kW];     // and of the tile's columns (tfc_col)
+  int ti[kW];
+};
+// phases 2-4: the interface list and the partial sums
+struct P2Smem {
+  // interface cells (row << 8 | output column): those that draw noise from the
+  // front, the others from the back, so that phase 3's warps are of one kind
+  uint16_t list[kTR * kW];
+  uint32_t nlist;  // how many of the first kind, and << 16 of the second
+  double part_mass[kWarps];
+  int part_itip[kWarps];
+};
+// melt tiles: S and mu of the halo columns of each warp's rows
+static constexpr int kHaloTerms = 2 * (kRowsPerWarp + 2);
+struct MeltHalo {
+  double s[kWarps][kHaloTerms], m[kWarps][kHaloTerms];
+};
+static_assert(sizeof(MeltHalo) <= sizeof(uint16_t) * kTR * kW, "a melt tile's halo terms use the list's room");
+template <bool TFC>
+struct alignas(128) TileSmem {
+  InSlot in;
+  StArr st;
+  StFlags fl;
+  alignas(16) P2Smem p2;
+  std::conditional_t<TFC, TfcTile, char> tf;
+  uint64_t full;
+  uint32_t vote;  // the tile's form (tile_vote), OR of every thread's
+};
 // Everything one phase group needs about a tile and its own lane.
 struct TileView {
   const StepCoef &K;
@@ -253,25 +307,13 @@ struct TileView {
 // them before it waits for its tile, so their latency hides under the load.
 struct LaneCols {
   double RT[2], C0[2], dK[3];
-  int tiT[2];       // TFC: the coarse column left of each of the lane's two columns
-  double tx[2];     // and the column's offset from it, in coarse cells
 };
-__device__ __forceinline__ CellGroups cell_groups(const TileView &V, int gx, int row) {
-  int iT, jT;
-  double x, y;
-  tfc_col(V.K, V.PS.i_left_end_T, gx, iT, x);
-  tfc_row(V.K, row, jT, y);
-  return groups_exact(V.K, tfc_T(V.K, V.PS.T_coarse, iT, x, jT, y));
-}
-
 template <bool TFC>
-__device__ __forceinline__ LaneCols lane_cols(const TileView &V) {
+static __device__ __forceinline__ LaneCols lane_cols(const TileView &V) {
   LaneCols L;
-  if constexpr (TFC) {  // per cell (cell_groups); no column differences
+  if constexpr (TFC) {  // per cell (cell_tfc); no column differences
     L.RT[0] = L.RT[1] = L.C0[0] = L.C0[1] = 0.0;
     L.dK[0] = L.dK[1] = L.dK[2] = 0.0;
-    tfc_col(V.K, V.PS.i_left_end_T, V.gi, L.tiT[0], L.tx[0]);
-    tfc_col(V.K, V.PS.i_left_end_T, V.gi + 1, L.tiT[1], L.tx[1]);
     return L;
   }
   const double2 RTv = ld2(V.T.RT + V.gi), C0v = ld2(V.T.C0 + V.gi);
@@ -282,15 +324,13 @@ __device__ __forceinline__ LaneCols lane_cols(const TileView &V) {
   L.dK[0] = V.T.DK[V.gi - 1];  // faces x-1|x for x = col .. col+2
   L.dK[1] = V.T.DK[V.gi];
   L.dK[2] = V.T.DK[V.gi + 1];
-  L.tiT[0] = L.tiT[1] = 0;
-  L.tx[0] = L.tx[1] = 0.0;
   return L;
 }
 
 // columns beyond the array (right-most tiles; zero-filled by TMA) become
 // bulk melt, so they never force the general path; no output reads them.
 // Returns whether it wrote (the group then synchronises).
-__device__ __forceinline__ bool fix_beyond(const TileView &V, InSlot &in) {
+static __device__ __forceinline__ bool fix_beyond(const TileView &V, InSlot &in) {
   if (V.x0 + kW + 4 <= V.K.nx) return false;
   for (int k = V.gtid; k < kTRin * kWin; k += kThreads) {
     const int rr = k / kWin, x = k % kWin;
@@ -302,15 +342,42 @@ __device__ __forceinline__ bool fix_beyond(const TileView &V, InSlot &in) {
   return true;
 }
 
+// S and mu of a cell of the halo columns x0-1 (side 0), x0+kW (side 1), at
+// global column g: the far-melt form where the cell has it, else the general
+// one (a cell's form does not depend on the tile)
+template <bool TFC>
+static __device__ __forceinline__ void halo_cell(const TileView &V, const TfcTile *tf, const double (&ma)[6], double pv,
+                                          double cv, int rr, int side, int g, double &Sh, double &mh) {
+  const Coef<double> &F = V.F;
+  const double dv = cv - F.cinf;
+  double RT, C0, KC = 0.0;
+  if constexpr (TFC) {
+    // C0 enters mu'' as (g + 1) C0, 0 at psi = -1 exactly: the liquid
+    // groups suffice there
+    cell_tfc(V.K, tf->kp, tfc_T(V.K, V.PS.T_coarse, tf->hiT[side], tf->hx[side], tf->tj[rr], tf->ty[rr]),
+             bits(pv) != kMinus1, RT, C0, KC);
+  } else {
+    RT = V.T.RT[g];
+    C0 = V.T.C0[g];
+  }
+  if (bits(pv) == kMinus1 && fabs(dv) <= F.melt_tiny) {
+    far_cell<TFC>(ma, cv, dv, RT, KC, Sh, mh);
+    return;
+  }
+  const double sv = dv / fma(2.0 * F.cinf, 1.0 - cv, dv);
+  cell_terms(F, pv, cv, sv, fabs(sv) < 1.0 / 9.0, RT, C0, Sh, mh);
+  if (TFC) mh += KC;
+}
+
 // ---- phase 1: per-cell terms of the input rows of group warp gw (rows gw,
 // gw+4, ...) and of the halo columns (group threads 64..99); st.liq and
 // st.sol must be 0 on entry
 template <bool TFC>
-__device__ __forceinline__ void phase1(const TileView &V, const LaneCols &LC, const InSlot &in, StSlot &st) {
+static __device__ __forceinline__ void phase1(const TileView &V, const LaneCols &LC, const InSlot &in, StArr &sa, StFlags &st,
+                                       const TfcTile *tf) {
   const Coef<double> &F = V.F;
   const int lane = V.lane, bc = V.bc;
   const double cinf = F.cinf;
-  constexpr double KL = -2.0 * kL0Liq;
   const double d_hi = F.ser_hi, d_lo = F.ser_lo;  // series range of delta (Coef)
   double RTa[2] = {LC.RT[0], LC.RT[1]}, C0a[2] = {LC.C0[0], LC.C0[1]}, KCa[2] = {0.0, 0.0};
   // per lane, bit q: psi is exactly +1 over the 3x3 neighbourhood of cell
@@ -349,8 +416,8 @@ __device__ __forceinline__ void phase1(const TileView &V, const LaneCols &LC, co
 #pragma unroll 1
   for (int rr = V.gw; rr < kTRin; rr += kWarps) {
     if (rr > rows_in) {  // beyond the array (last tile): never read by an output
-      st2(&st.S[rr][bc], 0.0, 0.0);
-      st2(&st.mu[rr][bc], 0.0, 0.0);
+      st2(&sa.S[rr][bc], 0.0, 0.0);
+      st2(&sa.mu[rr][bc], 0.0, 0.0);
       liq_rows |= 1u << rr;
       sol_rows |= 1u << rr;
       continue;
@@ -366,47 +433,33 @@ __device__ __forceinline__ void phase1(const TileView &V, const LaneCols &LC, co
     const bool far = __all_sync(FULL, liq2 && fmax(fabs(dv[0]), fabs(dv[1])) <= tiny);
     const bool bulk = !far && __all_sync(FULL, liq2 && fmax(dv[0], dv[1]) < d_hi && fmin(dv[0], dv[1]) > d_lo);
     if constexpr (TFC) {  // the melt forms need RT and K + C0 only
-      const int jT = st.tj[rr];
-      const double y = st.ty[rr];
+      const int jT = tf->tj[rr];
+      const double y = tf->ty[rr];
       if (jT != band_jT) {  // warp-uniform: jT depends on the row only
         band_jT = jT;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          const double *r0 = V.PS.T_coarse + (int64_t)jT * V.K.NxT_all + LC.tiT[q], *r1 = r0 + V.K.NxT_all;
+          const double tx = tf->tx[V.col + q];
+          const double *r0 = V.PS.T_coarse + (int64_t)jT * V.K.NxT_all + tf->ti[V.col + q], *r1 = r0 + V.K.NxT_all;
           const double f00 = r0[0], f10 = r0[1], f01 = r1[0], f11 = r1[1];
-          Pb[q] = fma(f10 - f00, LC.tx[q], f00);
-          Qb[q] = fma(f11 - f10 - f01 + f00, LC.tx[q], f01 - f00);
+          Pb[q] = fma(f10 - f00, tx, f00);
+          Qb[q] = fma(f11 - f10 - f01 + f00, tx, f01 - f00);
         }
       }
 #pragma unroll
       for (int q = 0; q < 2; ++q)
-        cell_tfc(V.K, st.kp, fma(Qb[q], y, Pb[q]), !(far || bulk), RTa[q], C0a[q], KCa[q]);
+        cell_tfc(V.K, tf->kp, fma(Qb[q], y, Pb[q]), !(far || bulk), RTa[q], C0a[q], KCa[q]);
     }
     uint32_t code;
     bool deep = false;
     if (far) {
-      // far melt: g = -1, q = 1, lam by its Taylor polynomial in delta
-      // (Coef::melt_a, six terms); mu'' = RT lam - 2 L0_Liq delta
-      // = delta (RT p + KL), lam = delta p
       code = 1u;
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        double p = ma[5];
-#pragma unroll
-        for (int k = 4; k >= 0; --k) p = fma(p, dv[q], ma[k]);
-        Sv[q] = cv[q] * (1.0 - cv[q]);
-        mv[q] = dv[q] * fma(RTa[q], p, KL);
-      }
+      for (int q = 0; q < 2; ++q) far_cell<TFC>(ma, cv[q], dv[q], RTa[q], KCa[q], Sv[q], mv[q]);
     } else if (bulk) {
-      // bulk melt: g = -1, q = 1
       code = 1u;
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const double c = cv[q], om = 1.0 - c;
-        const double sv = dv[q] / fma(2.0 * cinf, om, dv[q]);
-        Sv[q] = c * om;
-        mv[q] = fma(RTa[q], lam_series(sv), dv[q] * KL);
-      }
+      for (int q = 0; q < 2; ++q) bulk_cell<TFC>(cinf, cv[q], dv[q], RTa[q], KCa[q], Sv[q], mv[q]);
     } else {
       code = (__all_sync(FULL, liq2) ? 1u : 0u) | (__all_sync(FULL, sol2) ? 2u : 0u);
       // deep solid row: no cell's mu'' enters a flux, so S = mu'' = 0 gives
@@ -434,12 +487,12 @@ __device__ __forceinline__ void phase1(const TileView &V, const LaneCols &LC, co
         st.pmask[rr][lane] = (uint8_t)(L | (Sm << 4));
       }
     }
-    if (TFC && !deep) {  // mu = mu'' + (K + C0) of the cell itself
+    if (TFC && !deep && !far && !bulk) {  // mu = mu'' + (K + C0) of the cell itself
       mv[0] += KCa[0];
       mv[1] += KCa[1];
     }
-    st2(&st.S[rr][bc], Sv[0], Sv[1]);
-    st2(&st.mu[rr][bc], mv[0], mv[1]);
+    st2(&sa.S[rr][bc], Sv[0], Sv[1]);
+    st2(&sa.mu[rr][bc], mv[0], mv[1]);
     liq_rows |= (code & 1u) << rr;
     sol_rows |= ((code >> 1) & 1u) << rr;
   }
@@ -457,23 +510,11 @@ __device__ __forceinline__ void phase1(const TileView &V, const LaneCols &LC, co
     uint8_t hm = 3u;
     if (V.y0 - 1 + rr <= V.K.ny - 1) {
       const double pv = in.psi[rr][x], cv = in.c[rr][x];
-      const double dv = cv - cinf;
-      const double sv = dv / fma(2.0 * cinf, 1.0 - cv, dv);
-      if constexpr (TFC) {
-        // C0 enters mu'' as (g + 1) C0, 0 at psi = -1 exactly: the liquid
-        // groups suffice there
-        double RT, C0, KC;
-        cell_tfc(V.K, st.kp, tfc_T(V.K, V.PS.T_coarse, st.hiT[side], st.hx[side], st.tj[rr], st.ty[rr]),
-                 bits(pv) != kMinus1, RT, C0, KC);
-        cell_terms(F, pv, cv, sv, fabs(sv) < 1.0 / 9.0, RT, C0, Sh, mh);
-        mh += KC;
-      } else {
-        cell_terms(F, pv, cv, sv, fabs(sv) < 1.0 / 9.0, V.T.RT[g], V.T.C0[g], Sh, mh);
-      }
+      halo_cell<TFC>(V, tf, ma, pv, cv, rr, side, g, Sh, mh);
       hm = (pv <= -1.0 ? 1u : 0u) | (pv >= 1.0 ? 2u : 0u);
     }
-    st.S[rr][x] = Sh;
-    st.mu[rr][x] = mh;
+    sa.S[rr][x] = Sh;
+    sa.mu[rr][x] = mh;
     st.hmask[rr][side] = hm;
   }
 }
@@ -481,8 +522,8 @@ __device__ __forceinline__ void phase1(const TileView &V, const LaneCols &LC, co
 // ---- phase 2: group warp gw computes output rows 1 + 4gw .. 4 + 4gw:
 // fluxes, the c update into dn, the interface cells into the list (nlist
 // must be 0 on entry).  Returns the listed cells, 2 bits per output row.
-__device__ __forceinline__ uint32_t phase2(const TileView &V, const LaneCols &LC, const InSlot &in,
-                                           const StSlot &st, P2Smem &p2,
+static __device__ __forceinline__ uint32_t phase2(const TileView &V, const LaneCols &LC, const InSlot &in,
+                                           const StArr &sa, const StFlags &st, P2Smem &p2,
                                            double dn[kRowsPerWarp][2], double &mass, bool red) {
   const Coef<double> &F = V.F;
   const int lane = V.lane, bc = V.bc;
@@ -498,15 +539,15 @@ __device__ __forceinline__ uint32_t phase2(const TileView &V, const LaneCols &LC
     double q[3];
   };
   auto load_row = [&](int rr, Row &R) {
-    const double2 s = ld2(&st.S[rr][bc]), m = ld2(&st.mu[rr][bc]);
+    const double2 s = ld2(&sa.S[rr][bc]), m = ld2(&sa.mu[rr][bc]);
     R.s[0] = s.x;
     R.s[1] = s.y;
     R.m[0] = m.x;
     R.m[1] = m.y;
-    R.sl = st.S[rr][bc - 1];  // lane 0: the halo column x0-1
-    R.ml = st.mu[rr][bc - 1];
-    R.sr = st.S[rr][bc + 2];  // lane 31: the halo column x0+kW
-    R.mr = st.mu[rr][bc + 2];
+    R.sl = sa.S[rr][bc - 1];  // lane 0: the halo column x0-1
+    R.ml = sa.mu[rr][bc - 1];
+    R.sr = sa.S[rr][bc + 2];  // lane 31: the halo column x0+kW
+    R.mr = sa.mu[rr][bc + 2];
   };
   auto pairs = [](const Row &R) {
     Pairs P;
@@ -606,21 +647,26 @@ __device__ __forceinline__ uint32_t phase2(const TileView &V, const LaneCols &LC
         Sv &= ((lS >> k) & 1u) | (S << 1) | (((rS >> k) & 1u) << 3);
       }
       const uint32_t needs = ~((Lv & (Lv >> 1) & (Lv >> 2)) | (Sv & (Sv >> 1) & (Sv >> 2))) & V.outm;
-      const uint32_t cnt = __popc(needs);
-      uint32_t incl = cnt;  // inclusive warp scan of the counts
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(FULL, incl, o);
-        if (lane >= o) incl += v;
-      }
-      const uint32_t total = __shfl_sync(FULL, incl, 31);
-      int base = 0;
-      if (lane == 31 && total) base = atomicAdd(&p2.nlist, (int)total);
-      base = __shfl_sync(FULL, base, 31);
-      uint32_t off = (uint32_t)base + incl - cnt;
-#pragma unroll
-      for (int q = 0; q < 2; ++q)
-        if ((needs >> q) & 1u) p2.list[off++] = (uint16_t)((rr << 8) | (V.col + q));
+      // cells that draw noise (phi_cell's own test; here it only sorts the list)
+      const double2 ps2 = ld2(&in.psi[rr][bc]);
+      const uint32_t noisy =
+          F.noise_amp > 0.0 ? (fma(-ps2.x, ps2.x, 1.0) > 1.0e-3 ? 1u : 0u) | (fma(-ps2.y, ps2.y, 1.0) > 1.0e-3 ? 2u : 0u)
+                            : 3u;
+      // the lanes with such a cell (n) and with another listed one (t), per cell
+      const uint32_t n0 = __ballot_sync(FULL, needs & noisy & 1u), n1 = __ballot_sync(FULL, needs & noisy & 2u);
+      const uint32_t t0 = __ballot_sync(FULL, needs & ~noisy & 1u), t1 = __ballot_sync(FULL, needs & ~noisy & 2u);
+      const uint32_t add = (__popc(n0) + __popc(n1)) | ((__popc(t0) + __popc(t1)) << 16);
+      uint32_t base = 0u;
+      if (lane == 0 && add) base = atomicAdd(&p2.nlist, add);
+      base = __shfl_sync(FULL, base, 0);
+      const uint32_t below = (1u << lane) - 1u;
+      const uint32_t n_at = base & 0xFFFFu, t_at = kTR * kW - 1 - (base >> 16);
+      if (needs & 1u)
+        p2.list[(noisy & 1u) ? n_at + __popc(n0 & below) : t_at - __popc(t0 & below)] =
+            (uint16_t)((rr << 8) | V.col);
+      if (needs & 2u)
+        p2.list[(noisy & 2u) ? n_at + __popc(n0) + __popc(n1 & below) : t_at - __popc(t0) - __popc(t1 & below)] =
+            (uint16_t)((rr << 8) | (V.col + 1));
       needs_all |= needs << (2 * j);
     }
     rb = rc;
@@ -635,19 +681,18 @@ __device__ __forceinline__ uint32_t phase2(const TileView &V, const LaneCols &LC
 // ---- phase 3: the listed interface cells, one per group thread
 // (compute_phi, fun.cu:1143-1218); new psi into np[rr][x]
 template <bool TFC>
-__device__ __forceinline__ void phase3(const TileView &V, const InSlot &in, const P2Smem &p2,
+static __device__ __forceinline__ void phase3(const TileView &V, const InSlot &in, const P2Smem &p2, const TfcTile *tf,
                                        double (*np)[kWin], bool red, int &itip) {
-  const int nlist = p2.nlist;
+  const int na = (int)(p2.nlist & 0xFFFFu), nlist = na + (int)(p2.nlist >> 16);
   for (int idx = V.gtid; idx < nlist; idx += kThreads) {
-    const uint32_t e = p2.list[idx];
+    const uint32_t e = p2.list[idx < na ? idx : kTR * kW - 1 - (idx - na)];
     const int rr = (int)(e >> 8), x = (int)(e & 0xFFu) + 4;  // box column
     const int r = V.y0 - 1 + rr, g = V.x0 + x - 4;
     const double c00 = in.c[rr][x];
     double Anb, Ati;
     if constexpr (TFC) {
-      const CellGroups cg = cell_groups(V, g, r);
-      Anb = cg.Anb;
-      Ati = cg.Ati;
+      const double T = tfc_T(V.K, V.PS.T_coarse, tf->ti[x - 4], tf->tx[x - 4], tf->tj[rr], tf->ty[rr]);
+      drive_tfc(V.K, tf->kp, T, Anb, Ati);
     } else {
       Anb = V.T.Anb[g];
       Ati = V.T.Ati[g];
@@ -665,7 +710,7 @@ __device__ __forceinline__ void phase3(const TileView &V, const InSlot &in, cons
 
 // ---- phase 4: new psi and c of group warp gw's rows into the input tile
 // (after every group thread has finished phase 3)
-__device__ __forceinline__ void phase4_rows(const TileView &V, InSlot &in, const double (*np)[kWin],
+static __device__ __forceinline__ void phase4_rows(const TileView &V, InSlot &in, const double (*np)[kWin],
                                             uint32_t needs_all, const double dn[kRowsPerWarp][2], bool red,
                                             int &itip) {
   const int rbase = 1 + kRowsPerWarp * V.gw, bc = V.bc;
@@ -706,7 +751,7 @@ __device__ __forceinline__ void phase4_rows(const TileView &V, InSlot &in, const
 // < 64: row j, field, kind) and phi by plain stores; returns whether this
 // thread committed a bulk group (it then waits for its reads before the
 // tile's shared memory is reused)
-__device__ __forceinline__ bool store_tile(const TileView &V, InSlot &in, double *__restrict__ psi_n,
+static __device__ __forceinline__ bool store_tile(const TileView &V, InSlot &in, double *__restrict__ psi_n,
                                            double *__restrict__ c_n, double *__restrict__ phi_n, int bar) {
   const StepCoef &K = V.K;
   const int x0 = V.x0, y0 = V.y0;
@@ -766,12 +811,9 @@ __device__ __forceinline__ bool store_tile(const TileView &V, InSlot &in, double
   return any;
 }
 
-// the tile's partial sums, and the fused final reduction (the last tile to
-// finish sums every partial, in reduce_partials_kernel's order); scratch of
-// at least 256 doubles and 256 ints
-__device__ __forceinline__ void finish_tile(const TileView &V, P2Smem &p2, double mass, int itip,
-                                            BlockPartial *part, const FinalRed *FR, double *sm_m, int *sm_i,
-                                            int bar) {
+// the tile's partial sums (a dependent launch reduces them)
+static __device__ __forceinline__ void finish_tile(const TileView &V, P2Smem &p2, double mass, int itip,
+                                            BlockPartial *part, int bar) {
   if (!part) return;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mass += __shfl_down_sync(FULL, mass, o);
@@ -793,31 +835,258 @@ __device__ __forceinline__ void finish_tile(const TileView &V, P2Smem &p2, doubl
     b.pad = 0;
     *part = b;
   }
-  if (!FR) return;
-  if (V.gtid == 0) {
-    __threadfence();
-    p2.last = atomicAdd(FR->counter, 1u) == (unsigned)(FR->nparts - 1);
+}
+
+// ---- whole-tile forms: a tile whose input box is far melt (psi = -1 exactly,
+// |delta| <= melt_tiny) or deep solid (psi = +1 exactly) throughout needs
+// no masks, list or interface pass.  The CTA votes over every cell of the box
+// that an output reads (rows and columns outside the array are left out).  The ranges of delta are compared
+// by the high words of the doubles, on the safe side.  (Melt within the series
+// range only, the solute layer ahead of the front, keeps the phases: its rows
+// choose their form one by one, and a register form of that took 50 us on a
+// 2048^2 grid of such melt against 45.)
+enum : uint32_t { kNotMinus1 = 1u, kNotPlus1 = 2u, kNotFar = 4u, kNotFinite = 8u, kGaveUp = 16u };
+static __device__ __forceinline__ uint32_t hi_abs(double v) { return (uint32_t)__double2hiint(v) & 0x7fffffffu; }
+static __device__ __forceinline__ uint32_t tile_vote(const TileView &V, const InSlot &in) {
+  const Coef<double> &F = V.F;
+  const double cinf = F.cinf;
+  const int rows_in = V.K.ny - V.y0;
+  uint32_t m1 = 0u, p1 = 0u, dm = 0u;  // OR of psi's difference from -1 / +1, largest |delta| (high word)
+  auto cell = [&](double p, double c) {
+    const uint32_t lo = (uint32_t)__double2loint(p), hi = (uint32_t)__double2hiint(p);
+    m1 |= lo | (hi ^ 0xBFF00000u);
+    p1 |= lo | (hi ^ 0x3FF00000u);
+    dm = max(dm, hi_abs(c - cinf));
+  };
+#pragma unroll
+  for (int k = 0; k < (kTRin + kWarps - 1) / kWarps; ++k) {
+    const int rr = V.gw + kWarps * k;
+    if (rr < kTRin && rr <= rows_in) {
+      const double2 p = ld2(&in.psi[rr][V.bc]), c = ld2(&in.c[rr][V.bc]);
+      cell(p.x, c.x);
+      cell(p.y, c.y);
+    }
   }
-  gsync(bar);
-  if (!p2.last) return;
-  __threadfence();
-  final_reduce(*FR, sm_m, sm_i, V.gtid, [&] { gsync(bar); });
+  // the halo columns, one cell per thread, on the warps with a row fewer
+  if (V.gtid >= 64 && V.gtid < 64 + 2 * kTRin) {
+    const int rr = (V.gtid - 64) >> 1, side = V.gtid & 1;
+    if (rr <= rows_in && (side || V.x0 > 0)) cell(in.psi[rr][side ? kHaloR : kHaloL], in.c[rr][side ? kHaloR : kHaloL]);
+  }
+  return (m1 ? kNotMinus1 : 0u) | (p1 ? kNotPlus1 : 0u) | (dm < hi_abs(F.melt_tiny) ? 0u : kNotFar) |
+         (dm < 0x3FF00000u ? 0u : kNotFinite);
 }
 
-// tile (row tr, column tc) of the launch order: tile columns from the one
-// holding the front, tile rows of a column consecutive (they share halo rows
-// in L2)
-__device__ __forceinline__ void tile_of(int t, int nrt, int ncb, int f, int &tr, int &tc) {
-  tr = t % nrt;
-  tc = front_first_block(t / nrt, f, ncb);
+// new psi (constant pv) and c of the lane's two cells of the output rows of
+// its warp straight to global memory, with the ghost columns and rows they
+// copy to
+struct CellStore {
+  double *pr, *cr, *fr;  // the lane's cells of the row to store next
+  int64_t pitch;
+  bool live, left, right, ghost;
+  __device__ CellStore(const TileView &V, double *psi_n, double *c_n, double *phi_n) {
+    const StepCoef &K = V.K;
+    const int r = V.y0 + kRowsPerWarp * V.gw;
+    pitch = K.pitch;
+    const int64_t o = (int64_t)r * pitch + V.gi;
+    pr = psi_n + o;
+    cr = c_n + o;
+    fr = phi_n ? phi_n + o : nullptr;
+    live = V.gi < K.nx;          // (nx is even: both cells or neither)
+    left = V.gi == 0;            // ghost column 0
+    right = V.gi + 2 == K.nx;    // ghost column nx-1
+    ghost = (K.jmin >= r && K.jmin < r + kRowsPerWarp) || (K.jmax >= r && K.jmax < r + kRowsPerWarp);
+  }
+  // row r = y0 - 1 + rr, the next one of the warp
+  __device__ void put(const TileView &V, int rr, double pv, double c0, double c1, double *psi_n, double *c_n,
+                      double *phi_n) {
+    if (left) c0 = c1;
+    if (right) c1 = c0;
+    if (live) {
+      st2(pr, pv, pv);
+      st2(cr, c0, c1);
+      if (fr) st2(fr, pv, pv);
+      if (ghost) {
+        const int r = V.y0 - 1 + rr;
+        auto copy = [&](int row) {
+          const int64_t o = (int64_t)row * pitch + V.gi;
+          st2(psi_n + o, pv, pv);
+          st2(c_n + o, c0, c1);
+          if (phi_n) st2(phi_n + o, pv, pv);
+        };
+        if (r == V.K.jmin) copy(0);
+        if (r == V.K.jmax) copy(V.K.ny - 1);
+      }
+    }
+    pr += pitch;
+    cr += pitch;
+    if (fr) fr += pitch;
+  }
+};
+
+// a far-melt tile: psi stays -1; the c update of phases 1 and 2 with S and mu'' of
+// a warp's rows in registers (neighbour columns by shuffles, halo columns by
+// twelve lanes through scratch), stored straight to global memory.  The same
+// expressions as phases 1 and 2, so the same bits.  No row votes on its form,
+// so the arithmetic of the rows overlaps.  Returns the warp's part of the mass.
+template <bool TFC>
+static __device__ __forceinline__ double melt_tile(const TileView &V, const LaneCols &LC, const InSlot &in, MeltHalo &mh,
+                                            const TfcTile *tf, bool red, double *__restrict__ psi_n, double *__restrict__ c_n,
+                                            double *__restrict__ phi_n) {
+  const Coef<double> &F = V.F;
+  const int lane = V.lane, r0 = kRowsPerWarp * V.gw;
+  const double cinf = F.cinf, cflux4 = 0.25 * F.cflux, c_floor = F.c_floor;
+  const int rows_live = V.K.ny - 1 - V.y0;
+  const double(&ma)[6] = F.melt_a;
+  double *hs = mh.s[V.gw], *hm = mh.m[V.gw];  // halo terms of the warp's six rows, 2 per row
+  if (lane < kHaloTerms) {
+    const int rr = r0 + (lane >> 1), side = lane & 1;
+    double S = 0.0, m = 0.0;
+    if (rr <= V.K.ny - V.y0) {
+      const int x = side ? kHaloR : kHaloL;
+      halo_cell<TFC>(V, tf, ma, in.psi[rr][x], in.c[rr][x], rr, side, V.x0 - 4 + x, S, m);
+    }
+    hs[lane] = S;
+    hm[lane] = m;
+  }
+  __syncwarp();
+  struct Row {
+    double s[2], m[2], sl, sr, ml, mr;
+  };
+  int band_jT = -1;
+  double Pb[2] = {0.0, 0.0}, Qb[2] = {0.0, 0.0};
+  auto load_row = [&](int k, Row &R) {
+    const int rr = r0 + k;
+    const double2 cv = ld2(&in.c[rr][V.bc]);
+    const double cc[2] = {cv.x, cv.y};
+    const double dv[2] = {cv.x - cinf, cv.y - cinf};
+    double RT[2] = {LC.RT[0], LC.RT[1]}, KC[2] = {0.0, 0.0};
+    if constexpr (TFC) {
+      const int jT = tf->tj[rr];
+      const double y = tf->ty[rr];
+      if (jT != band_jT) {
+        band_jT = jT;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const double tx = tf->tx[V.col + q];
+          const double *t0 = V.PS.T_coarse + (int64_t)jT * V.K.NxT_all + tf->ti[V.col + q], *t1 = t0 + V.K.NxT_all;
+          const double f00 = t0[0], f10 = t0[1], f01 = t1[0], f11 = t1[1];
+          Pb[q] = fma(f10 - f00, tx, f00);
+          Qb[q] = fma(f11 - f10 - f01 + f00, tx, f01 - f00);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        double C0;
+        cell_tfc(V.K, tf->kp, fma(Qb[q], y, Pb[q]), false, RT[q], C0, KC[q]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) far_cell<TFC>(ma, cc[q], dv[q], RT[q], KC[q], R.s[q], R.m[q]);
+    R.sl = __shfl_up_sync(FULL, R.s[1], 1);
+    R.ml = __shfl_up_sync(FULL, R.m[1], 1);
+    R.sr = __shfl_down_sync(FULL, R.s[0], 1);
+    R.mr = __shfl_down_sync(FULL, R.m[0], 1);
+    if (lane == 0) {
+      R.sl = hs[2 * k];
+      R.ml = hm[2 * k];
+    }
+    if (lane == 31) {
+      R.sr = hs[2 * k + 1];
+      R.mr = hm[2 * k + 1];
+    }
+  };
+  struct Pairs {
+    double q[3];
+  };
+  auto pairs = [](const Row &R) {
+    Pairs P;
+    P.q[0] = R.sl + R.s[0];
+    P.q[1] = R.s[0] + R.s[1];
+    P.q[2] = R.s[1] + R.sr;
+    return P;
+  };
+  auto vface = [](const Row &A, const Row &B, double jv[2]) {
+    const double pp[4] = {A.sl + B.sl, A.s[0] + B.s[0], A.s[1] + B.s[1], A.sr + B.sr};
+#pragma unroll
+    for (int q = 0; q < 2; ++q) jv[q] = __dmul_rn(fma(6.0, pp[q + 1], pp[q] + pp[q + 2]), B.m[q] - A.m[q]);
+  };
+  CellStore out(V, psi_n, c_n, phi_n);
+  double mass = 0.0, jv_lo[2], jv_hi[2];
+  Row rb, rc;
+  Pairs pa, pb, pc;
+  {
+    Row ra;
+    load_row(0, ra);
+    load_row(1, rb);
+    vface(ra, rb, jv_lo);
+    pa = pairs(ra);
+    pb = pairs(rb);
+  }
+#pragma unroll
+  for (int j = 0; j < kRowsPerWarp; ++j) {
+    load_row(j + 2, rc);
+    pc = pairs(rc);
+    vface(rb, rc, jv_hi);
+    const double mm[4] = {rb.ml, rb.m[0], rb.m[1], rb.mr};
+    const double2 cv2 = ld2(&in.c[r0 + 1 + j][V.bc]);
+    const double cv[2] = {cv2.x, cv2.y};
+    double jh[3], dn[2];
+#pragma unroll
+    for (int fc = 0; fc < 3; ++fc)
+      jh[fc] = __dmul_rn(fma(6.0, pb.q[fc], pa.q[fc] + pc.q[fc]), mm[fc + 1] - mm[fc] + LC.dK[fc]);
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      dn[q] = fmax(fma(cflux4, (jh[q + 1] - jh[q]) + (jv_hi[q] - jv_lo[q]), cv[q]), c_floor);
+    if (r0 + 1 + j <= rows_live) {
+      if (red) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+          if ((V.outm >> q) & 1u) mass += dn[q];
+      }
+      out.put(V, r0 + 1 + j, -1.0, dn[0], dn[1], psi_n, c_n, phi_n);
+    }
+    rb = rc;
+    pa = pb;
+    pb = pc;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) jv_lo[q] = jv_hi[q];
+  }
+  return mass;
 }
 
-// ---------------------------------------------------------------- one tile per CTA
+// a deep solid tile: S = 0 in every cell, so every flux is 0 and psi and c
+// stay (itip: the last interior column, as phase 4 counts it)
+static __device__ __forceinline__ double solid_tile(const TileView &V, const InSlot &in, bool red,
+                                             double *__restrict__ psi_n, double *__restrict__ c_n,
+                                             double *__restrict__ phi_n, int &itip) {
+  const int r0 = kRowsPerWarp * V.gw, rows_live = V.K.ny - 1 - V.y0, nx = V.K.nx;
+  const double c_floor = V.F.c_floor;
+  CellStore out(V, psi_n, c_n, phi_n);
+  double mass = 0.0;
+#pragma unroll
+  for (int j = 0; j < kRowsPerWarp; ++j) {
+    const int rr = r0 + 1 + j;
+    if (rr > rows_live) break;
+    const double2 c = ld2(&in.c[rr][V.bc]);
+    const double dn[2] = {fmax(c.x, c_floor), fmax(c.y, c_floor)};
+    if (red) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        if ((V.outm >> q) & 1u) {
+          mass += dn[q];
+          itip = max(itip, V.gi + q == nx - 2 ? nx - 1 : V.gi + q);
+        }
+    }
+    out.put(V, rr, 1.0, dn[0], dn[1], psi_n, c_n, phi_n);
+  }
+  return mass;
+}
+
 // the input tile of a pull-back step: the same box as the TMA load (columns
 // x0-4 .. x0+kW+3, rows y0-1 .. y0+kTR, zeros outside the array), each
 // column i read from clamp(i + i_offset, 1, nx - 2), with c = cinf where that
 // is nx - 2 (the melt entering at the right edge)
-__device__ __forceinline__ void gather_pull_back(const StepCoef &K, const StepScalars &PS, int x0, int y0,
+static __device__ __forceinline__ void gather_pull_back(const StepCoef &K, const StepScalars &PS, int x0, int y0,
                                                  InSlot &in) {
   const double *__restrict__ psi = static_cast<const double *>(PS.src_psi);
   const double *__restrict__ c = static_cast<const double *>(PS.src_c);
@@ -836,23 +1105,49 @@ __device__ __forceinline__ void gather_pull_back(const StepCoef &K, const StepSc
   }
 }
 
-template <bool TFC>
+};
+
+// tile (row tr, column tc) of the launch order: tile columns from the one
+// holding the front, tile rows of a column consecutive (they share halo rows
+// in L2)
+__device__ __forceinline__ void tile_of(int t, int nrt, int ncb, int f, int &tr, int &tc) {
+  tr = t % nrt;
+  tc = front_first_block(t / nrt, f, ncb);
+}
+
+using Ops16 = TileOps<16>;
+// the persistent pipeline's rings
+constexpr int kRing = 3, kStage = 2;
+template <int TR>
+struct alignas(128) StSlot {
+  typename TileOps<TR>::StArr a;
+  typename TileOps<TR>::StFlags f;
+};
+template <int TR>
+struct alignas(128) PipeSmem64 {
+  typename TileOps<TR>::InSlot in[kRing];
+  StSlot<TR> st[kStage];
+  typename TileOps<TR>::P2Smem p2;
+  uint64_t in_full[kRing], in_empty[kRing], st_full[kStage], st_empty[kStage];
+  int abort;  // a wait gave up: every role stops
+};
+// ---------------------------------------------------------------- one tile per CTA
+template <int TR, bool TFC>
 __global__ void __launch_bounds__(kThreads, 5)
     tile_kernel_f64(const __grid_constant__ StepCoef K, const __grid_constant__ Coef<double> F,
                     const __grid_constant__ StepScalars PS, const __grid_constant__ CUtensorMap tm_psi,
                     const __grid_constant__ CUtensorMap tm_c, const double *__restrict__ tab, const int tab_len,
                     double *__restrict__ psi_n, double *__restrict__ c_n, double *__restrict__ phi_n,
-                    BlockPartial *partials, int *err, const __grid_constant__ FinalRed FR, const int wave) {
+                    BlockPartial *partials, int *err, const int wave_x, const int wave_y) {
+  using Ops = TileOps<TR>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  TileSmem64 &sm = *reinterpret_cast<TileSmem64 *>(smem_raw);
+  auto &sm = *reinterpret_cast<typename Ops::template TileSmem<TFC> *>(smem_raw);
   // blockIdx.x walks the tile rows of one tile column, blockIdx.y the tile
   // columns, from the one holding column PS.i_front
   const int f = max(PS.i_front, 0) / kW;
-  // tile t = blockIdx.y * gridDim.x + blockIdx.x of tile_of's order
   const int tr = (int)blockIdx.x, tc = front_first_block((int)blockIdx.y, f, (int)gridDim.y);
-  const int x0 = kW * tc, y0 = 1 + kTR * tr;
+  const int x0 = kW * tc, y0 = 1 + TR * tr;
   BlockPartial *part = partials ? partials + ((int64_t)tc * gridDim.x + tr) : nullptr;
-  const FinalRed *FRp = partials && FR.counter ? &FR : nullptr;
 
   if (smem_u32(smem_raw) & 127u) {  // TMA destinations must be 128-byte aligned
     if (threadIdx.x == 0) atomicExch(err, 2);
@@ -865,88 +1160,116 @@ __global__ void __launch_bounds__(kThreads, 5)
   if (threadIdx.x == 0) {
     mbar_init(&sm.full, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if (!pb) {
-      mbar_expect_tx(&sm.full, kTileBytes);
-      tma_load_2d(&sm.in.psi[0][0], &tm_psi, &sm.full, x0 - 4, y0 - 1);
-      tma_load_2d(&sm.in.c[0][0], &tm_c, &sm.full, x0 - 4, y0 - 1);
-    }
-    sm.st.liq = 0u;
-    sm.st.sol = 0u;
-    sm.p2.nlist = 0;
+    sm.fl.liq = sm.fl.sol = 0u;
+    sm.vote = 0u;
+    sm.p2.nlist = 0u;
   }
-  // the column table of this step (programmatic dependency on its kernel)
+  // the kernel before this one in the stream (the column table's, and with it
+  // every earlier one) has completed: its table and the fields are visible
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  // the step's final reduction (a programmatic dependent) may be scheduled now
+  if (threadIdx.x == 0 && !pb) {
+    mbar_expect_tx(&sm.full, Ops::kTileBytes);
+    tma_load_2d(&sm.in.psi[0][0], &tm_psi, &sm.full, x0 - 4, y0 - 1);
+    tma_load_2d(&sm.in.c[0][0], &tm_c, &sm.full, x0 - 4, y0 - 1);
+  }
+  // dependents of this step (its reduction, the next step) may be scheduled now
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const TileView V(K, F, PS, tab, tab_len, x0, y0, (int)threadIdx.x);
-  const LaneCols LC = lane_cols<TFC>(V);
-  if constexpr (TFC) {  // the row part of the cells' temperatures, once per tile row
-    if (threadIdx.x < kTRin) tfc_row(K, y0 - 1 + (int)threadIdx.x, sm.st.tj[threadIdx.x], sm.st.ty[threadIdx.x]);
-    if (threadIdx.x >= kTRin + 1 && threadIdx.x < kTRin + 3) {  // the halo columns x0-1, x0+kW
-      const int side = (int)threadIdx.x - (kTRin + 1);
-      tfc_col(K, PS.i_left_end_T, side ? x0 + kW : x0 - 1, sm.st.hiT[side], sm.st.hx[side]);
-    }
-    if (threadIdx.x == kTRin) {  // K + C0 about the temperature of the tile's centre
+  const typename Ops::TileView V(K, F, PS, tab, tab_len, x0, y0, (int)threadIdx.x);
+  const typename Ops::LaneCols LC = Ops::template lane_cols<TFC>(V);
+  const typename Ops::TfcTile *tf = nullptr;
+  if constexpr (TFC) {
+    typename Ops::TfcTile &T = sm.tf;
+    tf = &T;
+    // the column parts of the cells' temperatures, the row parts, and K + C0
+    // about the temperature of the tile's centre, once per tile
+    const int t = (int)threadIdx.x;
+    if (t < kW) tfc_col(K, PS.i_left_end_T, x0 + t, T.ti[t], T.tx[t]);
+    else if (t < kW + 2) tfc_col(K, PS.i_left_end_T, t == kW ? x0 - 1 : x0 + kW, T.hiT[t - kW], T.hx[t - kW]);
+    else if (t >= 96 && t < 96 + Ops::kTRin) tfc_row(K, y0 - 1 + t - 96, T.tj[t - 96], T.ty[t - 96]);
+    else if (t == 127) {
       int iT, jT;
       double x, y;
       tfc_col(K, PS.i_left_end_T, x0 + kW / 2, iT, x);
-      tfc_row(K, y0 + kTR / 2, jT, y);
-      sm.st.kp = kc_poly(K, tfc_T(K, PS.T_coarse, iT, x, jT, y));
+      tfc_row(K, y0 + TR / 2, jT, y);
+      T.kp = kc_poly(K, tfc_T(K, PS.T_coarse, iT, x, jT, y));
     }
   }
-  if (pb) gather_pull_back(K, PS, x0, y0, sm.in);
-  __syncthreads();  // barrier initialised, flags cleared (and the TFC row table written)
-  if (!pb) {
-    // bounded wait for the tile; if any thread gives up, the whole CTA skips
-    // the tile: no phase runs on a partly filled tile and nothing is stored.
-    // Thread 0 first waits (bounded again) for the load still in flight into
-    // this CTA's shared memory, and the CTA still reports a (zero) partial,
-    // so the fused final reduction keeps its count
+  if (pb) Ops::gather_pull_back(K, PS, x0, y0, sm.in);
+  __syncthreads();  // barrier initialised, flags cleared (and the TFC tables written)
+  bool gave_up = false;
+  if (!pb) {  // bounded wait for the tile
     const uint32_t limit = PS.wait_limit ? PS.wait_limit : kWaitLimit;
     uint32_t tries = 0;
-    bool gave_up = false;
     while (!mbar_try(&sm.full, 0, PS.wait_limit != 0)) {
       if (++tries >= limit) {
         gave_up = true;
         break;
       }
     }
-    if (__syncthreads_or(gave_up)) {
-      if (threadIdx.x == 0) {
-        atomicExch(err, 1);
-        for (uint32_t t = 0; t < kWaitLimit && !mbar_try_wait(&sm.full, 0); ++t) {
-        }
-      }
-      __syncthreads();
-      finish_tile(V, sm.p2, 0.0, 0, part, FRp, &sm.st.S[0][0], reinterpret_cast<int *>(&sm.st.mu[0][0]), 0);
-      return;
+  }
+  // pull the tile of the CTA that will start about one resident wave later
+  // (wave_y tile columns and wave_x tile rows on) into L2, so its loads
+  // overlap the rest of this wave's arithmetic
+  if (threadIdx.x == 0 && !pb && !gave_up) {
+    int nx = (int)blockIdx.x + wave_x, ny = (int)blockIdx.y + wave_y;
+    if (nx >= (int)gridDim.x) {
+      nx -= (int)gridDim.x;
+      ++ny;
+    }
+    if (ny < (int)gridDim.y) {
+      const int pc = front_first_block(ny, f, (int)gridDim.y);
+      tma_prefetch_2d(&tm_psi, kW * pc - 4, TR * nx);
+      tma_prefetch_2d(&tm_c, kW * pc - 4, TR * nx);
     }
   }
-  if (fix_beyond(V, sm.in)) __syncthreads();
-  phase1<TFC>(V, LC, sm.in, sm.st);
+  if (x0 + kW + 4 > K.nx) {  // (CTA-uniform) a thread that gave up leaves the tile alone
+    if (!gave_up) Ops::fix_beyond(V, sm.in);
+    __syncthreads();
+  }
+  {
+    uint32_t bad = gave_up ? (uint32_t)Ops::kGaveUp : Ops::tile_vote(V, sm.in);
+    bad = __reduce_or_sync(FULL, bad);
+    if (V.lane == 0 && bad) atomicOr(&sm.vote, bad);
+  }
   __syncthreads();
-  // phase 1 done: pull the tile of the CTA that will start about one resident
-  // wave later into L2, so its loads overlap the rest of this wave's arithmetic
-  if (threadIdx.x == 0 && wave > 0 && !pb) {
-    const unsigned nxt = blockIdx.y * gridDim.x + blockIdx.x + (unsigned)wave;
-    if (nxt < gridDim.x * gridDim.y) {
-      int pr, pc;
-      tile_of((int)nxt, (int)gridDim.x, (int)gridDim.y, f, pr, pc);
-      tma_prefetch_2d(&tm_psi, kW * pc - 4, kTR * pr);
-      tma_prefetch_2d(&tm_c, kW * pc - 4, kTR * pr);
-    }
-  }
+  const uint32_t vote = sm.vote;
   const bool red = part != nullptr;
   double mass = 0.0;
   int itip = 0;
-  double dn[kRowsPerWarp][2];
-  const uint32_t needs_all = phase2(V, LC, sm.in, sm.st, sm.p2, dn, mass, red);
+  if (vote & Ops::kGaveUp) {
+    // if any thread gives up, the whole CTA skips the tile: nothing is
+    // computed on a partly filled tile or stored.  Thread 0 first waits
+    // (bounded again) for the load still in flight into this CTA's shared
+    // memory, and the CTA still reports a (zero) partial
+    if (threadIdx.x == 0) {
+      atomicExch(err, 1);
+      for (uint32_t t = 0; t < kWaitLimit && !mbar_try_wait(&sm.full, 0); ++t) {
+      }
+    }
+    __syncthreads();
+    Ops::finish_tile(V, sm.p2, 0.0, 0, part, 0);
+    return;
+  }
+  const bool melt = !(vote & (Ops::kNotMinus1 | Ops::kNotFar));
+  if (melt || !(vote & (Ops::kNotPlus1 | Ops::kNotFinite))) {
+    if (melt)
+      mass = Ops::template melt_tile<TFC>(V, LC, sm.in, *reinterpret_cast<typename Ops::MeltHalo *>(sm.p2.list), tf, red,
+                                          psi_n, c_n, phi_n);
+    else
+      mass = Ops::solid_tile(V, sm.in, red, psi_n, c_n, phi_n, itip);
+    Ops::finish_tile(V, sm.p2, mass, itip, part, 0);
+    return;
+  }
+  Ops::template phase1<TFC>(V, LC, sm.in, sm.st, sm.fl, tf);
   __syncthreads();
-  phase3<TFC>(V, sm.in, sm.p2, sm.st.S, red, itip);  // S is free after phase 2
+  double dn[Ops::kRowsPerWarp][2];
+  const uint32_t needs_all = Ops::phase2(V, LC, sm.in, sm.st, sm.fl, sm.p2, dn, mass, red);
   __syncthreads();
-  phase4_rows(V, sm.in, sm.st.S, needs_all, dn, red, itip);
-  store_tile(V, sm.in, psi_n, c_n, phi_n, 0);
-  finish_tile(V, sm.p2, mass, itip, part, FRp, &sm.st.mu[0][0], reinterpret_cast<int *>(&sm.st.mu[8][0]), 0);
+  Ops::template phase3<TFC>(V, sm.in, sm.p2, tf, sm.st.S, red, itip);  // S is free after phase 2
+  __syncthreads();
+  Ops::phase4_rows(V, sm.in, sm.st.S, needs_all, dn, red, itip);
+  Ops::store_tile(V, sm.in, psi_n, c_n, phi_n, 0);
+  Ops::finish_tile(V, sm.p2, mass, itip, part, 0);
   // shared memory stays allocated until the copies have read it
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
@@ -983,19 +1306,19 @@ __device__ __forceinline__ bool pipe_wait(uint64_t *bar, uint32_t parity, volati
   return true;
 }
 
+template <int TR>
 __global__ void __launch_bounds__(kPipeThreads, 2)
     pipe_kernel_f64(const __grid_constant__ StepCoef K, const __grid_constant__ Coef<double> F,
                     const __grid_constant__ StepScalars PS, const __grid_constant__ CUtensorMap tm_psi,
                     const __grid_constant__ CUtensorMap tm_c, const double *__restrict__ tab, const int tab_len,
                     double *__restrict__ psi_n, double *__restrict__ c_n, double *__restrict__ phi_n,
-                    BlockPartial *partials, int *err, const __grid_constant__ FinalRed FR, const int nrt,
-                    const int ncb) {
+                    BlockPartial *partials, int *err, const int nrt, const int ncb) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  PipeSmem64 &sm = *reinterpret_cast<PipeSmem64 *>(smem_raw);
+  using Ops = TileOps<TR>;
+  PipeSmem64<TR> &sm = *reinterpret_cast<PipeSmem64<TR> *>(smem_raw);
   const int warp = threadIdx.x >> 5;
   const int ntiles = nrt * ncb;
   const int f = max(PS.i_front, 0) / kW;
-  const FinalRed *FRp = partials && FR.counter ? &FR : nullptr;
   const uint32_t limit = PS.wait_limit ? PS.wait_limit : kWaitLimit;
   const bool poll = PS.wait_limit != 0;
   volatile int *abort = &sm.abort;
@@ -1031,9 +1354,9 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
         if (k >= kRing && !pipe_wait(&sm.in_empty[s], ((k / kRing) - 1) & 1, abort, limit, err, poll)) break;
         int tr, tc;
         tile_of(t, nrt, ncb, f, tr, tc);
-        mbar_expect_tx(&sm.in_full[s], kTileBytes);
-        tma_load_2d(&sm.in[s].psi[0][0], &tm_psi, &sm.in_full[s], kW * tc - 4, kTR * tr);
-        tma_load_2d(&sm.in[s].c[0][0], &tm_c, &sm.in_full[s], kW * tc - 4, kTR * tr);
+        mbar_expect_tx(&sm.in_full[s], Ops::kTileBytes);
+        tma_load_2d(&sm.in[s].psi[0][0], &tm_psi, &sm.in_full[s], kW * tc - 4, TR * tr);
+        tma_load_2d(&sm.in[s].c[0][0], &tm_c, &sm.in_full[s], kW * tc - 4, TR * tr);
       }
       // loads still in flight into this CTA's shared memory complete before
       // it exits (bounded)
@@ -1057,14 +1380,14 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
       if (!group_and(ok, kBarP1)) break;
       int tr, tc;
       tile_of(t, nrt, ncb, f, tr, tc);
-      const TileView V(K, F, PS, tab, tab_len, kW * tc, 1 + kTR * tr, gtid);
+      const typename Ops::TileView V(K, F, PS, tab, tab_len, kW * tc, 1 + TR * tr, gtid);
       if (gtid == 0) {
-        sm.st[q].liq = 0u;
-        sm.st[q].sol = 0u;
+        sm.st[q].f.liq = 0u;
+        sm.st[q].f.sol = 0u;
       }
-      fix_beyond(V, sm.in[s]);
+      Ops::fix_beyond(V, sm.in[s]);
       gsync(kBarP1);
-      phase1<false>(V, lane_cols<false>(V), sm.in[s], sm.st[q]);
+      Ops::template phase1<false>(V, Ops::template lane_cols<false>(V), sm.in[s], sm.st[q].a, sm.st[q].f, nullptr);
       gsync(kBarP1);
       if (gtid == 0) mbar_arrive(&sm.st_full[q]);
     }
@@ -1078,22 +1401,21 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
     if (!group_and(pipe_wait(&sm.st_full[q], (k / kStage) & 1, abort, limit, err, poll), kBarP2)) break;
     int tr, tc;
     tile_of(t, nrt, ncb, f, tr, tc);
-    const TileView V(K, F, PS, tab, tab_len, kW * tc, 1 + kTR * tr, gtid);
+    const typename Ops::TileView V(K, F, PS, tab, tab_len, kW * tc, 1 + TR * tr, gtid);
     BlockPartial *part = partials ? partials + ((int64_t)tc * nrt + tr) : nullptr;
     const bool red = part != nullptr;
-    if (gtid == 0) sm.p2.nlist = 0;
+    if (gtid == 0) sm.p2.nlist = 0u;
     gsync(kBarP2);
     double mass = 0.0;
     int itip = 0;
-    double dn[kRowsPerWarp][2];
-    const uint32_t needs_all = phase2(V, lane_cols<false>(V), sm.in[s], sm.st[q], sm.p2, dn, mass, red);
+    double dn[Ops::kRowsPerWarp][2];
+    const uint32_t needs_all = Ops::phase2(V, Ops::template lane_cols<false>(V), sm.in[s], sm.st[q].a, sm.st[q].f, sm.p2, dn, mass, red);
     gsync(kBarP2);
-    phase3<false>(V, sm.in[s], sm.p2, sm.st[q].S, red, itip);  // S of the slot is free after phase 2
+    Ops::template phase3<false>(V, sm.in[s], sm.p2, nullptr, sm.st[q].a.S, red, itip);  // S of the slot is free after phase 2
     gsync(kBarP2);
-    phase4_rows(V, sm.in[s], sm.st[q].S, needs_all, dn, red, itip);
-    const bool issued = store_tile(V, sm.in[s], psi_n, c_n, phi_n, kBarP2);
-    finish_tile(V, sm.p2, mass, itip, part, FRp, &sm.st[q].mu[0][0], reinterpret_cast<int *>(&sm.st[q].mu[8][0]),
-                kBarP2);
+    Ops::phase4_rows(V, sm.in[s], sm.st[q].a.S, needs_all, dn, red, itip);
+    const bool issued = Ops::store_tile(V, sm.in[s], psi_n, c_n, phi_n, kBarP2);
+    Ops::finish_tile(V, sm.p2, mass, itip, part, kBarP2);
     // the slots are free once the bulk copies have read the input tile
     if (issued) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     gsync(kBarP2);
@@ -1107,67 +1429,91 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
 
 }  // namespace
 
+// Output rows of the tiles of an nx x ny step.  Low tiles share the latency of
+// a front tile (load, phases, stores in series, 12 to 21 us at 16 rows) among
+// more CTAs; high ones load and compute fewer halo rows.  The lines are where
+// they break even, in waves of five CTAs per SM of 16-row tiles (us a step with
+// a planar front, 4 / 8 / 16 rows): 512^2, 0.3 waves, 13.7 / 14.1 / 18.4; 768 x
+// 832, 0.8 waves, 12.4 / 13.9 / 24.0; 1024^2, 1.4 waves, 19.7 / 16.2 / 22.2;
+// 1536^2, 3.1 waves, 37.1 / 26.7 / 26.9; 2048^2, 5.5 waves, 61 / 42.3 / 37.1.
+// With the coarse-grid temperature a tile also sets up its temperature tables:
+// 768 x 832, 28.8 / 22.5 / 30.2 us a step, so 4 rows are left out.
+int tile_rows_f64(int nx, int ny, bool tfc) {
+  const int64_t tiles = (int64_t)((nx + kW - 1) / kW) * ((ny - 2 + 15) / 16), wave = 5 * (int64_t)sm_count();
+  return tiles >= 3 * wave ? 16 : tiles >= wave || tfc ? 8 : 4;
+}
+
 int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScalars &P, const TmaMaps &tm,
                         double *psi_n, double *c_n, double *phi_n, BlockPartial *partials, int max_partials,
                         int *nparts_out, int *err, cudaStream_t st) {
   const int nj = K.ny - 2;
   if (K.nx % 2 || K.pitch != K.nx) return -1;  // rows are copied in 16-byte units
-  const int nrt = (nj + kTR - 1) / kTR, ncb = (K.nx + kW - 1) / kW;
-  if (ncb > 65535 || (int64_t)nrt * ncb > (1 << 30)) return -1;
-  const int nparts = nrt * ncb;
-  if (partials && nparts > max_partials) return -1;
-  if (!tm.col_tab64 || tm.col_tab64_len < ncb * kW + kWin) return -1;
   // the coarse-grid temperature: per-cell groups, no column table (the
   // persistent pipeline has no TFC form and is not taken then)
   const bool tfc = K.tfc != 0;
   if (tfc && !P.T_coarse) return -1;
   const bool pipe = tm.pipeline != 0 && !tfc && !P.pull_back;
-  const int which = pipe ? 1 : tfc ? 2 : 0;
-  const size_t smem = pipe ? sizeof(PipeSmem64) : sizeof(TileSmem64);
-  const void *kfn = pipe ? (const void *)pipe_kernel_f64
-                         : tfc ? (const void *)tile_kernel_f64<true> : (const void *)tile_kernel_f64<false>;
-  static std::atomic<unsigned long long> attr_done[3];
+  const int TR = tm.rows;  // the tensor maps' box is TR + 2 rows high
+  if (!((TR == 4 && !tfc) || TR == 8 || TR == 16)) return -1;
+  const int nrt = (nj + TR - 1) / TR, ncb = (K.nx + kW - 1) / kW;
+  if (ncb > 65535 || (int64_t)nrt * ncb > (1 << 30)) return -1;
+  const int nparts = nrt * ncb;
+  if (partials && nparts > max_partials) return -1;
+  if (!tm.col_tab64 || tm.col_tab64_len < ncb * kW + kWin) return -1;
+  using Kfn = decltype(&tile_kernel_f64<16, false>);
+  static const Kfn tile_fn[2][3] = {{tile_kernel_f64<4, false>, tile_kernel_f64<8, false>, tile_kernel_f64<16, false>},
+                                    {nullptr, tile_kernel_f64<8, true>, tile_kernel_f64<16, true>}};
+  static const size_t tile_smem[2][3] = {
+      {sizeof(TileOps<4>::TileSmem<false>), sizeof(TileOps<8>::TileSmem<false>), sizeof(TileOps<16>::TileSmem<false>)},
+      {0, sizeof(TileOps<8>::TileSmem<true>), sizeof(TileOps<16>::TileSmem<true>)}};
+  const int sh = TR == 4 ? 0 : TR == 8 ? 1 : 2;
+  static const decltype(&pipe_kernel_f64<16>) pipe_fn[3] = {pipe_kernel_f64<4>, pipe_kernel_f64<8>, pipe_kernel_f64<16>};
+  static const size_t pipe_smem[3] = {sizeof(PipeSmem64<4>), sizeof(PipeSmem64<8>), sizeof(PipeSmem64<16>)};
+  const int which = pipe ? 6 + sh : 3 * tfc + sh;
+  const size_t smem = pipe ? pipe_smem[sh] : tile_smem[tfc][sh];
+  const void *kfn = pipe ? (const void *)pipe_fn[sh] : (const void *)tile_fn[tfc][sh];
+  static std::atomic<unsigned long long> attr_done[9];
   if (!smem_limit_once(kfn, (int)smem, attr_done[which])) return -3;
-  static std::atomic<int> resident_of[3][64];
+  static std::atomic<int> resident_of[9][64];
   const int resident = resident_ctas(kfn, pipe ? kPipeThreads : kThreads, smem, resident_of[which]);
   if (resident <= 0) return -3;
-  if (!tfc)
-    column_table_kernel_f64<<<(tm.col_tab64_len + kTabBlock - 2) / (kTabBlock - 1), kTabBlock, 0, st>>>(
-        K, P.d0, P.d1, tm.col_tab64_len, tm.col_tab64);
-  cudaLaunchConfig_t cfg = {};
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
+  // every kernel of the step is a programmatic dependent of the one before it
+  // in the stream: it is scheduled while that one drains and waits
+  // (griddepcontrol.wait) before it reads or writes what the other may touch
+  cudaLaunchConfig_t cfg = {};
+  cfg.stream = st;
   cfg.attrs = at;
-  // a programmatic dependent of the table kernel only: the tile kernel issues
-  // its TMA loads before griddepcontrol.wait, which is safe after the table
-  // kernel (it writes no field) but not after the previous step's kernels,
-  // so a TFC step (no table kernel) launches in plain stream order
-  cfg.numAttrs = tfc ? 0 : 1;
+  cfg.numAttrs = 1;
   const double *tab = tm.col_tab64;
-  // the final reduction is a programmatic dependent launch after the step
-  FinalRed fr = tm.red;
-  fr.partials = partials;
-  fr.nparts = nparts;
-  FinalRed none = fr;
-  none.counter = nullptr;
-  cudaError_t e;
+  cudaError_t e = cudaSuccess;
+  if (!tfc) {
+    cfg.gridDim = dim3((tm.col_tab64_len + kTabBlock - 2) / (kTabBlock - 1));
+    cfg.blockDim = dim3(kTabBlock);
+    e = cudaLaunchKernelEx(&cfg, column_table_kernel_f64, K, P.d0, P.d1, tm.col_tab64_len, tm.col_tab64);
+    if (e != cudaSuccess) return -3;
+  }
+  cfg.dynamicSmemBytes = smem;
   if (pipe) {
     // persistent: every CTA resident at once, each walking tiles b, b + G, ...
     cfg.gridDim = dim3((unsigned)std::min(resident, nparts));
     cfg.blockDim = dim3(kPipeThreads);
-    e = cudaLaunchKernelEx(&cfg, pipe_kernel_f64, K, F, P, tm.psi, tm.c, tab, tm.col_tab64_len, psi_n, c_n, phi_n,
-                           partials, err, none, nrt, ncb);
+    e = cudaLaunchKernelEx(&cfg, pipe_fn[sh], K, F, P, tm.psi, tm.c, tab, tm.col_tab64_len, psi_n, c_n, phi_n,
+                           partials, err, nrt, ncb);
   } else {
     // column-major: consecutive CTAs share a column strip and its halo rows in L2
     cfg.gridDim = dim3(nrt, ncb);
     cfg.blockDim = dim3(kThreads);
-    e = cudaLaunchKernelEx(&cfg, tfc ? tile_kernel_f64<true> : tile_kernel_f64<false>, K, F, P, tm.psi, tm.c, tab,
-                           tm.col_tab64_len, psi_n, c_n, phi_n, partials, err, none, resident);
+    e = cudaLaunchKernelEx(&cfg, tile_fn[tfc][sh], K, F, P, tm.psi, tm.c, tab, tm.col_tab64_len, psi_n, c_n, phi_n,
+                           partials, err, resident % nrt, resident / nrt);
   }
   if (e != cudaSuccess) return -3;
+  // the final reduction is a programmatic dependent launch after the step
+  FinalRed fr = tm.red;
+  fr.partials = partials;
+  fr.nparts = nparts;
   if (partials && (fr.mass_out || fr.itip_out) && launch_reduce_partials_dep(fr, st)) return -3;
   if (nparts_out) *nparts_out = nparts;
   return 0;
