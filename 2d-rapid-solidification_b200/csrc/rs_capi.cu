@@ -73,7 +73,6 @@ struct rs_ctx {
   float *mlp_w;        // its FP32 parameters (device)
   uint16_t *mlp_b16;   // FP16 W2 (32 x 32) and W3 padded to 8 rows (device)
   unsigned long long *mlp_audit;  // max error bits of mu'' and dG, fallback and audit counts
-  unsigned int *red_counter;  // fused final reduction of the FP32 tile kernel (device, 0 between launches)
   int use_tma;         // RS_OPT_TMA
   uint32_t wait_limit; // RS_OPT_WAIT_LIMIT (0: the kernels' default)
   int pipeline;        // RS_OPT_PIPELINE
@@ -353,8 +352,6 @@ int rs_create(const rs_params *p, rs_ctx **out) {
   if (e == cudaSuccess) e = cudaMalloc(&c->row_g, sizeof(double) * p->ny_all);
   if (e == cudaSuccess) e = cudaMalloc(&c->d_err, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(c->d_err, 0, sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&c->red_counter, sizeof(unsigned int));
-  if (e == cudaSuccess) e = cudaMemset(c->red_counter, 0, sizeof(unsigned int));
   c->col_tab_len = rs::col_tab_len(p->nx_all);
   if (e == cudaSuccess) e = cudaMalloc(&c->col_tab, sizeof(float) * rs::kColTabFields * c->col_tab_len);
   c->col_tab64_len = rs::col_tab64_len(p->nx_all);
@@ -375,7 +372,6 @@ int rs_destroy(rs_ctx *c) {
   cudaFree(c->row_f);
   cudaFree(c->row_g);
   cudaFree(c->d_err);
-  cudaFree(c->red_counter);
   cudaFree(c->col_tab);
   cudaFree(c->col_tab64);
   cudaFree(c->mlp_w);
@@ -462,8 +458,7 @@ int rs_step(rs_ctx *c, const rs_fields *cur, const rs_fields *next, const rs_ste
   const bool out_aligned =
       ((uintptr_t)next->psi % vec) == 0 && ((uintptr_t)next->c % vec) == 0 && ((uintptr_t)next->phi % vec) == 0;
   const int rows = cur->precision == RS_F64 ? rs::tile_rows_f64(c->p.nx_all, c->p.ny_all, c->p.tfc != 0)
-                   : c->p.tfc               ? rs::kTfcTileRows32
-                                            : rs::kTileRows;
+                                            : rs::tile_rows_f32(c->p.nx_all, c->p.ny_all, c->p.tfc != 0, c->surr.w != nullptr);
   const int box_rows = rows + 2;
   if (c->use_tma && out_aligned && field_map(c, cur->psi, cur->precision, box_rows, &tm.psi) &&
       field_map(c, cur->c, cur->precision, box_rows, &tm.c)) {
@@ -476,7 +471,6 @@ int rs_step(rs_ctx *c, const rs_fields *cur, const rs_fields *next, const rs_ste
     tm.rows = rows;
     tm.red = {};
     if (red) {  // both tile kernels reduce their partials themselves
-      tm.red.counter = c->red_counter;
       tm.red.mass_offset =
           cur->precision == RS_F32 ? (double)(c->p.nx_all - 2) * (c->p.ny_all - 2) * c->p.cinf : 0.0;
       tm.red.mass_out = a->mass_out;
@@ -559,7 +553,6 @@ int rs_device_status(rs_ctx *c, rs_stream_t stream) {
     return cuda_check("rs_device_status");
   if (h) {
     cudaMemsetAsync(c->d_err, 0, sizeof(int), st);
-    cudaMemsetAsync(c->red_counter, 0, sizeof(unsigned int), st);  // an aborted launch may have left it counting
     return fail(RS_E_STATE, "a device-side wait gave up (pipeline stalled); results of the affected steps are invalid");
   }
   return RS_OK;

@@ -154,15 +154,14 @@ int launch_mass_partials(int precision, const StepCoef &K, const void *c, double
              : -3;
 }
 
-__global__ void __launch_bounds__(128) reduce_partials_dep_kernel(const FinalRed FR) {
-  __shared__ double s_m[256];
-  __shared__ int s_i[256];
+__global__ void __launch_bounds__(kRedThreads) reduce_partials_dep_kernel(const FinalRed FR) {
   pdl_wait();  // the kernel that wrote the partials has completed, its writes visible
-  final_reduce(FR, s_m, s_i, (int)threadIdx.x, [] { __syncthreads(); });
+  pdl_trigger();
+  final_reduce(FR);
 }
 
 int launch_reduce_partials_dep(const FinalRed &FR, cudaStream_t st) {
-  return launch_dep(reduce_partials_dep_kernel, dim3(1), dim3(128), st, FR) == cudaSuccess ? 0 : -3;
+  return launch_dep(reduce_partials_dep_kernel, dim3(1), dim3(kRedThreads), st, FR) == cudaSuccess ? 0 : -3;
 }
 
 // ---------------------------------------------------------------- precise tip

@@ -18,11 +18,12 @@ struct Same {  // (the kernel's own parameter types: no deduction from the argum
   using type = T;
 };
 template <typename... Args>
-cudaError_t launch_dep(void (*kernel)(Args...), dim3 grid, dim3 block, cudaStream_t st,
-                       typename Same<Args>::type... args) {
+cudaError_t launch_dep_smem(void (*kernel)(Args...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                            const typename Same<Args>::type &...args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -30,6 +31,11 @@ cudaError_t launch_dep(void (*kernel)(Args...), dim3 grid, dim3 block, cudaStrea
   cfg.attrs = at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <typename... Args>
+cudaError_t launch_dep(void (*kernel)(Args...), dim3 grid, dim3 block, cudaStream_t st,
+                       const typename Same<Args>::type &...args) {
+  return launch_dep_smem(kernel, grid, block, 0, st, args...);
 }
 
 // Per-block partial results of a grid pass: sum of interior c (FP64) and the
@@ -72,75 +78,57 @@ __device__ __forceinline__ void block_partial(double mass, int itip, BlockPartia
 // Inputs of the TMA-staged FP32 kernel: descriptors of the current psi and c
 // fields (built on the host) and the context's per-column table workspace.
 struct SurrArgs;
-// Final reduction of the per-tile partials fused into the tile kernel: the
-// last CTA to finish (a counter in device memory, reset by that CTA) sums
-// them in the order of reduce_partials_kernel.  counter == nullptr: none.
+// The final reduction of a launch's partials (a dependent launch).
 struct FinalRed {
-  unsigned int *counter;
   const BlockPartial *partials;
   int nparts;
   double mass_offset;
   double *mass_out;
   int32_t *itip_out;
 };
-// The fused final reduction, run by the 128 threads of the CTA that finished
-// last: the partials are summed in a fixed order (slot v =
-// 0..255 adds partials v, v + 256, ... in turn, then a tree over the slots).
-// Each thread takes slots tid and tid + 128 and issues eight 16-byte loads
-// per slot before adding any of them, so the pass costs a few L2 round trips
-// rather than one per partial.  sm_m / sm_i: 256 doubles / ints of shared
-// scratch; sync(): the barrier of the 128 threads.
-template <typename Sync>
-__device__ __forceinline__ void final_reduce(const FinalRed &FR, double *sm_m, int *sm_i, int tid, Sync sync) {
-  constexpr int kB = 8;
+// It runs on one CTA of kRedThreads: slot v = 0 .. kRedThreads-1 adds partials v,
+// v + kRedThreads, ... in turn (four 16-byte loads in flight), then a tree over
+// each warp's slots and over the warps.  The next step waits for it, so its
+// latency counts: 128 threads with a tree in shared memory took 3.5 us for
+// 2048 partials.
+constexpr int kRedThreads = 1024;
+__device__ __forceinline__ void final_reduce(const FinalRed &FR) {
+  constexpr int kB = 4;
   static_assert(sizeof(BlockPartial) == 16, "a partial is one 16-byte load");
-  const int n = FR.nparts;
+  __shared__ double s_m[kRedThreads / 32];
+  __shared__ int s_i[kRedThreads / 32];
+  const int tid = threadIdx.x, n = FR.nparts;
   const double2 *P = reinterpret_cast<const double2 *>(FR.partials);
   auto itip_of = [](double2 x) { return (int)(uint32_t)(unsigned long long)__double_as_longlong(x.y); };
-  double m[2] = {0.0, 0.0};
-  int it[2] = {0, 0};
-  int j = 0;
-  for (; (j + kB) * 256 <= n; j += kB) {
-    double2 x[2][kB];
+  double m = 0.0;
+  int it = 0;
+  for (int k = tid; k < n; k += kB * kRedThreads) {
+    double2 x[kB];
 #pragma unroll
-    for (int s = 0; s < 2; ++s)
+    for (int u = 0; u < kB; ++u)
+      x[u] = k + u * kRedThreads < n ? __ldcg(P + k + u * kRedThreads) : make_double2(0.0, 0.0);
 #pragma unroll
-      for (int u = 0; u < kB; ++u) x[s][u] = __ldcg(P + tid + 128 * s + (j + u) * 256);
-#pragma unroll
-    for (int s = 0; s < 2; ++s)
-#pragma unroll
-      for (int u = 0; u < kB; ++u) {
-        m[s] += x[s][u].x;
-        it[s] = max(it[s], itip_of(x[s][u]));
-      }
-  }
-  for (; j * 256 < n; ++j)
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int k = tid + 128 * s + j * 256;
-      if (k < n) {
-        const double2 x = __ldcg(P + k);
-        m[s] += x.x;
-        it[s] = max(it[s], itip_of(x));
-      }
+    for (int u = 0; u < kB; ++u) {
+      m += x[u].x;
+      it = max(it, itip_of(x[u]));
     }
+  }
 #pragma unroll
-  for (int s = 0; s < 2; ++s) {
-    sm_m[tid + 128 * s] = m[s];
-    sm_i[tid + 128 * s] = it[s];
+  for (int o = 16; o > 0; o >>= 1) m += __shfl_down_sync(0xffffffffu, m, o);
+  it = __reduce_max_sync(0xffffffffu, it);
+  if ((tid & 31) == 0) {
+    s_m[tid >> 5] = m;
+    s_i[tid >> 5] = it;
   }
-  sync();
-  for (int sz = 128; sz > 0; sz >>= 1) {
-    if (tid < sz) {
-      sm_m[tid] += sm_m[tid + sz];
-      sm_i[tid] = max(sm_i[tid], sm_i[tid + sz]);
-    }
-    sync();
-  }
+  __syncthreads();
+  if (tid >= 32) return;
+  m = s_m[tid];
+  it = __reduce_max_sync(0xffffffffu, s_i[tid]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m += __shfl_down_sync(0xffffffffu, m, o);
   if (tid == 0) {
-    if (FR.mass_out) *FR.mass_out = sm_m[0] + FR.mass_offset;
-    if (FR.itip_out) *FR.itip_out = max(1, sm_i[0]);  // get_itip_all_grain starts at 1
-    if (FR.counter) *FR.counter = 0u;
+    if (FR.mass_out) *FR.mass_out = m + FR.mass_offset;
+    if (FR.itip_out) *FR.itip_out = max(1, it);  // get_itip_all_grain starts at 1
   }
 }
 
@@ -152,7 +140,7 @@ struct TmaMaps {
   double *col_tab64;  // kColTabFields arrays of col_tab64_len doubles (FP64 step)
   int col_tab64_len;
   const SurrArgs *surr;  // learned CALPHAD surrogate, or nullptr (exact)
-  FinalRed red;          // counter, offset and outputs (partials, nparts set by the launcher)
+  FinalRed red;          // offset and outputs (partials, nparts set by the launcher)
   int pipeline;          // the persistent warp-role kernel instead of one tile per CTA
   int rows;              // output rows of a tile (the maps' boxes are two rows higher)
 };
@@ -163,6 +151,7 @@ constexpr int kTmaBoxW64 = kTileOutW64 + 8;      // its input columns
 constexpr int kTileRows = 16;    // output rows of a tile
 constexpr int kTmaBoxH = kTileRows + 2;  // input rows of a tile
 int tile_rows_f64(int nx, int ny, bool tfc);  // output rows of an FP64 tile: 4, 8 or 16
+int tile_rows_f32(int nx, int ny, bool tfc, bool network);  // and of an FP32 tile
 constexpr int kTfcTileRows32 = 8;        // output rows of an FP32 coarse-grid-temperature tile
 constexpr int kColTabFields = 5;
 // length of the per-column table (entry k is column k - 4) for nx_all columns
@@ -191,7 +180,7 @@ int launch_step_f32_tma(const StepCoef &K, const Coef<float> &F, const StepScala
 int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScalars &P, const TmaMaps &tm,
                         double *psi_n, double *c_n, double *phi_n, BlockPartial *partials, int max_partials,
                         int *nparts_out, int *err, cudaStream_t st);
-// The final reduction of FR (counter unused) as a programmatic dependent of
+// The final reduction of FR as a programmatic dependent of
 // the kernel just launched on st, which wrote the partials: it is scheduled
 // while that kernel runs and waits for its completion on the device
 // (griddepcontrol.wait), so no host-side launch gap follows the step.  (A

@@ -7,30 +7,40 @@
 //     temperature (t_terms in FP64, get_delta fun.cu:1610-1619), rounded to
 //     FP32, plus the FP64 column differences of the composition-independent
 //     part of mu;
-//   * tile_kernel, launched as a programmatic dependent of the table kernel:
-//     its CTAs start, issue their TMA loads, and wait for the table only
-//     where they first read it.
+//   * tile_kernel.
+// Both are programmatic dependent launches: they are scheduled while the
+// kernel before them drains and wait for it on the device, so a run's steps
+// follow one another without launch gaps.
 //
-// A CTA of 128 threads owns a tile of 16 output rows x 128 output columns
-// (x0 .. x0+127, x0 a multiple of 128).  Its input, 18 rows x 136 columns
-// (x0-4 .. x0+131, so the TMA x coordinate stays 16-byte aligned), arrives in
-// shared memory by one TMA box per field.  Four adjacent columns per lane.
-//   phase 1  per-cell S = q(psi) c (1-c) and mu'' (below) of the 18 input
+// A CTA of 128 threads owns a tile of TR output rows x 128 output columns
+// (x0 .. x0+127, x0 a multiple of 128; TR = 4, 8 or 16 by tile_rows_f32, 32 in
+// ensembles too).  Its input, TR + 2 rows x 136 columns (x0-4 .. x0+131, so the
+// TMA x coordinate stays 16-byte aligned), arrives in shared memory by one TMA
+// box per field.  Four adjacent columns per lane.  The CTA votes on the tile's
+// form: a tile of far melt takes its c update from registers straight to
+// global memory, one of deep solid is copied; any other takes the phases:
+//   phase 1  per-cell S = q(psi) c (1-c) and mu'' (below) of the input
 //            rows into shared memory, with per-row flags "every psi == -1" /
 //            "== +1" and per-lane phi masks; the halo columns x0-1 and
 //            x0+128 are computed by 36 threads of warps 2 and 3 (one input
 //            row fewer than warps 0 and 1);
-//   phase 2  each warp computes 4 output rows: fluxes through the faces from
+//   phase 2  each warp computes its output rows: fluxes through the faces from
 //            the shared S and mu'', the c update (kept in registers); cells
-//            whose 3x3 phi neighbourhood is not uniformly +-1 are listed;
+//            whose 3x3 phi neighbourhood is not uniformly +-1 are listed,
+//            those that draw noise apart from the others;
 //   phase 3  the listed interface cells are updated one per thread
 //            (phi_cell), so a tile's interface work is spread over the CTA;
 //   phase 4  new psi and c are written into the shared tile, ghost columns
 //            copied there, and each output row leaves by one bulk async copy
 //            per field (ghost rows by one more, except in row-band mode);
 //   partials when the caller wants the solute mass or the coarse tip, each
-//            CTA writes its partial sums and the last CTA to finish reduces
-//            them all (same order as the separate reduction kernel).
+//            CTA writes its partial sums and a dependent launch reduces them.
+// What bounds it: a 2048^2 grid ahead of a planar front (20.6 us a step, 23.7
+// without the melt form and the chained launches; floor 10.3, a plain copy of
+// its fields by this tiling 17.3) its instruction issue (1100 instructions a
+// warp for 512 cells of far melt, half of them arithmetic) and the chain of a
+// CTA; small grids (256^2: 6.1 us, 12.0 with 16-row tiles) and fronts the chain
+// of the phases.
 // Arithmetic:
 //   * mu = K(T) + C0(T) + mu'' with C0 = -D - (L0_BCC - L0_Liq)(1 - 2 cinf)/2
 //     (D, K(T) as in rs_step.cu), so
@@ -53,10 +63,10 @@
 //     row-band mode).
 // Launch order: the tile columns from the one holding the front
 // (front_first_block), whose interface and network work is the slowest.
-// After phase 1 each CTA prefetches into L2 the input tile of the block
-// launched one resident wave later, so the tiles of the next wave arrive
-// while this wave computes (the CTAs of a wave otherwise load, compute and
-// store in step).
+// Once its own tile has arrived each CTA prefetches into L2 the input tile of
+// the block launched one resident wave later, so the tiles of the next wave
+// arrive while this wave computes (the CTAs of a wave otherwise load, compute
+// and store in step).
 // The coarse-grid temperature (TFC, interpolate_temperature fun.cu:1580-1608)
 // takes tile_kernel_tfc alone: every cell evaluates its CALPHAD groups from its
 // own bilinear temperature (K + C0 by its Taylor polynomial about the tile's
@@ -104,7 +114,9 @@ struct alignas(128) TileSmemT {
   alignas(16) float mu[kRin][kWin];
   // TFC: K + C0 of every cell in FP64 (the face terms are its differences)
   alignas(16) double kc[TFC ? kRin : 1][TFC ? kWin : 2];
-  uint16_t list[TR * kW];   // interface cells: row << 8 | output column
+  // interface cells (row << 8 | output column): those that draw noise from the
+  // front, the others from the back, so that phase 3's warps are of one kind
+  uint16_t list[TR * kW];
   uint8_t pmask[kRin][32];  // per lane: bits 0-3 psi <= -1, bits 4-7 psi >= 1 of its four cells
   uint8_t hmask[kRin][2];   // halo cells: bit 0 psi <= -1, bit 1 psi >= 1
   Mask liq, sol;            // bit r: every cell of input row r has psi == -1 / +1
@@ -113,19 +125,17 @@ struct alignas(128) TileSmemT {
   std::conditional_t<TFC, KcPoly, char> kp;  // TFC: K + C0 near the tile's temperature
   double hx[2];             // TFC: column part of the halo columns' temperatures
   int hiT[2];
-  int nlist;
+  uint32_t nlist;  // how many of the first kind, and << 16 of the second
+  uint32_t vote;   // the tile's form, OR of every thread's
   double part_mass[kWarps];
   int part_itip[kWarps];
   uint64_t full;
-  int last;  // this CTA finished last (fused final reduction)
 };
 using TileSmem = TileSmemT<kTR>;
 
 static_assert(offsetof(TileSmem, psi) % 128 == 0 && offsetof(TileSmem, d) % 128 == 0 &&
                   offsetof(TileSmemT<8>, d) % 128 == 0 && offsetof(TileSmemT<32>, d) % 128 == 0,
               "TMA destinations start on 128-byte boundaries");
-static_assert(sizeof(TileSmemT<8>::S) >= 256 * sizeof(double) && sizeof(TileSmemT<8>::mu) >= 256 * sizeof(int),
-              "the final reduction's scratch fits S and mu");
 static_assert((kWin * sizeof(float)) % 16 == 0, "rows stay 16-byte aligned for float4 and bulk copies");
 
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
@@ -148,6 +158,50 @@ __device__ __forceinline__ void cell_terms(const Coef<float> &F, float pv, float
   mu = -(g + 1.f) * C0 - dv * fmaf(2.f * L0half, g, L0sum) + RT * lam;
 }
 
+// A far-melt cell (psi = -1 exactly, |delta| <= melt_tiny): g = -1, q = 1, lam
+// by its Taylor polynomial in delta (Coef::melt_a);
+// mu'' = RT lam - 2 L0_Liq delta = delta (RT p + KL), lam = delta p.  Rounded
+// products: the phases and the melt tiles give the same bits.
+// M: its constants in registers (an ensemble's live in global memory, where
+// the tile's own stores would have them read again for every row)
+struct MeltC {
+  float cinf, tiny, a0, a1, a2, a3;
+  __device__ explicit MeltC(const Coef<float> &F)
+      : cinf(F.cinf), tiny(F.melt_tiny), a0(F.melt_a[0]), a1(F.melt_a[1]), a2(F.melt_a[2]), a3(F.melt_a[3]) {}
+};
+__device__ __forceinline__ void far_cell(const MeltC &M, float dv, float RT, float &S, float &mu) {
+  constexpr float KL = (float)(-2.0 * kL0Liq);
+  const float c = M.cinf + dv, om = 1.f - c;
+  float p = fmaf(M.a3, dv, M.a2);
+  p = fmaf(p, dv, M.a1);
+  p = fmaf(p, dv, M.a0);
+  S = __fmul_rn(c, om);
+  mu = __fmul_rn(dv, fmaf(RT, p, KL));
+}
+// A bulk-melt cell (psi = -1 exactly, delta in the series range): mu'' =
+// -2 L0_Liq delta + RT 2 atanh(s), atanh to s^7 (relative truncation below
+// 2.6e-9 for |s| < 1/9).
+__device__ __forceinline__ void bulk_cell(const MeltC &M, float dv, float RT, float &S, float &mu) {
+  constexpr float KL = (float)(-2.0 * kL0Liq);
+  const float c = M.cinf + dv, om = 1.f - c;
+  const float sv = __fdividef(dv, fmaf(M.cinf + M.cinf, om, dv));
+  const float s2 = sv * sv;
+  float p = fmaf(s2, 1.f / 7.f, 1.f / 5.f);
+  p = fmaf(s2, p, 1.f / 3.f);
+  const float ath = fmaf(sv * s2, p, sv);  // atanh(s); lam = 2 atanh(s)
+  S = __fmul_rn(c, om);
+  mu = fmaf(RT + RT, ath, __fmul_rn(dv, KL));
+}
+// a cell of the halo columns: the far-melt form where the cell has it, else
+// the general one (a cell's form does not depend on the tile)
+__device__ __forceinline__ void halo_cell(const Coef<float> &F, const MeltC &M, float pv, float dv, float RT, float C0,
+                                          float &S, float &mu) {
+  if (__float_as_uint(pv) == 0xBF800000u && fabsf(dv) <= M.tiny)
+    far_cell(M, dv, RT, S, mu);
+  else
+    cell_terms(F, pv, dv, RT, C0, S, mu);
+}
+
 // shared -> global bulk copy (16-byte aligned addresses, size a multiple of 16)
 __device__ __forceinline__ void bulk_store(void *gdst, const void *ssrc, uint32_t bytes) {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gdst), "r"(smem_u32(ssrc)),
@@ -160,6 +214,8 @@ __device__ __forceinline__ void bulk_store(void *gdst, const void *ssrc, uint32_
 // neighbouring thread, so blocks overlap by one column and write 127 entries.
 constexpr int kTabBlock = 128;
 // kc: kTabBlock doubles of shared scratch
+// (griddepcontrol.wait before the table is written: the previous step's tiles
+// have read it)
 __device__ __forceinline__ void table_block(const StepCoef &K, const double d0, const double d1, const int len,
                                             float *__restrict__ tab, const int blk, double *kc) {
   const int k = blk * (kTabBlock - 1) + threadIdx.x;  // table entry; column k - 4
@@ -170,6 +226,7 @@ __device__ __forceinline__ void table_block(const StepCoef &K, const double d0, 
   const double C0 = -D - 0.5 * (kL0Bcc - kL0Liq) * (1.0 - 2.0 * K.cinf);
   kc[threadIdx.x] = 0.5 * (tt.dGs + tt.dGl) + 0.5 * (kL0Bcc + kL0Liq) * (1.0 - 2.0 * K.cinf) + tt.RT * K.Lref + C0;
   __syncthreads();
+  pdl_wait();
   if (threadIdx.x == kTabBlock - 1 || k >= len) return;
   tab[kTabRT * len + k] = (float)tt.RT;
   tab[kTabC0 * len + k] = (float)C0;
@@ -200,7 +257,7 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
                                           const float *__restrict__ tab, const int tab_len, float *__restrict__ psi_n,
                                           float *__restrict__ c_n, float *__restrict__ phi_n, BlockPartial *part,
                                           int *err, const SurrArgs &SA, const int tr, const int tc,
-                                          const FinalRed *FR, const Prefetch &prefetch) {
+                                          const Prefetch &prefetch) {
   // the tile's shape (these hide the single-run constants of the same names)
   constexpr int kTR = TR, kTRin = TR + 2, kRowsPerWarp = TR / kWarps;
   static_assert(TR % kWarps == 0 && kRowsPerWarp * 4 <= 32, "output rows split evenly over the warps");
@@ -229,14 +286,10 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
   if (threadIdx.x == 0) {
     mbar_init(&sm.full, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if (!pb) {
-      mbar_expect_tx(&sm.full, kTileBytes);
-      tma_load_2d(&sm.psi[0][0], tm_psi, &sm.full, x0 - 4, y0 - 1);
-      tma_load_2d(&sm.d[0][0], tm_c, &sm.full, x0 - 4, y0 - 1);
-    }
     sm.liq = 0;
     sm.sol = 0;
-    sm.nlist = 0;
+    sm.nlist = 0u;
+    sm.vote = 0u;
   }
 
   const int col = 4 * lane;  // tile column of this lane's first cell
@@ -249,19 +302,23 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
   // launch constants of the row loops in registers (one read of the
   // arguments, which may live in global memory for the ensemble)
   const int ny = K.ny, nx = K.nx;
-  const float cinf = F.cinf, tiny = F.melt_tiny;
-  const float ma0 = F.melt_a[0], ma1 = F.melt_a[1], ma2 = F.melt_a[2], ma3 = F.melt_a[3];
-  const float two_cinf = F.cinf + F.cinf;
+  const MeltC M(F);
+  const float tiny = M.tiny;
   const float cflux4 = 0.25f * F.cflux;
   const float floor_d = F.c_floor - F.cinf;
-  constexpr float KL = (float)(-2.0 * kL0Liq);
   const float d_hi = F.ser_hi, d_lo = F.ser_lo;  // series range of delta (Coef)
   constexpr uint32_t kMinus1 = 0xBF800000u, kPlus1 = 0x3F800000u;
 
-  // the column table of this step (programmatic dependency on its kernel)
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  // the step's final reduction (a programmatic dependent) may be scheduled now
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // the kernel before this one in the stream (the column table's, and with it
+  // every earlier one) has completed: its table and the fields are visible
+  pdl_wait();
+  if (threadIdx.x == 0 && !pb) {
+    mbar_expect_tx(&sm.full, kTileBytes);
+    tma_load_2d(&sm.psi[0][0], tm_psi, &sm.full, x0 - 4, y0 - 1);
+    tma_load_2d(&sm.d[0][0], tm_c, &sm.full, x0 - 4, y0 - 1);
+  }
+  // dependents of this step (its reduction, the next step) may be scheduled now
+  pdl_trigger();
   const float *tRT = tab + kTabRT * tab_len + 4, *tC0 = tab + kTabC0 * tab_len + 4;
   const float *tDK = tab + kTabDK * tab_len + 4;
   float4 RTv = make_float4(0.f, 0.f, 0.f, 0.f), C0v = RTv, dKv = RTv;
@@ -381,8 +438,7 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
       }
     }
   };
-  // the partial sums of this tile and the fused final reduction (the last
-  // CTA to finish sums every partial, in reduce_partials_kernel's order)
+  // the partial sums of this tile (a dependent launch reduces them)
   auto finish = [&](double mass, int itip) {
     if (!part) return;
 #pragma unroll
@@ -405,17 +461,6 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
       b.pad = 0;
       *part = b;
     }
-    if (!FR) return;
-    if (threadIdx.x == 0) {
-      __threadfence();
-      sm.last = atomicAdd(FR->counter, 1u) == (unsigned)(FR->nparts - 1);
-    }
-    __syncthreads();
-    if (!sm.last) return;
-    __threadfence();
-    double *sm_m = reinterpret_cast<double *>(&sm.S[0][0]);  // S and mu are free now
-    int *sm_i = reinterpret_cast<int *>(&sm.mu[0][0]);
-    final_reduce(*FR, sm_m, sm_i, (int)threadIdx.x, [] { __syncthreads(); });
   };
   if (pb) {
     const float *__restrict__ gpsi = static_cast<const float *>(PS.src_psi);
@@ -435,43 +480,215 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     }
   }
   __syncthreads();  // barrier initialised, flags cleared (a pull-back tile gathered)
-  if (!pb) {
-    // bounded wait for the tile; if any thread gives up, the whole CTA skips
-    // the tile: no phase runs on a partly filled tile and nothing is stored.
-    // Thread 0 first waits (bounded again) for the load still in flight into
-    // this CTA's shared memory, and the CTA still reports a (zero) partial,
-    // so the fused final reduction keeps its count
+  bool gave_up = false;
+  if (!pb) {  // bounded wait for the tile
     const uint32_t limit = PS.wait_limit ? PS.wait_limit : kWaitLimit;
     uint32_t tries = 0;
-    bool gave_up = false;
     while (!mbar_try(&sm.full, 0, PS.wait_limit != 0)) {
       if (++tries >= limit) {
         gave_up = true;
         break;
       }
     }
-    if (__syncthreads_or(gave_up)) {
-      if (threadIdx.x == 0) {
-        atomicExch(err, 1);
-        for (uint32_t t = 0; t < kWaitLimit && !mbar_try_wait(&sm.full, 0); ++t) {
-        }
-      }
-      __syncthreads();
-      finish(0.0, 0);
-      return;
-    }
+    // pull the tile of the CTA that will start about one resident wave later
+    // into L2, so its loads overlap the rest of this wave's arithmetic
+    if (threadIdx.x == 0 && !gave_up) prefetch();
   }
   // columns beyond the array (right-most tiles; zero-filled by TMA) become
   // bulk melt, so they never force the general path; no output reads them
-  if (x0 + kW + 4 > K.nx) {
-    for (int k = threadIdx.x; k < kTRin * kWin; k += kThreads) {
-      const int rr = k / kWin, x = k % kWin;
-      if (x0 - 4 + x >= K.nx) {
-        sm.psi[rr][x] = -1.f;
-        sm.d[rr][x] = 0.f;
+  // (a thread that gave up leaves the tile alone)
+  if (x0 + kW + 4 > nx) {
+    if (!gave_up)
+      for (int k = threadIdx.x; k < kTRin * kWin; k += kThreads) {
+        const int rr = k / kWin, x = k % kWin;
+        if (x0 - 4 + x >= nx) {
+          sm.psi[rr][x] = -1.f;
+          sm.d[rr][x] = 0.f;
+        }
+      }
+    __syncthreads();
+  }
+  // ---- the tile's form: far melt (psi = -1 exactly, |delta| <= melt_tiny; melt
+  // in the series range too, with its rows' votes, cost the far melt more than
+  // it gained: 2048^2 all melt 18.3 -> 19.5 us) or deep solid (psi = +1 exactly) in every cell of the box that an output reads
+  // (rows and columns outside the array are left out) needs no masks, list or
+  // interface pass
+  constexpr uint32_t kNotMinus1 = 1u, kNotPlus1 = 2u, kNotFar = 4u, kNotFinite = 8u, kGaveUp = 16u;
+  {
+    uint32_t m1 = 0u, p1 = 0u, dm = 0u;  // OR of psi's difference from -1 / +1, largest |delta| (bits)
+    auto cell = [&](float p, float d) {
+      m1 |= __float_as_uint(p) ^ kMinus1;
+      p1 |= __float_as_uint(p) ^ kPlus1;
+      dm = max(dm, __float_as_uint(d) & 0x7fffffffu);
+    };
+    uint32_t bad = kGaveUp;
+    if (!gave_up) {
+#pragma unroll
+      for (int k = 0; k < (kTRin + kWarps - 1) / kWarps; ++k) {
+        const int rr = warp + kWarps * k;
+        if (rr < kTRin && rr <= ny - y0) {
+          const float4 p4 = ld4(&sm.psi[rr][bc]), d4 = ld4(&sm.d[rr][bc]);
+          cell(p4.x, d4.x);
+          cell(p4.y, d4.y);
+          cell(p4.z, d4.z);
+          cell(p4.w, d4.w);
+        }
+      }
+      if (threadIdx.x >= kHalo0 && threadIdx.x < kHalo0 + 2 * kTRin) {  // the halo columns, one cell per thread
+        const int rr = ((int)threadIdx.x - kHalo0) >> 1, side = ((int)threadIdx.x - kHalo0) & 1;
+        const int x = side ? kHaloR : kHaloL;
+        if (rr <= ny - y0 && (side || x0 > 0)) cell(sm.psi[rr][x], sm.d[rr][x]);
+      }
+      bad = (m1 ? kNotMinus1 : 0u) | (p1 ? kNotPlus1 : 0u) | (dm <= __float_as_uint(tiny) ? 0u : kNotFar) |
+            (dm < 0x3F800000u ? 0u : kNotFinite);
+    }
+    bad = __reduce_or_sync(FULL, bad);
+    if (lane == 0 && bad) atomicOr(&sm.vote, bad);
+  }
+  __syncthreads();
+  const uint32_t vote = sm.vote;
+  const bool red = part != nullptr;
+  double mass = 0.0;
+  int itip = 0;
+  if (vote & kGaveUp) {
+    // if any thread gives up, the whole CTA skips the tile: nothing is
+    // computed on a partly filled tile or stored.  Thread 0 first waits
+    // (bounded again) for the load still in flight into this CTA's shared
+    // memory, and the CTA still reports a (zero) partial
+    if (threadIdx.x == 0) {
+      atomicExch(err, 1);
+      for (uint32_t t = 0; t < kWaitLimit && !mbar_try_wait(&sm.full, 0); ++t) {
       }
     }
     __syncthreads();
+    finish(0.0, 0);
+    return;
+  }
+  const bool melt = !TFC && !(vote & (kNotMinus1 | kNotFar));
+  if (melt || !(vote & (kNotPlus1 | kNotFinite))) {
+    // the warp's output rows straight from registers to global memory, with
+    // the ghost columns and rows they copy to (nx is a multiple of 4: a lane's
+    // cells are all inside the array or all beyond it)
+    const int r0 = kRowsPerWarp * warp;  // input row before the warp's first output row
+    const int64_t o0 = (int64_t)(y0 + r0) * K.pitch + gi;
+    const bool inside = gi < nx, ghost = (K.jmin >= y0 + r0 && K.jmin < y0 + r0 + kRowsPerWarp) ||
+                                         (K.jmax >= y0 + r0 && K.jmax < y0 + r0 + kRowsPerWarp);
+    const float pv = melt ? -1.f : 1.f;
+    auto put = [&](int j, float (&v)[4]) {
+      if (gi == 0) v[0] = v[1];         // ghost column 0
+      if (gi + 4 == nx) v[3] = v[2];    // ghost column nx-1
+      if (!inside) return;
+      auto row = [&](int64_t o) {
+        st4(psi_n + o, pv, pv, pv, pv);
+        st4(c_n + o, v[0], v[1], v[2], v[3]);
+        if (phi_n) st4(phi_n + o, pv, pv, pv, pv);
+      };
+      row(o0 + (int64_t)j * K.pitch);
+      if (ghost) {
+        if (y0 + r0 + j == K.jmin) row(gi);
+        if (y0 + r0 + j == K.jmax) row((int64_t)(ny - 1) * K.pitch + gi);
+      }
+    };
+    if (!melt) {  // deep solid: S = 0 in every cell, so every flux is 0 and psi and c stay
+#pragma unroll
+      for (int j = 0; j < kRowsPerWarp; ++j) {
+        if (y0 + r0 + j > ny - 2) break;
+        const float4 d4 = ld4(&sm.d[r0 + 1 + j][bc]);
+        float v[4] = {fmaxf(d4.x, floor_d), fmaxf(d4.y, floor_d), fmaxf(d4.z, floor_d), fmaxf(d4.w, floor_d)};
+        if (red) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if ((outm >> q) & 1u) {
+              mass += (double)v[q];
+              itip = max(itip, gi + q == nx - 2 ? nx - 1 : gi + q);
+            }
+        }
+        put(j, v);
+      }
+      finish(mass, itip);
+      return;
+    }
+    if constexpr (!TFC) {
+      // far melt: phases 1 and 2 with S and mu'' of the warp's rows in
+      // registers (the same expressions, so the same bits); halo columns by a
+      // lane per cell through scratch
+      float *hs = &sm.S[warp][0], *hm = &sm.mu[warp][0];
+      if (lane < 2 * (kRowsPerWarp + 2)) {
+        const int rr = r0 + (lane >> 1), x = (lane & 1) ? kHaloR : kHaloL;
+        float Sh = 0.f, mh = 0.f;
+        if (rr <= ny - y0) far_cell(M, sm.d[rr][x], tRT[x0 - 4 + x], Sh, mh);
+        hs[lane] = Sh;
+        hm[lane] = mh;
+      }
+      __syncwarp();
+      if constexpr (SURR) {
+        dKv = ld4(tDK + gi);
+        dKl = tDK[gi - 1];
+      }
+      const float dKm[5] = {dKl, dKv.x, dKv.y, dKv.z, dKv.w};
+      struct MRow {
+        float s[4], m[4], d[4], sl, sr, ml, mr, q[5];
+      };
+      auto melt_row = [&](int k, MRow &R) {
+        const float4 d4 = ld4(&sm.d[r0 + k][bc]);
+        R.d[0] = d4.x; R.d[1] = d4.y; R.d[2] = d4.z; R.d[3] = d4.w;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) far_cell(M, R.d[q], RTa[q], R.s[q], R.m[q]);
+        R.sl = __shfl_up_sync(FULL, R.s[3], 1);
+        R.ml = __shfl_up_sync(FULL, R.m[3], 1);
+        R.sr = __shfl_down_sync(FULL, R.s[0], 1);
+        R.mr = __shfl_down_sync(FULL, R.m[0], 1);
+        if (lane == 0) {
+          R.sl = hs[2 * k];
+          R.ml = hm[2 * k];
+        }
+        if (lane == 31) {
+          R.sr = hs[2 * k + 1];
+          R.mr = hm[2 * k + 1];
+        }
+        R.q[0] = R.sl + R.s[0];
+        R.q[1] = R.s[0] + R.s[1];
+        R.q[2] = R.s[1] + R.s[2];
+        R.q[3] = R.s[2] + R.s[3];
+        R.q[4] = R.s[3] + R.sr;
+      };
+      auto melt_face = [&](const MRow &A, const MRow &B, float jv[4]) {
+        const float pp[6] = {A.sl + B.sl,         A.s[0] + B.s[0], A.s[1] + B.s[1],
+                             A.s[2] + B.s[2], A.s[3] + B.s[3], A.sr + B.sr};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) jv[q] = __fmul_rn(fmaf(6.f, pp[q + 1], pp[q] + pp[q + 2]), B.m[q] - A.m[q]);
+      };
+      MRow a, b, c;
+      float lo[4], hi[4];
+      melt_row(0, a);
+      melt_row(1, b);
+      melt_face(a, b, lo);
+#pragma unroll
+      for (int j = 0; j < kRowsPerWarp; ++j) {
+        melt_row(j + 2, c);
+        melt_face(b, c, hi);
+        const float mm[6] = {b.ml, b.m[0], b.m[1], b.m[2], b.m[3], b.mr};
+        float jh[5], v[4];
+#pragma unroll
+        for (int f = 0; f < 5; ++f) jh[f] = __fmul_rn(fmaf(6.f, b.q[f], a.q[f] + c.q[f]), mm[f + 1] - mm[f] + dKm[f]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = fmaxf(fmaf(cflux4, (jh[q + 1] - jh[q]) + (hi[q] - lo[q]), b.d[q]), floor_d);
+        if (y0 + r0 + j <= ny - 2) {
+          if (red) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if ((outm >> q) & 1u) mass += (double)v[q];
+          }
+          put(j, v);
+        }
+        a = b;
+        b = c;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) lo[q] = hi[q];
+      }
+      finish(mass, 0);
+      return;
+    }
   }
 
   // ---- phase 1: per-cell terms; warp w takes input rows w, w+4, ...
@@ -527,28 +744,11 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
       // mu'' = RT lam - 2 L0_Liq delta = delta (RT p + KL), lam = delta p
       code = 1u | 4u;  // 4: every cell in the exact melt form
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float c = cinf + dv[q], om = 1.f - c;
-        float p = fmaf(ma3, dv[q], ma2);
-        p = fmaf(p, dv[q], ma1);
-        p = fmaf(p, dv[q], ma0);
-        Sv[q] = c * om;
-        mv[q] = dv[q] * fmaf(RTa[q], p, KL);
-      }
+      for (int q = 0; q < 4; ++q) far_cell(M, dv[q], RTa[q], Sv[q], mv[q]);
     } else if (TFC ? bulk : __all_sync(FULL, liq4 && dmx < d_hi && dmn > d_lo)) {
       code = 1u | 4u;  // 4: every cell in the series form
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float c = cinf + dv[q], om = 1.f - c;
-        const float sv = __fdividef(dv[q], fmaf(two_cinf, om, dv[q]));
-        const float s2 = sv * sv;
-        // atanh(s) to s^7: relative truncation below 2.6e-9 for |s| < 1/9
-        float p = fmaf(s2, 1.f / 7.f, 1.f / 5.f);
-        p = fmaf(s2, p, 1.f / 3.f);
-        const float ath = fmaf(sv * s2, p, sv);  // atanh(s); lam = 2 atanh(s)
-        Sv[q] = c * om;
-        mv[q] = fmaf(RTa[q] + RTa[q], ath, dv[q] * KL);
-      }
+      for (int q = 0; q < 4; ++q) bulk_cell(M, dv[q], RTa[q], Sv[q], mv[q]);
     } else {
       const bool sol4 = band == kPlus1 && bor == kPlus1;
       code = (__all_sync(FULL, liq4) ? 1u : 0u) | (__all_sync(FULL, sol4) ? 2u : 0u);
@@ -632,9 +832,9 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
         double RT, C0;
         cell_tfc(K, sm.kp, tfc_T(K, PS.T_coarse, sm.hiT[side], sm.hx[side], sm.tj[rr], sm.ty[rr]),
                  __float_as_uint(pv) != kMinus1, RT, C0, kh);
-        cell_terms(F, pv, sm.d[rr][x], (float)RT, (float)C0, Sh, mh);
+        halo_cell(F, M, pv, sm.d[rr][x], (float)RT, (float)C0, Sh, mh);
       } else {
-        cell_terms(F, pv, sm.d[rr][x], tRT[g], tC0[g], Sh, mh);
+        halo_cell(F, M, pv, sm.d[rr][x], tRT[g], tC0[g], Sh, mh);
       }
       hm = (pv <= -1.f ? 1u : 0u) | (pv >= 1.f ? 2u : 0u);
     }
@@ -673,16 +873,9 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
   }
   const float dKa[5] = {dKl, dKv.x, dKv.y, dKv.z, dKv.w};  // faces x-1|x for x = col .. col+4
   __syncthreads();
-  // phase 1 done: pull the tile of the CTA that will start about one resident
-  // wave later into L2, so its loads overlap the rest of this wave's
-  // arithmetic (issued after the own load and phase 1, it measured fastest)
-  if (threadIdx.x == 0 && !pb) prefetch();
 
   // ---- phase 2: warp w computes output rows 1 + 4w .. 4 + 4w of the tile
   const Mask liq = sm.liq, sol = sm.sol;
-  const bool red = part != nullptr;
-  double mass = 0.0;
-  int itip = 0;
   struct Row {
     float s[4], m[4], sl, sr, ml, mr, q[5];  // q[f]: S pair sum of the face left of cell f (f = 0..4)
     double k[4], kl, kr;                     // TFC: K + C0 of the cells and of their neighbours
@@ -806,21 +999,28 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
         Sv &= (S << 1) | ((lf >> (8 * k + 7)) & 1u) | (((rt >> (8 * k + 4)) & 1u) << 5);
       }
       const uint32_t needs = ~((Lv & (Lv >> 1) & (Lv >> 2)) | (Sv & (Sv >> 1) & (Sv >> 2))) & outm;
-      const uint32_t cnt = __popc(needs);
-      uint32_t incl = cnt;  // inclusive warp scan of the counts
+      // cells that draw noise (phi_cell's own test; here it only sorts the list)
+      uint32_t noisy = 0xFu;
+      if (F.noise_amp > 0.f) {
+        const float4 p4 = ld4(&sm.psi[rr][bc]);
+        noisy = (fmaf(-p4.x, p4.x, 1.f) > 1.0e-3f ? 1u : 0u) | (fmaf(-p4.y, p4.y, 1.f) > 1.0e-3f ? 2u : 0u) |
+                (fmaf(-p4.z, p4.z, 1.f) > 1.0e-3f ? 4u : 0u) | (fmaf(-p4.w, p4.w, 1.f) > 1.0e-3f ? 8u : 0u);
+      }
+      // inclusive warp scan of the counts of both kinds (packed as in nlist)
+      const uint32_t cnt = __popc(needs & noisy) | (__popc(needs & ~noisy) << 16);
+      uint32_t incl = cnt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const uint32_t v = __shfl_up_sync(FULL, incl, o);
         if (lane >= o) incl += v;
       }
-      const uint32_t total = __shfl_sync(FULL, incl, 31);
-      int base = 0;
-      if (lane == 31 && total) base = atomicAdd(&sm.nlist, (int)total);
-      base = __shfl_sync(FULL, base, 31);
-      uint32_t off = (uint32_t)base + incl - cnt;
+      uint32_t base = 0u;
+      if (lane == 31 && incl) base = atomicAdd(&sm.nlist, incl);
+      base = __shfl_sync(FULL, base, 31) + incl - cnt;
+      uint32_t n_at = base & 0xFFFFu, t_at = kTR * kW - 1 - (base >> 16);
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if ((needs >> q) & 1u) sm.list[off++] = (uint16_t)((rr << 8) | (col + q));
+        if ((needs >> q) & 1u) sm.list[((noisy >> q) & 1u) ? n_at++ : t_at--] = (uint16_t)((rr << 8) | (col + q));
       needs_all |= needs << (4 * j);
     }
     ra = rb;
@@ -831,7 +1031,8 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
   __syncthreads();
 
   // ---- phase 3: interface cells, one per thread (compute_phi, fun.cu:1143-1218)
-  const int nlist = sm.nlist;
+  const int na = (int)(sm.nlist & 0xFFFFu), nlist = na + (int)(sm.nlist >> 16);
+  auto listed = [&](int idx) { return (uint32_t)sm.list[idx < na ? idx : kTR * kW - 1 - (idx - na)]; };
   if constexpr (SURR) {
     // network driving force of the listed cells, 16 per warp pass, into the
     // mu'' slots of those cells (mu'' is not read after phase 2)
@@ -841,7 +1042,7 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
 #pragma unroll 1
       for (int base = 16 * warp; base < nlist; base += 16 * kWarps) {
         const int ia = base + g, ib = ia + 8;
-        const uint32_t ea = sm.list[min(ia, nlist - 1)], eb = sm.list[min(ib, nlist - 1)];
+        const uint32_t ea = listed(min(ia, nlist - 1)), eb = listed(min(ib, nlist - 1));
         const int ra = (int)(ea >> 8), xa = (int)(ea & 0xFFu) + 4, rb = (int)(eb >> 8), xb = (int)(eb & 0xFFu) + 4;
         float in0[3], in1[3], o0[2], o1[2];
         net_inputs(ra, xa, in0);
@@ -857,7 +1058,7 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     __syncthreads();
   }
   for (int idx = threadIdx.x; idx < nlist; idx += kThreads) {
-    const uint32_t e = sm.list[idx];
+    const uint32_t e = listed(idx);
     const int rr = (int)(e >> 8), x = (int)(e & 0xFFu) + 4;  // box column
     const int r = y0 - 1 + rr, g = x0 + x - 4;
     const float c00 = F.cinf + sm.d[rr][x];
@@ -983,35 +1184,39 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
-template <bool SURR>
+// the tile of the block launched one resident wave later (wave_y tile columns
+// and wave_x tile rows on), into L2
+struct WavePrefetch {
+  const CUtensorMap *psi, *c;
+  int f, wave_x, wave_y, TR;
+  __device__ void operator()() const {
+    int bx = (int)blockIdx.x + wave_x, by = (int)blockIdx.y + wave_y;
+    if (bx >= (int)gridDim.x) {
+      bx -= (int)gridDim.x;
+      ++by;
+    }
+    if (by >= (int)gridDim.y) return;
+    const int pc = front_first_block(by, f, (int)gridDim.y);
+    tma_prefetch_2d(psi, kW * pc - 4, TR * bx);
+    tma_prefetch_2d(c, kW * pc - 4, TR * bx);
+  }
+};
+
+template <bool SURR, int TR>
 __global__ void __launch_bounds__(kThreads, SURR ? 4 : 5)
     tile_kernel(const __grid_constant__ StepCoef K, const __grid_constant__ Coef<float> F,
                 const __grid_constant__ StepScalars PS, const __grid_constant__ CUtensorMap tm_psi,
                 const __grid_constant__ CUtensorMap tm_c, const float *__restrict__ tab, const int tab_len,
                 float *__restrict__ psi_n, float *__restrict__ c_n, float *__restrict__ phi_n, BlockPartial *partials,
-                int *err, const __grid_constant__ SurrArgs SA, const __grid_constant__ FinalRed FR,
-                const int wave) {
+                int *err, const __grid_constant__ SurrArgs SA, const int wave_x, const int wave_y) {
   // blockIdx.x walks the tile rows of one tile column (they share halo rows
   // in L2), blockIdx.y the tile columns, from the one holding column PS.i_front
   const int f = max(PS.i_front, 0) / kW;
   const int tr = blockIdx.x;
   const int tc = front_first_block((int)blockIdx.y, f, (int)gridDim.y);
-  // the block launched `wave` (CTAs resident at once) positions later
-  const unsigned nxt = blockIdx.y * gridDim.x + blockIdx.x + (unsigned)wave;
-  int pf_tr = -1, pf_tc = -1;
-  if (wave > 0 && nxt < gridDim.x * gridDim.y) {
-    pf_tr = (int)(nxt % gridDim.x);
-    pf_tc = front_first_block((int)(nxt / gridDim.x), f, (int)gridDim.y);
-  }
-  auto prefetch = [&]() {
-    if (pf_tc >= 0) {
-      tma_prefetch_2d(&tm_psi, kW * pf_tc - 4, kTR * pf_tr);
-      tma_prefetch_2d(&tm_c, kW * pf_tc - 4, kTR * pf_tr);
-    }
-  };
-  tile_body<SURR, kTR>(K, F, PS, &tm_psi, &tm_c, tab, tab_len, psi_n, c_n, phi_n,
-                  partials ? partials + ((int64_t)tc * gridDim.x + tr) : nullptr, err, SA, tr, tc,
-                  partials && FR.counter ? &FR : nullptr, prefetch);
+  tile_body<SURR, TR>(K, F, PS, &tm_psi, &tm_c, tab, tab_len, psi_n, c_n, phi_n,
+                      partials ? partials + ((int64_t)tc * gridDim.x + tr) : nullptr, err, SA, tr, tc,
+                      WavePrefetch{&tm_psi, &tm_c, f, wave_x, wave_y, TR});
 }
 
 // The coarse-grid temperature (TFC): tiles of kTfcTileRows32 output rows, whose
@@ -1023,27 +1228,15 @@ __global__ void __launch_bounds__(kThreads, 5)
                     const __grid_constant__ StepScalars PS, const __grid_constant__ CUtensorMap tm_psi,
                     const __grid_constant__ CUtensorMap tm_c, const float *__restrict__ tab, const int tab_len,
                     float *__restrict__ psi_n, float *__restrict__ c_n, float *__restrict__ phi_n,
-                    BlockPartial *partials, int *err, const __grid_constant__ FinalRed FR, const int wave) {
+                    BlockPartial *partials, int *err, const int wave_x, const int wave_y) {
   const int f = max(PS.i_front, 0) / kW;
   const int tr = blockIdx.x;
   const int tc = front_first_block((int)blockIdx.y, f, (int)gridDim.y);
-  const unsigned nxt = blockIdx.y * gridDim.x + blockIdx.x + (unsigned)wave;
-  int pf_tr = -1, pf_tc = -1;
-  if (wave > 0 && nxt < gridDim.x * gridDim.y) {
-    pf_tr = (int)(nxt % gridDim.x);
-    pf_tc = front_first_block((int)(nxt / gridDim.x), f, (int)gridDim.y);
-  }
-  auto prefetch = [&]() {
-    if (pf_tc >= 0) {
-      tma_prefetch_2d(&tm_psi, kW * pf_tc - 4, kTfcTR * pf_tr);
-      tma_prefetch_2d(&tm_c, kW * pf_tc - 4, kTfcTR * pf_tr);
-    }
-  };
   const SurrArgs none = {};
-  tile_body<false, kTfcTR, decltype(prefetch), true>(
+  tile_body<false, kTfcTR, WavePrefetch, true>(
       K, F, PS, &tm_psi, &tm_c, tab, tab_len, psi_n, c_n, phi_n,
       partials ? partials + ((int64_t)tc * gridDim.x + tr) : nullptr, err, none, tr, tc,
-      partials && FR.counter ? &FR : nullptr, prefetch);
+      WavePrefetch{&tm_psi, &tm_c, f, wave_x, wave_y, kTfcTR});
 }
 
 // ---------------------------------------------------------------- ensemble
@@ -1061,6 +1254,8 @@ __device__ __forceinline__ double ens_d0(const EnsRun &R, const double l) {
 
 __global__ void __launch_bounds__(kTabBlock) ens_table_kernel(const EnsRun *__restrict__ runs,
                                                               const int32_t *__restrict__ tblk) {
+  pdl_wait();  // the runs' state
+  pdl_trigger();
   const int32_t e = tblk[blockIdx.x];
   const EnsRun &R = runs[e >> 16];
   if (!R.active) return;
@@ -1076,6 +1271,7 @@ template <bool SURR, int SHAPE>
 __global__ void __launch_bounds__(kThreads, min_ctas(SURR, shape_rows(SHAPE)))
     ens_tile_kernel(const EnsRun *__restrict__ runs, const int32_t *__restrict__ order, int *err, const int wave) {
   constexpr int TR = shape_rows(SHAPE);
+  pdl_wait();  // the runs' state
   const int32_t e = order[blockIdx.x];
   const EnsRun &R = runs[e >> 16];
   if (!R.active) return;
@@ -1100,11 +1296,12 @@ __global__ void __launch_bounds__(kThreads, min_ctas(SURR, shape_rows(SHAPE)))
   };
   const int nrt = R.nrt[SHAPE];
   tile_body<SURR, TR>(R.K, R.F, PS, &R.map_psi[SHAPE][par], &R.map_c[SHAPE][par], R.tab, R.tab_len, R.psi[par ^ 1],
-                      R.c[par ^ 1], nullptr, nullptr, err, SURR ? R.surr : none, t % nrt, t / nrt, nullptr,
-                      prefetch);
+                      R.c[par ^ 1], nullptr, nullptr, err, SURR ? R.surr : none, t % nrt, t / nrt, prefetch);
 }
 
 __global__ void ens_advance_kernel(EnsRun *runs, const int nruns) {
+  pdl_wait();
+  pdl_trigger();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= nruns || !runs[r].active) return;
   runs[r].step += 1;
@@ -1189,7 +1386,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas(SURR, shape_rows(SHAPE)))
         const int nrt = R.nrt[SHAPE];
         tile_body<SURR, TR>(R.K, R.F, PS, &R.map_psi[SHAPE][par], &R.map_c[SHAPE][par], R.tab, R.tab_len,
                             R.psi[par ^ 1], R.c[par ^ 1], nullptr, nullptr, err, SURR ? R.surr : none, t % nrt,
-                            t / nrt, nullptr, prefetch);
+                            t / nrt, prefetch);
         __syncthreads();  // every thread is done with the tile's barrier and shared memory
         if (threadIdx.x == 0) mbar_inval(&sm.full);
         if (__syncthreads_or(*(volatile int *)err != 0)) dead = true;
@@ -1217,36 +1414,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas(SURR, shape_rows(SHAPE)))
 // doing phases 2-4 of tile k and its bulk stores; mbarrier hand-offs, named
 // barriers per group, every wait bounded.  Same arithmetic, expression for
 // expression, as tile_body.
-struct alignas(128) InSlot32 {  // both arrays are TMA destinations: 128-byte aligned
-  alignas(128) float psi[kTRin][kWin];
-  alignas(128) float d[kTRin][kWin];
-};
-struct alignas(16) StSlot32 {
-  float S[kTRin][kWin];  // after phase 2: new psi of the listed cells
-  float mu[kTRin][kWin];
-  uint8_t pmask[kTRin][32];  // per lane: bits 0-3 psi <= -1, bits 4-7 psi >= 1 of its four cells
-  uint8_t hmask[kTRin][2];   // halo cells: bit 0 psi <= -1, bit 1 psi >= 1
-  uint32_t liq, sol;         // bit r: every cell of input row r has psi == -1 / +1
-};
-struct P2Smem32 {
-  uint16_t list[kTR * kW];  // interface cells: row << 8 | output column
-  int nlist;
-  int last;
-  double part_mass[kWarps];
-  int part_itip[kWarps];
-};
 constexpr int kRing = 3, kStage = 2;
-struct alignas(128) PipeSmem32 {
-  InSlot32 in[kRing];
-  StSlot32 st[kStage];
-  P2Smem32 p2;
-  uint64_t in_full[kRing], in_empty[kRing], st_full[kStage], st_empty[kStage];
-  int abort;
-};
-static_assert(sizeof(InSlot32) % 128 == 0 && offsetof(InSlot32, psi) % 128 == 0 && offsetof(InSlot32, d) % 128 == 0,
-              "ring slots and their TMA destinations stay 128-byte aligned");
-static_assert(offsetof(PipeSmem32, in) % 128 == 0, "the ring starts on a 128-byte boundary");
-constexpr uint32_t kTileBytes32 = 2u * kTRin * kWin * sizeof(float);
 constexpr uint32_t kMinus1f = 0xBF800000u, kPlus1f = 0x3F800000u;
 constexpr int kPipeThreads = 32 + 2 * kThreads;
 enum { kBarP1 = 1, kBarP2 = 2 };
@@ -1281,6 +1449,34 @@ __device__ __forceinline__ bool pipe_wait(uint64_t *bar, uint32_t parity, volati
   return true;
 }
 
+template <int TR>
+struct Pipe32 {
+static constexpr int kTR = TR, kTRin = TR + 2, kRowsPerWarp = TR / kWarps;
+static constexpr uint32_t kTileBytes32 = 2u * kTRin * kWin * sizeof(float);
+struct alignas(128) InSlot32 {  // both arrays are TMA destinations: 128-byte aligned
+  alignas(128) float psi[kTRin][kWin];
+  alignas(128) float d[kTRin][kWin];
+};
+struct alignas(16) StSlot32 {
+  float S[kTRin][kWin];  // after phase 2: new psi of the listed cells
+  float mu[kTRin][kWin];
+  uint8_t pmask[kTRin][32];  // per lane: bits 0-3 psi <= -1, bits 4-7 psi >= 1 of its four cells
+  uint8_t hmask[kTRin][2];   // halo cells: bit 0 psi <= -1, bit 1 psi >= 1
+  uint32_t liq, sol;         // bit r: every cell of input row r has psi == -1 / +1
+};
+struct P2Smem32 {
+  uint16_t list[kTR * kW];  // as TileSmemT's
+  uint32_t nlist;
+  double part_mass[kWarps];
+  int part_itip[kWarps];
+};
+struct alignas(128) PipeSmem32 {
+  InSlot32 in[kRing];
+  StSlot32 st[kStage];
+  P2Smem32 p2;
+  uint64_t in_full[kRing], in_empty[kRing], st_full[kStage], st_empty[kStage];
+  int abort;
+};
 // one phase group's view of a tile and of its own lane
 struct View32 {
   const StepCoef &K;
@@ -1304,7 +1500,7 @@ struct View32 {
   }
 };
 
-__device__ __forceinline__ void fix_beyond32(const View32 &V, InSlot32 &in) {
+static __device__ __forceinline__ void fix_beyond32(const View32 &V, InSlot32 &in) {
   if (V.x0 + kW + 4 <= V.K.nx) return;
   for (int k = V.gtid; k < kTRin * kWin; k += kThreads) {
     const int rr = k / kWin, x = k % kWin;
@@ -1317,11 +1513,10 @@ __device__ __forceinline__ void fix_beyond32(const View32 &V, InSlot32 &in) {
 
 // phase 1 of the group warp's input rows and of the halo columns (st.liq and
 // st.sol 0 on entry)
-__device__ __forceinline__ void phase1_32(const View32 &V, const InSlot32 &in, StSlot32 &st) {
+static __device__ __forceinline__ void phase1_32(const View32 &V, const InSlot32 &in, StSlot32 &st) {
   const Coef<float> &F = V.F;
+  const MeltC M(F);
   const int lane = V.lane, bc = V.bc;
-  const float two_cinf = F.cinf + F.cinf;
-  constexpr float KL = (float)(-2.0 * kL0Liq);
   const float d_hi = F.ser_hi, d_lo = F.ser_lo;  // series range of delta (Coef)
   const float4 RTv = ld4(V.tRT + V.gi), C0v = ld4(V.tC0 + V.gi);
   const float RTa[4] = {RTv.x, RTv.y, RTv.z, RTv.w}, C0a[4] = {C0v.x, C0v.y, C0v.z, C0v.w};
@@ -1368,28 +1563,12 @@ __device__ __forceinline__ void phase1_32(const View32 &V, const InSlot32 &in, S
       code = 1u;
       st.pmask[rr][lane] = 0x0Fu;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float c = F.cinf + dv[q], om = 1.f - c;
-        float p = fmaf(F.melt_a[3], dv[q], F.melt_a[2]);
-        p = fmaf(p, dv[q], F.melt_a[1]);
-        p = fmaf(p, dv[q], F.melt_a[0]);
-        Sv[q] = c * om;
-        mv[q] = dv[q] * fmaf(RTa[q], p, KL);
-      }
+      for (int q = 0; q < 4; ++q) far_cell(M, dv[q], RTa[q], Sv[q], mv[q]);
     } else if (__all_sync(FULL, liq4 && dmx < d_hi && dmn > d_lo)) {
       code = 1u;
       st.pmask[rr][lane] = 0x0Fu;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float c = F.cinf + dv[q], om = 1.f - c;
-        const float sv = __fdividef(dv[q], fmaf(two_cinf, om, dv[q]));
-        const float s2 = sv * sv;
-        float p = fmaf(s2, 1.f / 7.f, 1.f / 5.f);
-        p = fmaf(s2, p, 1.f / 3.f);
-        const float ath = fmaf(sv * s2, p, sv);
-        Sv[q] = c * om;
-        mv[q] = fmaf(RTa[q] + RTa[q], ath, dv[q] * KL);
-      }
+      for (int q = 0; q < 4; ++q) bulk_cell(M, dv[q], RTa[q], Sv[q], mv[q]);
     } else {
       const bool sol4 = band == kPlus1f && bor == kPlus1f;
       code = (__all_sync(FULL, liq4) ? 1u : 0u) | (__all_sync(FULL, sol4) ? 2u : 0u);
@@ -1424,7 +1603,7 @@ __device__ __forceinline__ void phase1_32(const View32 &V, const InSlot32 &in, S
     uint8_t hm = 3u;
     if (V.y0 - 1 + rr <= V.K.ny - 1) {
       const float pv = in.psi[rr][x];
-      cell_terms(F, pv, in.d[rr][x], V.tRT[g], V.tC0[g], Sh, mh);
+      halo_cell(F, M, pv, in.d[rr][x], V.tRT[g], V.tC0[g], Sh, mh);
       hm = (pv <= -1.f ? 1u : 0u) | (pv >= 1.f ? 2u : 0u);
     }
     st.S[rr][x] = Sh;
@@ -1435,7 +1614,7 @@ __device__ __forceinline__ void phase1_32(const View32 &V, const InSlot32 &in, S
 
 // phase 2 of the group warp's output rows (nlist 0 on entry); returns the
 // listed cells, 4 bits per output row
-__device__ __forceinline__ uint32_t phase2_32(const View32 &V, const InSlot32 &in, const StSlot32 &st, P2Smem32 &p2,
+static __device__ __forceinline__ uint32_t phase2_32(const View32 &V, const InSlot32 &in, const StSlot32 &st, P2Smem32 &p2,
                                               float dn[kRowsPerWarp][4], double &mass, bool red) {
   const Coef<float> &F = V.F;
   const int lane = V.lane, bc = V.bc;
@@ -1535,21 +1714,28 @@ __device__ __forceinline__ uint32_t phase2_32(const View32 &V, const InSlot32 &i
         Sv &= (S << 1) | ((lf >> (8 * k + 7)) & 1u) | (((rt >> (8 * k + 4)) & 1u) << 5);
       }
       const uint32_t needs = ~((Lv & (Lv >> 1) & (Lv >> 2)) | (Sv & (Sv >> 1) & (Sv >> 2))) & V.outm;
-      const uint32_t cnt = __popc(needs);
+      // cells that draw noise (phi_cell's own test; here it only sorts the list)
+      uint32_t noisy = 0xFu;
+      if (F.noise_amp > 0.f) {
+        const float4 p4 = ld4(&in.psi[rr][bc]);
+        noisy = (fmaf(-p4.x, p4.x, 1.f) > 1.0e-3f ? 1u : 0u) | (fmaf(-p4.y, p4.y, 1.f) > 1.0e-3f ? 2u : 0u) |
+                (fmaf(-p4.z, p4.z, 1.f) > 1.0e-3f ? 4u : 0u) | (fmaf(-p4.w, p4.w, 1.f) > 1.0e-3f ? 8u : 0u);
+      }
+      // inclusive warp scan of the counts of both kinds (packed as in nlist)
+      const uint32_t cnt = __popc(needs & noisy) | (__popc(needs & ~noisy) << 16);
       uint32_t incl = cnt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const uint32_t v = __shfl_up_sync(FULL, incl, o);
         if (lane >= o) incl += v;
       }
-      const uint32_t total = __shfl_sync(FULL, incl, 31);
-      int base = 0;
-      if (lane == 31 && total) base = atomicAdd(&p2.nlist, (int)total);
-      base = __shfl_sync(FULL, base, 31);
-      uint32_t off = (uint32_t)base + incl - cnt;
+      uint32_t base = 0u;
+      if (lane == 31 && incl) base = atomicAdd(&p2.nlist, incl);
+      base = __shfl_sync(FULL, base, 31) + incl - cnt;
+      uint32_t n_at = base & 0xFFFFu, t_at = kTR * kW - 1 - (base >> 16);
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if ((needs >> q) & 1u) p2.list[off++] = (uint16_t)((rr << 8) | (V.col + q));
+        if ((needs >> q) & 1u) p2.list[((noisy >> q) & 1u) ? n_at++ : t_at--] = (uint16_t)((rr << 8) | (V.col + q));
       needs_all |= needs << (4 * j);
     }
     ra = rb;
@@ -1561,11 +1747,11 @@ __device__ __forceinline__ uint32_t phase2_32(const View32 &V, const InSlot32 &i
 }
 
 // phase 3: listed interface cells, one per group thread; new psi into np
-__device__ __forceinline__ void phase3_32(const View32 &V, const InSlot32 &in, const P2Smem32 &p2,
+static __device__ __forceinline__ void phase3_32(const View32 &V, const InSlot32 &in, const P2Smem32 &p2,
                                           float (*np)[kWin], bool red, int &itip) {
-  const int nlist = p2.nlist;
+  const int na = (int)(p2.nlist & 0xFFFFu), nlist = na + (int)(p2.nlist >> 16);
   for (int idx = V.gtid; idx < nlist; idx += kThreads) {
-    const uint32_t e = p2.list[idx];
+    const uint32_t e = p2.list[idx < na ? idx : kTR * kW - 1 - (idx - na)];
     const int rr = (int)(e >> 8), x = (int)(e & 0xFFu) + 4;
     const int r = V.y0 - 1 + rr, g = V.x0 + x - 4;
     const float c00 = V.F.cinf + in.d[rr][x];
@@ -1581,7 +1767,7 @@ __device__ __forceinline__ void phase3_32(const View32 &V, const InSlot32 &in, c
 }
 
 // phase 4: new psi and c of the group warp's rows into the input tile
-__device__ __forceinline__ void phase4_32(const View32 &V, InSlot32 &in, const float (*np)[kWin], uint32_t needs_all,
+static __device__ __forceinline__ void phase4_32(const View32 &V, InSlot32 &in, const float (*np)[kWin], uint32_t needs_all,
                                           const float dn[kRowsPerWarp][4], bool red, int &itip) {
   const int rbase = 1 + kRowsPerWarp * V.gw, bc = V.bc;
 #pragma unroll
@@ -1605,7 +1791,7 @@ __device__ __forceinline__ void phase4_32(const View32 &V, InSlot32 &in, const f
 
 // ghost columns, bulk copies of the rows (group threads < 64) and phi;
 // returns whether this thread committed a bulk group
-__device__ __forceinline__ bool store_tile32(const View32 &V, InSlot32 &in, float *__restrict__ psi_n,
+static __device__ __forceinline__ bool store_tile32(const View32 &V, InSlot32 &in, float *__restrict__ psi_n,
                                              float *__restrict__ c_n, float *__restrict__ phi_n, int bar) {
   const StepCoef &K = V.K;
   const int x0 = V.x0, y0 = V.y0;
@@ -1664,10 +1850,9 @@ __device__ __forceinline__ bool store_tile32(const View32 &V, InSlot32 &in, floa
   return any;
 }
 
-// the tile's partial sums and the fused final reduction (scratch of at least
-// 256 doubles and 256 ints)
-__device__ __forceinline__ void finish32(const View32 &V, P2Smem32 &p2, double mass, int itip, BlockPartial *part,
-                                         const FinalRed *FR, double *sm_m, int *sm_i, int bar) {
+// the tile's partial sums (a dependent launch reduces them)
+static __device__ __forceinline__ void finish32(const View32 &V, P2Smem32 &p2, double mass, int itip, BlockPartial *part,
+                                         int bar) {
   if (!part) return;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mass += __shfl_down_sync(FULL, mass, o);
@@ -1689,35 +1874,30 @@ __device__ __forceinline__ void finish32(const View32 &V, P2Smem32 &p2, double m
     b.pad = 0;
     *part = b;
   }
-  if (!FR) return;
-  if (V.gtid == 0) {
-    __threadfence();
-    p2.last = atomicAdd(FR->counter, 1u) == (unsigned)(FR->nparts - 1);
-  }
-  gsync(bar);
-  if (!p2.last) return;
-  __threadfence();
-  final_reduce(*FR, sm_m, sm_i, V.gtid, [&] { gsync(bar); });
 }
 
+};
+static_assert(sizeof(Pipe32<16>::InSlot32) % 128 == 0 && offsetof(Pipe32<16>::InSlot32, psi) % 128 == 0 && offsetof(Pipe32<16>::InSlot32, d) % 128 == 0,
+              "ring slots and their TMA destinations stay 128-byte aligned");
+static_assert(offsetof(Pipe32<16>::PipeSmem32, in) % 128 == 0, "the ring starts on a 128-byte boundary");
 __device__ __forceinline__ void tile_of32(int t, int nrt, int ncb, int f, int &tr, int &tc) {
   tr = t % nrt;
   tc = front_first_block(t / nrt, f, ncb);
 }
 
+template <int TR>
 __global__ void __launch_bounds__(kPipeThreads, 2)
     pipe_kernel_f32(const __grid_constant__ StepCoef K, const __grid_constant__ Coef<float> F,
                     const __grid_constant__ StepScalars PS, const __grid_constant__ CUtensorMap tm_psi,
                     const __grid_constant__ CUtensorMap tm_c, const float *__restrict__ tab, const int tab_len,
                     float *__restrict__ psi_n, float *__restrict__ c_n, float *__restrict__ phi_n,
-                    BlockPartial *partials, int *err, const __grid_constant__ FinalRed FR, const int nrt,
-                    const int ncb) {
+                    BlockPartial *partials, int *err, const int nrt, const int ncb) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  PipeSmem32 &sm = *reinterpret_cast<PipeSmem32 *>(smem_raw);
+  using Ops = Pipe32<TR>;
+  auto &sm = *reinterpret_cast<typename Ops::PipeSmem32 *>(smem_raw);
   const int warp = threadIdx.x >> 5;
   const int ntiles = nrt * ncb;
   const int f = max(PS.i_front, 0) / kW;
-  const FinalRed *FRp = partials && FR.counter ? &FR : nullptr;
   const uint32_t limit = PS.wait_limit ? PS.wait_limit : kWaitLimit;
   const bool poll = PS.wait_limit != 0;
   volatile int *abort = &sm.abort;
@@ -1750,9 +1930,9 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
         if (k >= kRing && !pipe_wait(&sm.in_empty[s], ((k / kRing) - 1) & 1, abort, limit, err, poll)) break;
         int tr, tc;
         tile_of32(t, nrt, ncb, f, tr, tc);
-        mbar_expect_tx(&sm.in_full[s], kTileBytes32);
-        tma_load_2d(&sm.in[s].psi[0][0], &tm_psi, &sm.in_full[s], kW * tc - 4, kTR * tr);
-        tma_load_2d(&sm.in[s].d[0][0], &tm_c, &sm.in_full[s], kW * tc - 4, kTR * tr);
+        mbar_expect_tx(&sm.in_full[s], Ops::kTileBytes32);
+        tma_load_2d(&sm.in[s].psi[0][0], &tm_psi, &sm.in_full[s], kW * tc - 4, TR * tr);
+        tma_load_2d(&sm.in[s].d[0][0], &tm_c, &sm.in_full[s], kW * tc - 4, TR * tr);
       }
       // only the last kRing loads can still be in flight: they land before the CTA exits
       for (int q = max(k - kRing, 0); q < k; ++q)
@@ -1771,14 +1951,14 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
       if (!group_and(ok, kBarP1)) break;
       int tr, tc;
       tile_of32(t, nrt, ncb, f, tr, tc);
-      const View32 V(K, F, PS, tab, tab_len, kW * tc, 1 + kTR * tr, gtid);
+      const typename Ops::View32 V(K, F, PS, tab, tab_len, kW * tc, 1 + TR * tr, gtid);
       if (gtid == 0) {
         sm.st[q].liq = 0u;
         sm.st[q].sol = 0u;
       }
-      fix_beyond32(V, sm.in[s]);
+      Ops::fix_beyond32(V, sm.in[s]);
       gsync(kBarP1);
-      phase1_32(V, sm.in[s], sm.st[q]);
+      Ops::phase1_32(V, sm.in[s], sm.st[q]);
       gsync(kBarP1);
       if (gtid == 0) mbar_arrive(&sm.st_full[q]);
     }
@@ -1792,22 +1972,21 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
     if (!group_and(pipe_wait(&sm.st_full[q], (k / kStage) & 1, abort, limit, err, poll), kBarP2)) break;
     int tr, tc;
     tile_of32(t, nrt, ncb, f, tr, tc);
-    const View32 V(K, F, PS, tab, tab_len, kW * tc, 1 + kTR * tr, gtid);
+    const typename Ops::View32 V(K, F, PS, tab, tab_len, kW * tc, 1 + TR * tr, gtid);
     BlockPartial *part = partials ? partials + ((int64_t)tc * nrt + tr) : nullptr;
     const bool red = part != nullptr;
-    if (gtid == 0) sm.p2.nlist = 0;
+    if (gtid == 0) sm.p2.nlist = 0u;
     gsync(kBarP2);
     double mass = 0.0;
     int itip = 0;
-    float dn[kRowsPerWarp][4];
-    const uint32_t needs_all = phase2_32(V, sm.in[s], sm.st[q], sm.p2, dn, mass, red);
+    float dn[Ops::kRowsPerWarp][4];
+    const uint32_t needs_all = Ops::phase2_32(V, sm.in[s], sm.st[q], sm.p2, dn, mass, red);
     gsync(kBarP2);
-    phase3_32(V, sm.in[s], sm.p2, sm.st[q].S, red, itip);
+    Ops::phase3_32(V, sm.in[s], sm.p2, sm.st[q].S, red, itip);
     gsync(kBarP2);
-    phase4_32(V, sm.in[s], sm.st[q].S, needs_all, dn, red, itip);
-    const bool issued = store_tile32(V, sm.in[s], psi_n, c_n, phi_n, kBarP2);
-    finish32(V, sm.p2, mass, itip, part, FRp, reinterpret_cast<double *>(&sm.st[q].mu[0][0]),
-             reinterpret_cast<int *>(&sm.st[q].mu[8][0]), kBarP2);
+    Ops::phase4_32(V, sm.in[s], sm.st[q].S, needs_all, dn, red, itip);
+    const bool issued = Ops::store_tile32(V, sm.in[s], psi_n, c_n, phi_n, kBarP2);
+    Ops::finish32(V, sm.p2, mass, itip, part, kBarP2);
     if (issued) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     gsync(kBarP2);
     if (gtid == 0) {
@@ -1853,9 +2032,12 @@ int launch_ensemble(const EnsRun *runs, int nruns, const int32_t *tblk, int ntbl
   static std::atomic<int> wave_of[2][kTileShapes][64];
   const int wave = resident_ctas((const void *)kfn, kThreads, smem, wave_of[surr][shape]);
   if (wave < 0) return -3;
-  ens_table_kernel<<<ntblk, kTabBlock, 0, st>>>(runs, tblk);
-  kfn<<<ntiles, kThreads, smem, st>>>(runs, order, err, wave);
-  if (advance) ens_advance_kernel<<<(nruns + 63) / 64, 64, 0, st>>>(const_cast<EnsRun *>(runs), nruns);
+  if (launch_dep(ens_table_kernel, dim3(ntblk), dim3(kTabBlock), st, runs, tblk) != cudaSuccess ||
+      launch_dep_smem(kfn, dim3(ntiles), dim3(kThreads), smem, st, runs, order, err, wave) != cudaSuccess)
+    return -3;
+  if (advance && launch_dep(ens_advance_kernel, dim3((nruns + 63) / 64), dim3(64), st, const_cast<EnsRun *>(runs),
+                            nruns) != cudaSuccess)
+    return -3;
   return 0;
 }
 
@@ -1893,115 +2075,83 @@ int launch_ensemble_walk(EnsRun *runs, int nruns, const int32_t *tblk, int ntblk
   return 0;
 }
 
+// Output rows of the tiles of an nx x ny FP32 step, as tile_rows_f64, in waves
+// of five CTAs per SM of 16 x 128 tiles (us a step with a planar front, 4 / 8 /
+// 16 rows): 256^2, 0.04 waves, 6.2 / 8.3 / 12.2; 1024^2, 0.7 waves, 8.7 / 10.7 /
+// 16.0; 1280^2, 1.1 waves, 12.6 / 11.4 / 15.2; 2048 x 1536, 2.1 waves, 20.9 /
+// 18.1 / 19.3 (all melt 19.1 / 16.5 / 14.6); 2048^2, 2.8 waves, 26.6 / 22.9 /
+// 21.1.  The network's tiles at the front take two to three times as long:
+// 1024^2 19.1 / 26.0 / 45.6; 1536^2, 1.6 waves, 29.8 / 28.0 / 41.1; 2048 x 3072,
+// 4.2 waves, 67 / 47.9 / 49.5; 4096^2, 11 waves, 146 / 98 / 80.
+int tile_rows_f32(int nx, int ny, bool tfc, bool network) {
+  if (tfc) return kTfcTR;
+  const int64_t tiles = (int64_t)((nx + kW - 1) / kW) * ((ny - 2 + 15) / 16), wave = 5 * (int64_t)sm_count();
+  if (network) return 2 * tiles >= 9 * wave ? 16 : 2 * tiles >= 3 * wave ? 8 : 4;
+  return tiles >= 2 * wave ? 16 : tiles >= wave ? 8 : 4;
+}
+
 int launch_step_f32_tma(const StepCoef &K, const Coef<float> &F, const StepScalars &P, const TmaMaps &tm,
                         float *psi_n, float *c_n, float *phi_n, BlockPartial *partials, int max_partials,
                         int *nparts_out, int *err, cudaStream_t st) {
-  const int nj = K.ny - 2;
   if (K.nx % 4 || K.pitch != K.nx) return -1;  // rows are copied in 16-byte units
+  const bool surr = tm.surr != nullptr, tfc = K.tfc != 0;
+  // the coarse-grid temperature has no table kernel, surrogate or pipeline
+  if (tfc && (!P.T_coarse || surr)) return -1;
+  const bool pipe = tm.pipeline != 0 && !surr && !tfc && !P.pull_back;  // the persistent warp-role kernel (exact path)
+  const int TR = tm.rows;  // the tensor maps' box is TR + 2 rows high
+  if (tfc ? TR != kTfcTR : (TR != 4 && TR != 8 && TR != 16)) return -1;
   // column-major: consecutive CTAs share a column strip and its halo rows in L2
-  const dim3 grid((nj + kTR - 1) / kTR, (K.nx + kW - 1) / kW), block(kThreads);
-  if (grid.y > 65535 || (int64_t)grid.x * grid.y > (1 << 30)) return -1;
-  const int nparts = grid.x * grid.y;
+  const int nrt = (K.ny - 2 + TR - 1) / TR, ncb = (K.nx + kW - 1) / kW;
+  if (ncb > 65535 || (int64_t)nrt * ncb > (1 << 30)) return -1;
+  const int nparts = nrt * ncb;
   if (partials && nparts > max_partials) return -1;
-  if (tm.col_tab_len < (int)grid.y * kW + kWin) return -1;
-  const bool surr = tm.surr != nullptr;
-  if (K.tfc) {
-    // the coarse-grid temperature: no table kernel, so the tile kernel runs
-    // in plain stream order (it issues its TMA loads before
-    // griddepcontrol.wait, which is safe only after the table kernel); the
-    // maps' boxes are kTfcTR + 2 rows high
-    if (!P.T_coarse || surr) return -1;
-    const dim3 tg((nj + kTfcTR - 1) / kTfcTR, grid.y);
-    const int np = (int)(tg.x * tg.y);
-    if (partials && np > max_partials) return -1;
-    const size_t tsmem = sizeof(TileSmemT<kTfcTR, true>);
-    static std::atomic<unsigned long long> tattr{0};
-    if (!smem_limit_once((const void *)tile_kernel_tfc, (int)tsmem, tattr)) return -3;
-    static std::atomic<int> twave[64];
-    const int wave = resident_ctas((const void *)tile_kernel_tfc, kThreads, tsmem, twave);
-    if (wave < 0) return -3;
-    cudaLaunchConfig_t tc = {};
-    tc.gridDim = tg;
-    tc.blockDim = block;
-    tc.dynamicSmemBytes = tsmem;
-    tc.stream = st;
-    FinalRed fr = tm.red;
-    fr.partials = partials;
-    fr.nparts = np;
-    FinalRed none = fr;
-    none.counter = nullptr;
-    const float *tab = tm.col_tab;
-    if (cudaLaunchKernelEx(&tc, tile_kernel_tfc, K, F, P, tm.psi, tm.c, tab, tm.col_tab_len, psi_n, c_n, phi_n,
-                           partials, err, none, wave) != cudaSuccess)
-      return -3;
-    if (partials && (fr.mass_out || fr.itip_out) && launch_reduce_partials_dep(fr, st)) return -3;
-    if (nparts_out) *nparts_out = np;
-    return 0;
-  }
-  if (tm.pipeline && !surr && !P.pull_back) {  // the persistent warp-role kernel (exact path)
-    const int nrt = (int)grid.x, ncb = (int)grid.y;
-    const size_t psmem = sizeof(PipeSmem32);
-    static std::atomic<unsigned long long> pattr{0};
-    if (!smem_limit_once((const void *)pipe_kernel_f32, (int)psmem, pattr)) return -3;
-    static std::atomic<int> president[64];
-    const int res = resident_ctas((const void *)pipe_kernel_f32, kPipeThreads, psmem, president);
-    if (res <= 0) return -3;
-    column_table_kernel<<<(tm.col_tab_len + kTabBlock - 2) / (kTabBlock - 1), kTabBlock, 0, st>>>(
-        K, P.d0, P.d1, tm.col_tab_len, tm.col_tab);
-    cudaLaunchConfig_t pc = {};
-    pc.gridDim = dim3((unsigned)std::min(res, nparts));
-    pc.blockDim = dim3(kPipeThreads);
-    pc.dynamicSmemBytes = psmem;
-    pc.stream = st;
-    cudaLaunchAttribute pa[1];
-    pa[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    pa[0].val.programmaticStreamSerializationAllowed = 1;
-    pc.attrs = pa;
-    pc.numAttrs = 1;
-    // the final reduction is a programmatic dependent launch after the step
-    FinalRed pfr = tm.red;
-    pfr.partials = partials;
-    pfr.nparts = nparts;
-    FinalRed none = pfr;
-    none.counter = nullptr;
-    const float *ptab = tm.col_tab;
-    if (cudaLaunchKernelEx(&pc, pipe_kernel_f32, K, F, P, tm.psi, tm.c, ptab, tm.col_tab_len, psi_n, c_n, phi_n,
-                           partials, err, none, nrt, ncb) != cudaSuccess)
-      return -3;
-    if (partials && (pfr.mass_out || pfr.itip_out) && launch_reduce_partials_dep(pfr, st)) return -3;
-    if (nparts_out) *nparts_out = nparts;
-    return 0;
-  }
-  const size_t smem = sizeof(TileSmem);
-  auto kfn = surr ? tile_kernel<true> : tile_kernel<false>;
-  static std::atomic<unsigned long long> attr_done[2];
-  if (!smem_limit_once((const void *)kfn, (int)smem, attr_done[surr])) return -3;
-  static std::atomic<int> wave_of[2][64];
-  const int wave = resident_ctas((const void *)kfn, kThreads, smem, wave_of[surr]);
-  if (wave < 0) return -3;
-  SurrArgs sa = {};
-  if (surr) sa = *tm.surr;
-  column_table_kernel<<<(tm.col_tab_len + kTabBlock - 2) / (kTabBlock - 1), kTabBlock, 0, st>>>(K, P.d0, P.d1, tm.col_tab_len, tm.col_tab);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
+  if (tm.col_tab_len < ncb * kW + kWin) return -1;
+  const int sh = TR == 4 ? 0 : TR == 8 ? 1 : 2;
+  using Tile = decltype(&tile_kernel<false, 16>);
+  static const Tile tile_fn[2][3] = {{tile_kernel<false, 4>, tile_kernel<false, 8>, tile_kernel<false, 16>},
+                                     {tile_kernel<true, 4>, tile_kernel<true, 8>, tile_kernel<true, 16>}};
+  static const decltype(&pipe_kernel_f32<16>) pipe_fn[3] = {pipe_kernel_f32<4>, pipe_kernel_f32<8>, pipe_kernel_f32<16>};
+  static const size_t tile_smem[3] = {sizeof(TileSmemT<4>), sizeof(TileSmemT<8>), sizeof(TileSmemT<16>)};
+  static const size_t pipe_smem[3] = {sizeof(Pipe32<4>::PipeSmem32), sizeof(Pipe32<8>::PipeSmem32),
+                                      sizeof(Pipe32<16>::PipeSmem32)};
+  const int which = tfc ? 9 : pipe ? 6 + sh : 3 * surr + sh;
+  const void *kfn = tfc    ? (const void *)tile_kernel_tfc
+                    : pipe ? (const void *)pipe_fn[sh]
+                           : (const void *)tile_fn[surr][sh];
+  const size_t smem = tfc ? sizeof(TileSmemT<kTfcTR, true>) : pipe ? pipe_smem[sh] : tile_smem[sh];
+  const dim3 block(pipe ? kPipeThreads : kThreads);
+  static std::atomic<unsigned long long> attr_done[10];
+  if (!smem_limit_once(kfn, (int)smem, attr_done[which])) return -3;
+  static std::atomic<int> resident_of[10][64];
+  const int resident = resident_ctas(kfn, (int)block.x, smem, resident_of[which]);
+  if (resident <= 0) return -3;
+  // every kernel of the step is a programmatic dependent of the one before it
+  // in the stream (rs_step_f64t.cu)
   const float *tab = tm.col_tab;
+  cudaError_t e = cudaSuccess;
+  if (!tfc)
+    e = launch_dep(column_table_kernel, dim3((tm.col_tab_len + kTabBlock - 2) / (kTabBlock - 1)), dim3(kTabBlock), st,
+                   K, P.d0, P.d1, tm.col_tab_len, tm.col_tab);
+  if (e != cudaSuccess) return -3;
+  const dim3 grid(nrt, ncb);
+  const int wx = resident % nrt, wy = resident / nrt;
+  if (tfc) {
+    e = launch_dep_smem(tile_kernel_tfc, grid, block, smem, st, K, F, P, tm.psi, tm.c, tab, tm.col_tab_len, psi_n, c_n,
+                        phi_n, partials, err, wx, wy);
+  } else if (pipe) {
+    e = launch_dep_smem(pipe_fn[sh], dim3((unsigned)std::min(resident, nparts)), block, smem, st, K, F, P, tm.psi, tm.c,
+                        tab, tm.col_tab_len, psi_n, c_n, phi_n, partials, err, nrt, ncb);
+  } else {
+    SurrArgs sa = {};
+    if (surr) sa = *tm.surr;
+    e = launch_dep_smem(tile_fn[surr][sh], grid, block, smem, st, K, F, P, tm.psi, tm.c, tab, tm.col_tab_len, psi_n,
+                        c_n, phi_n, partials, err, sa, wx, wy);
+  }
+  if (e != cudaSuccess) return -3;
   // the final reduction is a programmatic dependent launch after the step
   FinalRed fr = tm.red;
   fr.partials = partials;
   fr.nparts = nparts;
-  FinalRed none = fr;
-  none.counter = nullptr;
-  if (cudaLaunchKernelEx(&cfg, kfn, K, F, P, tm.psi, tm.c, tab, tm.col_tab_len, psi_n, c_n, phi_n, partials, err,
-                         sa, none, wave) != cudaSuccess)
-    return -3;
   if (partials && (fr.mass_out || fr.itip_out) && launch_reduce_partials_dep(fr, st)) return -3;
   if (nparts_out) *nparts_out = nparts;
   return 0;

@@ -40,8 +40,9 @@ def state(p, kind, seed):
     return s
 
 
-# FP64 tiles of 64 columns: 4 rows below one wave of 740 16-row tiles, 8 below three, then 16
-SIZES = [(64, 18), (130, 19), (258, 8), (320, 66), (2048, 371), (2050, 372), (2048, 1127), (2110, 1045)]
+# FP64 tiles of 64 columns: 4 rows below one wave of 740 16-row tiles, 8 below three, then 16; FP32 tiles of
+# 128: 4 below one, 8 below two
+SIZES = [(64, 18), (128, 19), (260, 8), (320, 66), (2048, 371), (2052, 372), (2048, 1127), (2112, 1045), (2048, 1500)]
 
 
 @pytest.mark.parametrize("dtype", ["f64", "f32"])
