@@ -444,7 +444,7 @@ int rs_step(rs_ctx *c, const rs_fields *cur, const rs_fields *next, const rs_ste
   if (cur->psi == next->psi || cur->c == next->c || (next->phi && (next->phi == cur->psi || next->phi == cur->c)))
     return fail(RS_E_INVALID, "rs_step: cur and next alias");
   if (c->p.tfc && !a->T_coarse) return fail(RS_E_INVALID, "rs_step: TFC needs T_coarse");
-  const rs::StepScalars P = step_scalars(c, a, cur);
+  rs::StepScalars P = step_scalars(c, a, cur);
   cudaStream_t st = (cudaStream_t)stream;
   c->pb_cur = a->pull_back ? cur->psi : nullptr;
   c->pb_offset = a->pull_back ? a->i_offset : 0;
@@ -453,26 +453,32 @@ int rs_step(rs_ctx *c, const rs_fields *cur, const rs_fields *next, const rs_ste
   int lr;
   rs::TmaMaps tm;
   const rs::TmaMaps *tmp = nullptr;
-  // the TMA kernels store whole rows by 16-byte bulk copies
+  // the tile kernels load rows by TMA boxes and store them in 16-byte units;
+  // where a field's rows are not 16-byte aligned they copy element by element
+  // (2x the register kernel's speed all the same), with the exact evaluation
   const uintptr_t vec = 16;
   const bool out_aligned =
       ((uintptr_t)next->psi % vec) == 0 && ((uintptr_t)next->c % vec) == 0 && ((uintptr_t)next->phi % vec) == 0;
-  const int rows = cur->precision == RS_F64 ? rs::tile_rows_f64(c->p.nx_all, c->p.ny_all, c->p.tfc != 0)
-                                            : rs::tile_rows_f32(c->p.nx_all, c->p.ny_all, c->p.tfc != 0, c->surr.w != nullptr);
-  const int box_rows = rows + 2;
-  if (c->use_tma && out_aligned && field_map(c, cur->psi, cur->precision, box_rows, &tm.psi) &&
-      field_map(c, cur->c, cur->precision, box_rows, &tm.c)) {
+  const bool f64 = cur->precision == RS_F64, tfc = c->p.tfc != 0;
+  const rs::SurrArgs *surr = c->surr.w && !f64 ? &c->surr : nullptr;
+  const int nx = c->p.nx_all, ny = c->p.ny_all;
+  if (c->use_tma) {
+    tm.rows = f64 ? rs::tile_rows_f64(nx, ny, tfc) : rs::tile_rows_f32(nx, ny, tfc, surr != nullptr);
+    if (!(out_aligned && field_map(c, cur->psi, cur->precision, tm.rows + 2, &tm.psi) &&
+          field_map(c, cur->c, cur->precision, tm.rows + 2, &tm.c))) {
+      P.raw = 1;
+      surr = nullptr;
+      if (!f64) tm.rows = rs::tile_rows_f32(nx, ny, tfc, false);
+    }
     tm.col_tab = c->col_tab;
     tm.col_tab_len = c->col_tab_len;
     tm.col_tab64 = c->col_tab64;
     tm.col_tab64_len = c->col_tab64_len;
-    tm.surr = c->surr.w && cur->precision == RS_F32 ? &c->surr : nullptr;
+    tm.surr = surr;
     tm.pipeline = c->pipeline;
-    tm.rows = rows;
     tm.red = {};
     if (red) {  // both tile kernels reduce their partials themselves
-      tm.red.mass_offset =
-          cur->precision == RS_F32 ? (double)(c->p.nx_all - 2) * (c->p.ny_all - 2) * c->p.cinf : 0.0;
+      tm.red.mass_offset = f64 ? 0.0 : (double)(nx - 2) * (ny - 2) * c->p.cinf;
       tm.red.mass_out = a->mass_out;
       tm.red.itip_out = a->itip_out;
     }

@@ -250,6 +250,9 @@ struct StepScalars {
   // the current fields (the tile kernels gather a pull-back step's shifted
   // tile through them instead of a TMA box)
   const void *src_psi, *src_c;
+  // the fields' rows are not 16-byte aligned: the tile kernels copy their
+  // tiles in element by element and store cells by plain stores
+  int32_t raw;
 };
 
 }  // namespace rs

@@ -11,8 +11,8 @@
 //   * ghost cells (compute_boundary_individual, fun.cu:1220-1230) are written
 //     by the cell they copy, corners included.
 //
-// Three kernels: this file's register-prefetch kernel (unaligned fields,
-// RS_OPT_TMA = 0) and the TMA-staged tile kernels of rs_step_f32.cu (FP32) and
+// Three kernels: this file's register-prefetch kernel (RS_OPT_TMA = 0)
+// and the TMA-staged tile kernels of rs_step_f32.cu (FP32) and
 // rs_step_f64t.cu (FP64): frozen and coarse-grid temperature, pull-back steps
 // included (those gather their shifted tile).
 //

@@ -540,6 +540,16 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target, int
   return __syncthreads_and(ok) != 0;
 }
 
+// one element from global to shared memory, asynchronously (nothing is read and
+// 0 is written where !in); cp_async_wait: the thread's copies have arrived
+template <typename R>
+__device__ __forceinline__ void cp_async_elem(R *dst, const R *src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(smem_u32(dst)), "l"(src), "n"((int)sizeof(R)),
+               "r"(in ? (int)sizeof(R) : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // L2 prefetch of the box a tma_load_2d at (x, y) would copy (no shared memory,
 // no barrier; the same 16-byte alignment of x as the load)
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap *map, int x, int y) {

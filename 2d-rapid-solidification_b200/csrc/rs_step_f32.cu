@@ -251,7 +251,8 @@ __global__ void __launch_bounds__(kTabBlock) column_table_kernel(const StepCoef 
 // part: this tile's partial (mass, coarse tip), or nullptr.
 // TR: output rows of the tile (8, 16 or 32; the tensor maps' box is TR + 2
 // rows high).
-template <bool SURR, int TR, typename Prefetch, bool TFC = false>
+// RAW: the fields' rows are not 16-byte aligned (any nx).
+template <bool SURR, int TR, typename Prefetch, bool TFC = false, bool RAW = false>
 __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &F, const StepScalars &PS,
                                           const CUtensorMap *tm_psi, const CUtensorMap *tm_c,
                                           const float *__restrict__ tab, const int tab_len, float *__restrict__ psi_n,
@@ -282,7 +283,8 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
   // (pull_back, fun.cu:1469-1492): no TMA box has that shape, so the CTA
   // gathers its tile instead (same box, zeros outside the array, delta = 0
   // where the source is column nx - 2: the melt entering at the right edge)
-  const bool pb = PS.pull_back != 0;
+  // (and so it does on rows that are not 16-byte aligned, unshifted)
+  const bool pb = RAW || PS.pull_back != 0;
   if (threadIdx.x == 0) {
     mbar_init(&sm.full, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -465,7 +467,18 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
   if (pb) {
     const float *__restrict__ gpsi = static_cast<const float *>(PS.src_psi);
     const float *__restrict__ gd = static_cast<const float *>(PS.src_c);
-    for (int k = threadIdx.x; k < kTRin * kWin; k += kThreads) {
+    if (!PS.pull_back) {
+      for (int k = threadIdx.x; k < kTRin * kWin; k += kThreads) {
+        const int rr = k / kWin, x = k % kWin;
+        const int row = y0 - 1 + rr, g = x0 - 4 + x;
+        const bool inside = row <= ny - 1 && g >= 0 && g <= nx - 1;
+        const int64_t o = inside ? (int64_t)row * K.pitch + g : 0;
+        cp_async_elem(&sm.psi[rr][x], gpsi + o, inside);
+        cp_async_elem(&sm.d[rr][x], gd + o, inside);
+      }
+      cp_async_wait();
+    }
+    else for (int k = threadIdx.x; k < kTRin * kWin; k += kThreads) {
       const int rr = k / kWin, x = k % kWin;
       const int row = y0 - 1 + rr, g = x0 - 4 + x;
       float pv = 0.f, dv = 0.f;
@@ -480,6 +493,24 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     }
   }
   __syncthreads();  // barrier initialised, flags cleared (a pull-back tile gathered)
+  // one interior cell by plain stores, with the ghost cells that copy it
+  auto raw_cell = [&](int r, int g, float pv, float dv) {
+    if (g < 1 || g > nx - 2) return;
+    auto at = [&](int row, int col) {
+      const int64_t o = (int64_t)row * K.pitch + col;
+      psi_n[o] = pv;
+      c_n[o] = dv;
+      if (phi_n) phi_n[o] = clamp1(pv);
+    };
+    auto all = [&](int row) {
+      at(row, g);
+      if (g == 1) at(row, 0);
+      if (g == nx - 2) at(row, nx - 1);
+    };
+    all(r);
+    if (r == K.jmin) all(0);
+    if (r == K.jmax) all(ny - 1);
+  };
   bool gave_up = false;
   if (!pb) {  // bounded wait for the tile
     const uint32_t limit = PS.wait_limit ? PS.wait_limit : kWaitLimit;
@@ -575,6 +606,11 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
                                          (K.jmax >= y0 + r0 && K.jmax < y0 + r0 + kRowsPerWarp);
     const float pv = melt ? -1.f : 1.f;
     auto put = [&](int j, float (&v)[4]) {
+      if constexpr (RAW) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) raw_cell(y0 + r0 + j, gi + q, pv, v[q]);
+        return;
+      }
       if (gi == 0) v[0] = v[1];         // ghost column 0
       if (gi + 4 == nx) v[3] = v[2];    // ghost column nx-1
       if (!inside) return;
@@ -1123,6 +1159,15 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     }
   }
   const int nrow = min(kTR, K.ny - 1 - y0);  // output rows of this tile inside the interior
+  if constexpr (RAW) {
+    __syncthreads();
+    for (int k = threadIdx.x; k < nrow * kW; k += kThreads) {
+      const int j = k / kW, x = k % kW;
+      raw_cell(y0 + j, x0 + x, sm.psi[1 + j][4 + x], sm.d[1 + j][4 + x]);
+    }
+    finish(mass, itip);
+    return;
+  }
   const int ncol = min(kW, K.nx - x0);       // columns of this tile inside the array (a multiple of 4)
   if (x0 == 0 || x0 + kW >= K.nx) {
     // ghost columns 0 and nx-1 (compute_boundary_individual, fun.cu:1220-1230)
@@ -1202,7 +1247,7 @@ struct WavePrefetch {
   }
 };
 
-template <bool SURR, int TR>
+template <bool SURR, int TR, bool RAW>
 __global__ void __launch_bounds__(kThreads, SURR ? 4 : 5)
     tile_kernel(const __grid_constant__ StepCoef K, const __grid_constant__ Coef<float> F,
                 const __grid_constant__ StepScalars PS, const __grid_constant__ CUtensorMap tm_psi,
@@ -1214,7 +1259,7 @@ __global__ void __launch_bounds__(kThreads, SURR ? 4 : 5)
   const int f = max(PS.i_front, 0) / kW;
   const int tr = blockIdx.x;
   const int tc = front_first_block((int)blockIdx.y, f, (int)gridDim.y);
-  tile_body<SURR, TR>(K, F, PS, &tm_psi, &tm_c, tab, tab_len, psi_n, c_n, phi_n,
+  tile_body<SURR, TR, WavePrefetch, false, RAW>(K, F, PS, &tm_psi, &tm_c, tab, tab_len, psi_n, c_n, phi_n,
                       partials ? partials + ((int64_t)tc * gridDim.x + tr) : nullptr, err, SA, tr, tc,
                       WavePrefetch{&tm_psi, &tm_c, f, wave_x, wave_y, TR});
 }
@@ -1223,6 +1268,7 @@ __global__ void __launch_bounds__(kThreads, SURR ? 4 : 5)
 // per-cell K + C0 (FP64) fits beside the tile with six CTAs per SM; per-cell
 // CALPHAD groups instead of the column table.
 constexpr int kTfcTR = kTfcTileRows32;
+template <bool RAW>
 __global__ void __launch_bounds__(kThreads, 5)
     tile_kernel_tfc(const __grid_constant__ StepCoef K, const __grid_constant__ Coef<float> F,
                     const __grid_constant__ StepScalars PS, const __grid_constant__ CUtensorMap tm_psi,
@@ -1233,7 +1279,7 @@ __global__ void __launch_bounds__(kThreads, 5)
   const int tr = blockIdx.x;
   const int tc = front_first_block((int)blockIdx.y, f, (int)gridDim.y);
   const SurrArgs none = {};
-  tile_body<false, kTfcTR, WavePrefetch, true>(
+  tile_body<false, kTfcTR, WavePrefetch, true, RAW>(
       K, F, PS, &tm_psi, &tm_c, tab, tab_len, psi_n, c_n, phi_n,
       partials ? partials + ((int64_t)tc * gridDim.x + tr) : nullptr, err, none, tr, tc,
       WavePrefetch{&tm_psi, &tm_c, f, wave_x, wave_y, kTfcTR});
@@ -2093,36 +2139,43 @@ int tile_rows_f32(int nx, int ny, bool tfc, bool network) {
 int launch_step_f32_tma(const StepCoef &K, const Coef<float> &F, const StepScalars &P, const TmaMaps &tm,
                         float *psi_n, float *c_n, float *phi_n, BlockPartial *partials, int max_partials,
                         int *nparts_out, int *err, cudaStream_t st) {
-  if (K.nx % 4 || K.pitch != K.nx) return -1;  // rows are copied in 16-byte units
+  const bool raw = P.raw != 0;
+  if ((K.nx % 4 && !raw) || K.pitch != K.nx) return -1;  // rows are copied in 16-byte units
   const bool surr = tm.surr != nullptr, tfc = K.tfc != 0;
   // the coarse-grid temperature has no table kernel, surrogate or pipeline
   if (tfc && (!P.T_coarse || surr)) return -1;
-  const bool pipe = tm.pipeline != 0 && !surr && !tfc && !P.pull_back;  // the persistent warp-role kernel (exact path)
+  if (raw && surr) return -1;
+  const bool pipe = tm.pipeline != 0 && !surr && !tfc && !P.pull_back && !raw;  // the persistent warp-role kernel (exact path)
   const int TR = tm.rows;  // the tensor maps' box is TR + 2 rows high
   if (tfc ? TR != kTfcTR : (TR != 4 && TR != 8 && TR != 16)) return -1;
   // column-major: consecutive CTAs share a column strip and its halo rows in L2
-  const int nrt = (K.ny - 2 + TR - 1) / TR, ncb = (K.nx + kW - 1) / kW;
+  // (raw: the tile that holds the last interior column writes the ghost column)
+  const int nrt = (K.ny - 2 + TR - 1) / TR, ncb = (K.nx - raw + kW - 1) / kW;
   if (ncb > 65535 || (int64_t)nrt * ncb > (1 << 30)) return -1;
   const int nparts = nrt * ncb;
   if (partials && nparts > max_partials) return -1;
   if (tm.col_tab_len < ncb * kW + kWin) return -1;
   const int sh = TR == 4 ? 0 : TR == 8 ? 1 : 2;
-  using Tile = decltype(&tile_kernel<false, 16>);
-  static const Tile tile_fn[2][3] = {{tile_kernel<false, 4>, tile_kernel<false, 8>, tile_kernel<false, 16>},
-                                     {tile_kernel<true, 4>, tile_kernel<true, 8>, tile_kernel<true, 16>}};
+  using Tile = decltype(&tile_kernel<false, 16, false>);
+  static const Tile tile_fn[3][3] = {  // [exact, network, exact on unaligned rows][height]
+      {tile_kernel<false, 4, false>, tile_kernel<false, 8, false>, tile_kernel<false, 16, false>},
+      {tile_kernel<true, 4, false>, tile_kernel<true, 8, false>, tile_kernel<true, 16, false>},
+      {tile_kernel<false, 4, true>, tile_kernel<false, 8, true>, tile_kernel<false, 16, true>}};
+  const auto tfc_fn = raw ? tile_kernel_tfc<true> : tile_kernel_tfc<false>;
+  const int row = raw ? 2 : surr;
   static const decltype(&pipe_kernel_f32<16>) pipe_fn[3] = {pipe_kernel_f32<4>, pipe_kernel_f32<8>, pipe_kernel_f32<16>};
   static const size_t tile_smem[3] = {sizeof(TileSmemT<4>), sizeof(TileSmemT<8>), sizeof(TileSmemT<16>)};
   static const size_t pipe_smem[3] = {sizeof(Pipe32<4>::PipeSmem32), sizeof(Pipe32<8>::PipeSmem32),
                                       sizeof(Pipe32<16>::PipeSmem32)};
-  const int which = tfc ? 9 : pipe ? 6 + sh : 3 * surr + sh;
-  const void *kfn = tfc    ? (const void *)tile_kernel_tfc
+  const int which = tfc ? 12 + raw : pipe ? 9 + sh : 3 * row + sh;
+  const void *kfn = tfc    ? (const void *)tfc_fn
                     : pipe ? (const void *)pipe_fn[sh]
-                           : (const void *)tile_fn[surr][sh];
+                           : (const void *)tile_fn[row][sh];
   const size_t smem = tfc ? sizeof(TileSmemT<kTfcTR, true>) : pipe ? pipe_smem[sh] : tile_smem[sh];
   const dim3 block(pipe ? kPipeThreads : kThreads);
-  static std::atomic<unsigned long long> attr_done[10];
+  static std::atomic<unsigned long long> attr_done[14];
   if (!smem_limit_once(kfn, (int)smem, attr_done[which])) return -3;
-  static std::atomic<int> resident_of[10][64];
+  static std::atomic<int> resident_of[14][64];
   const int resident = resident_ctas(kfn, (int)block.x, smem, resident_of[which]);
   if (resident <= 0) return -3;
   // every kernel of the step is a programmatic dependent of the one before it
@@ -2136,7 +2189,7 @@ int launch_step_f32_tma(const StepCoef &K, const Coef<float> &F, const StepScala
   const dim3 grid(nrt, ncb);
   const int wx = resident % nrt, wy = resident / nrt;
   if (tfc) {
-    e = launch_dep_smem(tile_kernel_tfc, grid, block, smem, st, K, F, P, tm.psi, tm.c, tab, tm.col_tab_len, psi_n, c_n,
+    e = launch_dep_smem(tfc_fn, grid, block, smem, st, K, F, P, tm.psi, tm.c, tab, tm.col_tab_len, psi_n, c_n,
                         phi_n, partials, err, wx, wy);
   } else if (pipe) {
     e = launch_dep_smem(pipe_fn[sh], dim3((unsigned)std::min(resident, nparts)), block, smem, st, K, F, P, tm.psi, tm.c,
@@ -2144,7 +2197,7 @@ int launch_step_f32_tma(const StepCoef &K, const Coef<float> &F, const StepScala
   } else {
     SurrArgs sa = {};
     if (surr) sa = *tm.surr;
-    e = launch_dep_smem(tile_fn[surr][sh], grid, block, smem, st, K, F, P, tm.psi, tm.c, tab, tm.col_tab_len, psi_n,
+    e = launch_dep_smem(tile_fn[row][sh], grid, block, smem, st, K, F, P, tm.psi, tm.c, tab, tm.col_tab_len, psi_n,
                         c_n, phi_n, partials, err, sa, wx, wy);
   }
   if (e != cudaSuccess) return -3;

@@ -217,7 +217,9 @@ struct Tab {
 // phases -> stores of its four warps, and a tile at the front takes long (its
 // phase 3 alone 6 to 8 rounds at 16 rows), so a grid whose 16-row tiles would
 // leave SMs idle takes lower ones (tile_rows).
-template <int TR>
+// RAW: the fields' rows are not 16-byte aligned (any nx): the tile is copied in
+// element by element, the cells leave by plain stores.
+template <int TR, bool RAW = false>
 struct TileOps {
 static constexpr int kTR = TR, kTRin = TR + 2;  // output and input rows
 static constexpr int kRowsPerWarp = TR / kWarps;
@@ -756,6 +758,14 @@ static __device__ __forceinline__ bool store_tile(const TileView &V, InSlot &in,
   const StepCoef &K = V.K;
   const int x0 = V.x0, y0 = V.y0;
   const int nrow = min(kTR, K.ny - 1 - y0);  // output rows of this tile inside the interior
+  if constexpr (RAW) {
+    gsync(bar);
+    for (int k = V.gtid; k < nrow * kW; k += kThreads) {
+      const int j = k / kW, x = k % kW;
+      raw_cell(V, y0 + j, x0 + x, in.psi[1 + j][4 + x], in.c[1 + j][4 + x], psi_n, c_n, phi_n);
+    }
+    return false;
+  }
   const int ncol = min(kW, K.nx - x0);       // columns of this tile inside the array (even)
   if (x0 == 0 || x0 + kW >= K.nx) {
     // ghost columns 0 and nx-1 (compute_boundary_individual, fun.cu:1220-1230)
@@ -876,9 +886,33 @@ static __device__ __forceinline__ uint32_t tile_vote(const TileView &V, const In
          (dm < 0x3FF00000u ? 0u : kNotFinite);
 }
 
+// one interior cell by plain stores, with the ghost cells that copy it (others
+// are left out)
+static __device__ __forceinline__ void raw_cell(const TileView &V, int r, int g, double pv, double c,
+                                                double *__restrict__ psi_n, double *__restrict__ c_n,
+                                                double *__restrict__ phi_n) {
+  const StepCoef &K = V.K;
+  if (g < 1 || g > K.nx - 2) return;
+  auto put = [&](int row, int col) {
+    const int64_t o = (int64_t)row * K.pitch + col;
+    psi_n[o] = pv;
+    c_n[o] = c;
+    if (phi_n) phi_n[o] = clamp1(pv);
+  };
+  auto row = [&](int rw) {
+    put(rw, g);
+    if (g == 1) put(rw, 0);
+    if (g == K.nx - 2) put(rw, K.nx - 1);
+  };
+  row(r);
+  if (r == K.jmin) row(0);
+  if (r == K.jmax) row(K.ny - 1);
+}
+
 // new psi (constant pv) and c of the lane's two cells of the output rows of
 // its warp straight to global memory, with the ghost columns and rows they
 // copy to
+// (raw: rows not 16-byte aligned, any nx; cell by cell)
 struct CellStore {
   double *pr, *cr, *fr;  // the lane's cells of the row to store next
   int64_t pitch;
@@ -899,6 +933,12 @@ struct CellStore {
   // row r = y0 - 1 + rr, the next one of the warp
   __device__ void put(const TileView &V, int rr, double pv, double c0, double c1, double *psi_n, double *c_n,
                       double *phi_n) {
+    if constexpr (RAW) {
+      const int r = V.y0 - 1 + rr;
+      raw_cell(V, r, V.gi, pv, c0, psi_n, c_n, phi_n);
+      raw_cell(V, r, V.gi + 1, pv, c1, psi_n, c_n, phi_n);
+      return;
+    }
     if (left) c0 = c1;
     if (right) c1 = c0;
     if (live) {
@@ -1086,10 +1126,23 @@ static __device__ __forceinline__ double solid_tile(const TileView &V, const InS
 // x0-4 .. x0+kW+3, rows y0-1 .. y0+kTR, zeros outside the array), each
 // column i read from clamp(i + i_offset, 1, nx - 2), with c = cinf where that
 // is nx - 2 (the melt entering at the right edge)
-static __device__ __forceinline__ void gather_pull_back(const StepCoef &K, const StepScalars &PS, int x0, int y0,
-                                                 InSlot &in) {
+// A step on unaligned rows (RAW) copies the same box, unshifted.
+static __device__ __forceinline__ void gather_box(const StepCoef &K, const StepScalars &PS, int x0, int y0,
+                                                  InSlot &in) {
   const double *__restrict__ psi = static_cast<const double *>(PS.src_psi);
   const double *__restrict__ c = static_cast<const double *>(PS.src_c);
+  if (!PS.pull_back) {
+    for (int k = threadIdx.x; k < kTRin * kWin; k += kThreads) {
+      const int rr = k / kWin, x = k % kWin;
+      const int row = y0 - 1 + rr, g = x0 - 4 + x;
+      const bool inside = row <= K.ny - 1 && g >= 0 && g <= K.nx - 1;
+      const int64_t o = inside ? (int64_t)row * K.pitch + g : 0;
+      cp_async_elem(&in.psi[rr][x], psi + o, inside);
+      cp_async_elem(&in.c[rr][x], c + o, inside);
+    }
+    cp_async_wait();
+    return;
+  }
   for (int k = threadIdx.x; k < kTRin * kWin; k += kThreads) {
     const int rr = k / kWin, x = k % kWin;
     const int row = y0 - 1 + rr, g = x0 - 4 + x;
@@ -1132,14 +1185,14 @@ struct alignas(128) PipeSmem64 {
   int abort;  // a wait gave up: every role stops
 };
 // ---------------------------------------------------------------- one tile per CTA
-template <int TR, bool TFC>
+template <int TR, bool TFC, bool RAW>
 __global__ void __launch_bounds__(kThreads, 5)
     tile_kernel_f64(const __grid_constant__ StepCoef K, const __grid_constant__ Coef<double> F,
                     const __grid_constant__ StepScalars PS, const __grid_constant__ CUtensorMap tm_psi,
                     const __grid_constant__ CUtensorMap tm_c, const double *__restrict__ tab, const int tab_len,
                     double *__restrict__ psi_n, double *__restrict__ c_n, double *__restrict__ phi_n,
                     BlockPartial *partials, int *err, const int wave_x, const int wave_y) {
-  using Ops = TileOps<TR>;
+  using Ops = TileOps<TR, RAW>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   auto &sm = *reinterpret_cast<typename Ops::template TileSmem<TFC> *>(smem_raw);
   // blockIdx.x walks the tile rows of one tile column, blockIdx.y the tile
@@ -1155,8 +1208,8 @@ __global__ void __launch_bounds__(kThreads, 5)
   }
   // a pull-back step reads column clamp(i + i_offset, 1, nx - 2) for column i
   // (pull_back, fun.cu:1469-1492): no TMA box has that shape, so the CTA
-  // gathers its tile (gather_pull_back) instead
-  const bool pb = PS.pull_back != 0;
+  // gathers its tile (gather_box) instead; so it does on unaligned rows
+  const bool pb = RAW || PS.pull_back != 0;
   if (threadIdx.x == 0) {
     mbar_init(&sm.full, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1194,7 +1247,7 @@ __global__ void __launch_bounds__(kThreads, 5)
       T.kp = kc_poly(K, tfc_T(K, PS.T_coarse, iT, x, jT, y));
     }
   }
-  if (pb) Ops::gather_pull_back(K, PS, x0, y0, sm.in);
+  if (pb) Ops::gather_box(K, PS, x0, y0, sm.in);
   __syncthreads();  // barrier initialised, flags cleared (and the TFC tables written)
   bool gave_up = false;
   if (!pb) {  // bounded wait for the tile
@@ -1447,34 +1500,39 @@ int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScal
                         double *psi_n, double *c_n, double *phi_n, BlockPartial *partials, int max_partials,
                         int *nparts_out, int *err, cudaStream_t st) {
   const int nj = K.ny - 2;
-  if (K.nx % 2 || K.pitch != K.nx) return -1;  // rows are copied in 16-byte units
+  const bool raw = P.raw != 0;
+  if ((K.nx % 2 && !raw) || K.pitch != K.nx) return -1;  // rows are copied in 16-byte units
   // the coarse-grid temperature: per-cell groups, no column table (the
   // persistent pipeline has no TFC form and is not taken then)
   const bool tfc = K.tfc != 0;
   if (tfc && !P.T_coarse) return -1;
-  const bool pipe = tm.pipeline != 0 && !tfc && !P.pull_back;
+  const bool pipe = tm.pipeline != 0 && !tfc && !P.pull_back && !raw;
   const int TR = tm.rows;  // the tensor maps' box is TR + 2 rows high
   if (!((TR == 4 && !tfc) || TR == 8 || TR == 16)) return -1;
-  const int nrt = (nj + TR - 1) / TR, ncb = (K.nx + kW - 1) / kW;
+  // (raw: the tile that holds the last interior column writes the ghost column)
+  const int nrt = (nj + TR - 1) / TR, ncb = (K.nx - raw + kW - 1) / kW;
   if (ncb > 65535 || (int64_t)nrt * ncb > (1 << 30)) return -1;
   const int nparts = nrt * ncb;
   if (partials && nparts > max_partials) return -1;
   if (!tm.col_tab64 || tm.col_tab64_len < ncb * kW + kWin) return -1;
-  using Kfn = decltype(&tile_kernel_f64<16, false>);
-  static const Kfn tile_fn[2][3] = {{tile_kernel_f64<4, false>, tile_kernel_f64<8, false>, tile_kernel_f64<16, false>},
-                                    {nullptr, tile_kernel_f64<8, true>, tile_kernel_f64<16, true>}};
+  using Kfn = decltype(&tile_kernel_f64<16, false, false>);
+  static const Kfn tile_fn[2][2][3] = {  // [raw][tfc][height]
+      {{tile_kernel_f64<4, false, false>, tile_kernel_f64<8, false, false>, tile_kernel_f64<16, false, false>},
+       {nullptr, tile_kernel_f64<8, true, false>, tile_kernel_f64<16, true, false>}},
+      {{tile_kernel_f64<4, false, true>, tile_kernel_f64<8, false, true>, tile_kernel_f64<16, false, true>},
+       {nullptr, tile_kernel_f64<8, true, true>, tile_kernel_f64<16, true, true>}}};
   static const size_t tile_smem[2][3] = {
       {sizeof(TileOps<4>::TileSmem<false>), sizeof(TileOps<8>::TileSmem<false>), sizeof(TileOps<16>::TileSmem<false>)},
       {0, sizeof(TileOps<8>::TileSmem<true>), sizeof(TileOps<16>::TileSmem<true>)}};
   const int sh = TR == 4 ? 0 : TR == 8 ? 1 : 2;
   static const decltype(&pipe_kernel_f64<16>) pipe_fn[3] = {pipe_kernel_f64<4>, pipe_kernel_f64<8>, pipe_kernel_f64<16>};
   static const size_t pipe_smem[3] = {sizeof(PipeSmem64<4>), sizeof(PipeSmem64<8>), sizeof(PipeSmem64<16>)};
-  const int which = pipe ? 6 + sh : 3 * tfc + sh;
+  const int which = pipe ? 12 + sh : 6 * raw + 3 * tfc + sh;
   const size_t smem = pipe ? pipe_smem[sh] : tile_smem[tfc][sh];
-  const void *kfn = pipe ? (const void *)pipe_fn[sh] : (const void *)tile_fn[tfc][sh];
-  static std::atomic<unsigned long long> attr_done[9];
+  const void *kfn = pipe ? (const void *)pipe_fn[sh] : (const void *)tile_fn[raw][tfc][sh];
+  static std::atomic<unsigned long long> attr_done[15];
   if (!smem_limit_once(kfn, (int)smem, attr_done[which])) return -3;
-  static std::atomic<int> resident_of[9][64];
+  static std::atomic<int> resident_of[15][64];
   const int resident = resident_ctas(kfn, pipe ? kPipeThreads : kThreads, smem, resident_of[which]);
   if (resident <= 0) return -3;
   cudaLaunchAttribute at[1];
@@ -1506,7 +1564,7 @@ int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScal
     // column-major: consecutive CTAs share a column strip and its halo rows in L2
     cfg.gridDim = dim3(nrt, ncb);
     cfg.blockDim = dim3(kThreads);
-    e = cudaLaunchKernelEx(&cfg, tile_fn[tfc][sh], K, F, P, tm.psi, tm.c, tab, tm.col_tab64_len, psi_n, c_n, phi_n,
+    e = cudaLaunchKernelEx(&cfg, tile_fn[raw][tfc][sh], K, F, P, tm.psi, tm.c, tab, tm.col_tab64_len, psi_n, c_n, phi_n,
                            partials, err, resident % nrt, resident / nrt);
   }
   if (e != cudaSuccess) return -3;

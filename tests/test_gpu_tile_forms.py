@@ -45,9 +45,14 @@ def state(p, kind, seed):
 SIZES = [(64, 18), (128, 19), (260, 8), (320, 66), (2048, 371), (2052, 372), (2048, 1127), (2112, 1045), (2048, 1500)]
 
 
+# rows that are not 16-byte aligned: a last tile column of one cell more or less than full, of the ghost column alone
+ODD_SIZES = [(63, 18), (65, 19), (66, 20), (129, 66), (131, 22), (257, 40), (2047, 371), (2049, 372), (2049, 1127),
+             (2111, 1045)]
+
+
 @pytest.mark.parametrize("dtype", ["f64", "f32"])
 @pytest.mark.parametrize("kind", ["melt", "layer", "solid", "front"])
-@pytest.mark.parametrize("nx,ny", SIZES)
+@pytest.mark.parametrize("nx,ny", SIZES + ODD_SIZES)
 def test_tile_forms_match_the_oracle(nx, ny, kind, dtype):
     p = configs.small(nx, ny, i_tip_target=nx // 2, G=5e6, V=0.5, noise_amplitude=0.02, seed=9)
     d = pyoracle.derive(p)
@@ -96,3 +101,55 @@ def test_tfc_tile_forms_match_the_oracle(nx, ny):
     o = pyoracle.step(p, d, s, 0, T_fine=Tf)
     g = download(p, nxt)
     assert maxabs(g.psi, o.psi) <= 1e-13 and maxabs(g.c, o.c) <= 1e-13
+
+
+@pytest.mark.parametrize("periodic", [1, 0])
+@pytest.mark.parametrize("off", [None, -3, 0, 5])
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("nx,shift", [(129, 0), (67, 0), (128, 1)])
+def test_unaligned_rows_shifts_and_ghosts(nx, shift, dtype, off, periodic):
+    """Odd row lengths, and aligned ones in buffers that start one element off
+    (every row unaligned): with and without a fused pull-back, both boundary
+    kinds, every ghost cell compared."""
+    dt = torch.float64 if dtype == "f64" else torch.float32
+    p = configs.small(nx, 37, i_tip_target=nx // 2, G=5e6, V=0.5, noise_amplitude=0.02, seed=9, periodic_j=periodic)
+    d = pyoracle.derive(p)
+    s = state(p, "front", nx)
+    if dt == torch.float32:
+        s.psi[:] = s.phi[:] = s.psi.astype(np.float32)
+        s.c[:] = (s.c - p.cinf).astype(np.float32).astype(np.float64) + p.cinf
+    ctx = lib.Context(p)
+    cur, nxt = upload(p, s, dt), lib.FieldSet(p, dt, with_phi=True)
+    for fs in (cur, nxt):
+        for k in ("psi", "c", "phi"):
+            t = getattr(fs, k)
+            if t is not None and shift:
+                buf = torch.empty(t.numel() + shift, dtype=dt, device="cuda")
+                v = buf[shift:].view(t.shape)
+                v.copy_(t)
+                setattr(fs, k, v)
+    ctx.step(cur, nxt, 3, i_offset_history=1, l_offset_Vp=0.2, pull_back=off)
+    ctx.device_status()
+    so = s if off is None else pyoracle.pull_back(p, s, off)
+    o = pyoracle.step(p, d, so, 3, 1, 0.2)
+    g = download(p, nxt)
+    tol_psi, tol_c = (1e-13, 1e-13) if dt == torch.float64 else (5e-6, 5e-8)
+    assert maxabs(g.psi, o.psi) <= tol_psi and maxabs(g.phi, o.phi) <= tol_psi and maxabs(g.c, o.c) <= tol_c
+
+
+@pytest.mark.parametrize("nx", [129, 2047])
+def test_unaligned_rows_with_a_network_set_stay_exact(nx):
+    """Rows that are not 16-byte aligned take the exact evaluation whether or not
+    a network is set, and audit nothing."""
+    from rapidsolid import surrogate
+    p = configs.small(nx, 40, i_tip_target=nx // 2, G=5e6, V=0.5)
+    s = state(p, "front", 5)
+    ctx = lib.Context(p)
+    cur, a, b = upload(p, s, torch.float32), lib.FieldSet(p, torch.float32), lib.FieldSet(p, torch.float32)
+    ctx.step(cur, a, 0)
+    box = surrogate.fitted_box()
+    box.y_scale[0] = box.y_scale[1] = 100.0
+    ctx.set_surrogate(torch.from_numpy(surrogate.init_weights(1)).cuda(), box)
+    ctx.step(cur, b, 0)
+    assert torch.equal(a.psi, b.psi) and torch.equal(a.c, b.c)
+    assert ctx.surrogate_audit()[2:] == (0, 0)
