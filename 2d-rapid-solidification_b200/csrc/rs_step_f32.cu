@@ -468,13 +468,19 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     const float *__restrict__ gpsi = static_cast<const float *>(PS.src_psi);
     const float *__restrict__ gd = static_cast<const float *>(PS.src_c);
     if (!PS.pull_back) {
-      for (int k = threadIdx.x; k < kTRin * kWin; k += kThreads) {
-        const int rr = k / kWin, x = k % kWin;
-        const int row = y0 - 1 + rr, g = x0 - 4 + x;
-        const bool inside = row <= ny - 1 && g >= 0 && g <= nx - 1;
-        const int64_t o = inside ? (int64_t)row * K.pitch + g : 0;
-        cp_async_elem(&sm.psi[rr][x], gpsi + o, inside);
-        cp_async_elem(&sm.d[rr][x], gd + o, inside);
+      // a warp per row, every fourth row; columns lane, lane + 32, ...
+      for (int rr = warp; rr < kTRin; rr += kWarps) {
+        const int row = y0 - 1 + rr;
+        const int64_t o = (int64_t)min(row, ny - 1) * K.pitch + x0 - 4 + lane;
+#pragma unroll
+        for (int q = 0; q < (kWin + 31) / 32; ++q) {
+          const int x = lane + 32 * q, g = x0 - 4 + x;
+          const bool inside = row <= ny - 1 && g >= 0 && g <= nx - 1;
+          if (x < kWin) {
+            cp_async_elem(&sm.psi[rr][x], gpsi + (inside ? o + 32 * q : 0), inside);
+            cp_async_elem(&sm.d[rr][x], gd + (inside ? o + 32 * q : 0), inside);
+          }
+        }
       }
       cp_async_wait();
     }
@@ -607,8 +613,12 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     const float pv = melt ? -1.f : 1.f;
     auto put = [&](int j, float (&v)[4]) {
       if constexpr (RAW) {
+        // through the warp's row of mu, so that each store is of 32 adjacent cells
+        st4(&sm.mu[warp][4 * lane], v[0], v[1], v[2], v[3]);
+        __syncwarp();
 #pragma unroll
-        for (int q = 0; q < 4; ++q) raw_cell(y0 + r0 + j, gi + q, pv, v[q]);
+        for (int q = 0; q < 4; ++q) raw_cell(y0 + r0 + j, x0 + lane + 32 * q, pv, sm.mu[warp][lane + 32 * q]);
+        __syncwarp();
         return;
       }
       if (gi == 0) v[0] = v[1];         // ghost column 0
@@ -648,7 +658,7 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
       // far melt: phases 1 and 2 with S and mu'' of the warp's rows in
       // registers (the same expressions, so the same bits); halo columns by a
       // lane per cell through scratch
-      float *hs = &sm.S[warp][0], *hm = &sm.mu[warp][0];
+      float *hs = &sm.S[warp][0], *hm = &sm.S[warp][kWin / 2];
       if (lane < 2 * (kRowsPerWarp + 2)) {
         const int rr = r0 + (lane >> 1), x = (lane & 1) ? kHaloR : kHaloL;
         float Sh = 0.f, mh = 0.f;

@@ -916,8 +916,10 @@ static __device__ __forceinline__ void raw_cell(const TileView &V, int r, int g,
 struct CellStore {
   double *pr, *cr, *fr;  // the lane's cells of the row to store next
   int64_t pitch;
+  double *stage;  // RAW: a row of shared memory of the warp's own
   bool live, left, right, ghost;
-  __device__ CellStore(const TileView &V, double *psi_n, double *c_n, double *phi_n) {
+  __device__ CellStore(const TileView &V, double *stage_, double *psi_n, double *c_n, double *phi_n)
+      : stage(stage_) {
     const StepCoef &K = V.K;
     const int r = V.y0 + kRowsPerWarp * V.gw;
     pitch = K.pitch;
@@ -935,8 +937,11 @@ struct CellStore {
                       double *phi_n) {
     if constexpr (RAW) {
       const int r = V.y0 - 1 + rr;
-      raw_cell(V, r, V.gi, pv, c0, psi_n, c_n, phi_n);
-      raw_cell(V, r, V.gi + 1, pv, c1, psi_n, c_n, phi_n);
+      st2(stage + V.col, c0, c1);  // so that each store is of 32 adjacent cells
+      __syncwarp();
+      raw_cell(V, r, V.x0 + V.lane, pv, stage[V.lane], psi_n, c_n, phi_n);
+      raw_cell(V, r, V.x0 + V.lane + 32, pv, stage[V.lane + 32], psi_n, c_n, phi_n);
+      __syncwarp();
       return;
     }
     if (left) c0 = c1;
@@ -970,7 +975,8 @@ struct CellStore {
 // so the arithmetic of the rows overlaps.  Returns the warp's part of the mass.
 template <bool TFC>
 static __device__ __forceinline__ double melt_tile(const TileView &V, const LaneCols &LC, const InSlot &in, MeltHalo &mh,
-                                            const TfcTile *tf, bool red, double *__restrict__ psi_n, double *__restrict__ c_n,
+                                            const TfcTile *tf, bool red, double *stage, double *__restrict__ psi_n,
+                                            double *__restrict__ c_n,
                                             double *__restrict__ phi_n) {
   const Coef<double> &F = V.F;
   const int lane = V.lane, r0 = kRowsPerWarp * V.gw;
@@ -1050,7 +1056,7 @@ static __device__ __forceinline__ double melt_tile(const TileView &V, const Lane
 #pragma unroll
     for (int q = 0; q < 2; ++q) jv[q] = __dmul_rn(fma(6.0, pp[q + 1], pp[q] + pp[q + 2]), B.m[q] - A.m[q]);
   };
-  CellStore out(V, psi_n, c_n, phi_n);
+  CellStore out(V, stage, psi_n, c_n, phi_n);
   double mass = 0.0, jv_lo[2], jv_hi[2];
   Row rb, rc;
   Pairs pa, pb, pc;
@@ -1096,12 +1102,12 @@ static __device__ __forceinline__ double melt_tile(const TileView &V, const Lane
 
 // a deep solid tile: S = 0 in every cell, so every flux is 0 and psi and c
 // stay (itip: the last interior column, as phase 4 counts it)
-static __device__ __forceinline__ double solid_tile(const TileView &V, const InSlot &in, bool red,
+static __device__ __forceinline__ double solid_tile(const TileView &V, const InSlot &in, bool red, double *stage,
                                              double *__restrict__ psi_n, double *__restrict__ c_n,
                                              double *__restrict__ phi_n, int &itip) {
   const int r0 = kRowsPerWarp * V.gw, rows_live = V.K.ny - 1 - V.y0, nx = V.K.nx;
   const double c_floor = V.F.c_floor;
-  CellStore out(V, psi_n, c_n, phi_n);
+  CellStore out(V, stage, psi_n, c_n, phi_n);
   double mass = 0.0;
 #pragma unroll
   for (int j = 0; j < kRowsPerWarp; ++j) {
@@ -1132,13 +1138,20 @@ static __device__ __forceinline__ void gather_box(const StepCoef &K, const StepS
   const double *__restrict__ psi = static_cast<const double *>(PS.src_psi);
   const double *__restrict__ c = static_cast<const double *>(PS.src_c);
   if (!PS.pull_back) {
-    for (int k = threadIdx.x; k < kTRin * kWin; k += kThreads) {
-      const int rr = k / kWin, x = k % kWin;
-      const int row = y0 - 1 + rr, g = x0 - 4 + x;
-      const bool inside = row <= K.ny - 1 && g >= 0 && g <= K.nx - 1;
-      const int64_t o = inside ? (int64_t)row * K.pitch + g : 0;
-      cp_async_elem(&in.psi[rr][x], psi + o, inside);
-      cp_async_elem(&in.c[rr][x], c + o, inside);
+    // a warp per row, every fourth row; columns lane, lane + 32, lane + 64
+    const int lane = threadIdx.x & 31;
+    for (int rr = threadIdx.x >> 5; rr < kTRin; rr += kWarps) {
+      const int row = y0 - 1 + rr;
+      const int64_t o = (int64_t)min(row, K.ny - 1) * K.pitch + x0 - 4 + lane;
+#pragma unroll
+      for (int q = 0; q < (kWin + 31) / 32; ++q) {
+        const int x = lane + 32 * q, g = x0 - 4 + x;
+        const bool inside = row <= K.ny - 1 && g >= 0 && g <= K.nx - 1;
+        if (x < kWin) {
+          cp_async_elem(&in.psi[rr][x], psi + (inside ? o + 32 * q : 0), inside);
+          cp_async_elem(&in.c[rr][x], c + (inside ? o + 32 * q : 0), inside);
+        }
+      }
     }
     cp_async_wait();
     return;
@@ -1260,6 +1273,22 @@ __global__ void __launch_bounds__(kThreads, 5)
       }
     }
   }
+  if constexpr (RAW) {
+    // as below, line by line
+    int bx = (int)blockIdx.x + wave_x, by = (int)blockIdx.y + wave_y;
+    if (bx >= (int)gridDim.x) {
+      bx -= (int)gridDim.x;
+      ++by;
+    }
+    if (by < (int)gridDim.y && !PS.pull_back) {
+      const int px = max(kW * front_first_block(by, f, (int)gridDim.y) - 4, 0), py = TR * bx;
+      for (int k = threadIdx.x; k < Ops::kTRin * 6 * 2; k += kThreads) {
+        const int row = min(py + (k >> 1) / 6, K.ny - 1), x = min(px + 16 * ((k >> 1) % 6), K.nx - 1);
+        const double *q = static_cast<const double *>((k & 1) ? PS.src_psi : PS.src_c) + (int64_t)row * K.pitch + x;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
+      }
+    }
+  }
   // pull the tile of the CTA that will start about one resident wave later
   // (wave_y tile columns and wave_x tile rows on) into L2, so its loads
   // overlap the rest of this wave's arithmetic
@@ -1307,9 +1336,9 @@ __global__ void __launch_bounds__(kThreads, 5)
   if (melt || !(vote & (Ops::kNotPlus1 | Ops::kNotFinite))) {
     if (melt)
       mass = Ops::template melt_tile<TFC>(V, LC, sm.in, *reinterpret_cast<typename Ops::MeltHalo *>(sm.p2.list), tf, red,
-                                          psi_n, c_n, phi_n);
+                                          sm.st.S[V.gw], psi_n, c_n, phi_n);
     else
-      mass = Ops::solid_tile(V, sm.in, red, psi_n, c_n, phi_n, itip);
+      mass = Ops::solid_tile(V, sm.in, red, sm.st.S[V.gw], psi_n, c_n, phi_n, itip);
     Ops::finish_tile(V, sm.p2, mass, itip, part, 0);
     return;
   }
