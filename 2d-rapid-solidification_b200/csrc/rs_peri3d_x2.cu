@@ -12,6 +12,17 @@
 // the melt are not lost below ulp(c); mu is carried as mu - c_off (only its
 // differences and s_i - r_i mu enter), with c_off folded into the s_i.
 //
+// What bounds it (512^3): memory where a plane is melt, the packed FMA pipe
+// where it is not.  Pure-melt planes (CTA vote over the box) take c - r1 as mu
+// straight from the loaded c, with no mu plane; a slot goes back to the load
+// engine when the last warp leaves the plane, so two plane loads of a CTA are
+// in flight (before: one, issued behind the next plane's arrival); ghost images
+// are written in a loop beside the path that most rows take, which also took
+// the register spills away.  All melt 574 us (86 % of the copy rate), a front
+// in 90 of the 512 planes 695 us, before 957 us.  The z chunk is the slowest
+// grid index: with it the fastest, x and y neighbours no longer share their
+// halos in L2 (629 and 736 us).
+//
 // Tile: output cells x0 .. x0+63 (x0 a multiple of 64, pairs start on even
 // x), rows y0+1 .. y0+14.  Input box per field and plane: x0-4 .. x0+67
 // (72 columns, TMA x 16-byte aligned) x y0 .. y0+15 (16 rows).  224 threads:
@@ -20,13 +31,14 @@
 #include <cuda.h>
 
 #include "rs_f32x2.cuh"
+#include "rs_kernels.cuh"
 #include "rs_peri3d.cuh"
 #include "rs_step_common.cuh"
 
 namespace rs {
 namespace {
 
-constexpr int kX2Threads = 224;
+constexpr int kX2Threads = 224, kX2Warps = kX2Threads / 32;
 constexpr int kX2BX = 64, kX2BXin = 72, kX2BY = 14, kX2BYin = 16;
 constexpr int kX2Plane = kX2BXin * kX2BYin;  // 1152 floats = 4608 bytes (36 x 128)
 constexpr int kX2Slots = 4, kX2MuSlots = 4;
@@ -41,6 +53,7 @@ struct X2Smem {
   // per plane (q mod 8): every cell of the box inside the array is pure melt,
   // phi1 == 1 and phi2 == 0 exactly
   int melt[8];
+  uint32_t passed;  // warps that have left a plane, summed over the planes
 };
 constexpr unsigned long long kOne2 = 0x3F8000003F800000ull, kAbs2 = 0x7FFFFFFF7FFFFFFFull;
 
@@ -86,6 +99,8 @@ __global__ void __launch_bounds__(kX2Threads, 3)
   const int zo1 = min(zo0 + k.z_chunk, k.nz - 1);
   if (zo0 >= zo1) return;
   const int zin0 = zo0 - 1, zin1 = zo1;
+  pdl_wait();
+  pdl_trigger();
   constexpr uint32_t kBytes = 3u * kX2Plane * sizeof(float);
   if (smem_u32(smem_raw) & 127u) {
     if (tid == 0) atomicExch(err, 2);
@@ -103,6 +118,7 @@ __global__ void __launch_bounds__(kX2Threads, 3)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int z = zin0; z <= min(zin1, zin0 + kX2Slots - 1); ++z) issue(z);
     for (int s = 0; s < 8; ++s) sm.melt[s] = 1;
+    sm.passed = 0u;
   }
   __syncthreads();
   int issued = min(zin1, zin0 + kX2Slots - 1);
@@ -116,24 +132,47 @@ __global__ void __launch_bounds__(kX2Threads, 3)
       }
     return true;
   };
-  auto mu_plane = [&](int z) {
+  // Planes of pure melt (outside the array counts as melt: no stencil of an
+  // output cell reaches it).  A quad of the box lies wholly inside or outside
+  // (nx % 4 == 0, x0 - 4 a multiple of 4); bit u: quad 4 (tid + kX2Threads u) outside.
+  constexpr int kQuads = (kX2Plane / 4 + kX2Threads - 1) / kX2Threads;
+  uint32_t outside = 0u;
+#pragma unroll
+  for (int u = 0; u < kQuads; ++u) {
+    const int e = 4 * (tid + kX2Threads * u), ax = x0 - 4 + e % kX2BXin, ay = yb + e / kX2BXin;
+    if (!(ax >= 0 && ax < k.nx && ay < k.ny)) outside |= 1u << u;
+  }
+  auto check_plane = [&](int z) {
     const bool got = wait_plane(z);
+    const int q = z - zin0, s = q % kX2Slots;
+    if (got) {
+      uint32_t diff = 0u;
+#pragma unroll
+      for (int u = 0; u < kQuads; ++u) {
+        const int e = 4 * (tid + kX2Threads * u);
+        if (e >= kX2Plane) break;  // (warp-uniform)
+        const uint4 a = *reinterpret_cast<const uint4 *>(&sm.in[s][0][e]);
+        const uint4 b = *reinterpret_cast<const uint4 *>(&sm.in[s][1][e]);
+        const uint32_t one = 0x3F800000u;
+        const uint32_t d = (a.x ^ one) | (a.y ^ one) | (a.z ^ one) | (a.w ^ one) | ((b.x | b.y | b.z | b.w) << 1);
+        if (!((outside >> u) & 1u)) diff |= d;
+      }
+      if (diff) sm.melt[q & 7] = 0;
+    }
+    return got;
+  };
+  // mu of plane z (already loaded)
+  auto mu_plane = [&](int z) {
     const int q = z - zin0, s = q % kX2Slots;
     float *mu = sm.mu[q % kX2MuSlots];
     const float *f1 = sm.in[s][0], *f2p = sm.in[s][1], *fc = sm.in[s][2];
-    if (got) {
-      bool all_melt = true;  // this thread's pairs inside the array
-      for (int e = 2 * tid; e < kX2Plane; e += 2 * kX2Threads) {
-        const f2 p1 = ld2(f1 + e), p2 = ld2(f2p + e);
-        st2(mu + e, mu2(k, p1, p2, ld2(fc + e)));
-        // a pair lies wholly inside or outside the array (nx % 4 == 0, even x)
-        const int ax = x0 - 4 + e % kX2BXin, ay = yb + e / kX2BXin;
-        const bool inside = ax >= 0 && ax < k.nx && ay < k.ny;
-        all_melt = all_melt && (!inside || ((unsigned long long)p1 == kOne2 && ((unsigned long long)p2 & kAbs2) == 0ull));
-      }
-      if (!all_melt) sm.melt[q & 7] = 0;
+    for (int e = 2 * tid; e < kX2Plane; e += 2 * kX2Threads) {  // (warp-uniform)
+      const f2 p1 = ld2(f1 + e), p2 = ld2(f2p + e), c = ld2(fc + e);
+      const bool melt = (unsigned long long)p1 == kOne2 && ((unsigned long long)p2 & kAbs2) == 0ull;
+      // a warp of pure melt: g_1 = 1 and g_2 = g_3 = 0, so mu2 is c - r1 in
+      // one rounding
+      st2(mu + e, __all_sync(0xffffffffu, melt) ? sub2(c, bc(k.r1)) : mu2(k, p1, p2, c));
     }
-    return got;
   };
   auto drain = [&](int from) {
     if (tid == 0)
@@ -144,8 +183,8 @@ __global__ void __launch_bounds__(kX2Threads, 3)
         }
       }
   };
-  bool ok = mu_plane(zin0);
-  ok = mu_plane(zin0 + 1) && ok;
+  bool ok = check_plane(zin0);
+  ok = check_plane(zin0 + 1) && ok;
   if (!__syncthreads_and(ok)) {
     drain(zin0);
     return;
@@ -157,88 +196,105 @@ __global__ void __launch_bounds__(kX2Threads, 3)
   const int ry = 2 * warp;                             // first output row of the thread (tile row)
   const int ec = (ry + 1) * kX2BXin + 2 * lane + 4;    // box element of its first cell (even)
   const int64_t plane = (int64_t)k.nx * k.ny;
-  const bool xedge = !(v0 && v1) || gx == 1 || gx + 1 == k.nx - 2;  // a ghost column is involved
+  const bool xedge = !(v0 && v1);                      // one output, whose image is a ghost column
 
-  for (int z = zo0; z < zo1; ++z) {
-    // one barrier per plane: after it every thread has finished plane z-1,
-    // so the input slot of plane z-2 takes the load of plane z+2 (mu has
-    // four slots: mu(z+1) overwrites mu(z-3))
-    if (!__syncthreads_and(mu_plane(z + 1))) {
+  // mu is stored for the planes that the general form reads, ahead of the
+  // barrier while the march is in it; a march that enters it from pure melt
+  // makes up for the missing planes behind the barrier.  Uniform over the CTA.
+  int64_t out0 = (int64_t)zo0 * plane + (int64_t)(yb + 1 + ry) * k.nx + gx;  // the pair's first cell in plane z
+  int mu_done = zin0 - 1;   // mu of planes .. mu_done stands, as far as the ring goes
+  bool general = false;
+  for (int z = zo0; z < zo1; ++z, out0 += plane) {
+    // one barrier per plane: the flags and mu of planes .. z+1 stand behind it
+    // (mu has four slots: mu(z+1) overwrites mu(z-3))
+    const bool got = check_plane(z + 1);
+    if (general && got) mu_plane(z + 1);
+    if (general) mu_done = z + 1;
+    if (!__syncthreads_and(got)) {
+      issued = min(zin1, z + 2);
       drain(z + 1);
       return;
     }
-    if (z + 2 <= zin1 && z + 2 > issued) {
-      if (tid == 0) issue(z + 2);
-      issued = z + 2;
-    }
     const int q = z - zin0;
     // planes z-1 .. z+1 pure melt wherever a stencil of an output cell
-    // reaches (the flag of plane z+3 is re-armed here: its computation,
-    // mu_plane(z+3) before the barrier of iteration z+2, is separated from
-    // this write by the barrier of z+1)
+    // reaches (the flag of plane z+3 is re-armed here: check_plane(z+3), before
+    // the barrier of iteration z+2, is separated from this write by the barrier
+    // of z+1)
     const bool melt3 = sm.melt[(q - 1) & 7] && sm.melt[q & 7] && sm.melt[(q + 1) & 7];
     if (tid == 0) sm.melt[(q + 3) & 7] = 1;
+    if (!melt3 && mu_done < z + 1) {
+      for (int w = max(z - 1, mu_done + 1); w <= z + 1; ++w) mu_plane(w);
+      mu_done = z + 1;
+      __syncthreads();
+    }
+    general = !melt3;
     const float *c1 = sm.in[q % kX2Slots][0], *c2 = sm.in[q % kX2Slots][1], *cc = sm.in[q % kX2Slots][2];
     const float *d1 = sm.in[(q - 1) % kX2Slots][0], *d2 = sm.in[(q - 1) % kX2Slots][1];
     const float *u1 = sm.in[(q + 1) % kX2Slots][0], *u2 = sm.in[(q + 1) % kX2Slots][1];
     const float *mu = sm.mu[q % kX2MuSlots], *mud = sm.mu[(q - 1) % kX2MuSlots], *muu = sm.mu[(q + 1) % kX2MuSlots];
-    const double Tz = k.G_T == 0.0 ? k.T_ref : k.T_ref + k.G_T * ((double)z - k.z_T - k.V_T * (double)step);
-    const double B1 = k.B11 + k.B12 * Tz, B2 = k.B21 + k.B22 * Tz;
-    // s_i - r_i c_off: the fields hold c - c_off, so mu - c_off is what mu2 returns
-    const f2 s1 = bc((float)(B1 - k.r1d * k.c_off)), s2 = bc((float)(-B1 - B2 - k.r2d * k.c_off)),
-             s3 = bc((float)(-B1 + B2 - k.r3d * k.c_off));
-    const int zg = z == 1 ? 0 : (z == k.nz - 2 ? k.nz - 1 : -1);
+    const int zd = z == 1 ? -1 : (z == k.nz - 2 ? 1 : 0);  // planes 0 and nz-1 copy their neighbours
     // stores: the pair, and every ghost cell that images one of its cells
-    auto store_pair = [&](int gy, f2 n1, f2 n2, f2 nc) {
-      const int yg = gy == k.ny - 2 ? 0 : (gy == 1 ? k.ny - 1 : -1);
-      const int64_t o = (int64_t)z * plane + (int64_t)gy * k.nx + gx;
-      if (!xedge && (yg & zg) < 0) {
+    // (rows and planes: uniform over the warp; columns: the pairs (0, 1) and
+    // (nx-2, nx-1), one cell and its image each)
+    auto store_row = [&](int64_t o, f2 n1, f2 n2, f2 nc) {  // o: the pair's first cell
+      if (!xedge) {
         st2(o1 + o, n1);
         st2(o2 + o, n2);
         st2(oc + o, nc);
       } else {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int x = gx + h;
-          if (!(h ? v1 : v0)) continue;
-          const float a = h ? hi_of(n1) : lo_of(n1), bb = h ? hi_of(n2) : lo_of(n2), cv = h ? hi_of(nc) : lo_of(nc);
-          const int xg = x == k.nx - 2 ? 0 : (x == 1 ? k.nx - 1 : -1);
-          const int xs[2] = {x, xg}, ys[2] = {gy, yg}, zs[2] = {z, zg};
-#pragma unroll
-          for (int ia = 0; ia < 2; ++ia)
-#pragma unroll
-            for (int ib = 0; ib < 2; ++ib)
-#pragma unroll
-              for (int ic = 0; ic < 2; ++ic) {
-                if (xs[ia] < 0 || ys[ib] < 0 || zs[ic] < 0) continue;
-                const int64_t oo = (int64_t)zs[ic] * plane + (int64_t)ys[ib] * k.nx + xs[ia];
-                o1[oo] = a;
-                o2[oo] = bb;
-                oc[oo] = cv;
-              }
+        const float a = v1 ? hi_of(n1) : lo_of(n1), b2 = v1 ? hi_of(n2) : lo_of(n2), cv = v1 ? hi_of(nc) : lo_of(nc);
+        const int64_t oi = o + (v1 ? 1 : 0), og = oi + (v1 ? k.nx - 2 : 2 - k.nx);
+        o1[oi] = a, o1[og] = a;
+        o2[oi] = b2, o2[og] = b2;
+        oc[oi] = cv, oc[og] = cv;
+      }
+    };
+    auto store_pair = [&](int r, f2 n1, f2 n2, f2 nc) {
+      const int64_t o = out0 + r * k.nx;
+      store_row(o, n1, n2, nc);
+      const int gy = yb + 1 + ry + r;
+      const int yd = gy == k.ny - 2 ? 2 - k.ny : (gy == 1 ? k.ny - 2 : 0);  // to the image row, plane
+      if (yd | zd) {
+#pragma unroll 1
+        for (int im = 1; im < 4; ++im) {
+          if (((im & 1) && !yd) || ((im & 2) && !zd)) continue;
+          store_row(o + (im & 1 ? (int64_t)yd * k.nx : 0) + (im & 2 ? zd * plane : 0), n1, n2, nc);
         }
       }
     };
     if (any && melt3) {
       // pure-melt neighbourhood: phi1 and phi2 stay exactly 1 and 0 (every
-      // phase term and Laplacian is a zero there) and every face mobility is
-      // phi1 + phi1' = 2 exactly (the solid terms vanish), so the solute
-      // update is c + sum_d cf_d 2 ((mu+ - mu) + (mu- - mu)), the general
-      // form's value bit for bit
+      // phase term and Laplacian is a zero there), mu is c - r1 and every face
+      // mobility is phi1 + phi1' = 2 exactly (the solid terms vanish), so the
+      // solute update is c + sum_d cf_d 2 ((mu+ - mu) + (mu- - mu)), the
+      // general form's value bit for bit, and mu needs no plane of its own
+      const float *cd = sm.in[(q - 1) % kX2Slots][2], *cu = sm.in[(q + 1) % kX2Slots][2];
+      const f2 r1 = bc(k.r1);
+      f2 w[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) w[r] = ld2(cc + ec + (r - 1) * kX2BXin);
+      const f2 c0[2] = {w[1], w[2]};
+#pragma unroll
+      for (int r = 0; r < 4; ++r) w[r] = sub2(w[r], r1);
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const int gy = yb + 1 + ry + r;
         if (gy > k.ny - 2) break;
         const int e = ec + r * kX2BXin;
-        const f2 m0 = ld2(mu + e);
-        const f2 Lm = ld2(mu + e - 2), Rm = ld2(mu + e + 2);
-        auto face_m = [&](f2 mp, f2 mm) { return mul2(bc(2.f), add2(sub2(mp, m0), sub2(mm, m0))); };
-        f2 nc = fma2(face_m(pk(hi_of(m0), lo_of(Rm)), pk(hi_of(Lm), lo_of(m0))), bc(k.cfx), ld2(cc + e));
-        nc = fma2(face_m(ld2(mu + e + kX2BXin), ld2(mu + e - kX2BXin)), bc(k.cfy), nc);
-        nc = fma2(face_m(ld2(muu + e), ld2(mud + e)), bc(k.cfz), nc);
-        store_pair(gy, bc(1.f), bc(0.f), nc);
+        const f2 m0 = w[r + 1];
+        const f2 Lm = sub2(ld2(cc + e - 2), r1), Rm = sub2(ld2(cc + e + 2), r1);
+        auto face_m = [&](f2 mp, f2 mm) { return add2(sub2(mp, m0), sub2(mm, m0)); };
+        f2 nc = fma2(face_m(pk(hi_of(m0), lo_of(Rm)), pk(hi_of(Lm), lo_of(m0))), bc(2.f * k.cfx), c0[r]);  // (the 2: exact)
+        nc = fma2(face_m(w[r + 2], w[r]), bc(2.f * k.cfy), nc);
+        nc = fma2(face_m(sub2(ld2(cu + e), r1), sub2(ld2(cd + e), r1)), bc(2.f * k.cfz), nc);
+        store_pair(r, bc(1.f), bc(0.f), nc);
       }
     } else if (any) {
+      const double Tz = k.G_T == 0.0 ? k.T_ref : k.T_ref + k.G_T * ((double)z - k.z_T - k.V_T * (double)step);
+      const double B1 = k.B11 + k.B12 * Tz, B2 = k.B21 + k.B22 * Tz;
+      // s_i - r_i c_off: the fields hold c - c_off, so mu - c_off is what mu2 returns
+      const f2 s1 = bc((float)(B1 - k.r1d * k.c_off)), s2 = bc((float)(-B1 - B2 - k.r2d * k.c_off)),
+               s3 = bc((float)(-B1 + B2 - k.r3d * k.c_off));
       // column window rows ry-1 .. ry+2 of phi1, phi2, mu (pairs)
       f2 w1[4], w2[4], wm[4];
 #pragma unroll
@@ -332,9 +388,13 @@ __global__ void __launch_bounds__(kX2Threads, 3)
         f2 nc = fma2(face2(x1p, x2p, mxp, x1m, x2m, mxm), bc(k.cfx), ld2(cc + e));
         nc = fma2(face2(y1p, y2p, myp, y1m, y2m, mym), bc(k.cfy), nc);
         nc = fma2(face2(z1p, z2p, mzp, z1m, z2m, mzm), bc(k.cfz), nc);
-        store_pair(gy, n1, n2, nc);
+        store_pair(r, n1, n2, nc);
       }
     }
+    // the last warp that leaves plane z hands the slot of plane z-1 to the load
+    // of plane z+3, without waiting for plane z+2 first: two loads in flight
+    __syncwarp();
+    if (lane == 0 && arrive_count(&sm.passed) % kX2Warps == kX2Warps - 1 && z + 3 <= zin1) issue(z + 3);
   }
 }
 
@@ -388,8 +448,7 @@ int launch_peri3d_step_x2(const rs3_params &p, const P3Maps &m, float *o1, float
   const int which = (a1 ? 2 : 0) + (sd ? 1 : 0);
   if (!smem_limit_once((const void *)kfn, (int)smem, attr[which])) return -3;
   const dim3 grid((p.nx + kX2BX - 1) / kX2BX, (p.ny - 2 + kX2BY - 1) / kX2BY, (p.nz - 2 + k.z_chunk - 1) / k.z_chunk);
-  kfn<<<grid, kX2Threads, smem, st>>>(k, m.phi1, m.phi2, m.c, o1, o2, oc, step, err);
-  return 0;
+  return launch_dep_smem(kfn, grid, dim3(kX2Threads), smem, st, k, m.phi1, m.phi2, m.c, o1, o2, oc, step, err) == cudaSuccess ? 0 : -3;
 }
 
 }  // namespace rs

@@ -480,6 +480,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// counts an arrival at a shared counter and returns the count before it: what
+// the arriving lane's warp read (ordered by a __syncwarp) happens before what
+// the thread that sees the last count does next
+__device__ __forceinline__ uint32_t arrive_count(uint32_t *count) {
+  uint32_t old;
+  asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(old) : "r"(smem_u32(count)) : "memory");
+  return old;
+}
 // non-blocking: whether the phase has completed now (try_wait may suspend the
 // thread for a while first; a wait bounded by a count of test_wait polls
 // gives up after that many polls, which the tests use to reach the give-up
