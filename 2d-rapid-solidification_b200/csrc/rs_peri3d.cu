@@ -10,29 +10,44 @@
 //
 // The FP32 step runs on packed FP32 pairs (rs_peri3d_x2.cu); this file's
 // step kernel is the FP64 one.
-// Kernel: a CTA owns a column of BX x BY output cells (x, y) and marches
-// through a chunk of z planes.  Every input plane (BX+4 (FP32) or BX+2 (FP64)
-// columns x BY+2 rows of phi1, phi2 and c) arrives by one 3D TMA box per
-// field into a four-slot ring; the load of plane z+2 is in flight while plane
-// z is computed.  mu of each plane (tile plus x/y halo) is computed once into
-// a four-slot ring.  Outputs go straight to global memory (32 consecutive x
-// per warp), and each output that a ghost cell images (x = 1, nx-2; y = 1,
-// ny-2; z = 1, nz-2) is written to its ghost cells too, which is what the
-// reference's boundary kernels leave there.
+// Kernel: a CTA owns a column of 32 x 16 output cells (x, y) and marches
+// through a chunk of z planes.  Every input plane (34 columns x 18 rows of
+// phi1, phi2 and c) arrives by one 3D TMA box per field into a six-slot ring;
+// the last warp that leaves plane z issues the load into the slot of plane
+// z-1, so four planes are in flight while plane z is computed.  mu of each
+// plane (tile plus x/y halo) is computed once into a four-slot ring, where the
+// march is not in pure melt (there mu is c - r1).  Outputs go straight to
+// global memory (32 consecutive x per warp), and each output that a ghost cell
+// images (x = 1, nx-2; y = 1, ny-2; z = 1, nz-2) is written to its ghost cells
+// too, which is what the reference's boundary kernels leave there.
+// What bounds it (512 x 512 x 128): in melt the memory (333 us, 74 % of the
+// copy rate), in fronts the FP64 pipe (589 us; 180 FP64 instructions per cell,
+// 57 % of the pipe's rate at 16 warps per SM).  A front in two thirds of the
+// planes: 546 -> 486 us.  Measured beside it: four slots 519, 14-row tiles
+// with three CTAs per SM and four slots 532 (80 registers instead of 118).
 // Algorithmic bytes per cell-step: 3 fields read + 3 written.
 #include <cuda.h>
 
+#include "rs_kernels.cuh"
 #include "rs_peri3d_common.cuh"
 
 namespace rs {
 namespace {
 
-template <typename R>
+struct D3 {  // the tile: 32 x 16 output cells, two rows of a column per thread
+  static constexpr int BX = 32, BXin = 34, BY = 16, BYin = 18, kThreads = 256, K = BX * BY / kThreads;
+  static constexpr int kSlots = 6;            // input plane ring: 6 x 15 KB, two CTAs per SM
+  static constexpr int kPlane = BXin * BYin;  // elements of one field plane, 4896 bytes
+  static constexpr int kPlaneAl = 624;        // TMA destinations stay 128-byte aligned
+  static_assert(kPlaneAl >= kPlane && kPlaneAl * sizeof(double) % 128 == 0 && K == 2);
+};
+
 struct P3Smem {
-  alignas(128) R in[kP3Slots][3][P3Cfg<R>::kPlaneAl];  // [slot][field][row][col]
-  alignas(16) R mu[kP3MuSlots][P3Cfg<R>::kPlane];
-  uint64_t full[kP3Slots];
-  int melt[8];  // per plane (q mod 8): the box is pure melt inside the array (p3_melt)
+  alignas(128) double in[D3::kSlots][3][D3::kPlaneAl];  // [slot][field][row][col]
+  alignas(16) double mu[kP3MuSlots][D3::kPlane];
+  uint64_t full[D3::kSlots];
+  int melt[8];  // per plane (q mod 8): the box is pure melt inside the array (p3_melt_cell)
+  uint32_t passed;  // warps that have left a plane, summed over the planes
 };
 
 // mu = c - sum_i r_i g_i (computeMu, TiAg.cu:461-470)
@@ -41,59 +56,102 @@ __device__ __forceinline__ R mu_of(const K3<R> &k, R p1, R p2, R c) {
   const R p3 = R(1) - p1 - p2;
   return c - k.r1 * g3(p1, p2, p3) - k.r2 * g3(p2, p3, p1) - k.r3 * g3(p3, p1, p2);
 }
+// the same with the polynomials of g_i as multiply-adds,
+// 4 g = p^2 (15 - 5 p - 15 p^2 + 9 p^3 - 15 (1 - p) d^2), d = p_k - p_j
+__device__ __forceinline__ double mu_step(const K3<double> &k, double p1, double p2, double c) {
+  const double p3 = (1.0 - p1) - p2, d12 = p1 - p2, d23 = p2 - p3, d31 = p3 - p1;
+  auto g = [](double p, double d) {
+    const double a = fma(fma(fma(p, 9.0, -15.0), p, -5.0), p, 15.0);
+    return p * p * fma(fma(p, 15.0, -15.0), d * d, a);
+  };
+  return fma(g(p1, d23), -0.25 * k.r1, fma(g(p2, d31), -0.25 * k.r2, fma(g(p3, d12), -0.25 * k.r3, c)));
+}
 
-// SD: solid diffusivities Da or Db non-zero (the reference sets both to 0)
-template <typename R, bool SD>
-__global__ void __launch_bounds__(kP3Threads, sizeof(R) == 4 ? 3 : 2)
-    peri3d_kernel(const __grid_constant__ K3<R> k, const __grid_constant__ CUtensorMap m1,
+// A1: the a1 well terms are non-zero; SD: solid diffusivities Da or Db non-zero
+// (the reference sets all of them to 0)
+template <bool A1, bool SD>
+__global__ void __launch_bounds__(D3::kThreads, 2)
+    peri3d_kernel(const __grid_constant__ K3<double> k, const __grid_constant__ CUtensorMap m1,
                   const __grid_constant__ CUtensorMap m2, const __grid_constant__ CUtensorMap mc,
-                  R *__restrict__ o1, R *__restrict__ o2, R *__restrict__ oc, const int64_t step, int *err) {
-  using C = P3Cfg<R>;
+                  double *__restrict__ o1, double *__restrict__ o2, double *__restrict__ oc, const int64_t step,
+                  int *err) {
+  using C = D3;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  P3Smem<R> &sm = *reinterpret_cast<P3Smem<R> *>(smem_raw);
-  const int tid = threadIdx.x;
+  P3Smem &sm = *reinterpret_cast<P3Smem *>(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31;
   const int xb = C::BX * blockIdx.x;   // first box column (array x); outputs xb+1 .. xb+BX
-  const int yb = kP3BY * blockIdx.y;   // first box row (array y); outputs yb+1 .. yb+BY
+  const int yb = C::BY * blockIdx.y;   // first box row (array y); outputs yb+1 .. yb+BY
   const int zo0 = 1 + k.z_chunk * blockIdx.z;                 // first output plane
   const int zo1 = min(zo0 + k.z_chunk, k.nz - 1);            // one past the last
   if (zo0 >= zo1) return;
   const int zin0 = zo0 - 1, zin1 = zo1;  // input planes zin0 .. zin1
-  constexpr uint32_t kBytes = 3u * C::kPlane * sizeof(R);
+  pdl_wait();
+  pdl_trigger();
+  constexpr uint32_t kBytes = 3u * C::kPlane * sizeof(double);
   if (smem_u32(smem_raw) & 127u) {
     if (tid == 0) atomicExch(err, 2);
     return;
   }
-  static_assert((P3Cfg<R>::kPlaneAl * sizeof(R)) % 128 == 0, "TMA destinations 128-byte aligned");
   auto issue = [&](int z) {  // plane z into its ring slot
-    const int q = z - zin0, s = q % kP3Slots;
+    const int q = z - zin0, s = q % C::kSlots;
     mbar_expect_tx(&sm.full[s], kBytes);
     tma_load_3d(&sm.in[s][0][0], &m1, &sm.full[s], xb, yb, z);
     tma_load_3d(&sm.in[s][1][0], &m2, &sm.full[s], xb, yb, z);
     tma_load_3d(&sm.in[s][2][0], &mc, &sm.full[s], xb, yb, z);
   };
+  int issued = min(zin1, zin0 + C::kSlots - 1);  // last plane whose load was issued
   if (tid == 0) {
-    for (int s = 0; s < kP3Slots; ++s) mbar_init(&sm.full[s], 1);
+    for (int s = 0; s < C::kSlots; ++s) mbar_init(&sm.full[s], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    for (int z = zin0; z <= min(zin1, zin0 + kP3Slots - 1); ++z) issue(z);
+    for (int z = zin0; z <= issued; ++z) issue(z);
     for (int s = 0; s < 8; ++s) sm.melt[s] = 1;
+    sm.passed = 0u;
   }
   __syncthreads();
-  int issued = min(zin1, zin0 + kP3Slots - 1);  // last plane whose load was issued
-  // mu of plane z into its slot (tile and halo); false if its load never came
-  auto mu_plane = [&](int z) {
-    const int q = z - zin0, s = q % kP3Slots;
-    const bool got = p3_wait<R>(&sm.full[s], (uint32_t)((q / kP3Slots) & 1), err);
-    R *mu = sm.mu[q % kP3MuSlots];
-    const R *f1 = sm.in[s][0], *f2 = sm.in[s][1], *fc = sm.in[s][2];
-    if (got) {
-      bool all_melt = true;
-      for (int e = tid; e < C::kPlane; e += kP3Threads) {
-        mu[e] = mu_of(k, f1[e], f2[e], fc[e]);
-        all_melt = all_melt && p3_melt_cell(k, f1[e], f2[e], xb + e % C::BXin, yb + e / C::BXin);
-      }
-      if (!all_melt) sm.melt[q & 7] = 0;
+  // Planes of pure melt (p3_melt_cell; bit u: box element tid + C::kThreads u
+  // lies outside the array); false if the plane's load never came
+  constexpr int kElems = (C::kPlane + C::kThreads - 1) / C::kThreads;
+  uint32_t outside = 0u;
+#pragma unroll
+  for (int u = 0; u < kElems; ++u) {
+    const int e = tid + C::kThreads * u;
+    if (e >= C::kPlane || xb + e % C::BXin >= k.nx || yb + e / C::BXin >= k.ny) outside |= 1u << u;
+  }
+  auto wait_plane = [&](int z) {
+    const int q = z - zin0;
+    return p3_wait<double>(&sm.full[q % C::kSlots], (uint32_t)((q / C::kSlots) & 1), err);
+  };
+  // the words in which a cell differs from pure melt (phi1 == 1, phi2 == 0 of
+  // either sign), on the integer pipe
+  auto off_melt = [](double p1, double p2) {
+    return (uint32_t)(__double2hiint(p1) ^ 0x3FF00000) | (uint32_t)__double2loint(p1) |
+           ((uint32_t)__double2hiint(p2) << 1) | (uint32_t)__double2loint(p2);
+  };
+  auto check_plane = [&](int z) {
+    const int q = z - zin0, s = q % C::kSlots;
+    uint32_t diff = 0u;
+#pragma unroll
+    for (int u = 0; u < kElems; ++u) {
+      const int e = tid + C::kThreads * u;
+      if (!((outside >> u) & 1u)) diff |= off_melt(sm.in[s][0][e], sm.in[s][1][e]);
     }
-    return got;
+    if (diff) sm.melt[q & 7] = 0;
+  };
+  // mu of plane z (tile and halo, already loaded) into its slot, and its check
+  auto mu_plane = [&](int z) {
+    const int q = z - zin0, s = q % C::kSlots;
+    double *mu = sm.mu[q % kP3MuSlots];
+    const double *f1 = sm.in[s][0], *f2 = sm.in[s][1], *fc = sm.in[s][2];
+    uint32_t diff = 0u;
+#pragma unroll
+    for (int u = 0; u < kElems; ++u) {
+      const int e = tid + C::kThreads * u;
+      if (e >= C::kPlane) break;
+      const double p1 = f1[e], p2 = f2[e];
+      mu[e] = mu_step(k, p1, p2, fc[e]);
+      if (!((outside >> u) & 1u)) diff |= off_melt(p1, p2);
+    }
+    if (diff) sm.melt[q & 7] = 0;
   };
   // a load that did not arrive in time: wait (bounded) for every load still
   // in flight before the CTA leaves, so none lands in reused shared memory
@@ -102,12 +160,15 @@ __global__ void __launch_bounds__(kP3Threads, sizeof(R) == 4 ? 3 : 2)
       for (int z = from; z <= issued; ++z) {
         const int q = z - zin0;
         uint32_t tries = 0;
-        while (!mbar_try_wait(&sm.full[q % kP3Slots], (uint32_t)((q / kP3Slots) & 1)) && ++tries < kP3WaitLimit) {
+        while (!mbar_try_wait(&sm.full[q % C::kSlots], (uint32_t)((q / C::kSlots) & 1)) && ++tries < kP3WaitLimit) {
         }
       }
   };
-  bool ok = mu_plane(zin0);
-  ok = mu_plane(zin0 + 1) && ok;
+  const bool ok = wait_plane(zin0) && wait_plane(zin0 + 1);
+  if (ok) {
+    check_plane(zin0);
+    check_plane(zin0 + 1);
+  }
   if (!__syncthreads_and(ok)) {
     drain(zin0);
     return;
@@ -115,147 +176,180 @@ __global__ void __launch_bounds__(kP3Threads, sizeof(R) == 4 ? 3 : 2)
 
   // this thread's cells: column ix, a strip of K consecutive rows (the y
   // neighbours of the strip come from a register window)
-  constexpr int K = C::kCellsPerThread;
+  constexpr int K = C::K;
   const int ix = tid % C::BX, iy0 = (tid / C::BX) * K;
   const int gx = xb + 1 + ix;  // array x of the output
   const bool xin = gx <= k.nx - 2;
-  const int xg = gx == k.nx - 2 ? 0 : (gx == 1 ? k.nx - 1 : -1);  // ghost column it images
+  const int xd = gx == k.nx - 2 ? 2 - k.nx : (gx == 1 ? k.nx - 2 : 0);  // to the ghost column it images
+  const int e0 = (iy0 + 1) * C::BXin + ix + 1;                          // box element of the strip's first cell
   const int64_t plane = (int64_t)k.nx * k.ny;
-  const R third = R(1) / R(3);
+  int64_t out0 = (int64_t)zo0 * plane + (int64_t)(yb + 1 + iy0) * k.nx + gx;  // the strip's first cell in plane z
 
-  for (int z = zo0; z < zo1; ++z) {
-    // one barrier per plane: after it every thread has finished plane z-1,
-    // so the input slot of plane z-2 takes the load of plane z+2 (mu has
-    // four slots: mu(z+1) overwrites mu(z-3))
-    if (!__syncthreads_and(mu_plane(z + 1))) {
+  // mu is stored for the planes that the general form reads, ahead of the
+  // barrier while the march is in it; a march that enters it from pure melt
+  // makes up for the missing planes behind the barrier.  Uniform over the CTA.
+  int mu_done = zin0 - 1;  // mu of planes .. mu_done stands, as far as the ring goes
+  bool general = false;
+  for (int z = zo0; z < zo1; ++z, out0 += plane) {
+    // one barrier per plane: the flags and mu of planes .. z+1 stand behind it
+    // (mu has four slots: mu(z+1) overwrites mu(z-3))
+    const bool got = wait_plane(z + 1);
+    if (got) {
+      if (general) {
+        mu_plane(z + 1);
+        mu_done = z + 1;
+      } else {
+        check_plane(z + 1);
+      }
+    }
+    if (!__syncthreads_and(got)) {
+      issued = min(zin1, z + C::kSlots - 2);
       drain(z + 1);
       return;
     }
-    if (z + 2 <= zin1 && z + 2 > issued) {
-      if (tid == 0) issue(z + 2);
-      issued = z + 2;
-    }
     const int q = z - zin0;
     // planes z-1 .. z+1 pure melt wherever a stencil of an output cell reaches
-    // (p3_melt_cell); the flag of plane z+3 is re-armed here (its computation,
-    // mu_plane(z+3) before the barrier of iteration z+2, is separated from
-    // this write by the barrier of z+1)
+    // (p3_melt_cell); the flag of plane z+3 is re-armed here (check_plane(z+3),
+    // before the barrier of iteration z+2, is separated from this write by the
+    // barrier of z+1)
     const bool melt3 = sm.melt[(q - 1) & 7] && sm.melt[q & 7] && sm.melt[(q + 1) & 7];
     if (tid == 0) sm.melt[(q + 3) & 7] = 1;
-    const R *c1 = sm.in[q % kP3Slots][0], *c2 = sm.in[q % kP3Slots][1], *cc = sm.in[q % kP3Slots][2];
-    const R *d1 = sm.in[(q - 1) % kP3Slots][0], *d2 = sm.in[(q - 1) % kP3Slots][1];
-    const R *u1 = sm.in[(q + 1) % kP3Slots][0], *u2 = sm.in[(q + 1) % kP3Slots][1];
-    const R *mu = sm.mu[q % kP3MuSlots], *mud = sm.mu[(q - 1) % kP3MuSlots], *muu = sm.mu[(q + 1) % kP3MuSlots];
-    // the plane's B1, B2 (TiAg.cu:61-62) with the frozen T of this step
-    const double Tz = k.G_T == 0.0 ? k.T_ref : k.T_ref + k.G_T * ((double)z - k.z_T - k.V_T * (double)step);
-    const double B1 = k.B11 + k.B12 * Tz, B2 = k.B21 + k.B22 * Tz;
-    const R s1 = (R)B1, s2 = (R)(-B1 - B2), s3 = (R)(-B1 + B2);
-    const int zg = z == 1 ? 0 : (z == k.nz - 2 ? k.nz - 1 : -1);
+    if (!melt3 && mu_done < z + 1) {
+      for (int w = max(z - 1, mu_done + 1); w <= z + 1; ++w) mu_plane(w);
+      mu_done = z + 1;
+      __syncthreads();
+    }
+    general = !melt3;
+    const double *c1 = sm.in[q % C::kSlots][0], *c2 = sm.in[q % C::kSlots][1], *cc = sm.in[q % C::kSlots][2];
+    const int zd = z == 1 ? -1 : (z == k.nz - 2 ? 1 : 0);  // planes 0 and nz-1 copy their neighbours
     // the cell and every ghost cell that images it
-    auto store_cell = [&](int gy, R n1, R n2, R nc) {
-      const int yg = gy == k.ny - 2 ? 0 : (gy == 1 ? k.ny - 1 : -1);
-      if ((xg & yg & zg) < 0) {  // no ghost cell images this one
-        const int64_t o = (int64_t)z * plane + (int64_t)gy * k.nx + gx;
-        o1[o] = n1;
-        o2[o] = n2;
-        oc[o] = nc;
-      } else {
-        const int xs[2] = {gx, xg}, ys[2] = {gy, yg}, zs[2] = {z, zg};
-  #pragma unroll
-        for (int a = 0; a < 2; ++a)
-  #pragma unroll
-          for (int bq = 0; bq < 2; ++bq)
-  #pragma unroll
-            for (int cq = 0; cq < 2; ++cq) {
-              if (xs[a] < 0 || ys[bq] < 0 || zs[cq] < 0) continue;
-              const int64_t o = (int64_t)zs[cq] * plane + (int64_t)ys[bq] * k.nx + xs[a];
-              o1[o] = n1;
-              o2[o] = n2;
-              oc[o] = nc;
-            }
+    auto store_cell = [&](int r, double n1, double n2, double nc) {
+      const int gy = yb + 1 + iy0 + r;
+      if (gy > k.ny - 2) return;
+      const int64_t o = out0 + (int64_t)r * k.nx;
+      o1[o] = n1;
+      o2[o] = n2;
+      oc[o] = nc;
+      const int yd = gy == k.ny - 2 ? 2 - k.ny : (gy == 1 ? k.ny - 2 : 0);
+      if (xd | yd | zd) {
+#pragma unroll 1
+        for (int im = 1; im < 8; ++im) {
+          if (((im & 1) && !xd) || ((im & 2) && !yd) || ((im & 4) && !zd)) continue;
+          const int64_t og =
+              o + (im & 1 ? xd : 0) + (im & 2 ? (int64_t)yd * k.nx : 0) + (im & 4 ? zd * plane : 0);
+          o1[og] = n1;
+          o2[og] = n2;
+          oc[og] = nc;
+        }
       }
     };
     if (xin && melt3) {
-      // pure melt (p3_melt_cell): phi1, phi2 stay 1 and 0 and the face
-      // mobilities are 2, the values the general form gives bit for bit
-      const int e0 = (iy0 + 1) * C::BXin + ix + 1;
-      R wm[K + 2];
-  #pragma unroll
-      for (int r = 0; r < K + 2; ++r) wm[r] = mu[e0 + (r - 1) * C::BXin];
-  #pragma unroll
+      // pure melt (p3_melt_cell): phi1, phi2 stay 1 and 0, mu is c - r1 (g_1 = 1,
+      // g_2 = g_3 = 0) and the face mobilities are 2: the values the general
+      // form gives bit for bit, without a mu plane
+      const double *cd = sm.in[(q - 1) % C::kSlots][2], *cu = sm.in[(q + 1) % C::kSlots][2];
+      const double r1 = k.r1;
+      double w[K + 2];
+#pragma unroll
+      for (int r = 0; r < K + 2; ++r) w[r] = cc[e0 + (r - 1) * C::BXin];
+#pragma unroll
       for (int r = 0; r < K; ++r) {
-        const int gy = yb + 1 + iy0 + r;
-        if (gy > k.ny - 2) break;
         const int e = e0 + r * C::BXin;
-        const R m0 = wm[r + 1];
-        const R jx = R(2) * (mu[e + 1] - m0) - R(2) * (m0 - mu[e - 1]);
-        const R jy = R(2) * (wm[r + 2] - m0) - R(2) * (m0 - wm[r]);
-        const R jz = R(2) * (muu[e] - m0) - R(2) * (m0 - mud[e]);
-        store_cell(gy, R(1), R(0), cc[e] + (k.cfx * jx + k.cfy * jy + k.cfz * jz));
+        const double m0 = w[r + 1] - r1;
+        auto face = [&](double cp, double cm) { return 2.0 * (((cp - r1) - m0) + ((cm - r1) - m0)); };
+        double dc = face(cc[e + 1], cc[e - 1]) * k.cfx;
+        dc = fma(face(w[r + 2], w[r]), k.cfy, dc);
+        dc = fma(face(cu[e], cd[e]), k.cfz, dc);
+        store_cell(r, 1.0, 0.0, w[r + 1] + dc);
       }
     } else if (xin) {
-      const int e0 = (iy0 + 1) * C::BXin + ix + 1;  // box element of the strip's first cell
-      R w1[K + 2], w2[K + 2], wm[K + 2];            // the strip's column, rows iy0-1 .. iy0+K
-  #pragma unroll
+      const double *d1 = sm.in[(q - 1) % C::kSlots][0], *d2 = sm.in[(q - 1) % C::kSlots][1];
+      const double *u1 = sm.in[(q + 1) % C::kSlots][0], *u2 = sm.in[(q + 1) % C::kSlots][1];
+      const double *mu = sm.mu[q % kP3MuSlots], *mud = sm.mu[(q - 1) % kP3MuSlots],
+                   *muu = sm.mu[(q + 1) % kP3MuSlots];
+      // the plane's B1, B2 (TiAg.cu:61-62) with the frozen T of this step
+      const double Tz = k.G_T == 0.0 ? k.T_ref : k.T_ref + k.G_T * ((double)z - k.z_T - k.V_T * (double)step);
+      const double B1 = k.B11 + k.B12 * Tz, B2 = k.B21 + k.B22 * Tz;
+      const double s1 = B1, s2 = -B1 - B2, s3 = -B1 + B2;
+      double w1[K + 2], w2[K + 2], wm[K + 2];  // the strip's column, rows iy0-1 .. iy0+K
+#pragma unroll
       for (int r = 0; r < K + 2; ++r) {
         const int e = e0 + (r - 1) * C::BXin;
         w1[r] = c1[e];
         w2[r] = c2[e];
         wm[r] = mu[e];
       }
-  #pragma unroll
+#pragma unroll
       for (int r = 0; r < K; ++r) {
-        const int gy = yb + 1 + iy0 + r;
-        if (gy > k.ny - 2) break;
         const int e = e0 + r * C::BXin;
-        const R p1 = w1[r + 1], p2 = w2[r + 1], m0 = wm[r + 1], p3 = R(1) - p1 - p2;
-        const R d12 = p1 - p2, d23 = p2 - p3, d31 = p3 - p1;
-        // chemical driving forces (fcphi, TiAg.cu:514-516), with
-        // gp1(pi, pj, pk) = G_i and gp2(pi, pj, pk) = Q_i (pj - pk)
-        const R Q1 = R(7.5) * (p1 - R(1)) * (p1 * p1), Q2 = R(7.5) * (p2 - R(1)) * (p2 * p2),
-                Q3 = R(7.5) * (p3 - R(1)) * (p3 * p3);
-        const R G1 = R(3.75) * p1 * ((((R(3) * p1 - R(4)) * p1 - R(1)) * p1 + R(2)) + (R(3) * p1 - R(2)) * (d23 * d23));
-        const R G2 = R(3.75) * p2 * ((((R(3) * p2 - R(4)) * p2 - R(1)) * p2 + R(2)) + (R(3) * p2 - R(2)) * (d31 * d31));
-        const R G3 = R(3.75) * p3 * ((((R(3) * p3 - R(4)) * p3 - R(1)) * p3 + R(2)) + (R(3) * p3 - R(2)) * (d12 * d12));
-        const R o1w = s1 - k.r1 * m0, o2w = s2 - k.r2 * m0, o3w = s3 - k.r3 * m0;
-        const R A = Q1 * d23 * o1w, Bq = Q2 * d31 * o2w, Cq = Q3 * d12 * o3w;
+        const double p1 = w1[r + 1], p2 = w2[r + 1], m0 = wm[r + 1], p3 = (1.0 - p1) - p2;
+        const double d12 = p1 - p2, d23 = p2 - p3, d31 = p3 - p1;
+        const double p1s = p1 * p1, p2s = p2 * p2, p3s = p3 * p3;
+        // chemical driving forces (fcphi, TiAg.cu:514-516): gp2(pi, pj, pk) =
+        // Q_i (pj - pk), Q_i = 7.5 (p_i - 1) p_i^2, and gp1(pi, pj, pk) = G_i =
+        // 3.75 p_i (3 p_i^3 - 4 p_i^2 - p_i + 2 + (3 p_i - 2)(pj - pk)^2)
+        const double Q1 = fma(p1, 7.5, -7.5) * p1s, Q2 = fma(p2, 7.5, -7.5) * p2s, Q3 = fma(p3, 7.5, -7.5) * p3s;
+        auto G = [](double p, double d) {
+          const double a = fma(fma(fma(p, 11.25, -15.0), p, -3.75), p, 7.5);
+          return p * fma(fma(p, 11.25, -7.5), d * d, a);
+        };
+        const double G1 = G(p1, d23), G2 = G(p2, d31), G3 = G(p3, d12);
+        const double o1w = fma(m0, -k.r1, s1), o2w = fma(m0, -k.r2, s2), o3w = fma(m0, -k.r3, s3);
+        const double A = Q1 * d23 * o1w, Bq = Q2 * d31 * o2w, Cq = Q3 * d12 * o3w;
         // multi-well terms (fphi, TiAg.cu:522-527) with their shared factors
-        const R s12 = p1 * p2, s13 = p1 * p3, s23 = p2 * p3;
-        const R U1 = R(3) * s23 + R(3) * p1 + k.b * (p1 * p1), U2 = R(3) * s13 + R(3) * p2 + k.b * (p2 * p2),
-                U3 = R(3) * s12 + R(3) * p3 + k.b * (p3 * p3);
-        const R F1 = R(2) * p1 * (R(1) - p1) * (R(1) - R(2) * p1) + k.a1 * (s23 * s23) * (R(3) + R(2) * k.b * p1) +
-                     R(2) * k.a2 * p1 * (p3 * p3) * U2 + R(2) * k.a3 * p1 * (p2 * p2) * U3 +
-                     k.lam * (G1 * o1w - Bq + Cq);
-        const R F2 = R(2) * p2 * (R(1) - p2) * (R(1) - R(2) * p2) + R(2) * k.a1 * p2 * (p3 * p3) * U1 +
-                     k.a2 * (s13 * s13) * (R(3) + R(2) * k.b * p2) + R(2) * k.a3 * p2 * (p1 * p1) * U3 +
-                     k.lam * (A + G2 * o2w - Cq);
-        const R F3 = R(2) * p3 * (R(1) - p3) * (R(1) - R(2) * p3) + R(2) * k.a1 * p3 * (p2 * p2) * U1 +
-                     R(2) * k.a2 * p3 * (p1 * p1) * U2 + k.a3 * (s12 * s12) * (R(3) + R(2) * k.b * p3) +
-                     k.lam * (-A + Bq + G3 * o3w);
+        const double s12 = p1 * p2, s13 = p1 * p3, s23 = p2 * p3;
+        const double k2 = 2.0 * k.a2 * fma(s13, 3.0, p2 * fma(p2, k.b, 3.0));
+        const double k3 = 2.0 * k.a3 * fma(s12, 3.0, p3 * fma(p3, k.b, 3.0));
+        auto dw = [](double p) { return fma(fma(p, 4.0, -6.0), p, 2.0) * p; };  // 2p(1-p)(1-2p)
+        double F1 = fma(p1 * p3s, k2, dw(p1));
+        F1 = fma(p1 * p2s, k3, F1);
+        F1 = fma(fma(G1, o1w, Cq - Bq), k.lam, F1);
+        double F2 = fma(s13 * s13, fma(p2, 2.0 * k.b, 3.0) * k.a2, dw(p2));
+        F2 = fma(p2 * p1s, k3, F2);
+        F2 = fma(fma(G2, o2w, A - Cq), k.lam, F2);
+        double F3 = fma(p3 * p1s, k2, dw(p3));
+        F3 = fma(s12 * s12, fma(p3, 2.0 * k.b, 3.0) * k.a3, F3);
+        F3 = fma(fma(G3, o3w, Bq - A), k.lam, F3);
+        if constexpr (A1) {
+          const double k1 = 2.0 * k.a1 * fma(s23, 3.0, p1 * fma(p1, k.b, 3.0));
+          F1 = fma(s23 * s23, fma(p1, 2.0 * k.b, 3.0) * k.a1, F1);
+          F2 = fma(p2 * p3s, k1, F2);
+          F3 = fma(p3 * p2s, k1, F3);
+        }
         // neighbours
-        const R x1p = c1[e + 1], x1m = c1[e - 1], x2p = c2[e + 1], x2m = c2[e - 1];
-        const R z1p = u1[e], z1m = d1[e], z2p = u2[e], z2m = d2[e];
-        const R lap1 = (x1p + x1m - R(2) * p1) * k.dxi2 + (w1[r + 2] + w1[r] - R(2) * p1) * k.dyi2 +
-                       (z1p + z1m - R(2) * p1) * k.dzi2;
-        const R lap2 = (x2p + x2m - R(2) * p2) * k.dxi2 + (w2[r + 2] + w2[r] - R(2) * p2) * k.dyi2 +
-                       (z2p + z2m - R(2) * p2) * k.dzi2;
-        // phi_i' = phi_i - dt (2 mu_i - mu_j - mu_k) / 3 with mu_i = F_i - lap_i and
-        // lap_3 = -lap_1 - lap_2 (TiAg.cu:529-537)
-        const R n1 = p1 + k.dt * (lap1 - (R(2) * F1 - F2 - F3) * third);
-        const R n2 = p2 + k.dt * (lap2 - (R(2) * F2 - F1 - F3) * third);
+        const double x1p = c1[e + 1], x1m = c1[e - 1], x2p = c2[e + 1], x2m = c2[e - 1];
+        const double z1p = u1[e], z1m = d1[e], z2p = u2[e], z2m = d2[e];
+        auto lap = [&](double p, double xp, double xm, double yp, double ym, double zp, double zm) {
+          const double l = fma(fma(p, -2.0, yp + ym), k.dyi2, fma(p, -2.0, xp + xm) * k.dxi2);
+          return fma(fma(p, -2.0, zp + zm), k.dzi2, l);
+        };
+        const double lap1 = lap(p1, x1p, x1m, w1[r + 2], w1[r], z1p, z1m);
+        const double lap2 = lap(p2, x2p, x2m, w2[r + 2], w2[r], z2p, z2m);
+        // phi_i' = phi_i + dt lap_i - dt (2 F_i - F_j - F_k) / 3 with mu_i = F_i - lap_i
+        // and lap_3 = -lap_1 - lap_2 (TiAg.cu:529-537)
+        const double T3 = ((F1 + F2) + F3) * (k.dt * (1.0 / 3.0));
+        const double n1 = p1 + fma(lap1 - F1, k.dt, T3);
+        const double n2 = p2 + fma(lap2 - F2, k.dt, T3);
         // solute: face mobility (phi1 + phi1') / 2 (+ solid terms), TiAg.cu:543-552
-        auto mob = [&](R q1, R q2) {
-          R m = p1 + q1;
-          if constexpr (SD) m += k.Da2 * (p2 + q2) + k.Db2 * (p3 + R(1) - q1 - q2);
+        auto mob = [&](double q1, double q2) {
+          double m = p1 + q1;
+          if constexpr (SD) m = fma(((p3 + 1.0) - q1) - q2, k.Db2, fma(p2 + q2, k.Da2, m));
           return m;
         };
-        const R jx = mob(x1p, x2p) * (mu[e + 1] - m0) - mob(x1m, x2m) * (m0 - mu[e - 1]);
-        const R jy = mob(w1[r + 2], w2[r + 2]) * (wm[r + 2] - m0) - mob(w1[r], w2[r]) * (m0 - wm[r]);
-        const R jz = mob(z1p, z2p) * (muu[e] - m0) - mob(z1m, z2m) * (m0 - mud[e]);
-        const R nc = cc[e] + (k.cfx * jx + k.cfy * jy + k.cfz * jz);
-        store_cell(gy, n1, n2, nc);
+        auto face2 = [&](double qp1, double qp2, double mp, double qm1, double qm2, double mm) {
+          return fma(mob(qp1, qp2), mp - m0, mob(qm1, qm2) * (mm - m0));
+        };
+        double dc = face2(x1p, x2p, mu[e + 1], x1m, x2m, mu[e - 1]) * k.cfx;
+        dc = fma(face2(w1[r + 2], w2[r + 2], wm[r + 2], w1[r], w2[r], wm[r]), k.cfy, dc);
+        dc = fma(face2(z1p, z2p, muu[e], z1m, z2m, mud[e]), k.cfz, dc);
+        store_cell(r, n1, n2, cc[e] + dc);
       }
     }
+    // the last warp that leaves plane z hands the slot of plane z-1 to the load
+    // of plane z+3, without waiting for plane z+2 first: two loads in flight
+    __syncwarp();
+    if (lane == 0 && arrive_count(&sm.passed) % (C::kThreads / 32) == C::kThreads / 32 - 1 && z + C::kSlots - 1 <= zin1)
+      issue(z + C::kSlots - 1);
   }
 }
 
@@ -377,19 +471,22 @@ __global__ void peri3d_ghost_kernel(const K3<R> k, int axis, R *__restrict__ f1,
   fc[d1] = fc[s1];
 }
 
-template <typename R>
-int launch_step(const rs3_params &p, const P3Maps &m, R *o1, R *o2, R *oc, int64_t step, int *err, cudaStream_t st) {
-  using C = P3Cfg<R>;
-  const K3<R> k = make_k3<R>(p);
-  const size_t smem = sizeof(P3Smem<R>) + 128;
-  const bool sd = p.Da != 0.0 || p.Db != 0.0;
-  auto kfn = sd ? peri3d_kernel<R, true> : peri3d_kernel<R, false>;
-  static std::atomic<unsigned long long> attr[2];
-  if (!smem_limit_once((const void *)kfn, (int)smem, attr[sd])) return -3;
-  const dim3 grid((p.nx - 2 + C::BX - 1) / C::BX, (p.ny - 2 + kP3BY - 1) / kP3BY,
+int launch_step(const rs3_params &p, const P3Maps &m, double *o1, double *o2, double *oc, int64_t step, int *err,
+                cudaStream_t st) {
+  using C = D3;
+  const K3<double> k = make_k3<double>(p);
+  const size_t smem = sizeof(P3Smem) + 128;
+  const bool a1 = p.a1 != 0.0, sd = p.Da != 0.0 || p.Db != 0.0;
+  auto kfn = a1 ? (sd ? peri3d_kernel<true, true> : peri3d_kernel<true, false>)
+                : (sd ? peri3d_kernel<false, true> : peri3d_kernel<false, false>);
+  static std::atomic<unsigned long long> attr[4];
+  if (!smem_limit_once((const void *)kfn, (int)smem, attr[(a1 ? 2 : 0) + (sd ? 1 : 0)])) return -3;
+  const dim3 grid((p.nx - 2 + C::BX - 1) / C::BX, (p.ny - 2 + C::BY - 1) / C::BY,
                   (p.nz - 2 + k.z_chunk - 1) / k.z_chunk);
-  kfn<<<grid, kP3Threads, smem, st>>>(k, m.phi1, m.phi2, m.c, o1, o2, oc, step, err);
-  return 0;
+  return launch_dep_smem(kfn, grid, dim3(C::kThreads), smem, st, k, m.phi1, m.phi2, m.c, o1, o2, oc, step, err) ==
+                 cudaSuccess
+             ? 0
+             : -3;
 }
 
 }  // namespace
@@ -400,13 +497,13 @@ double peri3d_c_offset(const rs3_params &p) {  // clb at T_ref (TiAg.cu:67); c_r
   return (B1 - 0.5 * B2) / (p.A1 - 0.5 * p.A2) + p.A1;
 }
 
-int peri3d_box_width(int precision) { return precision == RS_F64 ? P3Cfg<double>::BXin : peri3d_x2_box_width(); }
-int peri3d_box_height(int precision) { return precision == RS_F64 ? kP3BY + 2 : peri3d_x2_box_height(); }
+int peri3d_box_width(int precision) { return precision == RS_F64 ? D3::BXin : peri3d_x2_box_width(); }
+int peri3d_box_height(int precision) { return precision == RS_F64 ? D3::BYin : peri3d_x2_box_height(); }
 
 int launch_peri3d_step(const rs3_params &p, const P3Maps &m, int precision, void *o1, void *o2, void *oc,
                        int64_t step, int *err, cudaStream_t st) {
   if (precision == RS_F64)
-    return launch_step<double>(p, m, (double *)o1, (double *)o2, (double *)oc, step, err, st);
+    return launch_step(p, m, (double *)o1, (double *)o2, (double *)oc, step, err, st);
   return launch_peri3d_step_x2(p, m, (float *)o1, (float *)o2, (float *)oc, step, err, st);
 }
 
