@@ -29,6 +29,7 @@
 #include <cuda.h>
 
 #include "rs_f32x2.cuh"
+#include "rs_kernels.cuh"
 #include "rs_peri3d_common.cuh"
 #include "rs_surrogate.cuh"
 
@@ -41,6 +42,8 @@ enum { kTT = 0, kTRT, kTdGl, kTdGs, kTAnb, kTAti, kTC0, kTdK };
 // the per-plane CALPHAD groups of one step: one thread per plane z of 0..nz-1
 __global__ void tinb_table_kernel(const K3<double> k, const int64_t step, double *__restrict__ tab) {
   const int z = blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_wait();
+  pdl_trigger();
   if (z >= k.nz) return;
   const double lref = log(k.c_ref / (1.0 - k.c_ref));
   auto terms = [&](int zz, double &T) {
@@ -478,11 +481,16 @@ __global__ void grains_init_kernel(const K3<R> k, const uint64_t seed, const dou
 // each lane rounds as the scalar FP32 operation), in the tiling of the TiAg
 // pair kernel (rs_peri3d_x2.cu): output cells x0 .. x0+63 (x0 a multiple of
 // 64, pairs start on even x), rows y0+1 .. y0+14; input box x0-4 .. x0+67 x
-// y0 .. y0+15 per field and plane by 3D TMA into a four-slot ring; 224
-// threads, warp w owns rows 2w, 2w+1, lane j the pair x0+2j, x0+2j+1.  mu''
-// and S of each plane (tile and halo) are computed once into four-slot rings,
-// so one barrier per plane suffices, as in tinb_kernel.  The surrogate path
-// keeps the scalar kernel.
+// y0 .. y0+15 per field and plane by 3D TMA into a four-slot ring, handed back
+// by the last warp that leaves a plane; 224 threads, warp w owns rows 2w, 2w+1,
+// lane j the pair x0+2j, x0+2j+1.  mu'' of each plane (tile and halo) is
+// computed once into a four-slot ring, S in the place of the plane's c (a thread
+// keeps the c of its own outputs), so one barrier per plane suffices and three
+// CTAs fit on an SM.  The surrogate path keeps the scalar kernel.
+// What bounds it (512 x 512 x 256): instruction issue (54 %, 256 per row of 64
+// cells in melt) and the latencies behind it; all melt 385 us, a front in 60 of
+// the 256 planes 628 -> 451 us.  Of that, the melt form of its own and the wider
+// melt polynomial gave 597 -> 494, the third CTA 494 -> 451.
 constexpr int kT2Threads = 224, kT2BX = 64, kT2BXin = 72, kT2BY = 14, kT2BYin = 16;
 constexpr unsigned long long kOne2 = 0x3F8000003F800000ull, kAbs2 = 0x7FFFFFFF7FFFFFFFull;
 __device__ __forceinline__ unsigned long long f2bits(f2 v) { return (unsigned long long)v; }
@@ -492,18 +500,18 @@ static_assert((kT2Plane * 4) % 128 == 0, "TMA destinations stay 128-byte aligned
 static_assert(kT2Threads == 32 * (kT2BY / 2) && kT2BX == 64, "a warp per row pair, a lane per column pair");
 
 struct T2Smem {
-  alignas(128) float in[kT2Slots][3][kT2Plane];
+  alignas(128) float in[kT2Slots][3][kT2Plane];  // phi1, phi2; c, replaced by S = q(phi1) c (1 - c)
   alignas(16) float mu[kT2MuSlots][kT2Plane];  // mu'' (FP32 form, see mu_cell)
-  alignas(16) float S[kT2MuSlots][kT2Plane];   // face-mobility terms q(phi1) c (1 - c)
   uint64_t full[kT2Slots];
   // per plane (q mod 8): every cell of the box inside the array is pure melt,
   // phi1 == 1 and phi2 == 0 exactly
   int melt[8];
+  uint32_t passed;  // warps that have left a plane, summed over the planes
 };
 
 // A1: the a1 well terms are non-zero; SD: solid diffusivities Da or Db non-zero
 template <bool A1, bool SD>
-__global__ void __launch_bounds__(kT2Threads, 2)
+__global__ void __launch_bounds__(kT2Threads, 3)
     tinb_x2_kernel(const __grid_constant__ K3<float> k, const __grid_constant__ CUtensorMap m1,
                    const __grid_constant__ CUtensorMap m2, const __grid_constant__ CUtensorMap mc,
                    float *__restrict__ o1, float *__restrict__ o2, float *__restrict__ oc, int *err) {
@@ -516,6 +524,8 @@ __global__ void __launch_bounds__(kT2Threads, 2)
   const int zo1 = min(zo0 + k.z_chunk, k.nz - 1);
   if (zo0 >= zo1) return;
   const int zin0 = zo0 - 1, zin1 = zo1;
+  pdl_wait();
+  pdl_trigger();
   constexpr uint32_t kBytes = 3u * kT2Plane * sizeof(float);
   if (smem_u32(smem_raw) & 127u) {
     if (tid == 0) atomicExch(err, 2);
@@ -533,6 +543,7 @@ __global__ void __launch_bounds__(kT2Threads, 2)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int z = zin0; z <= min(zin1, zin0 + kT2Slots - 1); ++z) issue(z);
     for (int s = 0; s < 8; ++s) sm.melt[s] = 1;
+    sm.passed = 0u;
   }
   __syncthreads();
   int issued = min(zin1, zin0 + kT2Slots - 1);
@@ -541,6 +552,25 @@ __global__ void __launch_bounds__(kT2Threads, 2)
   const f2 one = bc(1.f);
   constexpr float L0d = (float)(kL0Bcc - kL0Liq), L0s = (float)(kL0Bcc + kL0Liq), L0x = (float)(kL0Liq - kL0Bcc);
 
+  // this thread's pairs of a plane: its own two outputs (rows ry, ry + 1) and,
+  // for the first three warps, one of the halo that a stencil reaches (row
+  // above, row below, the pairs left and right).  A pair lies wholly inside or
+  // outside the array (nx % 4 == 0, even x); bit u: outside
+  const int ry = 2 * warp;                           // first output row of the thread (tile row)
+  const int ec = (ry + 1) * kT2BXin + 2 * lane + 4;  // box element of its first cell (even)
+  const int eh = warp == 0   ? 2 * lane + 4
+                 : warp == 1 ? (kT2BYin - 1) * kT2BXin + 2 * lane + 4
+                 : warp == 2 && lane < 2 * kT2BY
+                     ? (lane < kT2BY ? (1 + lane) * kT2BXin + 2 : (1 + lane - kT2BY) * kT2BXin + 4 + kT2BX)
+                     : -1;
+  uint32_t outside = 0u;
+#pragma unroll
+  for (int u = 0; u < 3; ++u) {
+    const int e = u < 2 ? ec + u * kT2BXin : max(eh, 0), ax = x0 - 4 + e % kT2BXin, ay = yb + e / kT2BXin;
+    if (!(ax >= 0 && ax < k.nx && ay < k.ny)) outside |= 1u << u;
+  }
+  f2 cn[2];  // c - c_ref of the thread's outputs in the plane that mu_plane saw last
+  const f2 q1m = fma2(bc(-k.AA1), one, bc(k.AA));  // q(1)
   // mu'' and S of plane z (tile and halo) into their ring slots
   auto mu_plane = [&](int z) {
     const int q = z - zin0, s = q % kT2Slots;
@@ -548,25 +578,26 @@ __global__ void __launch_bounds__(kT2Threads, 2)
     // a ghost plane images its neighbour, T included
     const PlaneT<float> t = plane_terms<float>(k.tab, z == 0 ? 1 : (z == k.nz - 1 ? k.nz - 2 : z));
     if (!got) return false;
-    float *mu = sm.mu[q % kT2MuSlots], *Sv = sm.S[q % kT2MuSlots];
-    const float *f1 = sm.in[s][0], *f2p = sm.in[s][1], *fc = sm.in[s][2];
+    float *mu = sm.mu[q % kT2MuSlots], *cS = sm.in[s][2];
+    const float *f1 = sm.in[s][0], *f2p = sm.in[s][1];
     bool all_melt = true;  // this thread's pairs inside the array
-    for (int e = 2 * tid; e < kT2Plane; e += 2 * kT2Threads) {
-      const f2 p1 = ld2(f1 + e), p2 = ld2(f2p + e), d = ld2(fc + e);
-      // a pair lies wholly inside or outside the array (nx % 4 == 0, even x)
-      const int ax = x0 - 4 + e % kT2BXin, ay = yb + e / kT2BXin;
-      const bool inside = ax >= 0 && ax < k.nx && ay < k.ny;
-      const bool melt = f2bits(p1) == kOne2 && (f2bits(p2) & kAbs2) == 0ull;
-      all_melt = all_melt && (melt || !inside);
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      const int e = u < 2 ? ec + u * kT2BXin : eh;
+      if (e < 0) break;
+      const f2 p1 = ld2(f1 + e), p2 = ld2(f2p + e), d = ld2(cS + e);
+      if (u < 2) cn[u] = d;
+      const bool melt = (f2bits(p1) == kOne2 && (f2bits(p2) & kAbs2) == 0ull) || ((outside >> u) & 1u);
+      all_melt = all_melt && melt;
       if (melt && fmaxf(fabsf(lo_of(d)), fabsf(hi_of(d))) <= k.melt_tiny) {
-        // far melt: g = -1, q(1) c (1 - c); lam by its Taylor polynomial
-        // (K3::melt_a), mu'' = d (RT p - 2 L0_Liq), lam = d p
-        f2 pp = fma2(bc(k.melt_a[3]), d, bc(k.melt_a[2]));
-        pp = fma2(pp, d, bc(k.melt_a[1]));
-        pp = fma2(pp, d, bc(k.melt_a[0]));
+        // far melt: g = -1, q(1) = 1, S = c (1 - c); lam by its Taylor
+        // polynomial (K3::melt_a), mu'' = d (RT p - 2 L0_Liq), lam = d p
+        f2 pp = fma2(bc(k.melt_a[7]), d, bc(k.melt_a[6]));
+#pragma unroll
+        for (int j = 5; j >= 0; --j) pp = fma2(pp, d, bc(k.melt_a[j]));
         const f2 c = add2(bc(c_ref), d);
         st2(mu + e, mul2(d, fma2(bc(t.RT), pp, bc((float)(-2.0 * kL0Liq)))));
-        st2(Sv + e, mul2(mul2(p1, fma2(bc(-k.AA1), p1, bc(k.AA))), mul2(c, sub2(one, c))));
+        st2(cS + e, mul2(q1m, mul2(c, sub2(one, c))));
         continue;
       }
       const f2 p3 = sub2(sub2(one, p1), p2);
@@ -587,9 +618,11 @@ __global__ void __launch_bounds__(kT2Threads, 2)
       f2 q1 = mul2(p1, fma2(bc(-k.AA1), p1, bc(k.AA)));
       if constexpr (SD) q1 = fma2(bc(k.Db2), p3, fma2(bc(k.Da2), p2, q1));
       st2(mu + e, m);
-      st2(Sv + e, mul2(q1, mul2(c, omc)));
+      st2(cS + e, mul2(q1, mul2(c, omc)));
     }
     if (!all_melt) sm.melt[q & 7] = 0;
+    // S was written where a later load lands
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     return true;
   };
   auto drain = [&](int from) {
@@ -611,22 +644,19 @@ __global__ void __launch_bounds__(kT2Threads, 2)
   const int gx = x0 + 2 * lane;                                        // array x of the pair's first cell
   const bool v0 = gx >= 1 && gx <= k.nx - 2, v1 = gx + 1 <= k.nx - 2;  // outputs
   const bool any = v0 || v1;
-  const int ry = 2 * warp;                           // first output row of the thread (tile row)
-  const int ec = (ry + 1) * kT2BXin + 2 * lane + 4;  // box element of its first cell (even)
   const int64_t plane = (int64_t)k.nx * k.ny;
-  const bool xedge = !(v0 && v1) || gx == 1 || gx + 1 == k.nx - 2;  // a ghost column is involved
+  const bool xedge = !(v0 && v1);                      // one output, whose image is a ghost column
   const f2 dt = bc(k.dt), dt3 = bc(k.dt * (1.f / 3.f));
 
-  for (int z = zo0; z < zo1; ++z) {
-    // one barrier per plane: afterwards the input slot of plane z-2 takes the
-    // load of plane z+2 (mu'' and S have four slots: plane z+1 overwrites z-3)
+  int64_t out0 = (int64_t)zo0 * plane + (int64_t)(yb + 1 + ry) * k.nx + gx;  // the pair's first cell in plane z
+  for (int z = zo0; z < zo1; ++z, out0 += plane) {
+    const f2 cz[2] = {cn[0], cn[1]};  // plane z
+    // one barrier per plane: the flags, mu'' and S of planes .. z+1 stand behind
+    // it (mu'' and S have four slots: plane z+1 overwrites z-3)
     if (!__syncthreads_and(mu_plane(z + 1))) {
+      issued = min(zin1, z + 2);
       drain(z + 1);
       return;
-    }
-    if (z + 2 <= zin1 && z + 2 > issued) {
-      if (tid == 0) issue(z + 2);
-      issued = z + 2;
     }
     const int q = z - zin0;
     // planes z-1 .. z+1 pure melt wherever a stencil of an output cell reaches:
@@ -636,42 +666,89 @@ __global__ void __launch_bounds__(kT2Threads, 2)
     // iteration z+2) is separated from this write by the barrier of z+1.
     const bool melt3 = sm.melt[(q - 1) & 7] && sm.melt[q & 7] && sm.melt[(q + 1) & 7];
     if (tid == 0) sm.melt[(q + 3) & 7] = 1;
-    if (!any) continue;
-    const float *c1 = sm.in[q % kT2Slots][0], *c2 = sm.in[q % kT2Slots][1], *cc = sm.in[q % kT2Slots][2];
+    if (any) {
+    const float *c1 = sm.in[q % kT2Slots][0], *c2 = sm.in[q % kT2Slots][1];
     const float *d1 = sm.in[(q - 1) % kT2Slots][0], *d2 = sm.in[(q - 1) % kT2Slots][1];
     const float *u1 = sm.in[(q + 1) % kT2Slots][0], *u2 = sm.in[(q + 1) % kT2Slots][1];
     const float *mu = sm.mu[q % kT2MuSlots], *mud = sm.mu[(q - 1) % kT2MuSlots], *muu = sm.mu[(q + 1) % kT2MuSlots];
-    const float *Sc = sm.S[q % kT2MuSlots], *Sd = sm.S[(q - 1) % kT2MuSlots], *Su = sm.S[(q + 1) % kT2MuSlots];
-    const PlaneT<float> t = plane_terms<float>(k.tab, z);
+    const float *Sc = sm.in[q % kT2Slots][2], *Sd = sm.in[(q - 1) % kT2Slots][2], *Su = sm.in[(q + 1) % kT2Slots][2];
     // z faces of mu'' add the melt's mu difference between the planes; a face
     // to a ghost plane has none (the ghost's mu'' is taken at this T)
-    const f2 dKu = bc(z + 1 < k.nz - 1 ? t.dK : 0.f);
+    const f2 dKu = bc(z + 1 < k.nz - 1 ? (float)k.tab[(int64_t)kTW * z + kTdK] : 0.f);
     const f2 dKd = bc(z - 1 > 0 ? (float)k.tab[(int64_t)kTW * (z - 1) + kTdK] : 0.f);
-    const int zg = z == 1 ? 0 : (z == k.nz - 2 ? k.nz - 1 : -1);
-    // column window rows ry-1 .. ry+2 of phi1, phi2, mu'', S (pairs)
-    f2 w1[4], w2[4], wm[4], ws[4];
+    const int zd = z == 1 ? -1 : (z == k.nz - 2 ? 1 : 0);  // planes 0 and nz-1 copy their neighbours
+    // stores: the pair, and every ghost cell that images one of its cells
+    // (rows and planes: uniform over the warp; columns: the pairs (0, 1) and
+    // (nx-2, nx-1), one cell and its image each)
+    auto store_row = [&](int64_t o, f2 n1, f2 n2, f2 nc) {  // o: the pair's first cell
+      if (!xedge) {
+        st2(o1 + o, n1);
+        st2(o2 + o, n2);
+        st2(oc + o, nc);
+      } else {
+        const float a = v1 ? hi_of(n1) : lo_of(n1), b2 = v1 ? hi_of(n2) : lo_of(n2), cv = v1 ? hi_of(nc) : lo_of(nc);
+        const int64_t oi = o + (v1 ? 1 : 0), og = oi + (v1 ? k.nx - 2 : 2 - k.nx);
+        o1[oi] = a, o1[og] = a;
+        o2[oi] = b2, o2[og] = b2;
+        oc[oi] = cv, oc[og] = cv;
+      }
+    };
+    auto store_pair = [&](int r, f2 n1, f2 n2, f2 nc) {
+      const int64_t o = out0 + r * k.nx;
+      store_row(o, n1, n2, nc);
+      const int gy = yb + 1 + ry + r;
+      const int yd = gy == k.ny - 2 ? 2 - k.ny : (gy == 1 ? k.ny - 2 : 0);  // to the image row, plane
+      if (yd | zd) {
+#pragma unroll 1
+        for (int im = 1; im < 4; ++im) {
+          if (((im & 1) && !yd) || ((im & 2) && !zd)) continue;
+          store_row(o + (im & 1 ? (int64_t)yd * k.nx : 0) + (im & 2 ? zd * plane : 0), n1, n2, nc);
+        }
+      }
+    };
+    // column window rows ry-1 .. ry+2 of mu'', S (pairs)
+    f2 wm[4], ws[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int e = ec + (r - 1) * kT2BXin;
+      wm[r] = ld2(mu + e);
+      ws[r] = ld2(Sc + e);
+    }
+    // the solute update of row r: face mobility (S + S') / 2 (the 1/2 is in cf)
+    auto solute = [&](int r, f2 cv) {
+      const int e = ec + r * kT2BXin;
+      const f2 m0 = wm[r + 1], S0 = ws[r + 1];
+      // x neighbours: (left, right) pairs from the pairs beside this one
+      const f2 Lm = ld2(mu + e - 2), Rm = ld2(mu + e + 2), Ls = ld2(Sc + e - 2), Rs = ld2(Sc + e + 2);
+      const f2 mxm = pk(hi_of(Lm), lo_of(m0)), mxp = pk(hi_of(m0), lo_of(Rm));
+      const f2 sxm = pk(hi_of(Ls), lo_of(S0)), sxp = pk(hi_of(S0), lo_of(Rs));
+      const f2 jx = fma2(add2(S0, sxp), sub2(mxp, m0), mul2(add2(S0, sxm), sub2(mxm, m0)));
+      const f2 jy = fma2(add2(S0, ws[r + 2]), sub2(wm[r + 2], m0), mul2(add2(S0, ws[r]), sub2(wm[r], m0)));
+      const f2 jz = fma2(add2(S0, ld2(Su + e)), add2(sub2(ld2(muu + e), m0), dKu),
+                         mul2(add2(S0, ld2(Sd + e)), sub2(sub2(ld2(mud + e), m0), dKd)));
+      return add2(cv, fma2(bc(k.cfz), jz, fma2(bc(k.cfy), jy, mul2(bc(k.cfx), jx))));
+    };
+    if (melt3) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        if (yb + 1 + ry + r > k.ny - 2) break;
+        store_pair(r, bc(1.f), bc(0.f), solute(r, cz[r]));
+      }
+    } else {
+    const PlaneT<float> t = plane_terms<float>(k.tab, z);
+    f2 w1[4], w2[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int e = ec + (r - 1) * kT2BXin;
       w1[r] = ld2(c1 + e);
       w2[r] = ld2(c2 + e);
-      wm[r] = ld2(mu + e);
-      ws[r] = ld2(Sc + e);
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-      const int gy = yb + 1 + ry + r;
-      if (gy > k.ny - 2) break;
+      if (yb + 1 + ry + r > k.ny - 2) break;
       const int e = ec + r * kT2BXin;
-      const f2 p1 = w1[r + 1], p2 = w2[r + 1], m0 = wm[r + 1], S0 = ws[r + 1];
-      const f2 cv = ld2(cc + e);
-      // x neighbours: (left, right) pairs from the pairs beside this one
-      const f2 Lm = ld2(mu + e - 2), Rm = ld2(mu + e + 2), Ls = ld2(Sc + e - 2), Rs = ld2(Sc + e + 2);
-      const f2 mxm = pk(hi_of(Lm), lo_of(m0)), mxp = pk(hi_of(m0), lo_of(Rm));
-      const f2 sxm = pk(hi_of(Ls), lo_of(S0)), sxp = pk(hi_of(S0), lo_of(Rs));
-
-      f2 n1 = bc(1.f), n2 = bc(0.f);
-      if (!melt3) {
+      const f2 p1 = w1[r + 1], p2 = w2[r + 1];
+      const f2 cv = cz[r];
       const f2 L1 = ld2(c1 + e - 2), R1 = ld2(c1 + e + 2), L2 = ld2(c2 + e - 2), R2 = ld2(c2 + e + 2);
       const f2 x1m = pk(hi_of(L1), lo_of(p1)), x1p = pk(hi_of(p1), lo_of(R1));
       const f2 x2m = pk(hi_of(L2), lo_of(p2)), x2p = pk(hi_of(p2), lo_of(R2));
@@ -720,45 +797,17 @@ __global__ void __launch_bounds__(kT2Threads, 2)
       const f2 lap2 = lap(p2, x2p, x2m, w2[r + 2], w2[r], ld2(u2 + e), ld2(d2 + e));
       // phi_i' = phi_i + dt lap_i - dt (2F_i - F_j - F_k) / 3
       const f2 T3 = mul2(add2(add2(F1, F2), F3), dt3);
-      n1 = fma2(F1, bc(-k.dt), add2(T3, fma2(lap1, dt, p1)));
-      n2 = fma2(F2, bc(-k.dt), add2(T3, fma2(lap2, dt, p2)));
-      }
-      // solute: face mobility (S + S') / 2 (the 1/2 is in cf)
-      const f2 jx = fma2(add2(S0, sxp), sub2(mxp, m0), mul2(add2(S0, sxm), sub2(mxm, m0)));
-      const f2 jy = fma2(add2(S0, ws[r + 2]), sub2(wm[r + 2], m0), mul2(add2(S0, ws[r]), sub2(wm[r], m0)));
-      const f2 jz = fma2(add2(S0, ld2(Su + e)), add2(sub2(ld2(muu + e), m0), dKu),
-                         mul2(add2(S0, ld2(Sd + e)), sub2(sub2(ld2(mud + e), m0), dKd)));
-      const f2 nc = add2(cv, fma2(bc(k.cfz), jz, fma2(bc(k.cfy), jy, mul2(bc(k.cfx), jx))));
-      // stores: the pair, and every ghost cell that images one of its cells
-      const int yg = gy == k.ny - 2 ? 0 : (gy == 1 ? k.ny - 1 : -1);
-      const int64_t o = (int64_t)z * plane + (int64_t)gy * k.nx + gx;
-      if (!xedge && (yg & zg) < 0) {
-        st2(o1 + o, n1);
-        st2(o2 + o, n2);
-        st2(oc + o, nc);
-      } else {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int x = gx + h;
-          if (!(h ? v1 : v0)) continue;
-          const float a = h ? hi_of(n1) : lo_of(n1), bb = h ? hi_of(n2) : lo_of(n2), cvv = h ? hi_of(nc) : lo_of(nc);
-          const int xg = x == k.nx - 2 ? 0 : (x == 1 ? k.nx - 1 : -1);
-          const int xs[2] = {x, xg}, ys[2] = {gy, yg}, zs[2] = {z, zg};
-#pragma unroll
-          for (int ia = 0; ia < 2; ++ia)
-#pragma unroll
-            for (int ib = 0; ib < 2; ++ib)
-#pragma unroll
-              for (int ic = 0; ic < 2; ++ic) {
-                if (xs[ia] < 0 || ys[ib] < 0 || zs[ic] < 0) continue;
-                const int64_t oo = (int64_t)zs[ic] * plane + (int64_t)ys[ib] * k.nx + xs[ia];
-                o1[oo] = a;
-                o2[oo] = bb;
-                oc[oo] = cvv;
-              }
-        }
-      }
+      const f2 n1 = fma2(F1, bc(-k.dt), add2(T3, fma2(lap1, dt, p1)));
+      const f2 n2 = fma2(F2, bc(-k.dt), add2(T3, fma2(lap2, dt, p2)));
+      store_pair(r, n1, n2, solute(r, cv));
     }
+    }
+    }
+    // the last warp that leaves plane z hands the slot of plane z-1 to the load
+    // of plane z+3, without waiting for plane z+2 first: two loads in flight
+    __syncwarp();
+    if (lane == 0 && arrive_count(&sm.passed) % (kT2Threads / 32) == kT2Threads / 32 - 1 && z + 3 <= zin1)
+      issue(z + 3);
   }
 }
 
@@ -769,8 +818,7 @@ int launch_tinb_x2(const K3<float> &k, const P3Maps &m, float *o1, float *o2, fl
   static std::atomic<unsigned long long> attr;
   if (!smem_limit_once((const void *)kfn, (int)smem, attr)) return -3;
   const dim3 grid((k.nx + kT2BX - 1) / kT2BX, (k.ny - 2 + kT2BY - 1) / kT2BY, (k.nz - 2 + k.z_chunk - 1) / k.z_chunk);
-  kfn<<<grid, kT2Threads, smem, st>>>(k, m.phi1, m.phi2, m.c, o1, o2, oc, err);
-  return 0;
+  return launch_dep_smem(kfn, grid, dim3(kT2Threads), smem, st, k, m.phi1, m.phi2, m.c, o1, o2, oc, err) == cudaSuccess ? 0 : -3;
 }
 
 template <typename R, bool SD, bool SURR>
@@ -799,7 +847,7 @@ int launch_tinb_step(const rs3_params &p, const P3Maps &m, int precision, void *
                      int *err, double *tab, const SurrArgs *surr, cudaStream_t st) {
   {
     K3<double> kt = make_k3<double>(p);
-    tinb_table_kernel<<<(p.nz + 127) / 128, 128, 0, st>>>(kt, step, tab);
+    launch_dep(tinb_table_kernel, dim3((p.nz + 127) / 128), dim3(128), st, kt, step, tab);
   }
   const bool sd = p.Da != 0.0 || p.Db != 0.0;
   SurrArgs none;

@@ -4,13 +4,15 @@ and fronts several times within a chunk, in whole planes and in parts of them.
 One step against the FP64 oracle, and every z chunk length bit for bit the
 same.  Tolerances: FP64 1e-13 (as the one-step oracle test); FP32 64 ulp of 1,
 2^-24 each: every term of an update is below 1 in size (dt lambda = 0.45,
-dt (2 / dx^2) 3 = 0.36) and some 50 roundings add up."""
+dt (2 / dx^2) 3 = 0.36) and some 50 roundings add up.  Ti-Nb in FP32: the
+roundings of mu are 16 ulp of its span, and reach c by the six faces of a cell,
+cf (S + S') each; those of phi are 64 ulp of 1 + the largest update."""
 import numpy as np
 import pytest
 import torch
 
 import pyoracle
-from rapidsolid import lib
+from rapidsolid import configs, lib
 from test_gpu_peri3d import params, run_gpu
 
 pytestmark = pytest.mark.gpu
@@ -18,7 +20,7 @@ pytestmark = pytest.mark.gpu
 TOL = {torch.float64: 1e-13, torch.float32: 64 * 2.0**-24}
 
 
-def fields(p, seed, off, base):
+def fields(p, seed, off, base, span=0.01):
     """Melt with slabs, single planes, single cells and a corner of mixed phase;
     the values are FP32 (c - off), ghost layers as images."""
     r = np.random.default_rng(seed)
@@ -36,7 +38,7 @@ def fields(p, seed, off, base):
             mixed[z, : p.ny // 2, p.nx // 3 :] = True
     a[mixed] = r.random(mixed.sum(), np.float32)
     b[mixed] = (1.0 - a[mixed]) * r.random(mixed.sum(), np.float32)
-    d = (base - off + 0.01 * (r.random(shape) - 0.5)).astype(np.float32)
+    d = (base - off + span * (r.random(shape) - 0.5)).astype(np.float32)
     out = [a.astype(np.float64), b.astype(np.float64), d.astype(np.float64) + off]
     for f in out:  # periodic x, y; no-flux z
         f[:, :, 0], f[:, :, -1] = f[:, :, -2], f[:, :, 1].copy()
@@ -55,7 +57,39 @@ def test_changes_between_melt_and_fronts(shape, dtype):
     ref = pyoracle.run3(p, f, 1)
     for x, y in zip(out, ref):
         assert np.abs(x - y).max() <= TOL[dtype]
+    same_for_every_chunk(lambda chunk: params(*shape, G_T=-2e-4, z_T=12.0, z_chunk=chunk), f, dtype)
+
+
+def same_for_every_chunk(make, f, dtype):
+    base = run_gpu(make(0), f, 3, dtype)
     for chunk in (1, 2, 5, 64):
-        q = params(*shape, G_T=-2e-4, z_T=12.0, z_chunk=chunk)
-        for x, y in zip(run_gpu(q, f, 3, dtype), run_gpu(p, f, 3, dtype)):
+        for x, y in zip(run_gpu(make(chunk), f, 3, dtype), base):
             assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("well", [0.0, 2.0])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("shape", [(4, 4, 4), (64, 16, 33), (68, 17, 40), (132, 31, 70), (36, 15, 5)])
+def test_tinb_changes_between_melt_and_fronts(shape, dtype, well):
+    """c within 0.0125 of c_ref = 0.9: both sides of the melt polynomial's range."""
+
+    def make(chunk):
+        p = configs.tinb_3d(nx=shape[0], ny=shape[1], nz=shape[2], z_front=12.0)
+        p.z_chunk, p.a1 = chunk, well
+        p.Da = 0.1 * well
+        return p
+
+    p = make(0)
+    f = fields(p, sum(shape), p.c_ref, p.c_ref, 0.025)
+    out, ref = run_gpu(p, f, 1, dtype), pyoracle.run3(p, f, 1)
+    if dtype == torch.float64:
+        tol_phi = tol_c = 1e-13 * (1.0 + max(np.abs(a - b).max() for a, b in zip(ref, f)))
+    else:
+        ulp = 2.0**-24
+        cf = 0.5 * p.dt * p.alpha * p.dx_inv**2
+        s_max = max(1.0, 0.25 * p.AA**2 / (p.AA - 1.0)) * 0.1 * 0.9 * 1.2 + 0.1 * well * 0.1
+        tol_phi = 64 * ulp * (1.0 + max(np.abs(ref[i] - f[i]).max() for i in (0, 1)))
+        tol_c = 64 * ulp + 6 * cf * 2 * s_max * 16 * ulp * np.ptp(pyoracle.mu3(p, *f))
+    assert max(np.abs(out[i] - ref[i]).max() for i in (0, 1)) <= tol_phi
+    assert np.abs(out[2] - ref[2]).max() <= tol_c
+    same_for_every_chunk(make, f, dtype)
