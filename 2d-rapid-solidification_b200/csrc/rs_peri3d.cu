@@ -474,15 +474,16 @@ __global__ void peri3d_ghost_kernel(const K3<R> k, int axis, R *__restrict__ f1,
 int launch_step(const rs3_params &p, const P3Maps &m, double *o1, double *o2, double *oc, int64_t step, int *err,
                 cudaStream_t st) {
   using C = D3;
-  const K3<double> k = make_k3<double>(p);
+  K3<double> k = make_k3<double>(p);
   const size_t smem = sizeof(P3Smem) + 128;
   const bool a1 = p.a1 != 0.0, sd = p.Da != 0.0 || p.Db != 0.0;
   auto kfn = a1 ? (sd ? peri3d_kernel<true, true> : peri3d_kernel<true, false>)
                 : (sd ? peri3d_kernel<false, true> : peri3d_kernel<false, false>);
   static std::atomic<unsigned long long> attr[4];
   if (!smem_limit_once((const void *)kfn, (int)smem, attr[(a1 ? 2 : 0) + (sd ? 1 : 0)])) return -3;
-  const dim3 grid((p.nx - 2 + C::BX - 1) / C::BX, (p.ny - 2 + C::BY - 1) / C::BY,
-                  (p.nz - 2 + k.z_chunk - 1) / k.z_chunk);
+  dim3 grid((p.nx - 2 + C::BX - 1) / C::BX, (p.ny - 2 + C::BY - 1) / C::BY);
+  k.z_chunk = p3_chunk(p, (int64_t)grid.x * grid.y, 2, 0.5);
+  grid.z = (p.nz - 2 + k.z_chunk - 1) / k.z_chunk;
   return launch_dep_smem(kfn, grid, dim3(C::kThreads), smem, st, k, m.phi1, m.phi2, m.c, o1, o2, oc, step, err) ==
                  cudaSuccess
              ? 0

@@ -6,6 +6,8 @@
 
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "rs_peri3d.cuh"
 #include "rs_step_common.cuh"
 
@@ -43,9 +45,36 @@ __device__ __forceinline__ R gp2(R pi, R pj, R pk) {
   return R(7.5) * (pi - R(1)) * (pi * pi) * (pj - pk);
 }
 
+// z planes per CTA where the caller leaves the choice (z_chunk == 0): the least
+// (waves + 1/2)(c + halo) of c = 32, 16, 8, 4, 2, halo being what the two planes
+// that a chunk reads beside those it writes cost, in planes.  The half wave
+// stands for the last one and for fronts, whose planes take longer than melt.
+// A march of 32 planes left small volumes with a few dozen CTAs, us per step:
+//             planes:  2     4     8     16    32
+//   TiAg FP32 128^3    23    24    36    42    79
+//             256^3    126   113   108   108   139
+//             512^3    812   715   672   658   664
+//   TiAg FP64 128^3    48    44    45    61    86
+//             256^3    262   223   211   209   227
+//   Ti-Nb FP32 256^3   172   145   133   133   148
+//   Ti-Nb FP64 256^3   521   426   381   348   366
+// The results do not depend on it.
+inline int p3_chunk(const rs3_params &p, int64_t tiles, int ctas_per_sm, double halo) {
+  if (p.z_chunk > 0) return p.z_chunk;
+  int best = 32;
+  double least = 1e300;
+  for (int c = 32; c >= 2; c /= 2) {
+    const double waves = (double)(tiles * ((p.nz - 2 + c - 1) / c)) / (148 * ctas_per_sm);
+    const double cost = (std::max(waves, 1.0) + 0.5) * (c + halo);
+    if (cost < least) least = cost, best = c;
+  }
+  return best;
+}
+
 template <typename R>
 struct K3 {  // kernel constants in the working precision
   int nx, ny, nz, z_chunk;
+  int count_chunk;  // the z chunk that the surrogate's counters stand for
   R dt, dxi, dyi, dzi, dxi2, dyi2, dzi2;
   R a1, a2, a3, b, lam, Da2, Db2, cfx, cfy, cfz;
   R r1, r2, r3;
@@ -69,7 +98,7 @@ K3<R> make_k3(const rs3_params &p) {
   k.nx = p.nx;
   k.ny = p.ny;
   k.nz = p.nz;
-  k.z_chunk = p.z_chunk > 0 ? p.z_chunk : 32;
+  k.z_chunk = k.count_chunk = p.z_chunk > 0 ? p.z_chunk : 32;
   k.dt = (R)p.dt;
   k.dxi = (R)p.dx_inv;
   k.dyi = (R)p.dy_inv;

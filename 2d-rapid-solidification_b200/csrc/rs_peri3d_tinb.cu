@@ -149,6 +149,7 @@ struct TSmem {
   alignas(16) float dG[3][SURR ? P3Cfg<R>::BX * kP3BY : 1];
   uint64_t full[kP3Slots];
   int melt[8];  // per plane (q mod 8): the box is pure melt inside the array (p3_melt_cell)
+  uint32_t passed;  // warps that have left a plane, summed over the planes
 };
 
 // SD: solid diffusivities Da or Db non-zero
@@ -170,6 +171,8 @@ __global__ void __launch_bounds__(kP3Threads, 2)
   const int zo1 = min(zo0 + k.z_chunk, k.nz - 1);
   if (zo0 >= zo1) return;
   const int zin0 = zo0 - 1, zin1 = zo1;
+  pdl_wait();
+  pdl_trigger();
   constexpr uint32_t kBytes = 3u * C::kPlane * sizeof(R);
   if (smem_u32(smem_raw) & 127u) {
     if (tid == 0) atomicExch(err, 2);
@@ -186,6 +189,7 @@ __global__ void __launch_bounds__(kP3Threads, 2)
   if (tid == 0) {
     for (int s = 0; s < kP3Slots; ++s) mbar_init(&sm.full[s], 1);
     for (int s = 0; s < 8; ++s) sm.melt[s] = 1;
+    sm.passed = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int z = zin0; z <= min(zin1, zin0 + kP3Slots - 1); ++z) issue(z);
   }
@@ -227,6 +231,15 @@ __global__ void __launch_bounds__(kP3Threads, 2)
       constexpr unsigned FULL = 0xffffffffu;
       const int warp = tid >> 5, lane = tid & 31;
       float *dg = sm.dG[q % 3];
+      // the counters count a cell as often as a march in chunks of count_chunk
+      // planes reads its plane (each chunk reads the plane before and the plane
+      // behind); once per plane, by the chunk that writes it
+      auto count = [&](unsigned long long *counter) {
+        const int cc = k.count_chunk;
+        if (!((z >= zo0 && z < zo1) || z == 0 || z == k.nz - 1)) return;
+        atomicAdd(counter, 1ull + (z > 0 && z % cc == 0 && z + 1 <= k.nz - 2) +
+                               (z < k.nz - 1 && z > cc && z == 1 + cc * ((z - 1) / cc)));
+      };
       const bool T_in = t.T >= SA.T_lo && t.T <= SA.T_hi;
       const float xT = (t.T - SA.T_mid) * SA.T_ihalf;
       for (int base = 32 * warp; base < C::kPlane; base += kP3Threads) {
@@ -255,13 +268,13 @@ __global__ void __launch_bounds__(kP3Threads, 2)
           if (audit) {
             atomicMax(&SA.audit[0], (unsigned long long)__float_as_uint(fabsf(m_net - m)));
             atomicMax(&SA.audit[1], (unsigned long long)__float_as_uint(fabsf(dG_net - dGv)));
-            atomicAdd(&SA.audit[3], 1ull);
+            count(&SA.audit[3]);
           } else if (net) {
             m = m_net;
             dGv = dG_net;
           }
         }
-        if (in && !melt && !inbox) atomicAdd(&SA.audit[2], 1ull);
+        if (in && !melt && !inbox) count(&SA.audit[2]);
         if (in) all_melt = all_melt && p3_melt_cell(k, p1, p2, xb + e % C::BXin, yb + e / C::BXin);
         if (in) {
           const float q1 = p1 * (k.AA - k.AA1 * p1) + (SD ? k.Da2 * p2 + k.Db2 * (1.f - p1 - p2) : 0.f);
@@ -301,8 +314,7 @@ __global__ void __launch_bounds__(kP3Threads, 2)
   const R third = R(1) / R(3);
 
   for (int z = zo0; z < zo1; ++z) {
-    // one barrier per plane (see rs_peri3d.cu): afterwards the input slot of
-    // plane z-2 takes the load of plane z+2
+    // one barrier per plane (see rs_peri3d.cu)
     if (!__syncthreads_and(mu_plane(z + 1))) {
       drain(z + 1);
       return;
@@ -812,27 +824,32 @@ __global__ void __launch_bounds__(kT2Threads, 3)
 }
 
 template <bool A1, bool SD>
-int launch_tinb_x2(const K3<float> &k, const P3Maps &m, float *o1, float *o2, float *oc, int *err, cudaStream_t st) {
+int launch_tinb_x2(const rs3_params &p, K3<float> k, const P3Maps &m, float *o1, float *o2, float *oc, int *err, cudaStream_t st) {
   const size_t smem = sizeof(T2Smem) + 128;
   auto kfn = tinb_x2_kernel<A1, SD>;
   static std::atomic<unsigned long long> attr;
   if (!smem_limit_once((const void *)kfn, (int)smem, attr)) return -3;
-  const dim3 grid((k.nx + kT2BX - 1) / kT2BX, (k.ny - 2 + kT2BY - 1) / kT2BY, (k.nz - 2 + k.z_chunk - 1) / k.z_chunk);
+  dim3 grid((k.nx + kT2BX - 1) / kT2BX, (k.ny - 2 + kT2BY - 1) / kT2BY);
+  k.z_chunk = p3_chunk(p, (int64_t)grid.x * grid.y, 3, 0.5);
+  grid.z = (k.nz - 2 + k.z_chunk - 1) / k.z_chunk;
   return launch_dep_smem(kfn, grid, dim3(kT2Threads), smem, st, k, m.phi1, m.phi2, m.c, o1, o2, oc, err) == cudaSuccess ? 0 : -3;
 }
 
 template <typename R, bool SD, bool SURR>
-int launch_tinb(const K3<R> &k, const P3Maps &m, R *o1, R *o2, R *oc, int64_t step, int *err, const SurrArgs &sa,
+int launch_tinb(const rs3_params &p, K3<R> k, const P3Maps &m, R *o1, R *o2, R *oc, int64_t step, int *err, const SurrArgs &sa,
                 cudaStream_t st) {
   using C = P3Cfg<R>;
   const size_t smem = sizeof(TSmem<R, SURR>) + 128;
   auto kfn = tinb_kernel<R, SD, SURR>;
   static std::atomic<unsigned long long> attr;
   if (!smem_limit_once((const void *)kfn, (int)smem, attr)) return -3;
-  const dim3 grid((k.nx - 2 + C::BX - 1) / C::BX, (k.ny - 2 + kP3BY - 1) / kP3BY,
-                  (k.nz - 2 + k.z_chunk - 1) / k.z_chunk);
-  kfn<<<grid, kP3Threads, smem, st>>>(k, m.phi1, m.phi2, m.c, o1, o2, oc, step, err, sa);
-  return 0;
+  dim3 grid((k.nx - 2 + C::BX - 1) / C::BX, (k.ny - 2 + kP3BY - 1) / kP3BY);
+  k.z_chunk = p3_chunk(p, (int64_t)grid.x * grid.y, 2, 2.0);  // (halo planes: logarithms, networks)
+  grid.z = (k.nz - 2 + k.z_chunk - 1) / k.z_chunk;
+  return launch_dep_smem(kfn, grid, dim3(kP3Threads), smem, st, k, m.phi1, m.phi2, m.c, o1, o2, oc, step, err, sa) ==
+                 cudaSuccess
+             ? 0
+             : -3;
 }
 
 }  // namespace
@@ -856,8 +873,8 @@ int launch_tinb_step(const rs3_params &p, const P3Maps &m, int precision, void *
     if (surr) return -4;
     K3<double> k = make_k3<double>(p);
     k.tab = tab;
-    return sd ? launch_tinb<double, true, false>(k, m, (double *)o1, (double *)o2, (double *)oc, step, err, none, st)
-              : launch_tinb<double, false, false>(k, m, (double *)o1, (double *)o2, (double *)oc, step, err, none,
+    return sd ? launch_tinb<double, true, false>(p, k, m, (double *)o1, (double *)o2, (double *)oc, step, err, none, st)
+              : launch_tinb<double, false, false>(p, k, m, (double *)o1, (double *)o2, (double *)oc, step, err, none,
                                                   st);
   }
   K3<float> k = make_k3<float>(p);
@@ -865,14 +882,14 @@ int launch_tinb_step(const rs3_params &p, const P3Maps &m, int precision, void *
   k.c_off = p.c_ref;
   float *f1 = (float *)o1, *f2 = (float *)o2, *fc = (float *)oc;
   if (surr)
-    return sd ? launch_tinb<float, true, true>(k, m, f1, f2, fc, step, err, *surr, st)
-              : launch_tinb<float, false, true>(k, m, f1, f2, fc, step, err, *surr, st);
+    return sd ? launch_tinb<float, true, true>(p, k, m, f1, f2, fc, step, err, *surr, st)
+              : launch_tinb<float, false, true>(p, k, m, f1, f2, fc, step, err, *surr, st);
   // the exact FP32 step on packed pairs
   const bool a1 = p.a1 != 0.0;
-  return a1 ? (sd ? launch_tinb_x2<true, true>(k, m, f1, f2, fc, err, st)
-                  : launch_tinb_x2<true, false>(k, m, f1, f2, fc, err, st))
-            : (sd ? launch_tinb_x2<false, true>(k, m, f1, f2, fc, err, st)
-                  : launch_tinb_x2<false, false>(k, m, f1, f2, fc, err, st));
+  return a1 ? (sd ? launch_tinb_x2<true, true>(p, k, m, f1, f2, fc, err, st)
+                  : launch_tinb_x2<true, false>(p, k, m, f1, f2, fc, err, st))
+            : (sd ? launch_tinb_x2<false, true>(p, k, m, f1, f2, fc, err, st)
+                  : launch_tinb_x2<false, false>(p, k, m, f1, f2, fc, err, st));
 }
 
 int launch_tinb_mu(const rs3_params &p, int precision, const void *f1, const void *f2, const void *fc, void *mu,

@@ -32,7 +32,7 @@
 
 #include "rs_f32x2.cuh"
 #include "rs_kernels.cuh"
-#include "rs_peri3d.cuh"
+#include "rs_peri3d_common.cuh"
 #include "rs_step_common.cuh"
 
 namespace rs {
@@ -409,7 +409,6 @@ int launch_peri3d_step_x2(const rs3_params &p, const P3Maps &m, float *o1, float
   k.nx = p.nx;
   k.ny = p.ny;
   k.nz = p.nz;
-  k.z_chunk = p.z_chunk > 0 ? p.z_chunk : 32;
   k.a1 = (float)p.a1;
   k.a2 = (float)p.a2;
   k.a3 = (float)p.a3;
@@ -447,7 +446,9 @@ int launch_peri3d_step_x2(const rs3_params &p, const P3Maps &m, float *o1, float
   static std::atomic<unsigned long long> attr[4];
   const int which = (a1 ? 2 : 0) + (sd ? 1 : 0);
   if (!smem_limit_once((const void *)kfn, (int)smem, attr[which])) return -3;
-  const dim3 grid((p.nx + kX2BX - 1) / kX2BX, (p.ny - 2 + kX2BY - 1) / kX2BY, (p.nz - 2 + k.z_chunk - 1) / k.z_chunk);
+  dim3 grid((p.nx + kX2BX - 1) / kX2BX, (p.ny - 2 + kX2BY - 1) / kX2BY);
+  k.z_chunk = p3_chunk(p, (int64_t)grid.x * grid.y, 3, 0.5);
+  grid.z = (p.nz - 2 + k.z_chunk - 1) / k.z_chunk;
   return launch_dep_smem(kfn, grid, dim3(kX2Threads), smem, st, k, m.phi1, m.phi2, m.c, o1, o2, oc, step, err) == cudaSuccess ? 0 : -3;
 }
 

@@ -446,7 +446,7 @@ int rs_ensemble_set_path(rs_ens *e, int32_t path);
  * solute coefficient per J/mol (Dl / (Gamma muk0 h0 v0) of the 2D model). */
 typedef struct rs3_params {
   int32_t nx, ny, nz;               /* extents incl. ghost layers (TiAg Nx, Ny, devNz) */
-  int32_t z_chunk;                  /* planes per CTA of the z march (0: 32) */
+  int32_t z_chunk;                  /* planes per CTA of the z march (0: by the volume) */
   double dt;                        /* DT */
   double dx_inv, dy_inv, dz_inv;    /* DXin, DYin, DZin */
   double a1, a2, a3, b;             /* three-phase well terms */

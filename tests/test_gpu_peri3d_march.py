@@ -12,8 +12,8 @@ import pytest
 import torch
 
 import pyoracle
-from rapidsolid import configs, lib
-from test_gpu_peri3d import params, run_gpu
+from rapidsolid import configs, lib, surrogate
+from test_gpu_peri3d import params, run_gpu, to_gpu, to_host
 
 pytestmark = pytest.mark.gpu
 
@@ -93,3 +93,30 @@ def test_tinb_changes_between_melt_and_fronts(shape, dtype, well):
     assert max(np.abs(out[i] - ref[i]).max() for i in (0, 1)) <= tol_phi
     assert np.abs(out[2] - ref[2]).max() <= tol_c
     same_for_every_chunk(make, f, dtype)
+
+
+def test_surrogate_counters_do_not_depend_on_the_chosen_chunk():
+    """z_chunk = 0 picks a chunk by the volume; the audit's counters stay those
+    of a march in chunks of 32 planes, and so do the fields."""
+    p = configs.tinb_3d(nx=68, ny=31, nz=70, z_front=12.0)
+    p2 = configs.scale()
+    p2.cinf = p.c_ref
+    w, box, _ = surrogate.train(p2, box=surrogate.fitted_box(), n_samples=1 << 14, epochs=1, batch=4096, seed=3,
+                                g_input=True)
+    f = fields(p, 7, p.c_ref, p.c_ref, 0.1)
+    out = []
+    for chunk in (0, 32):
+        p.z_chunk = chunk
+        ctx = lib.Context3(p)
+        ctx.set_surrogate(w, box)
+        a, b = to_gpu(p, f, torch.float32), lib.FieldSet3(p, torch.float32)
+        for k in range(3):
+            ctx.step(a, b, k)
+            a, b = b, a
+        torch.cuda.synchronize()
+        ctx.device_status()
+        out.append((to_host(a, p), ctx.surrogate_audit()))
+        ctx.close()
+    assert out[0][1] == out[1][1] and out[0][1][3] > 0
+    for x, y in zip(out[0][0], out[1][0]):
+        assert np.array_equal(x, y)
