@@ -205,11 +205,25 @@ class HostBuffer:
             pass
 
 
+_raw_stream = None  # () -> handle of the current stream of the current device
+
+
 def _stream(stream):
-    import torch
-    if stream is None:
-        stream = torch.cuda.current_stream()
-    return C.c_void_p(stream.cuda_stream)
+    global _raw_stream
+    if stream is not None:
+        return C.c_void_p(stream.cuda_stream)
+    if _raw_stream is None:
+        import torch
+        torch.cuda.current_stream()  # (initialises CUDA)
+        try:
+            raw, dev = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+            raw(dev())
+        except AttributeError:
+            _raw_stream = lambda: torch.cuda.current_stream().cuda_stream  # noqa: E731
+        else:
+            # no Stream object per call: 0.2 us instead of 1.3
+            _raw_stream = lambda: raw(dev())  # noqa: E731
+    return C.c_void_p(_raw_stream())
 
 
 class FieldSet:
@@ -228,9 +242,9 @@ class FieldSet:
         self.precision = _abi.RS_F64 if dtype == torch.float64 else _abi.RS_F32
 
     def fields(self):
-        return _abi.Fields(c=self.c.data_ptr(), psi=self.psi.data_ptr(),
-                           phi=None if self.phi is None else self.phi.data_ptr(),
-                           precision=self.precision, pitch=0)
+        # in the order of the declaration: keywords cost 0.5 us more
+        return _abi.Fields(self.c.data_ptr(), self.psi.data_ptr(), None if self.phi is None else self.phi.data_ptr(),
+                           self.precision, 0)
 
 
 class Context:
@@ -270,17 +284,10 @@ class Context:
     # ---- hot path
     def step(self, cur, nxt, step, i_offset_history=0, l_offset_Vp=0.0, pull_back=None,
              T_coarse=None, i_left_end=0, i_left_end_T=0, mass_out=None, itip_out=None, stream=None):
-        a = _abi.StepArgs()
-        a.step = step
-        a.i_offset_history = i_offset_history
-        a.pull_back = 0 if pull_back is None else 1
-        a.i_offset = 0 if pull_back is None else int(pull_back)
-        a.i_left_end = i_left_end
-        a.i_left_end_T = i_left_end_T
-        a.l_offset_Vp = l_offset_Vp
-        a.T_coarse = None if T_coarse is None else T_coarse.data_ptr()
-        a.mass_out = _addr(mass_out)
-        a.itip_out = _addr(itip_out)
+        # in the order of the declaration, one call
+        a = _abi.StepArgs(step, i_offset_history, 0 if pull_back is None else 1,
+                          0 if pull_back is None else int(pull_back), i_left_end, i_left_end_T, 0, l_offset_Vp,
+                          None if T_coarse is None else T_coarse.data_ptr(), _addr(mass_out), _addr(itip_out))
         fc, fn = cur.fields(), nxt.fields()
         check(self.lib.rs_step(self._h, C.byref(fc), C.byref(fn), C.byref(a), _stream(stream)))
 
@@ -448,8 +455,7 @@ class FieldSet3:
         self.precision = _abi.RS_F64 if dtype == torch.float64 else _abi.RS_F32
 
     def fields(self):
-        return _abi.Fields3(phi1=self.phi1.data_ptr(), phi2=self.phi2.data_ptr(), c=self.c.data_ptr(),
-                            precision=self.precision, reserved=0)
+        return _abi.Fields3(self.phi1.data_ptr(), self.phi2.data_ptr(), self.c.data_ptr(), self.precision, 0)
 
 
 class Context3:
