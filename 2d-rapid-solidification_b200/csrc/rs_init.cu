@@ -193,7 +193,7 @@ void launch_interpolate_temperature(const TfcCoef &T, const StepCoef &, const do
 // thread per coarse cell adds them in the reference's order (rows outer,
 // columns inner).  At 768 x 832 one thread per coarse cell, a hundred strided
 // loads in series, took 22 us; a warp per cell with the sum passed through
-// shuffles 8; this takes 4, bound by the latency of its loads and of the 100
+// shuffles 8; this takes 7, bound by the latency of its loads and of the 100
 // dependent additions.
 // psi is read through the pull_back column remap of i_offset (0: none), so
 // the source of a step whose shift was fused into rs_step sees the shifted

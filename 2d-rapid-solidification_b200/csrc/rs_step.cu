@@ -189,7 +189,7 @@ struct Strip {
       const R an = anisotropy<R>(F, p1, pr1, pl1, p2, p0, pr2, pl2, pr0, pl0, as, ak);
       const R c00 = Tr<R>::kDelta ? cinf + d1 : d1;
       const R Anb = TFC ? A1nb : col.A_nb, Ati = TFC ? A1ti : col.A_ti;
-      const R dG = (R(1) - c00) * Anb + c00 * Ati + c00 * (R(1) - c00) * R(kL0Liq - kL0Bcc);
+      const R dG = drive_dG<R>(c00, Anb, Ati);
       const R q = R(1) - p1 * p1;
       const R term = p1 - p1 * p1 * p1 + an + dG * (R(1.875) * (q * q)) * F.drive;
       R pn = p1 + Tr<R>::div(F.dt * ak, as * as) * term;

@@ -160,41 +160,51 @@ Coef<R> make_coef(const StepCoef &K) {
   return F;
 }
 
+// a product that no addition takes up.  Where both terms of a sum are products
+// the compiler is free to fuse either one, and chose differently in different
+// kernels that inline the same lines (the ensemble's walk differed from the
+// other paths by an ulp of psi); with one of them rounded there is no choice, so
+// a cell's phi does not depend on the kernel that evaluates it.
+__device__ __forceinline__ float mulr(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mulr(double a, double b) { return __dmul_rn(a, b); }
+
 // anisotropic operator of get_anisotropy (fun.cu:1030-1139)
 template <typename R>
 __device__ __forceinline__ R anisotropy(const Coef<R> &F, R phi00, R phi10, R phim0,
                                         R phi01, R phi0m, R phi11, R phim1, R phi1m, R phimm, R &as,
                                         R &ak) {
-  const R px = (phi10 - phim0) * F.inv_2dx;
-  const R py = (phi01 - phi0m) * F.inv_2dx;
-  const R g2 = px * px + py * py;
-  const R dxx = (phi10 - R(2) * phi00 + phim0) * F.inv_dx2;
-  const R dyy = (phi01 - R(2) * phi00 + phi0m) * F.inv_dx2;
-  const R dxy = (phi11 - phim1 - phi1m + phimm) * F.inv_4dx2;
-  const R lap = (R(2) / R(3)) * (dxx + dyy) +
-                (R(1) / R(3)) * (phi11 + phim1 + phi1m + phimm - R(4) * phi00) * F.inv_2dx2;
+  const R px = mulr(phi10 - phim0, F.inv_2dx);
+  const R py = mulr(phi01 - phi0m, F.inv_2dx);
+  const R py2 = mulr(py, py);
+  const R g2 = fma(px, px, py2);
+  const R dxx = mulr(phi10 - R(2) * phi00 + phim0, F.inv_dx2);
+  const R dyy = mulr(phi01 - R(2) * phi00 + phi0m, F.inv_dx2);
+  const R dxy = mulr(phi11 - phim1 - phi1m + phimm, F.inv_4dx2);
+  const R lap = fma(R(2) / R(3), dxx + dyy,
+                    mulr(mulr(R(1) / R(3), phi11 + phim1 + phi1m + phimm - R(4) * phi00), F.inv_2dx2));
   // |grad phi| > 1e-15 (fun.cu:1056)
   if (!(g2 > R(1.0e-30))) {
     as = F.as0;
     ak = F.ak0;
-    return (as * as) * lap;
+    return mulr(mulr(as, as), lap);
   }
   const R ig2 = Tr<R>::rcp(g2);
-  const R dtx = (px * dxy - py * dxx) * ig2;
-  const R dty = (px * dyy - py * dxy) * ig2;
+  const R dtx = mulr(fma(px, dxy, -mulr(py, dxx)), ig2);
+  const R dty = mulr(fma(px, dyy, -mulr(py, dxy)), ig2);
   R da1, da2;
   if (F.one_eps) {
-    const R C2 = (px * px - py * py) * ig2;
-    const R S2 = R(2) * px * py * ig2;
-    const R C4 = C2 * C2 - S2 * S2;
-    const R S4 = R(2) * S2 * C2;
+    const R C2 = mulr(fma(px, px, -py2), ig2);
+    const R S2 = mulr(mulr(R(2) * px, py), ig2);
+    const R C4 = fma(C2, C2, -mulr(S2, S2));
+    const R S4 = mulr(R(2) * S2, C2);
     const R np4 = F.k0 + F.k1 * C2 + F.k2 * S2 + F.k3 * C4 + F.k4 * S4;
-    const R d1 = R(2) * (F.k2 * C2 - F.k1 * S2) + R(4) * (F.k4 * C4 - F.k3 * S4);
-    const R d2 = R(-4) * (F.k1 * C2 + F.k2 * S2) - R(16) * (F.k3 * C4 + F.k4 * S4);
+    // (the factors 2, 4 and 16 round nothing)
+    const R d1 = R(2) * fma(F.k2, C2, -mulr(F.k1, S2)) + R(4) * fma(F.k4, C4, -mulr(F.k3, S4));
+    const R d2 = R(-4) * fma(F.k1, C2, mulr(F.k2, S2)) - R(16) * fma(F.k3, C4, mulr(F.k4, S4));
     ak = R(1) - R(3) * F.epk1 + R(4) * F.epk1 * np4;
     as = R(1) - R(3) * F.eps1 + R(4) * F.eps1 * np4;
-    da1 = R(4) * F.eps1 * d1;
-    da2 = R(4) * F.eps1 * d2;
+    da1 = mulr(R(4) * F.eps1, d1);
+    da2 = mulr(R(4) * F.eps1, d2);
   } else {
     // (eps1, eps2) form needs the sextic (n_x n_y n_z)^2: explicit directions
     const R ia = sqrt(ig2);
@@ -219,7 +229,9 @@ __device__ __forceinline__ R anisotropy(const Coef<R> &F, R phi00, R phi10, R ph
     da1 = (F.eps1 + R(3) * F.eps2) * dnp4_1 + R(66) * F.eps2 * dnp2_1;
     da2 = (F.eps1 + R(3) * F.eps2) * dnp4_2 + R(66) * F.eps2 * dnp2_2;
   }
-  return (as * as) * lap + R(2) * as * da1 * (dtx * px + dty * py) + (da2 * as + da1 * da1) * (dty * px - dtx * py);
+  R an = mulr(mulr(as, as), lap);
+  an = fma(mulr(R(2) * as, da1), fma(dtx, px, mulr(dty, py)), an);
+  return fma(fma(da2, as, mulr(da1, da1)), fma(dty, px, -mulr(dtx, py)), an);
 }
 
 __device__ __forceinline__ double t_fine_at(const StepCoef &K, const double *__restrict__ T, int ile, int i, int j) {
@@ -443,8 +455,9 @@ __device__ __forceinline__ R phi_cell_dG(const Coef<R> *__restrict__ Fp, R p00, 
   const Coef<R> &F = *Fp;
   R as, ak;
   const R an = anisotropy<R>(F, p00, p10, pm0, p01, p0m, p11, pm1, p1m, pmm, as, ak);
-  const R q = R(1) - p00 * p00;
-  const R term = p00 - p00 * p00 * p00 + an + dG * (R(1.875) * (q * q)) * F.drive;
+  const R q = fma(-p00, p00, R(1));
+  const R term =
+      fma(mulr(dG, mulr(R(1.875), mulr(q, q))), F.drive, fma(-mulr(p00, p00), p00, p00) + an);
   R pn = p00 + Tr<R>::div(F.dt * ak, as * as) * term;
   if (F.noise_amp > R(0) && q > R(1.0e-3)) {
     uint32_t x[4];
@@ -455,11 +468,18 @@ __device__ __forceinline__ R phi_cell_dG(const Coef<R> *__restrict__ Fp, R p00, 
   return pn > R(1) ? R(1) : pn;  // renormalisation (fun.cu:1252-1261)
 }
 
+// dG = Gl - Gs from the column's groups (fun.cu:1192-1193)
+template <typename R>
+__device__ __forceinline__ R drive_dG(R c00, R Anb, R Ati) {
+  const R omc = R(1) - c00;
+  return fma(mulr(c00, omc), R(kL0Liq - kL0Bcc), fma(omc, Anb, mulr(c00, Ati)));
+}
+
 template <typename R>
 __device__ __forceinline__ R phi_cell(const Coef<R> *__restrict__ Fp, R p00, R p10, R pm0, R p01, R p0m, R p11,
                                    R pm1, R p1m, R pmm, R c00, R Anb, R Ati, int64_t step, int64_t cell,
                                    uint32_t seed_lo, uint32_t seed_hi) {
-  const R dG = (R(1) - c00) * Anb + c00 * Ati + c00 * (R(1) - c00) * R(kL0Liq - kL0Bcc);
+  const R dG = drive_dG<R>(c00, Anb, Ati);
   return phi_cell_dG<R>(Fp, p00, p10, pm0, p01, p0m, p11, pm1, p1m, pmm, dG, step, cell, seed_lo, seed_hi);
 }
 

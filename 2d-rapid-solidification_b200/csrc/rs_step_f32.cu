@@ -432,7 +432,7 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     } else if (real) {
       if (!inbox) atomicAdd(&SA.audit[2], 1ull);
       if (audit) {
-        const float dG_ex = (1.f - c) * tAnb[gx] + c * tAti[gx] + c * (1.f - c) * (float)(kL0Liq - kL0Bcc);
+        const float dG_ex = drive_dG<float>(c, tAnb[gx], tAti[gx]);
         const float dG_net = fmaf(o[1], SA.y_scale[1], SA.y_mean[1]);
         atomicMax(&SA.audit[0], (unsigned long long)__float_as_uint(fabsf(mu_net - sm.mu[rr][b])));
         atomicMax(&SA.audit[1], (unsigned long long)__float_as_uint(fabsf(dG_net - dG_ex)));
@@ -1117,7 +1117,7 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
       Anb = tAnb[g];
       Ati = tAti[g];
     }
-    float dG = (1.f - c00) * Anb + c00 * Ati + c00 * (1.f - c00) * (float)(kL0Liq - kL0Bcc);
+    float dG = drive_dG<float>(c00, Anb, Ati);
     if constexpr (SURR) {  // driving force from the surrogate for in-box, unaudited cells
       float in[3];
       net_inputs(rr, x, in);
@@ -1811,7 +1811,7 @@ static __device__ __forceinline__ void phase3_32(const View32 &V, const InSlot32
     const int rr = (int)(e >> 8), x = (int)(e & 0xFFu) + 4;
     const int r = V.y0 - 1 + rr, g = V.x0 + x - 4;
     const float c00 = V.F.cinf + in.d[rr][x];
-    const float dG = (1.f - c00) * V.tAnb[g] + c00 * V.tAti[g] + c00 * (1.f - c00) * (float)(kL0Liq - kL0Bcc);
+    const float dG = drive_dG<float>(c00, V.tAnb[g], V.tAti[g]);
     const float res = phi_cell_dG<float>(
         &V.F, clamp1(in.psi[rr][x]), clamp1(in.psi[rr][x + 1]), clamp1(in.psi[rr][x - 1]),
         clamp1(in.psi[rr + 1][x]), clamp1(in.psi[rr - 1][x]), clamp1(in.psi[rr + 1][x + 1]),

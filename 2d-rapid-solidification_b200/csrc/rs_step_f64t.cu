@@ -699,7 +699,7 @@ static __device__ __forceinline__ void phase3(const TileView &V, const InSlot &i
       Anb = V.T.Anb[g];
       Ati = V.T.Ati[g];
     }
-    const double dG = (1.0 - c00) * Anb + c00 * Ati + c00 * (1.0 - c00) * (kL0Liq - kL0Bcc);
+    const double dG = drive_dG<double>(c00, Anb, Ati);
     const double res = phi_cell_dG<double>(
         &V.F, clamp1(in.psi[rr][x]), clamp1(in.psi[rr][x + 1]), clamp1(in.psi[rr][x - 1]),
         clamp1(in.psi[rr + 1][x]), clamp1(in.psi[rr - 1][x]), clamp1(in.psi[rr + 1][x + 1]),
