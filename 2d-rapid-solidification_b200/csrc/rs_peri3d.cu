@@ -482,7 +482,7 @@ int launch_step(const rs3_params &p, const P3Maps &m, double *o1, double *o2, do
   static std::atomic<unsigned long long> attr[4];
   if (!smem_limit_once((const void *)kfn, (int)smem, attr[(a1 ? 2 : 0) + (sd ? 1 : 0)])) return -3;
   dim3 grid((p.nx - 2 + C::BX - 1) / C::BX, (p.ny - 2 + C::BY - 1) / C::BY);
-  k.z_chunk = p3_chunk(p, (int64_t)grid.x * grid.y, 2, 0.5);
+  k.z_chunk = p3_chunk(p, (int64_t)grid.x * grid.y, 2, false);
   grid.z = (p.nz - 2 + k.z_chunk - 1) / k.z_chunk;
   return launch_dep_smem(kfn, grid, dim3(C::kThreads), smem, st, k, m.phi1, m.phi2, m.c, o1, o2, oc, step, err) ==
                  cudaSuccess

@@ -46,9 +46,14 @@ __device__ __forceinline__ R gp2(R pi, R pj, R pk) {
 }
 
 // z planes per CTA where the caller leaves the choice (z_chunk == 0): the least
-// (waves + 1/2)(c + halo) of c = 32, 16, 8, 4, 2, halo being what the two planes
-// that a chunk reads beside those it writes cost, in planes.  The half wave
-// stands for the last one and for fronts, whose planes take longer than melt.
+// (waves + extra)(c + halo) of c = 32, 16, 8, 4, 2, halo being what the two planes
+// that a chunk reads beside those it writes cost, in planes (1/2 where they are
+// loads, 3 where they are logarithms and network passes too).  The extra wave,
+// 1/2 or 1, stands for the last one and for fronts, whose planes take longer
+// than melt.  heavy: the second kind, whose fronts' z position decides more than
+// this knows; a lower chunk than 32 has to promise 15 % (over 90 volumes of 64
+// to 384 cells a side, fronts at 15 to 50 % of the height, against 32 planes:
+// network 0.64 of the time, at most 1.00; FP64 0.72, at most 1.00).
 // A march of 32 planes left small volumes with a few dozen CTAs, us per step:
 //             planes:  2     4     8     16    32
 //   TiAg FP32 128^3    23    24    36    42    79
@@ -59,14 +64,14 @@ __device__ __forceinline__ R gp2(R pi, R pj, R pk) {
 //   Ti-Nb FP32 256^3   172   145   133   133   148
 //   Ti-Nb FP64 256^3   521   426   381   348   366
 // The results do not depend on it.
-inline int p3_chunk(const rs3_params &p, int64_t tiles, int ctas_per_sm, double halo) {
+inline int p3_chunk(const rs3_params &p, int64_t tiles, int ctas_per_sm, bool heavy) {
   if (p.z_chunk > 0) return p.z_chunk;
   int best = 32;
   double least = 1e300;
   for (int c = 32; c >= 2; c /= 2) {
     const double waves = (double)(tiles * ((p.nz - 2 + c - 1) / c)) / (148 * ctas_per_sm);
-    const double cost = (std::max(waves, 1.0) + 0.5) * (c + halo);
-    if (cost < least) least = cost, best = c;
+    const double cost = (std::max(waves, 1.0) + (heavy ? 1.0 : 0.5)) * (c + (heavy ? 3.0 : 0.5));
+    if (cost < least) least = cost * (heavy && c == 32 ? 0.85 : 1.0), best = c;
   }
   return best;
 }

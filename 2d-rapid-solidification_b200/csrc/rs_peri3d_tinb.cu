@@ -836,7 +836,7 @@ int launch_tinb_x2(const rs3_params &p, K3<float> k, const P3Maps &m, float *o1,
   static std::atomic<unsigned long long> attr;
   if (!smem_limit_once((const void *)kfn, (int)smem, attr)) return -3;
   dim3 grid((k.nx + kT2BX - 1) / kT2BX, (k.ny - 2 + kT2BY - 1) / kT2BY);
-  k.z_chunk = p3_chunk(p, (int64_t)grid.x * grid.y, 3, 0.5);
+  k.z_chunk = p3_chunk(p, (int64_t)grid.x * grid.y, 3, false);
   grid.z = (k.nz - 2 + k.z_chunk - 1) / k.z_chunk;
   return launch_dep_smem(kfn, grid, dim3(kT2Threads), smem, st, k, m.phi1, m.phi2, m.c, o1, o2, oc, err) == cudaSuccess ? 0 : -3;
 }
@@ -847,7 +847,7 @@ int launch_tinb(const rs3_params &p, K3<R> k, const P3Maps &m, R *o1, R *o2, R *
   using C = P3Cfg<R>;
   const size_t smem = sizeof(TSmem<R, SURR>) + 128;
   dim3 grid((k.nx - 2 + C::BX - 1) / C::BX, (k.ny - 2 + kP3BY - 1) / kP3BY);
-  k.z_chunk = p3_chunk(p, (int64_t)grid.x * grid.y, 2, 2.0);  // (halo planes: logarithms, networks)
+  k.z_chunk = p3_chunk(p, (int64_t)grid.x * grid.y, 2, true);
   grid.z = (k.nz - 2 + k.z_chunk - 1) / k.z_chunk;
   const bool weigh = SURR && k.z_chunk != k.count_chunk;
   auto kfn = weigh ? tinb_kernel<R, SD, SURR, SURR> : tinb_kernel<R, SD, SURR>;

@@ -447,7 +447,7 @@ int launch_peri3d_step_x2(const rs3_params &p, const P3Maps &m, float *o1, float
   const int which = (a1 ? 2 : 0) + (sd ? 1 : 0);
   if (!smem_limit_once((const void *)kfn, (int)smem, attr[which])) return -3;
   dim3 grid((p.nx + kX2BX - 1) / kX2BX, (p.ny - 2 + kX2BY - 1) / kX2BY);
-  k.z_chunk = p3_chunk(p, (int64_t)grid.x * grid.y, 3, 0.5);
+  k.z_chunk = p3_chunk(p, (int64_t)grid.x * grid.y, 3, false);
   grid.z = (p.nz - 2 + k.z_chunk - 1) / k.z_chunk;
   return launch_dep_smem(kfn, grid, dim3(kX2Threads), smem, st, k, m.phi1, m.phi2, m.c, o1, o2, oc, step, err) == cudaSuccess ? 0 : -3;
 }
