@@ -56,20 +56,28 @@ void launch_pull_back(int precision, const StepCoef &K, const void *c, const voi
 // dependent of it.  The passes are programmatic dependents too: every kernel
 // here waits (griddepcontrol.wait) before it touches memory, so its launch
 // overlaps the kernel before it.  At 2048 x 2048 in FP64 (front at column 300)
-// itip takes 15, the precise tip 21 and the mass 9 us, 296 together before: the
-// tip's row scan was one thread's, and itip and mass read both fields.
+// itip takes 9, the row pass of the precise tip 10 and the mass 9 us, their
+// second kernels 3, 8 and 3, 296 together before: the tip's row scan was one
+// thread's, and itip and mass read both fields.  16 loads a lane in flight
+// instead of 32 make 14 and 13 of the row passes.
 // The largest column in [0, hi] with psi > 0 of a row, or -1: the whole warp
 // walks from the right end, kScan cells per lane and turn (their loads in
 // flight together), and stops at the first turn that finds one, so it reads
 // the melt ahead of the front only.
-constexpr int kScan = 16;
+constexpr int kScan = 32;
 // all of v in registers at once: without it the compiler loads and compares a
 // few cells at a time (itip of 2048 x 2048 in FP64: 27 us)
 #define RS_HOLD8(C, v, k)                                                                                  \
   "+" C(v[k]), "+" C(v[k + 1]), "+" C(v[k + 2]), "+" C(v[k + 3]), "+" C(v[k + 4]), "+" C(v[k + 5]), \
       "+" C(v[k + 6]), "+" C(v[k + 7])
-__device__ __forceinline__ void hold(double (&v)[kScan]) { asm volatile("" : RS_HOLD8("d", v, 0), RS_HOLD8("d", v, 8)); }
-__device__ __forceinline__ void hold(float (&v)[kScan]) { asm volatile("" : RS_HOLD8("f", v, 0), RS_HOLD8("f", v, 8)); }
+__device__ __forceinline__ void hold(double (&v)[kScan]) {
+  asm volatile("" : RS_HOLD8("d", v, 0), RS_HOLD8("d", v, 8), RS_HOLD8("d", v, 16));
+  asm volatile("" : RS_HOLD8("d", v, 24));
+}
+__device__ __forceinline__ void hold(float (&v)[kScan]) {
+  asm volatile("" : RS_HOLD8("f", v, 0), RS_HOLD8("f", v, 8), RS_HOLD8("f", v, 16));
+  asm volatile("" : RS_HOLD8("f", v, 24));
+}
 #undef RS_HOLD8
 template <typename R>
 __device__ __forceinline__ int last_solid(const R *__restrict__ row, int hi, int lane) {
@@ -322,9 +330,14 @@ __device__ int fit_parabola_d(const double *x, const double *y, double *x0, doub
 // of row j is the running tip int(itip), so row j offers f_j if its last solid
 // column is not behind that, else g_j, and becomes the tip if it is larger.
 // Here the block reads kFitRows rows at a time and takes the larger of f_j and
-// g_j over each group of 32; one warp then visits the groups that can raise
-// the tip, in order, and in a group the rows that do (ballots), with the
-// comparisons of the sequential scan.  The five quartic fits run on five lanes.
+// g_j over each group of 32.  Let M be the largest of them and m the first row
+// that has it.  No row offers more than M, so where M does not exceed the tip no
+// row raises it; and where m has it as f_m with a last solid column not behind
+// int(M), row m is reached with a tip below M, offers f_m = M and becomes the
+// tip, and no later row does: the scan's result at once.  Otherwise (f_j and g_j
+// of odd fields) one warp visits the groups that can raise the tip, in order,
+// and in a group the rows that do (ballots), with the comparisons of the
+// sequential scan.  The five quartic fits run on five lanes.
 constexpr int kFitThreads = 512;
 constexpr int kFitRows = 2048;
 constexpr int kFitGroups = kFitRows / 32;
@@ -359,6 +372,22 @@ __global__ void __launch_bounds__(kFitThreads) tip_fit_kernel(const StepCoef K, 
     __syncthreads();
     if (warp != 0) continue;
     const double m0 = s_max[lane], m1 = s_max[32 + lane];
+    double M = fmax(m0, m1);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) M = fmax(M, __shfl_xor_sync(0xffffffffu, M, o));
+    if (!(M > itip)) continue;
+    {
+      const unsigned lo = __ballot_sync(0xffffffffu, m0 == M), hi = __ballot_sync(0xffffffffu, m1 == M);
+      const int g = lo ? __ffs(lo) - 1 : 31 + __ffs(hi), r = 32 * g + lane;
+      const unsigned at = __ballot_sync(0xffffffffu, fmax(s_f[r], s_g[r]) == M);
+      const int l = __ffs(at) - 1;  // (a group's maximum is one of its rows')
+      if (at && __shfl_sync(0xffffffffu, (int)(s_f[r] == M && s_last[r] >= 0 && (double)s_last[r] >= floor(M)), l)) {
+        itip = M;
+        ti = (int)M;
+        tj = base + 32 * g + l;
+        continue;
+      }
+    }
     for (int g = 0; g < kFitGroups; ++g) {  // the next group that can raise the tip
       const unsigned long long can = ((unsigned long long)__ballot_sync(0xffffffffu, m1 > itip) << 32) |
                                      __ballot_sync(0xffffffffu, m0 > itip);

@@ -78,7 +78,7 @@ __global__ void sample_kernel(const double cinf, const double RR, const MlpBox b
 //   sums: the owner of a parameter (each CTA a share of them) adds the round's
 //     chunk sums to its chains, read over distributed shared memory.
 // At batch 4096 one thread per parameter and 32-way conflicting rows on 8 CTAs
-// took 205 us; this takes 27.  Shared-memory bandwidth bounds it (the 16-byte
+// took 205 us; this takes 30.  Shared-memory bandwidth bounds it (the 16-byte
 // weight broadcasts return 512 B each: 13 us), then the chain of its phases.
 constexpr int kChunk = 128;
 constexpr int kChains = 8;
