@@ -9,7 +9,8 @@
 //   * column_table_kernel_f64: the per-column CALPHAD groups of this step's
 //     frozen temperature (col_terms, get_delta fun.cu:1610-1619) in FP64;
 //   * tile_kernel_f64.
-// Both are programmatic dependent launches: they are scheduled while the
+// (Grids of one wave of CTAs: the second alone, its tiles computing their own
+// columns' groups.)  Both are programmatic dependent launches: they are scheduled while the
 // kernel before them drains and wait for it on the device, so a run's steps
 // follow one another without launch gaps (2048^2, all solid: 28.7 -> 26.4 us).
 //
@@ -43,7 +44,8 @@
 // What bounds it: a 2048^2 grid ahead of a planar front (34.8 us a step, 43.0
 // without the melt form and the chained launches, floor 20.5) its instruction
 // issue and the load -> compute -> store chain of a CTA; small grids (256^2:
-// 12.4 us, 15.0 with 16-row tiles) and fronts the chain of the phases.
+// 6.5 us, 12.1 with 16-row tiles and a table launch) and fronts the chain of the
+// phases.
 // Arithmetic (identical mathematics to the reference, regrouped as in the
 // FP32 tile kernel):
 //   * mu = K(T) + C0(T) + mu'', C0 = -D - (L0_BCC - L0_Liq)(1 - 2 cinf)/2, so
@@ -177,6 +179,22 @@ __device__ __forceinline__ void bulk_store(void *gdst, const void *ssrc, uint32_
                : "memory");
 }
 
+// The table entries of the column at temperature T (dK by the caller, from KC,
+// K + C0).  Out of line: the table kernel and the tiles that compute their own
+// columns run one copy of it, so their entries are the same bits.
+struct ColEntry {
+  double RT, C0, KC, Anb, Ati;
+};
+__device__ __noinline__ ColEntry col_entry(const double T, const double RR, const double cinf, const double Lref) {
+  StepCoef K;
+  K.RR = RR;
+  K.cinf = cinf;
+  K.Lref = Lref;
+  const ColT<double> ct = col_terms<double>(K, T);
+  const double C0 = -ct.D - 0.5 * (kL0Bcc - kL0Liq) * (1.0 - 2.0 * cinf);
+  return {ct.RT, C0, ct.Kc + C0, ct.A_nb, ct.A_ti};
+}
+
 // One thread per column, one exact FP64 col_terms each; K + C0 of the next
 // column comes from the neighbouring thread, so blocks overlap by one column
 // and write 127 entries.
@@ -190,18 +208,17 @@ __global__ void __launch_bounds__(kTabBlock) column_table_kernel_f64(const StepC
   const int k = blockIdx.x * (kTabBlock - 1) + threadIdx.x;  // table entry; column k - 4
   const int gi = min(max(k - 4, 0), K.nx - 1);
   const double T = (d0 + d1 * gi) * K.deltaT0 + K.Tmelt;  // get_delta, fun.cu:1610-1619
-  const ColT<double> ct = col_terms<double>(K, T);
-  const double C0 = -ct.D - 0.5 * (kL0Bcc - kL0Liq) * (1.0 - 2.0 * K.cinf);
-  kc[threadIdx.x] = ct.Kc + C0;
+  const ColEntry ct = col_entry(T, K.RR, K.cinf, K.Lref);
+  kc[threadIdx.x] = ct.KC;
   __syncthreads();
   // the previous step's tiles have read the table
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (threadIdx.x == kTabBlock - 1 || k >= len) return;
   tab[kTabRT * len + k] = ct.RT;
-  tab[kTabC0 * len + k] = C0;
+  tab[kTabC0 * len + k] = ct.C0;
   tab[kTabDK * len + k] = kc[threadIdx.x + 1] - kc[threadIdx.x];  // (K + C0)(i+1) - (K + C0)(i)
-  tab[kTabAnb * len + k] = ct.A_nb;
-  tab[kTabAti * len + k] = ct.A_ti;
+  tab[kTabAnb * len + k] = ct.Anb;
+  tab[kTabAti * len + k] = ct.Ati;
 }
 
 // the column table, indexed by column
@@ -1198,7 +1215,12 @@ struct alignas(128) PipeSmem64 {
   int abort;  // a wait gave up: every role stops
 };
 // ---------------------------------------------------------------- one tile per CTA
-template <int TR, bool TFC, bool RAW>
+// OWN: the CTA computes the table entries of its 72 columns itself, before it
+// waits for the kernel before it, and the step is one launch.  For grids whose
+// CTAs are all resident at once: theirs are scheduled, and compute the entries,
+// while the step before is still at work (256^2: 8.1 -> 6.5 us a step); on
+// larger ones every wave would compute them again.
+template <int TR, bool TFC, bool RAW, bool OWN = false>
 __global__ void __launch_bounds__(kThreads, 5)
     tile_kernel_f64(const __grid_constant__ StepCoef K, const __grid_constant__ Coef<double> F,
                     const __grid_constant__ StepScalars PS, const __grid_constant__ CUtensorMap tm_psi,
@@ -1230,6 +1252,28 @@ __global__ void __launch_bounds__(kThreads, 5)
     sm.vote = 0u;
     sm.p2.nlist = 0u;
   }
+  __shared__ alignas(16) double own_tab[OWN ? kColTabFields * kWin : 1];
+  if constexpr (OWN) {
+    // (as column_table_kernel_f64, entry k the column x0 - 4 + k; the last dK is
+    // no lane's)
+    __shared__ double kc[kWin];
+    const int k = (int)threadIdx.x;
+    ColEntry ct = {};
+    if (k < kWin) {
+      const int gi = min(max(x0 - 4 + k, 0), K.nx - 1);
+      ct = col_entry((PS.d0 + PS.d1 * gi) * K.deltaT0 + K.Tmelt, K.RR, K.cinf, K.Lref);
+      kc[k] = ct.KC;
+    }
+    __syncthreads();
+    if (k < kWin) {
+      own_tab[kTabRT * kWin + k] = ct.RT;
+      own_tab[kTabC0 * kWin + k] = ct.C0;
+      own_tab[kTabDK * kWin + k] = k + 1 < kWin ? kc[k + 1] - ct.KC : 0.0;
+      own_tab[kTabAnb * kWin + k] = ct.Anb;
+      own_tab[kTabAti * kWin + k] = ct.Ati;
+    }
+    __syncthreads();
+  }
   // the kernel before this one in the stream (the column table's, and with it
   // every earlier one) has completed: its table and the fields are visible
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -1240,7 +1284,8 @@ __global__ void __launch_bounds__(kThreads, 5)
   }
   // dependents of this step (its reduction, the next step) may be scheduled now
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const typename Ops::TileView V(K, F, PS, tab, tab_len, x0, y0, (int)threadIdx.x);
+  const typename Ops::TileView V(K, F, PS, OWN ? own_tab - x0 : tab, OWN ? kWin : tab_len, x0, y0,
+                                 (int)threadIdx.x);
   const typename Ops::LaneCols LC = Ops::template lane_cols<TFC>(V);
   const typename Ops::TfcTile *tf = nullptr;
   if constexpr (TFC) {
@@ -1545,6 +1590,7 @@ int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScal
   if (partials && nparts > max_partials) return -1;
   if (!tm.col_tab64 || tm.col_tab64_len < ncb * kW + kWin) return -1;
   using Kfn = decltype(&tile_kernel_f64<16, false, false>);
+  static const Kfn own_fn[2] = {tile_kernel_f64<4, false, false, true>, tile_kernel_f64<4, false, true, true>};
   static const Kfn tile_fn[2][2][3] = {  // [raw][tfc][height]
       {{tile_kernel_f64<4, false, false>, tile_kernel_f64<8, false, false>, tile_kernel_f64<16, false, false>},
        {nullptr, tile_kernel_f64<8, true, false>, tile_kernel_f64<16, true, false>}},
@@ -1556,13 +1602,27 @@ int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScal
   const int sh = TR == 4 ? 0 : TR == 8 ? 1 : 2;
   static const decltype(&pipe_kernel_f64<16>) pipe_fn[3] = {pipe_kernel_f64<4>, pipe_kernel_f64<8>, pipe_kernel_f64<16>};
   static const size_t pipe_smem[3] = {sizeof(PipeSmem64<4>), sizeof(PipeSmem64<8>), sizeof(PipeSmem64<16>)};
-  const int which = pipe ? 12 + sh : 6 * raw + 3 * tfc + sh;
   const size_t smem = pipe ? pipe_smem[sh] : tile_smem[tfc][sh];
-  const void *kfn = pipe ? (const void *)pipe_fn[sh] : (const void *)tile_fn[raw][tfc][sh];
-  static std::atomic<unsigned long long> attr_done[15];
-  if (!smem_limit_once(kfn, (int)smem, attr_done[which])) return -3;
-  static std::atomic<int> resident_of[15][64];
-  const int resident = resident_ctas(kfn, pipe ? kPipeThreads : kThreads, smem, resident_of[which]);
+  static std::atomic<unsigned long long> attr_done[17];
+  static std::atomic<int> resident_of[17][64];
+  const void *kfn;
+  auto resident_at = [&](int which) {
+    return smem_limit_once(kfn, (int)smem, attr_done[which])
+               ? resident_ctas(kfn, pipe ? kPipeThreads : kThreads, smem, resident_of[which])
+               : -1;
+  };
+  // a grid of one wave: the tiles compute their columns' entries themselves
+  bool own = TR == 4 && !tfc && !pipe;
+  int resident = 0;
+  if (own) {
+    kfn = (const void *)own_fn[raw];
+    resident = resident_at(15 + raw);
+    own = nparts <= resident;
+  }
+  if (!own) {
+    kfn = pipe ? (const void *)pipe_fn[sh] : (const void *)tile_fn[raw][tfc][sh];
+    resident = resident_at(pipe ? 12 + sh : 6 * raw + 3 * tfc + sh);
+  }
   if (resident <= 0) return -3;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1576,7 +1636,7 @@ int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScal
   cfg.numAttrs = 1;
   const double *tab = tm.col_tab64;
   cudaError_t e = cudaSuccess;
-  if (!tfc) {
+  if (!tfc && !own) {
     cfg.gridDim = dim3((tm.col_tab64_len + kTabBlock - 2) / (kTabBlock - 1));
     cfg.blockDim = dim3(kTabBlock);
     e = cudaLaunchKernelEx(&cfg, column_table_kernel_f64, K, P.d0, P.d1, tm.col_tab64_len, tm.col_tab64);
@@ -1593,7 +1653,7 @@ int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScal
     // column-major: consecutive CTAs share a column strip and its halo rows in L2
     cfg.gridDim = dim3(nrt, ncb);
     cfg.blockDim = dim3(kThreads);
-    e = cudaLaunchKernelEx(&cfg, tile_fn[raw][tfc][sh], K, F, P, tm.psi, tm.c, tab, tm.col_tab64_len, psi_n, c_n, phi_n,
+    e = cudaLaunchKernelEx(&cfg, own ? own_fn[raw] : tile_fn[raw][tfc][sh], K, F, P, tm.psi, tm.c, tab, tm.col_tab64_len, psi_n, c_n, phi_n,
                            partials, err, resident % nrt, resident / nrt);
   }
   if (e != cudaSuccess) return -3;
