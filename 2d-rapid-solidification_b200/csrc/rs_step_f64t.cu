@@ -1563,11 +1563,17 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
 // a planar front, 4 / 8 / 16 rows): 512^2, 0.3 waves, 13.7 / 14.1 / 18.4; 768 x
 // 832, 0.8 waves, 12.4 / 13.9 / 24.0; 1024^2, 1.4 waves, 19.7 / 16.2 / 22.2;
 // 1536^2, 3.1 waves, 37.1 / 26.7 / 26.9; 2048^2, 5.5 waves, 61 / 42.3 / 37.1.
+// A tall grid has front tiles enough for every SM at 8 or 16 rows, and then the
+// rows that a tile reads beside its own decide (with the mass, 4 / 8 / 16 rows):
+// 352 x 1568 19.7 / 18.1 / -; 128 x 1800 17.0 / 14.2 / -; 128 x 2500 18.2 /
+// 16.2 / 18.6; 160 x 3776 28.5 / 24.7 / 22.0; 96 x 4000 26.0 / 24.5 / 22.3.
 // With the coarse-grid temperature a tile also sets up its temperature tables:
 // 768 x 832, 28.8 / 22.5 / 30.2 us a step, so 4 rows are left out.
 int tile_rows_f64(int nx, int ny, bool tfc) {
   const int64_t tiles = (int64_t)((nx + kW - 1) / kW) * ((ny - 2 + 15) / 16), wave = 5 * (int64_t)sm_count();
-  return tiles >= 3 * wave ? 16 : tiles >= wave || tfc ? 8 : 4;
+  if (tfc) return tiles >= 3 * wave ? 16 : 8;
+  const int64_t rows = ny - 2, sms = sm_count();
+  return tiles >= 3 * wave || rows > 21 * sms ? 16 : tiles >= wave || rows > 10 * sms ? 8 : 4;
 }
 
 int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScalars &P, const TmaMaps &tm,
