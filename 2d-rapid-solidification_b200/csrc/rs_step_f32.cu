@@ -1401,6 +1401,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas(SURR, shape_rows(SHAPE)))
                                   reinterpret_cast<double *>(smem_raw));
         __syncthreads();  // the scratch is reused by the next block
       }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the scratch lies where tiles' loads land
     target += G;
     if (!grid_barrier(bar, target, err, barrier_limit)) dead = true;
     // tiles are handed out by a ticket counter (bar[1]): a CTA takes the next
@@ -1443,6 +1444,10 @@ __global__ void __launch_bounds__(kThreads, min_ctas(SURR, shape_rows(SHAPE)))
         tile_body<SURR, TR>(R.K, R.F, PS, &R.map_psi[SHAPE][par], &R.map_c[SHAPE][par], R.tab, R.tab_len,
                             R.psi[par ^ 1], R.c[par ^ 1], nullptr, nullptr, err, SURR ? R.surr : none, t % nrt,
                             t / nrt, prefetch);
+        // what this thread wrote into the input tile (the columns beyond the
+        // array; a far-melt or solid tile ends without the fence of the bulk
+        // stores) comes before the next tile's load into the same memory
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();  // every thread is done with the tile's barrier and shared memory
         if (threadIdx.x == 0) mbar_inval(&sm.full);
         if (__syncthreads_or(*(volatile int *)err != 0)) dead = true;
