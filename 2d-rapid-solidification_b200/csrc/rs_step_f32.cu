@@ -252,7 +252,9 @@ __global__ void __launch_bounds__(kTabBlock) column_table_kernel(const StepCoef 
 // TR: output rows of the tile (8, 16 or 32; the tensor maps' box is TR + 2
 // rows high).
 // RAW: the fields' rows are not 16-byte aligned (any nx).
-template <bool SURR, int TR, typename Prefetch, bool TFC = false, bool RAW = false>
+// AR: the surrogate's counters take every network cell as often as tiles of AR
+// rows read its row (twice where two of them do), whatever TR is.
+template <bool SURR, int TR, typename Prefetch, bool TFC = false, bool RAW = false, int AR = TR>
 __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &F, const StepScalars &PS,
                                           const CUtensorMap *tm_psi, const CUtensorMap *tm_c,
                                           const float *__restrict__ tab, const int tab_len, float *__restrict__ psi_n,
@@ -381,11 +383,22 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     const float dv = sm.d[rr][b];
     return __float_as_uint(sm.psi[rr][b]) == kMinus1 && dv < d_hi && dv > d_lo;
   };
+  // the counters' tiling (AR): the input rows of this tile that it reads too, and
+  // whether its last tile holds rows beyond the array, whose zeros leave no cell
+  // of row ny-1 deep solid
+  static_assert(AR % TR == 0, "the counters' tiles hold whole ones");
+  auto counted = [&](int rr) {
+    if (AR == TR || (rr >= 1 && rr <= kTR)) return true;
+    return rr == 0 ? (y0 - 1) % AR == 0 : (y0 - 1 + kTR) % AR == 0 || y0 + kTR == ny - 1;
+  };
+  const bool open_end = SURR && (ny - 2) % AR != 0;
+  auto open_row = [&](int rr) { return AR != TR && open_end && rr == kTR + 1 && y0 + kTR == ny - 1; };
   // a halo cell's mu'' enters only the face to the tile's edge column, whose
   // weight is 0 when psi is exactly +1 on both columns over rows rr-1..rr+1;
   // column -1 (left-most tile) enters no face at all (column 0 is a ghost)
   auto halo_mu_used = [&](int rr, int b) {
     if (b == kHaloL && x0 == 0) return false;
+    if (open_row(rr)) return true;
     const int b2 = b == kHaloL ? b + 1 : b - 1;
     bool solid = true;
     for (int r2 = max(rr - 1, 0); r2 <= min(rr + 1, kTRin - 1); ++r2)
@@ -398,6 +411,7 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
   // S = q(1) c (1 - c) = 0 there, so every face weight touching the cell is 0
   // and its mu'' enters no flux (0 times a finite difference)
   auto solid3 = [&](int rr) -> uint32_t {
+    if (open_row(rr)) return 0u;  // (warp-uniform)
     const int xh = lane == 0 ? kHaloL : kHaloR;
     uint32_t v = 0xFu;
     bool hs = true;  // the halo column beside lanes 0 and 31
@@ -429,7 +443,7 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     const float mu_net = fmaf(o[0], SA.y_scale[0], SA.y_mean[0]);
     if (inbox && !audit) {
       sm.mu[rr][b] = mu_net;
-    } else if (real) {
+    } else if (real && counted(rr)) {
       if (!inbox) atomicAdd(&SA.audit[2], 1ull);
       if (audit) {
         const float dG_ex = drive_dG<float>(c, tAnb[gx], tAti[gx]);
@@ -602,7 +616,8 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     return;
   }
   const bool melt = !TFC && !(vote & (kNotMinus1 | kNotFar));
-  if (melt || !(vote & (kNotPlus1 | kNotFinite))) {
+  // (a solid tile with such a row ny-1 takes the phases, where its cells are counted)
+  if (melt || !((vote & (kNotPlus1 | kNotFinite)) || (open_end && y0 + kTR >= ny - 1))) {
     // the warp's output rows straight from registers to global memory, with
     // the ghost columns and rows they copy to (nx is a multiple of 4: a lane's
     // cells are all inside the array or all beyond it)
@@ -1269,7 +1284,7 @@ __global__ void __launch_bounds__(kThreads, SURR ? 4 : 5)
   const int f = max(PS.i_front, 0) / kW;
   const int tr = blockIdx.x;
   const int tc = front_first_block((int)blockIdx.y, f, (int)gridDim.y);
-  tile_body<SURR, TR, WavePrefetch, false, RAW>(K, F, PS, &tm_psi, &tm_c, tab, tab_len, psi_n, c_n, phi_n,
+  tile_body<SURR, TR, WavePrefetch, false, RAW, SURR ? kTileRows : TR>(K, F, PS, &tm_psi, &tm_c, tab, tab_len, psi_n, c_n, phi_n,
                       partials ? partials + ((int64_t)tc * gridDim.x + tr) : nullptr, err, SA, tr, tc,
                       WavePrefetch{&tm_psi, &tm_c, f, wave_x, wave_y, TR});
 }

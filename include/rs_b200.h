@@ -364,8 +364,10 @@ int rs_mlp_forward(const rs_mlp_box *box, const float *d_w, int64_t n, const flo
  * with the coarse-grid temperature. */
 int rs_set_surrogate(rs_ctx *ctx, const float *d_w, const rs_mlp_box *box);
 /* Largest |surrogate - exact| of mu'' and dG over the audited cells and the
- * counts of fallback and audited cells since the last call; clears them.
- * Synchronizes the stream. */
+ * counts of fallback and audited cells since the last call; clears them.  A cell
+ * counts once per tile of 16 rows by 128 columns whose rows and neighbours hold
+ * it, whatever tiles the step takes (an ensemble on another tile shape counts
+ * by that shape).  Synchronizes the stream. */
 int rs_surrogate_audit(rs_ctx *ctx, double *max_err_mu, double *max_err_dG, int64_t *n_fallback,
                        int64_t *n_audit, rs_stream_t stream);
 
