@@ -21,7 +21,7 @@ struct alignas(64) EnsRun {
   StepCoef K;
   Coef<float> F;
   float *psi[2], *c[2];
-  float *tab;  // the run's column table (rs_step_f32.cu layout)
+  float *tab;  // the run's column table (rs_tile_f32.cuh layout)
   int32_t tab_len;
   int32_t nrt[kTileShapes], ntiles[kTileShapes];  // per tile shape: row tiles, tiles
   int32_t active;       // 0: the run is stepped outside the batched launch this step
@@ -35,7 +35,7 @@ struct alignas(64) EnsRun {
   SurrArgs surr;  // the run's learned CALPHAD surrogate (surr.w == nullptr: exact)
 };
 
-// launches of rs_step_f32.cu for the ensemble: table blocks listed by
+// launches of rs_ensemble.cu and rs_ensemble_walk.cu: table blocks listed by
 // (run, block of that run), tiles in `order` as run << 16 | tile of that run
 // surr: every run evaluates its cells through its surrogate (all runs have one)
 // shape: the tile shape (0 .. kTileShapes - 1) the order's tile indices refer to

@@ -169,13 +169,13 @@ int launch_step_f32(const StepCoef &K, const StepScalars &P, const float *psi, c
                     int *nblocks_out, const TmaMaps *tm, int *err, cudaStream_t st);
 template <typename R>
 struct Coef;
-// FP32 TMA-staged kernel (rs_step_f32.cu): frozen temperature, no pull-back.
+// FP32 TMA-staged kernel (rs_tile_f32.cuh): frozen temperature, no pull-back.
 // Launches the per-column table kernel and the tile kernel; nparts_out gets
 // the number of partials written.
 int launch_step_f32_tma(const StepCoef &K, const Coef<float> &F, const StepScalars &P, const TmaMaps &tm,
                         float *psi_n, float *c_n, float *phi_n, BlockPartial *partials, int max_partials,
                         int *nparts_out, int *err, cudaStream_t st);
-// FP64 TMA-staged kernel (rs_step_f64t.cu): frozen temperature, no pull-back,
+// FP64 TMA-staged kernel (rs_tile_f64.cuh): frozen temperature, no pull-back,
 // even nx_all; column table + tile kernel, final reduction fused.
 int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScalars &P, const TmaMaps &tm,
                         double *psi_n, double *c_n, double *phi_n, BlockPartial *partials, int max_partials,

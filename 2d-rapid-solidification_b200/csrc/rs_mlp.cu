@@ -4,7 +4,7 @@
 // Network: (T, c, phi) -> (mu'', dG), 3 -> 32 -> 32 -> 2, SiLU, inputs scaled
 // to [-1, 1] over the training box, outputs scaled by the box's
 // mean/scale.  mu'' is the chemical potential relative to the melt's column
-// value used by the FP32 tile kernel (rs_step_f32.cu),
+// value used by the FP32 tile kernel (rs_tile_f32.cuh),
 //   mu'' = -(g+1) C0(T) - delta (L0_BCC + L0_Liq + g (L0_BCC - L0_Liq)) + RT lam(c),
 // and dG = Gl - Gs = (1-c) A_Nb + c A_Ti + c (1-c) (L0_Liq - L0_BCC)
 // (fun.cu:1671-1720 regrouped, rs_common.cuh).  Targets are evaluated in FP64

@@ -1,6 +1,6 @@
 // rs_mlp.cuh — layout and device evaluation of the CALPHAD surrogate network
 // (3 -> 32 -> 32 -> 2, SiLU), shared by the training kernels (rs_mlp.cu) and
-// the surrogate form of the FP32 tile kernel (rs_step_f32.cu).
+// the surrogate form of the FP32 tile kernel (rs_tile_f32.cuh).
 #pragma once
 
 #include "rs_kernels.cuh"

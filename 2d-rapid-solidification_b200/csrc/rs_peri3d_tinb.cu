@@ -16,7 +16,7 @@
 //
 // FP64 carries mu itself.  FP32 sets hold delta = c - c_ref and the kernel
 // carries mu'' = mu - mu_ref(T), mu relative to the melt of composition c_ref
-// at the plane's T, in the form of the 2D FP32 tile kernel (rs_step_f32.cu):
+// at the plane's T, in the form of the 2D FP32 tile kernel (rs_tile_f32.cuh):
 //   mu'' = -(g+1) C0 - delta (L0_BCC + L0_Liq + g (L0_BCC - L0_Liq)) + RT lam,
 //   g = 1 - 2 g1,  C0 = -(dGs - dGl)/2 - (L0_BCC - L0_Liq)(1 - 2 c_ref)/2,
 //   lam = log(c/(1-c)) - log(c_ref/(1-c_ref)),

@@ -12,8 +12,8 @@
 //     by the cell they copy, corners included.
 //
 // Three kernels: this file's register-prefetch kernel (RS_OPT_TMA = 0)
-// and the TMA-staged tile kernels of rs_step_f32.cu (FP32) and
-// rs_step_f64t.cu (FP64): frozen and coarse-grid temperature, pull-back steps
+// and the TMA-staged tile kernels of rs_tile_f32.cuh (FP32) and
+// rs_tile_f64.cuh (FP64): frozen and coarse-grid temperature, pull-back steps
 // included (those gather their shifted tile).
 //
 // Layout of the work here: a warp owns a strip of 30 output columns (32 input
