@@ -454,22 +454,27 @@ int rs_step(rs_ctx *c, const rs_fields *cur, const rs_fields *next, const rs_ste
   rs::TmaMaps tm;
   const rs::TmaMaps *tmp = nullptr;
   // the tile kernels load rows by TMA boxes and store them in 16-byte units;
-  // where a field's rows are not 16-byte aligned they copy element by element
-  // (2x the register kernel's speed all the same), with the exact evaluation
+  // where a field's rows are not 16-byte aligned they copy element by element,
+  // with the exact evaluation, or the register kernel takes the step
   const uintptr_t vec = 16;
   const bool out_aligned =
       ((uintptr_t)next->psi % vec) == 0 && ((uintptr_t)next->c % vec) == 0 && ((uintptr_t)next->phi % vec) == 0;
   const bool f64 = cur->precision == RS_F64, tfc = c->p.tfc != 0;
   const rs::SurrArgs *surr = c->surr.w && !f64 ? &c->surr : nullptr;
   const int nx = c->p.nx_all, ny = c->p.ny_all;
-  if (c->use_tma) {
-    tm.rows = f64 ? rs::tile_rows_f64(nx, ny, tfc) : rs::tile_rows_f32(nx, ny, tfc, surr != nullptr);
+  bool tiles = c->use_tma != 0;
+  if (tiles) {
+    tm.rows = f64 ? rs::tile_rows_f64(nx, ny, tfc, a->pull_back != 0) : rs::tile_rows_f32(nx, ny, tfc, surr != nullptr);
     if (!(out_aligned && field_map(c, cur->psi, cur->precision, tm.rows + 2, &tm.psi) &&
           field_map(c, cur->c, cur->precision, tm.rows + 2, &tm.c))) {
       P.raw = 1;
       surr = nullptr;
       if (!f64) tm.rows = rs::tile_rows_f32(nx, ny, tfc, false);
+      tiles = f64 ? rs::raw_on_tiles_f64(nx, ny, tfc, a->pull_back != 0)
+                  : rs::raw_on_tiles_f32(nx, ny, tfc, a->pull_back != 0);
     }
+  }
+  if (tiles) {
     tm.col_tab = c->col_tab;
     tm.col_tab_len = c->col_tab_len;
     tm.col_tab64 = c->col_tab64;

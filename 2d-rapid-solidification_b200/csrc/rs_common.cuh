@@ -253,6 +253,9 @@ struct StepScalars {
   // the fields' rows are not 16-byte aligned: the tile kernels copy their
   // tiles in element by element and store cells by plain stores
   int32_t raw;
+  // the tile kernels let the next kernel of the stream be scheduled once their
+  // listed cells are done (0: as soon as they run)
+  int32_t late;
 };
 
 }  // namespace rs

@@ -150,8 +150,12 @@ constexpr int kTileOutW64 = 64;                  // output columns of an FP64 ti
 constexpr int kTmaBoxW64 = kTileOutW64 + 8;      // its input columns
 constexpr int kTileRows = 16;    // output rows of a tile
 constexpr int kTmaBoxH = kTileRows + 2;  // input rows of a tile
-int tile_rows_f64(int nx, int ny, bool tfc);  // output rows of an FP64 tile: 4, 8 or 16
+int tile_rows_f64(int nx, int ny, bool tfc, bool pull_back);  // output rows of an FP64 tile: 4, 8 or 16
 int tile_rows_f32(int nx, int ny, bool tfc, bool network);  // and of an FP32 tile
+// whether the tile kernels take a step on rows that are not 16-byte aligned (else
+// the register kernel)
+bool raw_on_tiles_f64(int nx, int ny, bool tfc, bool pull_back);
+bool raw_on_tiles_f32(int nx, int ny, bool tfc, bool pull_back);
 constexpr int kTfcTileRows32 = 8;        // output rows of an FP32 coarse-grid-temperature tile
 constexpr int kColTabFields = 5;
 // length of the per-column table (entry k is column k - 4) for nx_all columns

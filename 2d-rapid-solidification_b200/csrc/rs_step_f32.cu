@@ -23,11 +23,33 @@ __global__ void __launch_bounds__(kTabBlock) column_table_kernel(const StepCoef 
 // 21.1.  The network's tiles at the front take two to three times as long:
 // 1024^2 19.1 / 26.0 / 45.6; 1536^2, 1.6 waves, 29.8 / 28.0 / 41.1; 2048 x 3072,
 // 4.2 waves, 67 / 47.9 / 49.5; 4096^2, 11 waves, 146 / 98 / 80.
+// Tall grids, whose front tiles fill every SM by themselves, as in FP64 (planar,
+// cellular front): 64 x 8000, 0.7 waves, 18.9, 18.3 / 20, 19 / 18.1, 17.0; with
+// the network 67 / 53 / 50; 600 x 2300, 1 wave, network, in units of 16 rows 0.86
+// / 0.78 / 1.
 int tile_rows_f32(int nx, int ny, bool tfc, bool network) {
   if (tfc) return kTfcTR;
-  const int64_t tiles = (int64_t)((nx + kW - 1) / kW) * ((ny - 2 + 15) / 16), wave = 5 * (int64_t)sm_count();
-  if (network) return 2 * tiles >= 9 * wave ? 16 : 2 * tiles >= 3 * wave ? 8 : 4;
+  const int64_t sms = sm_count(), rows = ny - 2;
+  const int64_t tiles = (int64_t)((nx + kW - 1) / kW) * ((rows + 15) / 16), wave = 5 * sms;
+  if (rows > 28 * sms && (network || tiles < 2 * wave)) return 16;
+  if (network) return 2 * tiles >= 9 * wave ? 16 : 2 * tiles >= 3 * wave || (rows > 14 * sms && 20 * tiles >= 19 * wave) ? 8 : 4;
   return tiles >= 2 * wave ? 16 : tiles >= wave ? 8 : 4;
+}
+// Rows that are not 16-byte aligned: the tiles, which copy their boxes cell by
+// cell, but for grids of more than a wave and a half of them (at 4 rows a tile)
+// where the register kernel is the faster one with a cellular front and no noise
+// (us a step, register kernel / tiles): narrow ones, 319 x 2300 13.0 / 15.2, 417 x
+// 1568 12.6 / 13.5, 63 x 8000 14.2 / 20.2 (639 x 1600 16.9 / 12.8), and steps with
+// a shift, whose tiles load from two places: 1279 x 700 13.1 / 15.3, 4095 x 2048
+// 88 / 108 (639 x 640 11.5 / 10.5).  With the coarse-grid temperature narrow grids
+// of little more than one wave: 199 x 4002 1 / 1.14, 63 x 8002 31.4 / 43.9 (255 x
+// 6002, two waves, 1 / 0.95).
+bool raw_on_tiles_f32(int nx, int ny, bool tfc, bool pull_back) {
+  const int rows = tfc ? kTfcTR : 4;
+  const int64_t tiles = (int64_t)((nx - 1 + kW - 1) / kW) * ((ny - 2 + rows - 1) / rows), wave = 5 * (int64_t)sm_count();
+  const bool few = 2 * tiles <= 3 * wave;
+  if (tfc) return nx > 448 || tiles <= wave || !few;
+  return few || (!pull_back && nx > 432);
 }
 
 int launch_step_f32_tma(const StepCoef &K, const Coef<float> &F, const StepScalars &P, const TmaMaps &tm,
@@ -68,6 +90,17 @@ int launch_step_f32_tma(const StepCoef &K, const Coef<float> &F, const StepScala
   static std::atomic<int> resident_of[14][64];
   const int resident = resident_ctas(kfn, (int)block.x, smem, resident_of[which]);
   if (resident <= 0) return -3;
+  // the late trigger (rs_step_f64t.cu) where it pays: tiles of the coarse-grid
+  // temperature in few waves (96 x 3002, cellular: 0.95 -> 0.80 of the 16-row
+  // form), unaligned rows (1279 x 700, cellular: 13.6 -> 12.8 us; from 2.5 waves on
+  // it costs: 1023 x 1024 12.6 / 13.4), the network's higher tiles (320 x 2300 at 8
+  // rows: 41.9 -> 39.2), tall grids (64 x 8000 at 16 rows: 1.15 -> 1.01)
+  StepScalars Q = P;
+  const int64_t sms = sm_count();
+  Q.late = tfc    ? nparts < 3 * (int64_t)resident
+           : raw  ? 2 * (int64_t)nparts < 25 * sms
+           : surr ? TR > 4 && nparts < 3 * (int64_t)resident
+                  : !pipe && TR == 16 && K.ny - 2 > 28 * sms && nparts < 10 * sms;
   // every kernel of the step is a programmatic dependent of the one before it
   // in the stream (rs_step_f64t.cu)
   const float *tab = tm.col_tab;
@@ -79,15 +112,15 @@ int launch_step_f32_tma(const StepCoef &K, const Coef<float> &F, const StepScala
   const dim3 grid(nrt, ncb);
   const int wx = resident % nrt, wy = resident / nrt;
   if (tfc) {
-    e = launch_dep_smem(x.fn, grid, block, smem, st, K, F, P, tm.psi, tm.c, tab, tm.col_tab_len, psi_n, c_n,
+    e = launch_dep_smem(x.fn, grid, block, smem, st, K, F, Q, tm.psi, tm.c, tab, tm.col_tab_len, psi_n, c_n,
                         phi_n, partials, err, wx, wy);
   } else if (pipe) {
-    e = launch_dep_smem(x.fn, dim3((unsigned)std::min(resident, nparts)), block, smem, st, K, F, P, tm.psi, tm.c,
+    e = launch_dep_smem(x.fn, dim3((unsigned)std::min(resident, nparts)), block, smem, st, K, F, Q, tm.psi, tm.c,
                         tab, tm.col_tab_len, psi_n, c_n, phi_n, partials, err, nrt, ncb);
   } else {
     SurrArgs sa = {};
     if (surr) sa = *tm.surr;
-    e = launch_dep_smem(k.fn, grid, block, smem, st, K, F, P, tm.psi, tm.c, tab, tm.col_tab_len, psi_n,
+    e = launch_dep_smem(k.fn, grid, block, smem, st, K, F, Q, tm.psi, tm.c, tab, tm.col_tab_len, psi_n,
                         c_n, phi_n, partials, err, sa, wx, wy);
   }
   if (e != cudaSuccess) return -3;

@@ -38,19 +38,37 @@ __global__ void __launch_bounds__(kTabBlock) column_table_kernel_f64(const StepC
 // more CTAs; high ones load and compute fewer halo rows.  The lines are where
 // they break even, in waves of five CTAs per SM of 16-row tiles (us a step with
 // a planar front, 4 / 8 / 16 rows): 512^2, 0.3 waves, 13.7 / 14.1 / 18.4; 768 x
-// 832, 0.8 waves, 12.4 / 13.9 / 24.0; 1024^2, 1.4 waves, 19.7 / 16.2 / 22.2;
-// 1536^2, 3.1 waves, 37.1 / 26.7 / 26.9; 2048^2, 5.5 waves, 61 / 42.3 / 37.1.
+// 832, 0.8 waves, 13.8 / 12.4 / 17.5; 1024^2, 1.4 waves, 18.5 / 16.5 / 17.9;
+// 1536^2, 3.1 waves, 33.7 / 23.7 / 20.3; 2048^2, 5.5 waves, 57 / 41.3 / 38.9.
 // A tall grid has front tiles enough for every SM at 8 or 16 rows, and then the
-// rows that a tile reads beside its own decide (with the mass, 4 / 8 / 16 rows):
-// 352 x 1568 19.7 / 18.1 / -; 128 x 1800 17.0 / 14.2 / -; 128 x 2500 18.2 /
-// 16.2 / 18.6; 160 x 3776 28.5 / 24.7 / 22.0; 96 x 4000 26.0 / 24.5 / 22.3.
+// rows that a tile reads beside its own decide, and whether all tiles are resident
+// at once (planar, cellular front, 4 / 8 / 16 rows): 128 x 1800, 0.3 waves, 14.2,
+// 13.4 / 11.3, 10.9 / 15.8, 14.7; 352 x 1568, 0.8 waves, 15.8, 18.7 / 13.5, 18.4 /
+// 16.6, 16.2; 96 x 4000, 0.7 waves, 16.1, 22.0 / 14.8, 20.1 / 18.9, 17.5; 160 x
+// 3776, 0.96 waves, 24.2, 24.6 / 21.4, 21.7 / 19.3, 19.5; with a shift 28.3, 28.3 /
+// 24.1, 24.4 / 21.8, 21.4.  A step with a shift gathers its tiles cell by cell, so
+// their halo rows cost more: 640 x 1100, 0.9 waves, cellular, in units of the
+// 16-row tile without its whole-tile forms 1.12 / 1.04 / 0.99.
 // With the coarse-grid temperature a tile also sets up its temperature tables:
 // 768 x 832, 28.8 / 22.5 / 30.2 us a step, so 4 rows are left out.
-int tile_rows_f64(int nx, int ny, bool tfc) {
-  const int64_t tiles = (int64_t)((nx + kW - 1) / kW) * ((ny - 2 + 15) / 16), wave = 5 * (int64_t)sm_count();
+int tile_rows_f64(int nx, int ny, bool tfc, bool pull_back) {
+  const int64_t sms = sm_count(), rows = ny - 2;
+  const int64_t tiles = (int64_t)((nx + kW - 1) / kW) * ((rows + 15) / 16), wave = 5 * sms;
   if (tfc) return tiles >= 3 * wave ? 16 : 8;
-  const int64_t rows = ny - 2, sms = sm_count();
-  return tiles >= 3 * wave || rows > 21 * sms ? 16 : tiles >= wave || rows > 10 * sms ? 8 : 4;
+  if (tiles >= 3 * wave) return 16;
+  if (rows > 21 * sms && tiles >= 2 * wave) return 16;
+  if (2 * rows > 21 * sms && tiles < wave) return 20 * tiles >= 9 * wave ? 16 : 8;
+  if (pull_back && rows > 7 * sms && 4 * tiles >= 3 * wave && tiles < wave) return 16;
+  return 5 * tiles >= 4 * wave || rows > 10 * sms ? 8 : 4;
+}
+// Rows that are not 16-byte aligned: the tiles but for tall grids of two tile
+// columns, where the second is mostly empty, or whose tiles a shift makes dear
+// (95 x 4000: the register kernel 26.7 us a step with a planar front and noise,
+// 17.9 with a cellular one without, 16-row tiles 20.7, 20.0; 127 x 3000 with a
+// shift, cellular: 1.06 of the register kernel's time, without one 1.02, 0.71).
+bool raw_on_tiles_f64(int nx, int ny, bool tfc, bool pull_back) {
+  const int64_t columns = (nx - 1 + kW - 1) / kW, tiles = columns * ((ny - 2 + 15) / 16), wave = 5 * (int64_t)sm_count();
+  return tfc || columns != 2 || 20 * tiles < 9 * wave || (nx >= 104 && !pull_back);
 }
 
 int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScalars &P, const TmaMaps &tm,
@@ -73,15 +91,14 @@ int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScal
   if (partials && nparts > max_partials) return -1;
   if (!tm.col_tab64 || tm.col_tab64_len < ncb * kW + kWin) return -1;
   const int sh = TR == 4 ? 0 : TR == 8 ? 1 : 2;
-  auto aligned = [&](bool own) {
-    if (TR == 4)
-      return StepKernel64{own ? tile_kernel_f64<4, false, false, true> : tile_kernel_f64<4, false, false>,
-                          sizeof(TileOps<4>::TileSmem<false>)};
-    if (TR == 8) return StepKernel64{tile_kernel_f64<8, false, false>, sizeof(TileOps<8>::TileSmem<false>)};
-    return StepKernel64{tile_kernel_f64<16, false, false>, sizeof(TileOps<16>::TileSmem<false>)};
+  auto frozen = [&](bool own) {
+    return raw       ? raw_kernel_f64(TR, own)
+           : TR == 4 ? frozen_kernel<4, false>(own)
+           : TR == 8 ? frozen_kernel<8, false>(own)
+                     : frozen_kernel<16, false>(own);
   };
-  static std::atomic<unsigned long long> attr_done[17];
-  static std::atomic<int> resident_of[17][64];
+  static std::atomic<unsigned long long> attr_done[21];
+  static std::atomic<int> resident_of[21][64];
   StepKernel64 k = {};
   auto resident_at = [&](int which) {
     return smem_limit_once((const void *)k.fn, (int)k.smem, attr_done[which])
@@ -89,21 +106,30 @@ int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScal
                : -1;
   };
   // a grid of one wave: the tiles compute their columns' entries themselves
-  bool own = TR == 4 && !tfc && !pipe;
+  bool own = !tfc && !pipe;
   int resident = 0;
   if (own) {
-    k = raw ? raw_kernel_f64(TR, true) : aligned(true);
-    resident = resident_at(15 + raw);
+    k = frozen(true);
+    resident = resident_at(15 + 3 * raw + sh);
     own = nparts <= resident;
   }
   if (!own) {
     k = pipe  ? pipe_kernel_of_f64(TR)
         : tfc ? (raw ? tfc_raw_kernel_f64(TR) : tfc_kernel_f64(TR))
-        : raw ? raw_kernel_f64(TR, false)
-              : aligned(false);
+              : frozen(false);
     resident = resident_at(pipe ? 12 + sh : 6 * raw + 3 * tfc + sh);
   }
   if (resident <= 0) return -3;
+  // CTAs of the next step that are scheduled while this one's last tiles are at
+  // work fill the slots of SMs that have finished first, its front tiles, which
+  // are launched first, several to an SM.  Where a grid has few waves that costs
+  // more than the launch latency it hides: 96 x 4000 with a cellular front on
+  // 16-row tiles, 22.5 us a step with the early trigger, 18.5 with the late one;
+  // 768 x 832 on 8-row tiles 15.9 / 14.9; 1536^2, 3.1 waves of 16-row tiles, with
+  // a planar front 20.3 / 21.0.  (4-row tiles: no difference, and the early
+  // trigger lets those that compute their own columns start on them.)
+  StepScalars Q = P;
+  Q.late = TR > 4 && !tfc && !pipe && nparts < 15 * (int64_t)sm_count();
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -133,7 +159,7 @@ int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScal
     // column-major: consecutive CTAs share a column strip and its halo rows in L2
     cfg.gridDim = dim3(nrt, ncb);
     cfg.blockDim = dim3(kTileThreads64);
-    e = cudaLaunchKernelEx(&cfg, k.fn, K, F, P, tm.psi, tm.c, tab, tm.col_tab64_len, psi_n, c_n, phi_n, partials,
+    e = cudaLaunchKernelEx(&cfg, k.fn, K, F, Q, tm.psi, tm.c, tab, tm.col_tab64_len, psi_n, c_n, phi_n, partials,
                            err, resident % nrt, resident / nrt);
   }
   if (e != cudaSuccess) return -3;

@@ -5,9 +5,7 @@
 namespace rs {
 
 StepKernel64 raw_kernel_f64(int rows, bool own) {
-  if (rows == 4) return {own ? tile_kernel_f64<4, false, true, true> : tile_kernel_f64<4, false, true>, sizeof(TileOps<4>::TileSmem<false>)};
-  if (rows == 8) return {tile_kernel_f64<8, false, true>, sizeof(TileOps<8>::TileSmem<false>)};
-  return {tile_kernel_f64<16, false, true>, sizeof(TileOps<16>::TileSmem<false>)};
+  return rows == 4 ? frozen_kernel<4, true>(own) : rows == 8 ? frozen_kernel<8, true>(own) : frozen_kernel<16, true>(own);
 }
 
 }  // namespace rs

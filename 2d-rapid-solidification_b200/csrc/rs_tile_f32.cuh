@@ -319,8 +319,9 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     tma_load_2d(&sm.psi[0][0], tm_psi, &sm.full, x0 - 4, y0 - 1);
     tma_load_2d(&sm.d[0][0], tm_c, &sm.full, x0 - 4, y0 - 1);
   }
-  // dependents of this step (its reduction, the next step) may be scheduled now
-  pdl_trigger();
+  // dependents of this step (its reduction, the next step) may be scheduled now,
+  // or (late) once the tile's listed cells are done
+  if (!PS.late) pdl_trigger();
   const float *tRT = tab + kTabRT * tab_len + 4, *tC0 = tab + kTabC0 * tab_len + 4;
   const float *tDK = tab + kTabDK * tab_len + 4;
   float4 RTv = make_float4(0.f, 0.f, 0.f, 0.f), C0v = RTv, dKv = RTv;
@@ -390,13 +391,14 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     return rr == 0 ? (y0 - 1) % AR == 0 : (y0 - 1 + kTR) % AR == 0 || y0 + kTR == ny - 1;
   };
   const bool open_end = SURR && (ny - 2) % AR != 0;
-  auto open_row = [&](int rr) { return AR != TR && open_end && rr == kTR + 1 && y0 + kTR == ny - 1; };
+  auto open_row = [&](int rr) { return open_end && rr == kTR + 1 && y0 + kTR == ny - 1; };
   // a halo cell's mu'' enters only the face to the tile's edge column, whose
   // weight is 0 when psi is exactly +1 on both columns over rows rr-1..rr+1;
   // column -1 (left-most tile) enters no face at all (column 0 is a ghost)
   auto halo_mu_used = [&](int rr, int b) {
     if (b == kHaloL && x0 == 0) return false;
-    if (open_row(rr)) return true;
+    if constexpr (AR != TR)
+      if (open_row(rr)) return true;
     const int b2 = b == kHaloL ? b + 1 : b - 1;
     bool solid = true;
     for (int r2 = max(rr - 1, 0); r2 <= min(rr + 1, kTRin - 1); ++r2)
@@ -409,7 +411,8 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
   // S = q(1) c (1 - c) = 0 there, so every face weight touching the cell is 0
   // and its mu'' enters no flux (0 times a finite difference)
   auto solid3 = [&](int rr) -> uint32_t {
-    if (open_row(rr)) return 0u;  // (warp-uniform)
+    if constexpr (AR != TR)
+      if (open_row(rr)) return 0u;  // (warp-uniform)
     const int xh = lane == 0 ? kHaloL : kHaloR;
     uint32_t v = 0xFu;
     bool hs = true;  // the halo column beside lanes 0 and 31
@@ -614,8 +617,10 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     return;
   }
   const bool melt = !TFC && !(vote & (kNotMinus1 | kNotFar));
+  bool solid = !(vote & (kNotPlus1 | kNotFinite));
   // (a solid tile with such a row ny-1 takes the phases, where its cells are counted)
-  if (melt || !((vote & (kNotPlus1 | kNotFinite)) || (open_end && y0 + kTR >= ny - 1))) {
+  if constexpr (SURR) solid = solid && !(open_end && y0 + kTR >= ny - 1);
+  if (melt || solid) {
     // the warp's output rows straight from registers to global memory, with
     // the ghost columns and rows they copy to (nx is a multiple of 4: a lane's
     // cells are all inside the array or all beyond it)
@@ -1149,6 +1154,9 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
   }
   __syncthreads();
 
+  // (a whole-tile form, and a CTA that gave up, trigger by their end)
+  if (PS.late) pdl_trigger();
+
   // ---- phase 4: new psi and c into the tile rows
 #pragma unroll
   for (int j = 0; j < kRowsPerWarp; ++j) {
@@ -1270,6 +1278,8 @@ struct WavePrefetch {
   }
 };
 
+// (exact, 4 rows: 72 registers, so that seven CTAs fit on an SM; with 74 and six,
+// 96 x 4000 took 14.0 us a step instead of 10.5)
 template <bool SURR, int TR, bool RAW>
 __global__ void __launch_bounds__(kThreads, SURR ? 4 : 5)
     tile_kernel(const __grid_constant__ StepCoef K, const __grid_constant__ Coef<float> F,

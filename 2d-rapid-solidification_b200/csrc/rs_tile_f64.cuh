@@ -1183,8 +1183,9 @@ __device__ __forceinline__ void tile_of(int t, int nrt, int ncb, int f, int &tr,
 // OWN: the CTA computes the table entries of its 72 columns itself, before it
 // waits for the kernel before it, and the step is one launch.  For grids whose
 // CTAs are all resident at once: theirs are scheduled, and compute the entries,
-// while the step before is still at work (256^2: 8.1 -> 6.5 us a step); on
-// larger ones every wave would compute them again.
+// while the step before is still at work (256^2: 8.1 -> 6.5 us a step; 352 x 1568
+// with a cellular front on 16-row tiles: 18.5 -> 16.2); on larger ones every wave
+// would compute them again.
 template <int TR, bool TFC, bool RAW, bool OWN = false>
 __global__ void __launch_bounds__(kThreads, 5)
     tile_kernel_f64(const __grid_constant__ StepCoef K, const __grid_constant__ Coef<double> F,
@@ -1247,8 +1248,9 @@ __global__ void __launch_bounds__(kThreads, 5)
     tma_load_2d(&sm.in.psi[0][0], &tm_psi, &sm.full, x0 - 4, y0 - 1);
     tma_load_2d(&sm.in.c[0][0], &tm_c, &sm.full, x0 - 4, y0 - 1);
   }
-  // dependents of this step (its reduction, the next step) may be scheduled now
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // dependents of this step (its reduction, the next step) may be scheduled now,
+  // or (late) once the tile's phase 3 is done
+  if (!PS.late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const typename Ops::TileView V(K, F, PS, OWN ? own_tab - x0 : tab, OWN ? kWin : tab_len, x0, y0,
                                  (int)threadIdx.x);
   const typename Ops::LaneCols LC = Ops::template lane_cols<TFC>(V);
@@ -1359,6 +1361,8 @@ __global__ void __launch_bounds__(kThreads, 5)
   __syncthreads();
   Ops::template phase3<TFC>(V, sm.in, sm.p2, tf, sm.st.S, red, itip);  // S is free after phase 2
   __syncthreads();
+  // (a whole-tile form, and a CTA that gave up, trigger by their end)
+  if (PS.late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   Ops::phase4_rows(V, sm.in, sm.st.S, needs_all, dn, red, itip);
   Ops::store_tile(V, sm.in, psi_n, c_n, phi_n, 0);
   Ops::finish_tile(V, sm.p2, mass, itip, part, 0);
@@ -1377,6 +1381,11 @@ struct StepKernel64 {
   StepFn64 fn;
   size_t smem;
 };
+template <int TR, bool RAW>
+StepKernel64 frozen_kernel(bool own) {
+  return {own ? tile_kernel_f64<TR, false, RAW, true> : tile_kernel_f64<TR, false, RAW>,
+          sizeof(typename TileOps<TR>::template TileSmem<false>)};
+}
 StepKernel64 raw_kernel_f64(int rows, bool own);  // rs_step_f64t_raw.cu
 StepKernel64 tfc_kernel_f64(int rows);            // rs_step_f64t_tfc.cu
 StepKernel64 tfc_raw_kernel_f64(int rows);        // rs_step_f64t_tfc_raw.cu
