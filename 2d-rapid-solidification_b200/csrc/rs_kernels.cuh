@@ -153,7 +153,8 @@ constexpr int kTmaBoxH = kTileRows + 2;  // input rows of a tile
 int tile_rows_f64(int nx, int ny, bool tfc, bool pull_back);  // output rows of an FP64 tile: 4, 8 or 16
 int tile_rows_f32(int nx, int ny, bool tfc, bool network);  // and of an FP32 tile
 // whether the tile kernels take a step on rows that are not 16-byte aligned (else
-// the register kernel)
+// the register kernel, whose grid is 4 strips of 30 columns wide)
+constexpr bool register_grid_fits(int nx) { return ((nx - 2 + 29) / 30 + 3) / 4 <= 65535; }
 bool raw_on_tiles_f64(int nx, int ny, bool tfc, bool pull_back);
 bool raw_on_tiles_f32(int nx, int ny, bool tfc, bool pull_back);
 constexpr int kTfcTileRows32 = 8;        // output rows of an FP32 coarse-grid-temperature tile

@@ -48,6 +48,7 @@ bool raw_on_tiles_f32(int nx, int ny, bool tfc, bool pull_back) {
   const int rows = tfc ? kTfcTR : 4;
   const int64_t tiles = (int64_t)((nx - 1 + kW - 1) / kW) * ((ny - 2 + rows - 1) / rows), wave = 5 * (int64_t)sm_count();
   const bool few = 2 * tiles <= 3 * wave;
+  if (!register_grid_fits(nx)) return true;
   if (tfc) return nx > 448 || tiles <= wave || !few;
   return few || (!pull_back && nx > 432);
 }

@@ -68,6 +68,8 @@ int tile_rows_f64(int nx, int ny, bool tfc, bool pull_back) {
 // shift, cellular: 1.06 of the register kernel's time, without one 1.02, 0.71).
 bool raw_on_tiles_f64(int nx, int ny, bool tfc, bool pull_back) {
   const int64_t columns = (nx - 1 + kW - 1) / kW, tiles = columns * ((ny - 2 + 15) / 16), wave = 5 * (int64_t)sm_count();
+  if (!register_grid_fits(nx)) return true;
+  if (columns > 65535) return false;  // (the tiles' grid: 4194240 columns)
   return tfc || columns != 2 || 20 * tiles < 9 * wave || (nx >= 104 && !pull_back);
 }
 
