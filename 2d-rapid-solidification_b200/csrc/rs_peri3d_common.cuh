@@ -69,7 +69,7 @@ inline int p3_chunk(const rs3_params &p, int64_t tiles, int ctas_per_sm, bool he
   int best = 32;
   double least = 1e300;
   for (int c = 32; c >= 2; c /= 2) {
-    const double waves = (double)(tiles * ((p.nz - 2 + c - 1) / c)) / (148 * ctas_per_sm);
+    const double waves = (double)(tiles * ((p.nz - 2 + c - 1) / c)) / (sm_count() * ctas_per_sm);
     const double cost = (std::max(waves, 1.0) + (heavy ? 1.0 : 0.5)) * (c + (heavy ? 3.0 : 0.5));
     if (cost < least) least = cost * (heavy && c == 32 ? 0.85 : 1.0), best = c;
   }
