@@ -149,7 +149,6 @@ struct TSmem {
   alignas(16) float dG[3][SURR ? P3Cfg<R>::BX * kP3BY : 1];
   uint64_t full[kP3Slots];
   int melt[8];  // per plane (q mod 8): the box is pure melt inside the array (p3_melt_cell)
-  uint32_t passed;  // warps that have left a plane, summed over the planes
 };
 
 // SD: solid diffusivities Da or Db non-zero.  WEIGH: the surrogate's counters
@@ -191,7 +190,6 @@ __global__ void __launch_bounds__(kP3Threads, 2)
   if (tid == 0) {
     for (int s = 0; s < kP3Slots; ++s) mbar_init(&sm.full[s], 1);
     for (int s = 0; s < 8; ++s) sm.melt[s] = 1;
-    sm.passed = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int z = zin0; z <= min(zin1, zin0 + kP3Slots - 1); ++z) issue(z);
   }
@@ -869,10 +867,9 @@ int tinb_table_len(const rs3_params &p) { return kTW * p.nz; }
 
 int launch_tinb_step(const rs3_params &p, const P3Maps &m, int precision, void *o1, void *o2, void *oc, int64_t step,
                      int *err, double *tab, const SurrArgs *surr, cudaStream_t st) {
-  {
-    K3<double> kt = make_k3<double>(p);
-    launch_dep(tinb_table_kernel, dim3((p.nz + 127) / 128), dim3(128), st, kt, step, tab);
-  }
+  if (launch_dep(tinb_table_kernel, dim3((p.nz + 127) / 128), dim3(128), st, make_k3<double>(p), step, tab) !=
+      cudaSuccess)
+    return -3;  // (the step would read another step's table)
   const bool sd = p.Da != 0.0 || p.Db != 0.0;
   SurrArgs none;
   memset(&none, 0, sizeof(none));
