@@ -319,33 +319,39 @@ struct KcPoly {
   double a[7];   // A_Ti^(k)(T0) / k!
   int ok;        // T0 in [1945, 2746)
 };
-__device__ __forceinline__ KcPoly kc_poly(const StepCoef &K, double T0) {
-  KcPoly P;
-  P.lr = log_ref(T0);
+// K + C0's part of P; its logarithm, divisions and powers are a chain of some 300
+// cycles for one thread of a tile, the driving-force part as long for another
+__device__ __forceinline__ void kc_poly(const StepCoef &K, double T0, KcPoly &P) {
+  const LogRef lr = log_ref(T0);
+  P.lr = lr;
   P.ok = T0 >= 1945.0 && T0 < 2746.0;
   constexpr double c = -46.29 + 26.4711, d = -0.203475e-3, e = 0.35012e-6, f = -93399.0, h = 306.098e-25;
   const double b = (298.7367 - 131.229057) + K.RR * K.Lref;
-  const double T = T0, lT = P.lr.lT0, i1 = P.lr.iT0;
+  const double T = T0, lT = lr.lT0, i1 = lr.iT0;
   const double i2 = i1 * i1, i3 = i2 * i1, i4 = i2 * i2, i5 = i4 * i1, i6 = i3 * i3, i7 = i6 * i1;
   const double T2 = T * T, T3 = T2 * T, T4 = T2 * T2, T5 = T4 * T, T6 = T3 * T3;
   P.c[0] = groups_at(K, T, lT, false).KC;
   P.c[1] = b + c * (lT + 1.0) + 2.0 * d * T + 3.0 * e * T2 - f * i2 + 7.0 * h * T6;
-  P.c[2] = (c * i1 + 2.0 * d + 6.0 * e * T + 2.0 * f * i3 + 42.0 * h * T5) / 2.0;
-  P.c[3] = (-c * i2 + 6.0 * e - 6.0 * f * i4 + 210.0 * h * T4) / 6.0;
-  P.c[4] = (2.0 * c * i3 + 24.0 * f * i5 + 840.0 * h * T3) / 24.0;
-  P.c[5] = (-6.0 * c * i4 - 120.0 * f * i6 + 2520.0 * h * T2) / 120.0;
-  P.c[6] = (24.0 * c * i5 + 720.0 * f * i7 + 5040.0 * h * T) / 720.0;
+  P.c[2] = (c * i1 + 2.0 * d + 6.0 * e * T + 2.0 * f * i3 + 42.0 * h * T5) * 0.5;
+  P.c[3] = (-c * i2 + 6.0 * e - 6.0 * f * i4 + 210.0 * h * T4) * (1.0 / 6.0);
+  P.c[4] = (2.0 * c * i3 + 24.0 * f * i5 + 840.0 * h * T3) * (1.0 / 24.0);
+  P.c[5] = (-6.0 * c * i4 - 120.0 * f * i6 + 2520.0 * h * T2) * (1.0 / 120.0);
+  P.c[6] = (24.0 * c * i5 + 720.0 * f * i7 + 5040.0 * h * T) * (1.0 / 720.0);
+}
+__device__ __forceinline__ void drive_poly(double T0, KcPoly &P) {
   // G_Ti_Liq - G_Ti_BCC above 1941 K (fun.cu:1628-1647)
   constexpr double ab = 298.7367 + 182.426471, ac = -46.29 - 19.0900905, ad = 22.00832e-3, ae = -1.228863e-6,
                    af = -1400501.0;
-  P.a[0] = P.ok ? g_ti_liq(T, lT) - g_ti_bcc(T, lT) : 0.0;
+  const LogRef lr = log_ref(T0);
+  const double T = T0, lT = lr.lT0, i1 = lr.iT0, T2 = T * T;
+  const double i2 = i1 * i1, i3 = i2 * i1, i4 = i2 * i2, i5 = i4 * i1, i6 = i3 * i3, i7 = i6 * i1;
+  P.a[0] = T0 >= 1945.0 && T0 < 2746.0 ? g_ti_liq(T, lT) - g_ti_bcc(T, lT) : 0.0;
   P.a[1] = ab + ac * (lT + 1.0) + 2.0 * ad * T + 3.0 * ae * T2 - af * i2;
-  P.a[2] = (ac * i1 + 2.0 * ad + 6.0 * ae * T + 2.0 * af * i3) / 2.0;
-  P.a[3] = (-ac * i2 + 6.0 * ae - 6.0 * af * i4) / 6.0;
-  P.a[4] = (2.0 * ac * i3 + 24.0 * af * i5) / 24.0;
-  P.a[5] = (-6.0 * ac * i4 - 120.0 * af * i6) / 120.0;
-  P.a[6] = (24.0 * ac * i5 + 720.0 * af * i7) / 720.0;
-  return P;
+  P.a[2] = (ac * i1 + 2.0 * ad + 6.0 * ae * T + 2.0 * af * i3) * 0.5;
+  P.a[3] = (-ac * i2 + 6.0 * ae - 6.0 * af * i4) * (1.0 / 6.0);
+  P.a[4] = (2.0 * ac * i3 + 24.0 * af * i5) * (1.0 / 24.0);
+  P.a[5] = (-6.0 * ac * i4 - 120.0 * af * i6) * (1.0 / 120.0);
+  P.a[6] = (24.0 * ac * i5 + 720.0 * af * i7) * (1.0 / 720.0);
 }
 // the driving-force groups at T from P, or false where it does not apply
 __device__ __forceinline__ bool drive_eval(const KcPoly &P, double T, double &Anb, double &Ati) {

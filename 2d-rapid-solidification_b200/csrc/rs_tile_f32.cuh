@@ -351,12 +351,14 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
       const int side = (int)threadIdx.x - (kTRin + 1);
       tfc_col(K, PS.i_left_end_T, side ? x0 + kW : x0 - 1, sm.hiT[side], sm.hx[side]);
     }
-    if (threadIdx.x == kTRin) {
+    if (threadIdx.x == 64 || threadIdx.x == 96) {
       int iT, jT;
       double x, y;
       tfc_col(K, PS.i_left_end_T, x0 + kW / 2, iT, x);
       tfc_row(K, y0 + kTR / 2, jT, y);
-      sm.kp = kc_poly(K, tfc_T(K, PS.T_coarse, iT, x, jT, y));
+      const double T0 = tfc_T(K, PS.T_coarse, iT, x, jT, y);
+      if (threadIdx.x == 64) kc_poly(K, T0, sm.kp);
+      else drive_poly(T0, sm.kp);
     }
   }
   // TFC: all groups of one cell, the logarithm exact (halo and interface cells)
@@ -573,8 +575,11 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
       p1 |= __float_as_uint(p) ^ kPlus1;
       dm = max(dm, __float_as_uint(d) & 0x7fffffffu);
     };
-    uint32_t bad = kGaveUp;
-    if (!gave_up) {
+    uint32_t bad = gave_up ? kGaveUp : kNotMinus1 | kNotPlus1;
+    // (the coarse-grid temperature has no melt form: its tiles vote only where the
+    // first interior cell is solid; 2048^2 all melt, with the polynomials of K + C0
+    // and of the driving force on two threads, 63.5 -> 59 us a step)
+    if (!gave_up && (!TFC || __float_as_uint(sm.psi[1][5]) == kPlus1)) {
 #pragma unroll
       for (int k = 0; k < (kTRin + kWarps - 1) / kWarps; ++k) {
         const int rr = warp + kWarps * k;

@@ -971,9 +971,8 @@ struct CellStore {
 // twelve lanes through scratch), stored straight to global memory.  The same
 // expressions as phases 1 and 2, so the same bits.  No row votes on its form,
 // so the arithmetic of the rows overlaps.  Returns the warp's part of the mass.
-template <bool TFC>
 static __device__ __forceinline__ double melt_tile(const TileView &V, const LaneCols &LC, const InSlot &in, MeltHalo &mh,
-                                            const TfcTile *tf, bool red, double *stage, double *__restrict__ psi_n,
+                                            bool red, double *stage, double *__restrict__ psi_n,
                                             double *__restrict__ c_n,
                                             double *__restrict__ phi_n) {
   const Coef<double> &F = V.F;
@@ -987,7 +986,7 @@ static __device__ __forceinline__ double melt_tile(const TileView &V, const Lane
     double S = 0.0, m = 0.0;
     if (rr <= V.K.ny - V.y0) {
       const int x = side ? kHaloR : kHaloL;
-      halo_cell<TFC>(V, tf, ma, in.psi[rr][x], in.c[rr][x], rr, side, V.x0 - 4 + x, S, m);
+      halo_cell<false>(V, nullptr, ma, in.psi[rr][x], in.c[rr][x], rr, side, V.x0 - 4 + x, S, m);
     }
     hs[lane] = S;
     hm[lane] = m;
@@ -996,36 +995,13 @@ static __device__ __forceinline__ double melt_tile(const TileView &V, const Lane
   struct Row {
     double s[2], m[2], sl, sr, ml, mr;
   };
-  int band_jT = -1;
-  double Pb[2] = {0.0, 0.0}, Qb[2] = {0.0, 0.0};
   auto load_row = [&](int k, Row &R) {
     const int rr = r0 + k;
     const double2 cv = ld2(&in.c[rr][V.bc]);
     const double cc[2] = {cv.x, cv.y};
     const double dv[2] = {cv.x - cinf, cv.y - cinf};
-    double RT[2] = {LC.RT[0], LC.RT[1]}, KC[2] = {0.0, 0.0};
-    if constexpr (TFC) {
-      const int jT = tf->tj[rr];
-      const double y = tf->ty[rr];
-      if (jT != band_jT) {
-        band_jT = jT;
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const double tx = tf->tx[V.col + q];
-          const double *t0 = V.PS.T_coarse + (int64_t)jT * V.K.NxT_all + tf->ti[V.col + q], *t1 = t0 + V.K.NxT_all;
-          const double f00 = t0[0], f10 = t0[1], f01 = t1[0], f11 = t1[1];
-          Pb[q] = fma(f10 - f00, tx, f00);
-          Qb[q] = fma(f11 - f10 - f01 + f00, tx, f01 - f00);
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        double C0;
-        cell_tfc(V.K, tf->kp, fma(Qb[q], y, Pb[q]), false, RT[q], C0, KC[q]);
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 2; ++q) far_cell<TFC>(ma, cc[q], dv[q], RT[q], KC[q], R.s[q], R.m[q]);
+    for (int q = 0; q < 2; ++q) far_cell<false>(ma, cc[q], dv[q], LC.RT[q], 0.0, R.s[q], R.m[q]);
     R.sl = __shfl_up_sync(FULL, R.s[1], 1);
     R.ml = __shfl_up_sync(FULL, R.m[1], 1);
     R.sr = __shfl_down_sync(FULL, R.s[0], 1);
@@ -1264,12 +1240,14 @@ __global__ void __launch_bounds__(kThreads, 5)
     if (t < kW) tfc_col(K, PS.i_left_end_T, x0 + t, T.ti[t], T.tx[t]);
     else if (t < kW + 2) tfc_col(K, PS.i_left_end_T, t == kW ? x0 - 1 : x0 + kW, T.hiT[t - kW], T.hx[t - kW]);
     else if (t >= 96 && t < 96 + Ops::kTRin) tfc_row(K, y0 - 1 + t - 96, T.tj[t - 96], T.ty[t - 96]);
-    else if (t == 127) {
+    else if (t == 80 || t == 127) {  // (two warps)
       int iT, jT;
       double x, y;
       tfc_col(K, PS.i_left_end_T, x0 + kW / 2, iT, x);
       tfc_row(K, y0 + TR / 2, jT, y);
-      T.kp = kc_poly(K, tfc_T(K, PS.T_coarse, iT, x, jT, y));
+      const double T0 = tfc_T(K, PS.T_coarse, iT, x, jT, y);
+      if (t == 127) kc_poly(K, T0, T.kp);
+      else drive_poly(T0, T.kp);
     }
   }
   if (pb) Ops::gather_box(K, PS, x0, y0, sm.in);
@@ -1321,7 +1299,11 @@ __global__ void __launch_bounds__(kThreads, 5)
     __syncthreads();
   }
   {
-    uint32_t bad = gave_up ? (uint32_t)Ops::kGaveUp : Ops::tile_vote(V, sm.in);
+    // (the coarse-grid temperature has no melt form: a tile votes only where its
+    // first interior cell is solid)
+    uint32_t bad = gave_up ? (uint32_t)Ops::kGaveUp
+                   : TFC && bits(sm.in.psi[1][5]) != kPlus1 ? (uint32_t)(Ops::kNotMinus1 | Ops::kNotPlus1)
+                                                            : Ops::tile_vote(V, sm.in);
     bad = __reduce_or_sync(FULL, bad);
     if (V.lane == 0 && bad) atomicOr(&sm.vote, bad);
   }
@@ -1344,11 +1326,11 @@ __global__ void __launch_bounds__(kThreads, 5)
     Ops::finish_tile(V, sm.p2, 0.0, 0, part, 0);
     return;
   }
-  const bool melt = !(vote & (Ops::kNotMinus1 | Ops::kNotFar));
+  const bool melt = !TFC && !(vote & (Ops::kNotMinus1 | Ops::kNotFar));
   if (melt || !(vote & (Ops::kNotPlus1 | Ops::kNotFinite))) {
     if (melt)
-      mass = Ops::template melt_tile<TFC>(V, LC, sm.in, *reinterpret_cast<typename Ops::MeltHalo *>(sm.p2.list), tf, red,
-                                          sm.st.S[V.gw], psi_n, c_n, phi_n);
+      mass = Ops::melt_tile(V, LC, sm.in, *reinterpret_cast<typename Ops::MeltHalo *>(sm.p2.list), red, sm.st.S[V.gw], psi_n,
+                            c_n, phi_n);
     else
       mass = Ops::solid_tile(V, sm.in, red, sm.st.S[V.gw], psi_n, c_n, phi_n, itip);
     Ops::finish_tile(V, sm.p2, mass, itip, part, 0);
