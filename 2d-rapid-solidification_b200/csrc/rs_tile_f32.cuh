@@ -435,26 +435,32 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     in[1] = fmaf(sm.d[rr][b], SA.c_ihalf, cnA);
     in[2] = clamp1(sm.psi[rr][b]);
   };
+  // box and audit of one cell (in: net_inputs of it)
+  auto net_inbox = [&](int rr, int b, const float in[3]) {
+    const float T = SA.T_mid + in[0] / SA.T_ihalf, c = F.cinf + sm.d[rr][b];
+    return T >= SA.T_lo && T <= SA.T_hi && c >= SA.c_lo && c <= SA.c_hi;
+  };
+  auto net_audited = [&](int rr, int b) {
+    return surr_audit_cell(PS.step, (int64_t)(y0 - 1 + rr + K.j_offset) * K.nx + x0 + b - 4);
+  };
+  auto audit_store = [&](int rr, int b, const float o[2]) {  // (the exact mu'' is in place)
+    const int gx = x0 + b - 4;
+    const float dG_ex = drive_dG<float>(F.cinf + sm.d[rr][b], tAnb[gx], tAti[gx]);
+    const float mu_net = fmaf(o[0], SA.y_scale[0], SA.y_mean[0]), dG_net = fmaf(o[1], SA.y_scale[1], SA.y_mean[1]);
+    atomicMax(&SA.audit[0], (unsigned long long)__float_as_uint(fabsf(mu_net - sm.mu[rr][b])));
+    atomicMax(&SA.audit[1], (unsigned long long)__float_as_uint(fabsf(dG_net - dG_ex)));
+    atomicAdd(&SA.audit[3], 1ull);
+  };
   // store the surrogate mu'' of one cell, or keep the exact value already in
   // place (out-of-box and audited cells); audited cells record the errors
   auto net_store = [&](int rr, int b, const float in[3], const float o[2]) {
     const int gx = x0 + b - 4;
-    const float T = SA.T_mid + in[0] / SA.T_ihalf, c = F.cinf + sm.d[rr][b];
-    const bool inbox = T >= SA.T_lo && T <= SA.T_hi && c >= SA.c_lo && c <= SA.c_hi;
-    const bool real = gx >= 0 && gx <= K.nx - 1;
-    const bool audit = real && surr_audit_cell(PS.step, (int64_t)(y0 - 1 + rr + K.j_offset) * K.nx + gx);
-    const float mu_net = fmaf(o[0], SA.y_scale[0], SA.y_mean[0]);
+    const bool inbox = net_inbox(rr, b, in), real = gx >= 0 && gx <= K.nx - 1, audit = real && net_audited(rr, b);
     if (inbox && !audit) {
-      sm.mu[rr][b] = mu_net;
+      sm.mu[rr][b] = fmaf(o[0], SA.y_scale[0], SA.y_mean[0]);
     } else if (real && counted(rr)) {
       if (!inbox) atomicAdd(&SA.audit[2], 1ull);
-      if (audit) {
-        const float dG_ex = drive_dG<float>(c, tAnb[gx], tAti[gx]);
-        const float dG_net = fmaf(o[1], SA.y_scale[1], SA.y_mean[1]);
-        atomicMax(&SA.audit[0], (unsigned long long)__float_as_uint(fabsf(mu_net - sm.mu[rr][b])));
-        atomicMax(&SA.audit[1], (unsigned long long)__float_as_uint(fabsf(dG_net - dG_ex)));
-        atomicAdd(&SA.audit[3], 1ull);
-      }
+      if (audit) audit_store(rr, b, o);
     }
   };
   // the partial sums of this tile (a dependent launch reduces them)
@@ -622,10 +628,7 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
     return;
   }
   const bool melt = !TFC && !(vote & (kNotMinus1 | kNotFar));
-  bool solid = !(vote & (kNotPlus1 | kNotFinite));
-  // (a solid tile with such a row ny-1 takes the phases, where its cells are counted)
-  if constexpr (SURR) solid = solid && !(open_end && y0 + kTR >= ny - 1);
-  if (melt || solid) {
+  if (melt || !(vote & (kNotPlus1 | kNotFinite))) {
     // the warp's output rows straight from registers to global memory, with
     // the ghost columns and rows they copy to (nx is a multiple of 4: a lane's
     // cells are all inside the array or all beyond it)
@@ -673,6 +676,45 @@ __device__ __forceinline__ void tile_body(const StepCoef &K, const Coef<float> &
             }
         }
         put(j, v);
+      }
+      if constexpr (SURR) {
+        // row ny-1 at the counters' open end: its cells count, and the audited ones
+        // take the network, as the phases would have them
+        if (open_end && y0 + kTR >= ny - 1) {
+          const int rr = ny - y0, own = 4 + 32 * warp;
+          auto cells = [&](int b, bool real, int ba, int bb, uint32_t ma, uint32_t mb) {  // one lane's cell; two per pass
+            float in0[3], in1[3], o0[2], o1[2], Sx, mx;
+            bool audit = false;
+            if (real) {
+              net_inputs(rr, b, in0);
+              audit = net_audited(rr, b);
+              if (!net_inbox(rr, b, in0)) atomicAdd(&SA.audit[2], 1ull);
+            }
+            const uint32_t am = __ballot_sync(FULL, audit);
+            if (!am) return;
+            if (audit) {
+              cell_terms(F, sm.psi[rr][b], sm.d[rr][b], tRT[x0 + b - 4], tC0[x0 + b - 4], Sx, mx);
+              sm.mu[rr][b] = mx;
+            }
+            __syncwarp();
+            const SurrConst SC = surr_load(SA, lane);
+#pragma unroll 1
+            for (int h = 0; h < 32; h += 16) {
+              if (!(am >> h & 0xFFFFu)) continue;
+              net_inputs(rr, ba + h, in0);
+              net_inputs(rr, bb + h, in1);
+              surr_tile16(SC, in0, in1, o0, o1);
+              if ((lane & 3) == 0) {
+                if (am >> h & ma) audit_store(rr, ba + h, o0);
+                if (am >> h & mb) audit_store(rr, bb + h, o1);
+              }
+            }
+          };
+          const int g = lane >> 2;
+          cells(own + lane, true, own + g, own + g + 8, 1u << g, 256u << g);
+          if (warp == 3)  // the halo columns, lanes 0 and 1
+            cells(lane ? kHaloR : kHaloL, lane == 1 || (lane == 0 && x0 > 0), kHaloL, kHaloR, g ? 0u : 1u, g ? 0u : 2u);
+        }
       }
       finish(mass, itip);
       return;

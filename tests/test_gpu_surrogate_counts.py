@@ -101,3 +101,37 @@ def test_a_run_alone_reports_what_it_reports_in_an_ensemble(nx, ny):
     assert want[3] > 0
     assert tuple(got) == tuple(want)
     ens.close()
+
+
+# most columns solid: last tile rows of 4, 8 and 16 rows that hold a whole tile of solid
+@pytest.mark.parametrize("nx,ny", [(516, 58), (388, 200), (640, 66), (2048, 1122)])
+def test_solid_tiles_report_the_cells_of_row_ny_minus_1(nx, ny):
+    p = configs._ti10nb(configs.default_params(), nx, ny, 5e6, 0.5, T0=configs.T_SOLIDUS_TI10NB)
+    p.i_tip_target, p.noise_amplitude, p.seed = nx // 2, 0.01, 11
+    w, box, _ = surrogate.train(p, n_samples=1 << 12, epochs=1, batch=1024, seed=3)
+    box.c_hi = 0.5 * (box.c_lo + box.c_hi)  # part of the cells are out of the box
+    front = int(0.9 * nx)
+
+    def step(ctx):
+        a, b = lib.FieldSet(p, torch.float32), lib.FieldSet(p, torch.float32)
+        ctx.initial_planar(a, configs.C_LIQUID_TI10NB, configs.C_SOLID_AT_TLIQ, front)
+        a.psi[:, : front - 20] = 1.0
+        ctx.set_surrogate(w, box)
+        return a, b
+
+    ens = lib.Ensemble([p])
+    ea, eb = step(ens.ctx[0])
+    ens.bind(0, ea, eb)
+    ens.set_path(0)  # per-step launches, 16-row tiles
+    ens.steps(1)
+    torch.cuda.synchronize()
+    want = ens.ctx[0].surrogate_audit()
+    ctx = lib.Context(p)
+    a, b = step(ctx)
+    tip = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ctx.itip(a, tip)
+    pb = int(tip.item()) - p.i_tip_target
+    ctx.step(a, b, 0, i_offset_history=pb, l_offset_Vp=0.0, pull_back=pb)
+    assert tuple(ctx.surrogate_audit()) == tuple(want)
+    assert torch.equal(b.psi, eb.psi)
+    ens.close()
