@@ -464,12 +464,13 @@ int rs_step(rs_ctx *c, const rs_fields *cur, const rs_fields *next, const rs_ste
   const int nx = c->p.nx_all, ny = c->p.ny_all;
   bool tiles = c->use_tma != 0;
   if (tiles) {
-    tm.rows = f64 ? rs::tile_rows_f64(nx, ny, tfc, a->pull_back != 0) : rs::tile_rows_f32(nx, ny, tfc, surr != nullptr);
+    tm.rows = f64 ? rs::tile_rows_f64(nx, ny, tfc, a->pull_back != 0)
+                  : rs::tile_rows_f32(nx, ny, tfc, surr != nullptr, std::max(P.i_front, 0));
     if (!(out_aligned && field_map(c, cur->psi, cur->precision, tm.rows + 2, &tm.psi) &&
           field_map(c, cur->c, cur->precision, tm.rows + 2, &tm.c))) {
       P.raw = 1;
       surr = nullptr;
-      if (!f64) tm.rows = rs::tile_rows_f32(nx, ny, tfc, false);
+      if (!f64) tm.rows = rs::tile_rows_f32(nx, ny, tfc, false, -1);
       tiles = f64 ? rs::raw_on_tiles_f64(nx, ny, tfc, a->pull_back != 0)
                   : rs::raw_on_tiles_f32(nx, ny, tfc, a->pull_back != 0);
     }

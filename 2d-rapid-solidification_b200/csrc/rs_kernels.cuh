@@ -151,7 +151,8 @@ constexpr int kTmaBoxW64 = kTileOutW64 + 8;      // its input columns
 constexpr int kTileRows = 16;    // output rows of a tile
 constexpr int kTmaBoxH = kTileRows + 2;  // input rows of a tile
 int tile_rows_f64(int nx, int ny, bool tfc, bool pull_back);  // output rows of an FP64 tile: 4, 8 or 16
-int tile_rows_f32(int nx, int ny, bool tfc, bool network);  // and of an FP32 tile
+// and of an FP32 tile (i_front: the column of the front, < 0 on unaligned rows)
+int tile_rows_f32(int nx, int ny, bool tfc, bool network, int i_front);
 // whether the tile kernels take a step on rows that are not 16-byte aligned (else
 // the register kernel, whose grid is 4 strips of 30 columns wide)
 constexpr bool register_grid_fits(int nx) { return ((nx - 2 + 29) / 30 + 3) / 4 <= 65535; }

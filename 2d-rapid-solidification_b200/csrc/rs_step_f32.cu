@@ -27,11 +27,20 @@ __global__ void __launch_bounds__(kTabBlock) column_table_kernel(const StepCoef 
 // cellular front): 64 x 8000, 0.7 waves, 18.9, 18.3 / 20, 19 / 18.1, 17.0; with
 // the network 67 / 53 / 50; 600 x 2300, 1 wave, network, in units of 16 rows 0.86
 // / 0.78 / 1.
-int tile_rows_f32(int nx, int ny, bool tfc, bool network) {
+// And where the front's column, which i_tip_target gives, lies so near the border of
+// two tile columns that both hold it: twice the front tiles, for which 16 rows with the
+// late trigger are best (before the tile heights / rule without the border / now):
+// 448 x 3000, front at 134, 15.0, 15.4 / 16.7, 17.2 / 14.8, 15.4, network 35.1, 48.9 /
+// 41.7, 51.9 / 35.5, 49.7; 512 x 4000, front at 272, 1 / 1.07, 1.14 / 0.99, 1.00; the
+// front in the middle of a column 448 x 3000, 44, 14.8 / 12.8 / 14.6, network 40.9 /
+// 29.1 / 40.8: it keeps 8 rows.  Beyond 24 rows per SM the exact step takes 16
+// rows wherever the front is: 448 x 3600, cellular front at 153, 1 / 1.14 / 1.01.  (i_front < 0: unaligned rows, without these lines)
+int tile_rows_f32(int nx, int ny, bool tfc, bool network, int i_front) {
   if (tfc) return kTfcTR;
   const int64_t sms = sm_count(), rows = ny - 2;
   const int64_t tiles = (int64_t)((nx + kW - 1) / kW) * ((rows + 15) / 16), wave = 5 * sms;
-  if (rows > 28 * sms && (network || tiles < 2 * wave)) return 16;
+  if (rows > (network || i_front < 0 ? 28 : 24) * sms && (network || tiles < 2 * wave)) return 16;
+  if (i_front >= 0 && (i_front + 14) % kW < 34 && rows > (network ? 15 : 18) * sms && 2 * tiles < 5 * wave) return 16;
   if (network) return 2 * tiles >= 9 * wave ? 16 : 2 * tiles >= 3 * wave || (rows > 14 * sms && 20 * tiles >= 19 * wave) ? 8 : 4;
   return tiles >= 2 * wave ? 16 : tiles >= wave ? 8 : 4;
 }
@@ -101,7 +110,7 @@ int launch_step_f32_tma(const StepCoef &K, const Coef<float> &F, const StepScala
   Q.late = tfc    ? nparts < 3 * (int64_t)resident
            : raw  ? 2 * (int64_t)nparts < 25 * sms
            : surr ? TR > 4 && nparts < 3 * (int64_t)resident
-                  : !pipe && TR == 16 && K.ny - 2 > 28 * sms && nparts < 10 * sms;
+                  : !pipe && TR == 16 && K.ny - 2 > 18 * sms && nparts < 10 * sms;
   // every kernel of the step is a programmatic dependent of the one before it
   // in the stream (rs_step_f64t.cu)
   const float *tab = tm.col_tab;

@@ -114,7 +114,7 @@ def test_solid_tiles_report_the_cells_of_row_ny_minus_1(nx, ny):
 
     def step(ctx):
         a, b = lib.FieldSet(p, torch.float32), lib.FieldSet(p, torch.float32)
-        ctx.initial_planar(a, configs.C_LIQUID_TI10NB, configs.C_SOLID_AT_TLIQ, front)
+        ctx.initial_planar(a, configs.C_LIQUID_TI10NB, configs.C_SOLID_AT_TLIQ, 7)
         a.psi[:, : front - 20] = 1.0
         ctx.set_surrogate(w, box)
         return a, b
