@@ -96,9 +96,10 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 }
 
 // 2D tiled descriptor of one field (row pitch = nx_all elements), box of
-// kTmaBoxW32/64 x kTmaBoxH elements, zero fill outside the array.  Returns false
+// kTmaBoxW32/64 x box_rows elements, zero fill outside the array.  Returns false
 // when TMA cannot be used (alignment, driver entry point).
-// box_rows: the box height (input rows of a tile)
+// box_rows: the input rows of a tile, its output rows + 2: 6, 10 or 18, and 34 in
+// an ensemble's tallest shape
 bool encode_map(const rs_params &p, const void *ptr, int precision, int box_rows, CUtensorMap *out) {
   auto enc = encode_fn();
   const size_t es = precision == RS_F64 ? 8 : 4;
@@ -115,7 +116,7 @@ bool encode_map(const rs_params &p, const void *ptr, int precision, int box_rows
   return r == CUDA_SUCCESS;
 }
 
-// box_rows: kTmaBoxH, or kTfcTileRows32 + 2 for FP32 coarse-grid-temperature steps
+// box_rows: as encode_map
 bool field_map(rs_ctx *c, const void *ptr, int precision, int box_rows, CUtensorMap *out) {
   for (int k = 0; k < c->tma_n; ++k)
     if (c->tma[k].ptr == ptr && c->tma[k].precision == precision && c->tma[k].rows == box_rows) {

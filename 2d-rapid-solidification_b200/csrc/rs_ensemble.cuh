@@ -10,7 +10,7 @@
 namespace rs {
 
 // Tile shapes of the ensemble kernels: kW = 128 output columns by
-// shape_rows(s) output rows (shape 0 is the single-run kernel's 16 x 128).
+// shape_rows(s) output rows (shape 0: 16 rows, a run alone's tallest).
 constexpr int kTileShapes = 3;
 __host__ __device__ constexpr int shape_rows(int s) { return s == 1 ? 8 : s == 2 ? 32 : 16; }
 

@@ -175,14 +175,16 @@ int launch_step_f32(const StepCoef &K, const StepScalars &P, const float *psi, c
                     int *nblocks_out, const TmaMaps *tm, int *err, cudaStream_t st);
 template <typename R>
 struct Coef;
-// FP32 TMA-staged kernel (rs_tile_f32.cuh): frozen temperature, no pull-back.
-// Launches the per-column table kernel and the tile kernel; nparts_out gets
-// the number of partials written.
+// FP32 TMA-staged kernels (rs_tile_f32.cuh): the frozen and the coarse-grid
+// temperature, with or without a fused pull-back, the fields by TMA or, of rows
+// that TMA cannot address, element by element.  Launches the per-column table
+// kernel (frozen temperature) and the tile kernel; nparts_out gets the number of
+// partials written.
 int launch_step_f32_tma(const StepCoef &K, const Coef<float> &F, const StepScalars &P, const TmaMaps &tm,
                         float *psi_n, float *c_n, float *phi_n, BlockPartial *partials, int max_partials,
                         int *nparts_out, int *err, cudaStream_t st);
-// FP64 TMA-staged kernel (rs_tile_f64.cuh): frozen temperature, no pull-back,
-// even nx_all; column table + tile kernel, final reduction fused.
+// FP64 TMA-staged kernels (rs_tile_f64.cuh), the same calls.  (Frozen
+// temperature, a grid of one wave of CTAs: no table kernel.)
 int launch_step_f64_tma(const StepCoef &K, const Coef<double> &F, const StepScalars &P, const TmaMaps &tm,
                         double *psi_n, double *c_n, double *phi_n, BlockPartial *partials, int max_partials,
                         int *nparts_out, int *err, cudaStream_t st);

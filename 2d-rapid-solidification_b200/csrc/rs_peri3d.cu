@@ -21,9 +21,9 @@
 // images (x = 1, nx-2; y = 1, ny-2; z = 1, nz-2) is written to its ghost cells
 // too, which is what the reference's boundary kernels leave there.
 // What bounds it (512 x 512 x 128): in melt the memory (333 us, 74 % of the
-// copy rate), in fronts the FP64 pipe (589 us; 180 FP64 instructions per cell,
-// 57 % of the pipe's rate at 16 warps per SM).  A front in two thirds of the
-// planes: 546 -> 486 us.  Measured beside it: four slots 519, 14-row tiles
+// copy rate), in fronts the FP64 pipe (605 us; 191 FP64 instructions per cell,
+// 61 % of the pipe's rate at 16 warps per SM).  A front in two thirds of the
+// planes: 546 -> 476 to 486 us.  Measured beside it: four slots 519, 14-row tiles
 // with three CTAs per SM and four slots 532 (80 registers instead of 118).
 // Algorithmic bytes per cell-step: 3 fields read + 3 written.
 #include <cuda.h>
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(D3::kThreads, 2)
       }
     }
     // the last warp that leaves plane z hands the slot of plane z-1 to the load
-    // of plane z+3, without waiting for plane z+2 first: two loads in flight
+    // of plane z+5, without waiting for plane z+2 first: four loads in flight
     __syncwarp();
     if (lane == 0 && arrive_count(&sm.passed) % (C::kThreads / 32) == C::kThreads / 32 - 1 && z + C::kSlots - 1 <= zin1)
       issue(z + C::kSlots - 1);

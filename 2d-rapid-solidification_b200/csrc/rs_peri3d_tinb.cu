@@ -503,7 +503,7 @@ __global__ void grains_init_kernel(const K3<R> k, const uint64_t seed, const dou
 // computed once into a four-slot ring, S in the place of the plane's c (a thread
 // keeps the c of its own outputs), so one barrier per plane suffices and three
 // CTAs fit on an SM.  The surrogate path keeps the scalar kernel.
-// What bounds it (512 x 512 x 256): instruction issue (54 %, 256 per row of 64
+// What bounds it (512 x 512 x 256): instruction issue (62 %, 256 per row of 64
 // cells in melt) and the latencies behind it; all melt 385 us, a front in 60 of
 // the 256 planes 628 -> 451 us.  Of that, the melt form of its own and the wider
 // melt polynomial gave 597 -> 494, the third CTA 494 -> 451.

@@ -164,7 +164,9 @@ Coef<R> make_coef(const StepCoef &K) {
 // the compiler is free to fuse either one, and chose differently in different
 // kernels that inline the same lines (the ensemble's walk differed from the
 // other paths by an ulp of psi); with one of them rounded there is no choice, so
-// a cell's phi does not depend on the kernel that evaluates it.
+// a cell's phi is the same in the tile, pipeline and ensemble kernels.  (The
+// register kernel's own update and the form of the anisotropy with two strengths
+// keep such sums: there an ulp may differ between kernels.)
 __device__ __forceinline__ float mulr(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mulr(double a, double b) { return __dmul_rn(a, b); }
 

@@ -40,7 +40,7 @@
 //            CTA writes its partial sums and a dependent launch reduces them.
 // What bounds it: a 2048^2 grid ahead of a planar front (20.6 us a step, 23.7
 // without the melt form and the chained launches; floor 10.3, a plain copy of
-// its fields by this tiling 17.3) its instruction issue (1100 instructions a
+// its fields by this tiling 17.3) its instruction issue (1150 instructions a
 // warp for 512 cells of far melt, half of them arithmetic) and the chain of a
 // CTA; small grids (256^2: 6.1 us, 12.0 with 16-row tiles) and fronts the chain
 // of the phases.
@@ -75,7 +75,8 @@
 // own bilinear temperature (K + C0 by its Taylor polynomial about the tile's
 // centre temperature, kc_poly), keeps K + C0 in FP64 in shared memory, and the
 // faces add its differences, rounded to FP32, along both axes; tiles of 8
-// output rows, so that the FP64 array fits with five CTAs per SM.
+// output rows, so that the FP64 array fits with five CTAs per SM.  Its only
+// whole-tile form is the deep solid one.
 // Fields store psi and delta = c - cinf (include/rs_b200.h).
 #pragma once
 
@@ -108,7 +109,8 @@ enum { kTabRT = 0, kTabC0 = 1, kTabDK = 2, kTabAnb = 3, kTabAti = 4 };
 
 // Shared memory of one tile of TR output rows x kW output columns (input
 // TR + 2 rows); the ensemble kernels take TR = 8, 16 or 32 (kTileShapes), the
-// single-run kernel TR = kTR.
+// single-run kernels TR = 4, 8 or 16 (tile_rows_f32) and, with the coarse-grid
+// temperature, kTfcTileRows32.
 template <int TR, bool TFC = false>
 struct alignas(128) TileSmemT {
   static constexpr int kRin = TR + 2;  // input rows
@@ -1345,7 +1347,7 @@ __global__ void __launch_bounds__(kThreads, SURR ? 4 : 5)
 }
 
 // The coarse-grid temperature (TFC): tiles of kTfcTileRows32 output rows, whose
-// per-cell K + C0 (FP64) fits beside the tile with six CTAs per SM; per-cell
+// per-cell K + C0 (FP64) fits beside the tile with five CTAs per SM; per-cell
 // CALPHAD groups instead of the column table.
 constexpr int kTfcTR = kTfcTileRows32;
 template <bool RAW>

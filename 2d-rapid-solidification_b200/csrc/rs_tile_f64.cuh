@@ -25,7 +25,7 @@
 // votes on the tile's form:
 //   * far melt everywhere (the bulk of a run ahead of its front): the c update
 //     straight from registers to global memory (melt_tile), one barrier after
-//     the load;
+//     the load (frozen temperature only);
 //   * deep solid everywhere: psi and c stay (solid_tile);
 //   * anything else, the phases:
 //   phase 1  per-cell S = q(psi) c (1-c) and mu'' of the input rows into
@@ -74,10 +74,14 @@
 // fun.cu:1580-1608): no table kernel; every cell evaluates its CALPHAD groups
 // from its own bilinear temperature (K + C0 by its Taylor polynomial about
 // the tile's centre temperature, kc_poly, and C0 and the driving-force groups
-// likewise; cells out of the polynomials' range by the Gibbs functions) and
-// stores mu = mu'' + (K + C0), so the faces take plain differences of mu.
-// 768 x 832 with a cellular front: 22.5 us a step (41 with the Gibbs functions
-// per cell).
+// likewise, drive_poly on a second thread; cells out of the polynomials' range
+// by the Gibbs functions) and
+// stores mu = mu'' + (K + C0), so the faces take plain differences of mu.  Melt
+// tiles take the phases and only tiles whose first interior cell is solid vote
+// (2048^2 all melt: 59.2 us; 74.7 with the melt form and a vote in every
+// tile, of which most fail).  768 x 832 with a cellular front: 22.7 to 25.6 us a
+// step by where the front lies in its tile column (34.7 to 36.2 before the
+// polynomials and the 8-row tiles).
 //
 // Two kernels run these phases (same functions, same results bit for bit):
 //   * tile_kernel_f64: one tile per CTA of 128 threads, the phases in series
