@@ -33,14 +33,16 @@ __global__ void __launch_bounds__(kTabBlock) column_table_kernel(const StepCoef 
 // 448 x 3000, front at 134, 15.0, 15.4 / 16.7, 17.2 / 14.8, 15.4, network 35.1, 48.9 /
 // 41.7, 51.9 / 35.5, 49.7; 512 x 4000, front at 272, 1 / 1.07, 1.14 / 0.99, 1.00; the
 // front in the middle of a column 448 x 3000, 44, 14.8 / 12.8 / 14.6, network 40.9 /
-// 29.1 / 40.8: it keeps 8 rows.  Beyond 24 rows per SM the exact step takes 16
+// 29.1 / 40.8: it keeps 8 rows, and so does a front near column 0, where there is no
+// second tile column (448 x 3000, 16, 14.9 / 13.0 / 14.6, network 36.3 / 27.1 / 36.4).  Beyond 24 rows per SM the exact step takes 16
 // rows wherever the front is: 448 x 3600, cellular front at 153, 1 / 1.14 / 1.01.  (i_front < 0: unaligned rows, without these lines)
 int tile_rows_f32(int nx, int ny, bool tfc, bool network, int i_front) {
   if (tfc) return kTfcTR;
   const int64_t sms = sm_count(), rows = ny - 2;
   const int64_t tiles = (int64_t)((nx + kW - 1) / kW) * ((rows + 15) / 16), wave = 5 * sms;
   if (rows > (network || i_front < 0 ? 28 : 24) * sms && (network || tiles < 2 * wave)) return 16;
-  if (i_front >= 0 && (i_front + 14) % kW < 34 && rows > (network ? 15 : 18) * sms && 2 * tiles < 5 * wave) return 16;
+  const bool border = i_front >= kW - 14 && i_front < nx && (i_front + 14) % kW < 34;
+  if (border && rows > (network ? 15 : 18) * sms && 2 * tiles < 5 * wave) return 16;
   if (network) return 2 * tiles >= 9 * wave ? 16 : 2 * tiles >= 3 * wave || (rows > 14 * sms && 20 * tiles >= 19 * wave) ? 8 : 4;
   return tiles >= 2 * wave ? 16 : tiles >= wave ? 8 : 4;
 }

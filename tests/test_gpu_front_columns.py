@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("nx,ny", [(192, 2300), (260, 2702), (448, 3000), (388, 3600)])
 def test_fields_do_not_depend_on_where_the_front_is_said_to_be(nx, ny, network):
     out = []
-    for tip in (64, 114, 134):  # beside the offset, made up for below, i_tip_target orders the tiles and chooses their height
+    for tip in (64, 114, 134, 10):  # beside the offset, made up for below, i_tip_target orders the tiles and chooses their height
         p = configs._ti10nb(configs.default_params(), nx, ny, 5e6, 0.5, T0=configs.T_SOLIDUS_TI10NB)
         p.i_tip_target, p.noise_amplitude, p.seed = tip, 0.01, 5
         ctx = lib.Context(p)
