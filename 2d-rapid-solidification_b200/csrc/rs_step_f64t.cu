@@ -50,11 +50,15 @@ __global__ void __launch_bounds__(kTabBlock) column_table_kernel_f64(const StepC
 // their halo rows cost more: 640 x 1100, 0.9 waves, cellular, in units of the
 // 16-row tile without its whole-tile forms 1.12 / 1.04 / 0.99.
 // With the coarse-grid temperature a tile also sets up its temperature tables:
-// 768 x 832, 28.8 / 22.5 / 30.2 us a step, so 4 rows are left out.
+// 768 x 832, 28.8 / 22.5 / 30.2 us a step, so 4 rows are left out, and 16 pay from
+// 1.45 waves on (in units of the 16-row tile without its polynomials, planar front
+// at column 16, 8 / 16 rows): 1024^2, 1.4 waves, 0.65 / 0.74 (in a tile column's
+// middle 0.80 / 0.76); 1200^2, 1.9 waves, 0.87 / 0.71; 1400 x 1600, 3 waves less a
+// tile row, 1.13 / 0.86; 512 x 4002, 2.7 waves, 1.11 / 0.87.
 int tile_rows_f64(int nx, int ny, bool tfc, bool pull_back) {
   const int64_t sms = sm_count(), rows = ny - 2;
   const int64_t tiles = (int64_t)((nx + kW - 1) / kW) * ((rows + 15) / 16), wave = 5 * sms;
-  if (tfc) return tiles >= 3 * wave ? 16 : 8;
+  if (tfc) return 20 * tiles >= 29 * wave ? 16 : 8;
   if (tiles >= 3 * wave) return 16;
   if (rows > 21 * sms && tiles >= 2 * wave) return 16;
   if (2 * rows > 21 * sms && tiles < wave) return 20 * tiles >= 9 * wave ? 16 : 8;

@@ -73,3 +73,10 @@ def test_coarse_temperature_tiles_match_the_oracle(nx, ny, shift, dtype, kind, o
 @pytest.mark.parametrize("nx,shift", [(2049, 0), (2050, 1)])
 def test_coarse_temperature_16_row_tiles_on_unaligned_rows(nx, shift, off):
     run(nx, 1132, "f64", "front", off, shift)
+
+
+# the line between 8 and 16 rows in FP64 (1073 tiles of 16 x 64 on a B200): 1072, 1088, 1088 tiles
+@pytest.mark.parametrize("off", [None, 5])
+@pytest.mark.parametrize("nx,ny", [(1024, 1072), (1024, 1082), (1023, 1082)])
+def test_coarse_temperature_at_the_line_between_the_tile_heights(nx, ny, off):
+    run(nx, ny, "f64", "front", off, 0)
