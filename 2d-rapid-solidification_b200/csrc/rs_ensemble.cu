@@ -38,8 +38,15 @@ int launch_ensemble(const EnsRun *runs, int nruns, const int32_t *tblk, int ntbl
   static std::atomic<int> wave_of[2][kTileShapes][64];
   const int wave = resident_ctas((const void *)kfn, kThreads, smem, wave_of[surr][shape]);
   if (wave < 0) return -3;
-  if (launch_dep(ens_table_kernel, dim3(ntblk), dim3(kTabBlock), st, runs, tblk) != cudaSuccess ||
-      launch_dep_smem(kfn, dim3(ntiles), dim3(kThreads), smem, st, runs, order, err, wave) != cudaSuccess)
+  if (launch_dep(ens_table_kernel, dim3(ntblk), dim3(kTabBlock), st, runs, tblk) != cudaSuccess) return -3;
+  // tiles scheduled while the table kernel runs share the SMs out unevenly: below
+  // two waves that costs more than the launch latency it hides (us a step, tiles as
+  // a dependent launch / behind the tables): 415 tiles 20.5 / 18.5, 738 22.3 / 20.5,
+  // 1327 28.4 / 27.9 (490 18.5 / 20.5, 638 20.5 / 20.5); 2908 46.6 / 46.8, 3578
+  // 58.5 / 59.1; with the network 415 tiles 57.2 / 53.0, 638 63.9 / 58.6
+  if (ntiles < 2 * wave)
+    kfn<<<ntiles, kThreads, smem, st>>>(runs, order, err, wave);
+  else if (launch_dep_smem(kfn, dim3(ntiles), dim3(kThreads), smem, st, runs, order, err, wave) != cudaSuccess)
     return -3;
   if (advance && launch_dep(ens_advance_kernel, dim3((nruns + 63) / 64), dim3(64), st, const_cast<EnsRun *>(runs),
                             nruns) != cudaSuccess)
