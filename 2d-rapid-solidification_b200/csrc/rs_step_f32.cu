@@ -34,17 +34,26 @@ __global__ void __launch_bounds__(kTabBlock) column_table_kernel(const StepCoef 
 // 41.7, 51.9 / 35.5, 49.7; 512 x 4000, front at 272, 1 / 1.07, 1.14 / 0.99, 1.00; the
 // front in the middle of a column 448 x 3000, 44, 14.8 / 12.8 / 14.6, network 40.9 /
 // 29.1 / 40.8: it keeps 8 rows, and so does a front near column 0, where there is no
-// second tile column (448 x 3000, 16, 14.9 / 13.0 / 14.6, network 36.3 / 27.1 / 36.4).  Beyond 24 rows per SM the exact step takes 16
-// rows wherever the front is: 448 x 3600, cellular front at 153, 1 / 1.14 / 1.01.  (i_front < 0: unaligned rows, without these lines)
+// second tile column (448 x 3000, 16, 14.9 / 13.0 / 14.6, network 36.3 / 27.1 / 36.4).
+// The network's tiles of one column fit on the device at once at 4 rows up to 16 rows
+// per SM (at 8 up to 32): 192 x 3968, front at 104, 1 / 1.17 with 4 rows / 0.98 with
+// 8; 384 x 3968, 40, 1 / 0.84 / 0.70.  At a border below these lines 8 rows beat 4:
+// 512 x 2300, 121, 1 / 1.07 / 1.00; 192 x 2300, 134, network, 1 / 1.05 / 0.79.
+// Beyond 24 rows per SM the exact step takes 16 rows wherever the front is: 448 x
+// 3600, cellular front at 153, 1 / 1.14 / 1.01.  (i_front < 0: unaligned rows,
+// without these lines)
 int tile_rows_f32(int nx, int ny, bool tfc, bool network, int i_front) {
   if (tfc) return kTfcTR;
   const int64_t sms = sm_count(), rows = ny - 2;
   const int64_t tiles = (int64_t)((nx + kW - 1) / kW) * ((rows + 15) / 16), wave = 5 * sms;
   if (rows > (network || i_front < 0 ? 28 : 24) * sms && (network || tiles < 2 * wave)) return 16;
   const bool border = i_front >= kW - 14 && i_front < nx && (i_front + 14) % kW < 34;
-  if (border && rows > (network ? 15 : 18) * sms && 2 * tiles < 5 * wave) return 16;
-  if (network) return 2 * tiles >= 9 * wave ? 16 : 2 * tiles >= 3 * wave || (rows > 14 * sms && 20 * tiles >= 19 * wave) ? 8 : 4;
-  return tiles >= 2 * wave ? 16 : tiles >= wave ? 8 : 4;
+  if (border && rows > (network ? 16 : 18) * sms && 2 * tiles < 5 * wave) return 16;
+  if (network) {
+    if (2 * tiles >= 9 * wave) return 16;
+    return 2 * tiles >= 3 * wave || rows > 16 * sms || (rows > 14 * sms && (border || 20 * tiles >= 19 * wave)) ? 8 : 4;
+  }
+  return tiles >= 2 * wave ? 16 : tiles >= wave || (border && rows > 14 * sms) ? 8 : 4;
 }
 // Rows that are not 16-byte aligned: the tiles, which copy their boxes cell by
 // cell, but for grids of more than a wave and a half of them (at 4 rows a tile)
